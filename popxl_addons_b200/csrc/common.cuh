@@ -43,6 +43,30 @@ template <typename T> __device__ __forceinline__ void xl_store16(T* __restrict__
   *reinterpret_cast<uint4*>(p) = raw;
 }
 
+// 16 bytes from an address that is aligned to the element only: the one or two aligned 16-byte blocks that hold them, shifted
+// together. Every block read holds at least one of the 16 bytes.
+template <typename T> __device__ __forceinline__ uint4 xl_load16_any(const T* __restrict__ p) {
+  const uint32_t off = (uint32_t)((uintptr_t)p & 15);
+  const uint4* a = reinterpret_cast<const uint4*>((uintptr_t)p - off);
+  const uint4 lo = a[0];
+  if (off == 0) return lo;
+  const uint4 hi = a[1];
+  uint4 o;  // words off / 4 .. off / 4 + 4 of the eight; the selections are uniform over a row
+  uint32_t w0, w1, w2, w3, w4;
+  switch (off >> 2) {
+    case 0: w0 = lo.x; w1 = lo.y; w2 = lo.z; w3 = lo.w; w4 = hi.x; break;
+    case 1: w0 = lo.y; w1 = lo.z; w2 = lo.w; w3 = hi.x; w4 = hi.y; break;
+    case 2: w0 = lo.z; w1 = lo.w; w2 = hi.x; w3 = hi.y; w4 = hi.z; break;
+    default: w0 = lo.w; w1 = hi.x; w2 = hi.y; w3 = hi.z; w4 = hi.w; break;
+  }
+  const uint32_t sh = (off & 3) * 8;
+  o.x = __funnelshift_r(w0, w1, sh);
+  o.y = __funnelshift_r(w1, w2, sh);
+  o.z = __funnelshift_r(w2, w3, sh);
+  o.w = __funnelshift_r(w3, w4, sh);
+  return o;
+}
+
 __device__ __forceinline__ float xl_warp_sum(float v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);

@@ -878,14 +878,16 @@ XL_API int xl_attn_softmax_bwd(const void* p, void* dp, long long rows, int Sq, 
 }
 
 // ------------------------------------------------------------------------------------------------------------------
-// Cross-entropy on logits with the gradient fused: one CTA per row, three sweeps over the row (max, sum-exp, write);
-// the row (<= ~100 KB) stays in L2 between sweeps. loss_row[r] = -log softmax(x)[label]; dlogits = (softmax -
-// onehot) * grad_scale for valid rows, 0 for ignored rows. Mean reduction and its 1/count are applied by the caller.
+// Cross-entropy on logits with the gradient fused: one CTA per row, two sweeps over the row. The first keeps a running maximum
+// and sum of exponentials per thread, the second (from L1 / L2: a row has at most ~100 KB) writes the gradient.
+// loss_row[r] = -log softmax(x)[label]; dlogits = (softmax - onehot) * grad_scale for valid rows, 0 for ignored rows. Mean
+// reduction and its 1/count are applied by the caller. Rows of logits may start at any element; rows of dlogits start at
+// multiples of `ldd` elements, 16-byte aligned, and their padding (V .. ldd) is written as zeros.
 // ------------------------------------------------------------------------------------------------------------------
 template <typename T>
 __global__ void __launch_bounds__(512)
     ce_fwd_bwd_kernel(const T* __restrict__ logits, const int* __restrict__ labels, float* __restrict__ loss_row,
-                      T* __restrict__ dlogits, int V, int ignore_index, const float* __restrict__ grad_scale_ptr,
+                      T* __restrict__ dlogits, int V, int ldd, int ignore_index, const float* __restrict__ grad_scale_ptr,
                       float grad_scale) {
   constexpr int N = XlVec<T>::N;
   __shared__ float red[32];
@@ -894,32 +896,46 @@ __global__ void __launch_bounds__(512)
   const int label = labels[row];
   const bool valid = label != ignore_index && label >= 0 && label < V;
   const int nvec = V / N;
-  float mx = -INFINITY;
-  for (int i = threadIdx.x; i < nvec; i += blockDim.x) {
-    float a[N];
-    xl_load16(xr + i * N, a);
+  auto load = [&](int i, float (&a)[N]) {
+    const uint4 raw = xl_load16_any(xr + i * N);
+    const T* e = reinterpret_cast<const T*>(&raw);
 #pragma unroll
-    for (int k = 0; k < N; ++k) mx = fmaxf(mx, a[k]);
-  }
-  for (int i = nvec * N + threadIdx.x; i < V; i += blockDim.x) mx = fmaxf(mx, xl_to_float(xr[i]));
-  mx = xl_block_max(mx, red);
-  float sum = 0.f;
+    for (int k = 0; k < N; ++k) a[k] = xl_to_float(e[k]);
+  };
+  float mx = -INFINITY, sum = 0.f;
+#pragma unroll 2
   for (int i = threadIdx.x; i < nvec; i += blockDim.x) {
     float a[N];
-    xl_load16(xr + i * N, a);
+    load(i, a);
+    float m = mx;
+#pragma unroll
+    for (int k = 0; k < N; ++k) m = fmaxf(m, a[k]);
+    if (m != mx) { sum *= __expf(mx - m); mx = m; }  // from -inf: the sum is still 0
+    if (mx == -INFINITY) {  // masked so far: nothing to add, but a NaN stays one
+#pragma unroll
+      for (int k = 0; k < N; ++k) sum += a[k] != a[k] ? a[k] : 0.f;
+      continue;
+    }
 #pragma unroll
     for (int k = 0; k < N; ++k) sum += __expf(a[k] - mx);
   }
-  for (int i = nvec * N + threadIdx.x; i < V; i += blockDim.x) sum += __expf(xl_to_float(xr[i]) - mx);
+  for (int i = nvec * N + threadIdx.x; i < V; i += blockDim.x) {
+    const float v = xl_to_float(xr[i]), m = fmaxf(mx, v);
+    if (m != mx) { sum *= __expf(mx - m); mx = m; }
+    sum += mx == -INFINITY ? (v != v ? v : 0.f) : __expf(v - mx);
+  }
+  const float top = xl_block_max(mx, red);
+  if (mx != top) sum *= __expf(mx - top);  // a thread without a finite value has the sum 0 (or NaN, which stays)
   sum = xl_block_sum(sum, red);
-  const float lse = mx + logf(sum);
+  const float lse = top + logf(sum);
   if (threadIdx.x == 0) loss_row[row] = valid ? lse - xl_to_float(xr[label]) : 0.f;
   if (dlogits == nullptr) return;
   const float gs = valid ? (grad_scale_ptr ? *grad_scale_ptr * grad_scale : grad_scale) : 0.f;
-  T* dr = dlogits + row * V;
+  T* dr = dlogits + row * ldd;
+#pragma unroll 2
   for (int i = threadIdx.x; i < nvec; i += blockDim.x) {
     float a[N];
-    xl_load16(xr + i * N, a);
+    load(i, a);
 #pragma unroll
     for (int k = 0; k < N; ++k) {
       float p = __expf(a[k] - lse);
@@ -933,14 +949,15 @@ __global__ void __launch_bounds__(512)
     if (i == label) p -= 1.f;
     dr[i] = xl_from_float<T>(p * gs);
   }
+  for (int i = V + threadIdx.x; i < ldd; i += blockDim.x) dr[i] = xl_from_float<T>(0.f);
 }
-XL_API int xl_ce_fwd_bwd(const void* logits, const int* labels, float* loss_row, void* dlogits, long long rows, int V,
+// logits (rows, V) contiguous; dlogits (rows, V) with row stride ldd >= V whose rows are 16-byte aligned (one row: any ldd).
+XL_API int xl_ce_fwd_bwd(const void* logits, const int* labels, float* loss_row, void* dlogits, long long rows, int V, int ldd,
                          int ignore_index, const float* grad_scale_ptr, float grad_scale, int dtype, cudaStream_t s) {
   const int vec = dtype == XL_F32 ? 4 : 8;
-  if ((V * (dtype == XL_F32 ? 4 : 2)) % 16 != 0 && rows > 1) return -1;  // rows must stay 16-byte aligned
-  (void)vec;
+  if (rows < 1 || V < 1 || ldd < V || (((uintptr_t)dlogits) & 15) || (rows > 1 && ldd % vec != 0)) return -1;
   XL_DISPATCH_DTYPE(dtype, T, {
-    ce_fwd_bwd_kernel<T><<<(unsigned)rows, 512, 0, s>>>((const T*)logits, labels, loss_row, (T*)dlogits, V, ignore_index,
+    ce_fwd_bwd_kernel<T><<<(unsigned)rows, 512, 0, s>>>((const T*)logits, labels, loss_row, (T*)dlogits, V, ldd, ignore_index,
                                                        grad_scale_ptr, grad_scale);
   });
   return (int)cudaGetLastError();

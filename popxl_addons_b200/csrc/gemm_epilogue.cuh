@@ -22,6 +22,13 @@ __device__ __forceinline__ float apply_act(float v, int act) {
   return v;
 }
 
+__device__ __forceinline__ float epilogue_bias(const EpilogueParams& p, int col) {
+  if (!p.bias) return 0.f;
+  if (p.bias_dtype == XL_F32) return ((const float*)p.bias)[col];
+  if (p.bias_dtype == XL_BF16) return __bfloat162float(((const __nv_bfloat16*)p.bias)[col]);
+  return __half2float(((const __half*)p.bias)[col]);
+}
+
 // One thread's 32 consecutive accumulator columns (row `crow`, columns col0 .. col0 + 31) -> scale, bias, activation,
 // optional accumulation into the old contents, conversion and store. The caller has checked row < M and col0 < N.
 __device__ __forceinline__ void epilogue_store_32cols(const EpilogueParams& p, const uint32_t (&r)[32], uint8_t* crow,

@@ -75,7 +75,9 @@ _attn_bwd_dq = _sig("xl_attn_bwd_dq_tcgen05", _c_p, _c_ll, _c_ll, _c_p, _c_ll, _
                     _c_p)
 _attn_bwd_plan = _sig("xl_attn_bwd_plan", _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_p)
 _sm_bwd = _sig("xl_attn_softmax_bwd", _c_p, _c_p, _c_ll, _c_int, _c_int, _c_f, _c_int, _c_int, _c_p)
-_ce = _sig("xl_ce_fwd_bwd", _c_p, _c_p, _c_p, _c_p, _c_ll, _c_int, _c_int, _c_p, _c_f, _c_int, _c_p)
+_ce = _sig("xl_ce_fwd_bwd", _c_p, _c_p, _c_p, _c_p, _c_ll, _c_int, _c_int, _c_int, _c_p, _c_f, _c_int, _c_p)
+_pack_rows16 = _sig("xl_pack_rows16", _c_p, _c_ll, _c_p, _c_ll, _c_ll, _c_int, _c_p)
+_unpack_rows16 = _sig("xl_unpack_rows16", _c_p, _c_ll, _c_p, _c_ll, _c_int, _c_p)
 _gemm = _sig("xl_gemm_tcgen05", _c_p, _c_p, _c_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_ll, _c_ll, _c_ll,
              _c_ll, _c_ll, _c_ll, _c_int, _c_int, _c_p, _c_int, _c_int, _c_int, _c_p, _c_f, _c_p, _c_int, _c_p, _c_int,
              _c_int, _c_p, _c_p)
@@ -414,14 +416,34 @@ def sgd_cuda(w, g, *rest, has_momentum, **attrs):
     return w
 
 
+def _padded_rows(t) -> bool:
+    """Rows of less than 16 bytes of padding in an allocation that holds the last row's padding too."""
+    pad = t.stride(-2) - t.shape[-1]
+    if t.stride(-1) != 1 or not 0 < pad * t.element_size() < 16:
+        return False
+    dense = t.stride(-2)
+    for d in range(t.dim() - 2, -1, -1):
+        if t.stride(d) != dense:
+            return False
+        dense *= t.shape[d]
+    return (t.storage_offset() + dense) * t.element_size() <= t.untyped_storage().nbytes()
+
+
 @native("sum")
 def sum_cuda(a, axis, keepdims):
     """Sum over the leading axes of a contiguous tensor (bias gradients: over the token rows): column sums in fp32,
     added in a fixed order."""
-    if axis is None or keepdims or not _ok(a) or a.dim() < 2:
+    if axis is None or keepdims or a.dim() < 2:
         return NotImplemented
     axes = sorted(int(x) % a.dim() for x in axis)
     if axes != list(range(len(axes))) or len(axes) == a.dim():
+        return NotImplemented
+    width = None
+    if len(axes) == a.dim() - 1 and _padded_rows(a):
+        # rows with padding behind (the gradient of an odd number of classes): summed with it, which is dropped again
+        width = a.shape[-1]
+        a = torch.as_strided(a, (*a.shape[:-1], a.stride(-2)), a.stride(), a.storage_offset())
+    if not _ok(a):
         return NotImplemented
     cols = 1
     for d in a.shape[len(axes):]:
@@ -437,7 +459,7 @@ def sum_cuda(a, axis, keepdims):
         return NotImplemented
     _check(rc, "col_sum")
     _count("col_sum")
-    return out
+    return out if width is None else out[:width]
 
 
 @native("accumulate_mean_")
@@ -534,6 +556,28 @@ def _major(t: torch.Tensor, contraction_last: bool):
     return None
 
 
+def _aligned_operand(t: torch.Tensor) -> torch.Tensor:
+    """A 2-D GEMM operand whose rows (or, transposed, columns) all start on 16-byte boundaries: `t`, or a copy with padded
+    rows. The copy costs two passes over the operand; without it the product would leave the tcgen05 kernels."""
+    src = t if t.stride(1) == 1 else t.t()
+    if t.dtype not in (torch.bfloat16, torch.float16) or (src.stride(0) % 8 == 0 and t.data_ptr() % 16 == 0):
+        return t
+    rows, cols = src.shape
+    dst = torch.empty((rows, (cols + 7) // 8 * 8), dtype=t.dtype, device=t.device)
+    _check(_pack_rows16(src.data_ptr(), src.stride(0), dst.data_ptr(), dst.stride(0), rows, cols, _stream()), "pack_rows")
+    _count("pack_rows")
+    dst = dst[:, :cols]
+    return dst if src is t else dst.t()
+
+
+def _without_gaps(t: torch.Tensor) -> torch.Tensor:
+    """Contiguous copy of 16-bit rows with padding behind them."""
+    y = torch.empty(t.shape, dtype=t.dtype, device=t.device)
+    _check(_unpack_rows16(t.data_ptr(), t.stride(0), y.data_ptr(), t.shape[0], t.shape[1], _stream()), "unpack_rows")
+    _count("unpack_rows")
+    return y
+
+
 # Plain GEMMs with N > 128 run on CTA pairs (tcgen05 cta_group::2, 256 x 256 tiles: measured 1.15 to 1.22x the single-CTA
 # kernel on the transformer shapes); collective epilogues, the all-gather prologue and causal products keep the
 # single-CTA kernel. XL_GEMM_CTA_PAIRS=0 switches the pairs off.
@@ -562,8 +606,12 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, bias: Optional[torch.Tensor] = Non
     if a.dim() not in (2, 3) or b.dim() != a.dim():
         return NotImplemented
     ma, mb = _major(a, True), _major(b, False)
-    if ma is None or mb is None:
+    if ma is None or mb is None or 0 in a.shape or 0 in b.shape:
         return NotImplemented
+    plain = comm is None and gather is None and accumulate <= 2 and not batched
+    if plain:
+        a, b = _aligned_operand(a), _aligned_operand(b)
+        ma, mb = _major(a, True), _major(b, False)
     (a_mn, lda), (b_mn, ldb) = ma, mb
     M, K = a.shape[-2], a.shape[-1]
     N = b.shape[-1]
@@ -576,9 +624,15 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, bias: Optional[torch.Tensor] = Non
         return NotImplemented
     if lda % 8 or ldb % 8 or a.data_ptr() % 16 or b.data_ptr() % 16 or (batched and (sa % 8 or sb % 8)):
         return NotImplemented
+    gaps = None
     if out is None:
         out_dtype = out_dtype or a.dtype
-        out = torch.empty((batch, M, N) if batched else (M, N), dtype=out_dtype, device=a.device)
+        if plain and N % 8 and out_dtype in (torch.bfloat16, torch.float16):
+            # 16-bit rows that do not start on 16-byte boundaries: multiplied into padded rows, then copied together
+            gaps = torch.empty((M, (N + 7) // 8 * 8), dtype=out_dtype, device=a.device)
+            out = gaps[:, :N]
+        else:
+            out = torch.empty((batch, M, N) if batched else (M, N), dtype=out_dtype, device=a.device)
     if out.dtype not in _CODE or out.stride(-1) != 1 or out.dim() != a.dim():
         return NotImplemented
     if accumulate == 4 and (rs_dst is None or comm is None or out.shape[-2] * comm.world != M):
@@ -586,7 +640,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, bias: Optional[torch.Tensor] = Non
     ldc = out.stride(-2)
     stride_c = out.stride(0) if batched else 0
     esz = out.element_size()
-    if (ldc * esz) % 16 or out.data_ptr() % 16 or (batched and (stride_c * esz) % 16):
+    if not plain and ((ldc * esz) % 16 or out.data_ptr() % 16 or (batched and (stride_c * esz) % 16)):
         return NotImplemented
     if bias is not None and not (bias.is_cuda and bias.is_contiguous() and bias.dtype in _CODE and bias.numel() == N):
         return NotImplemented
@@ -624,7 +678,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, bias: Optional[torch.Tensor] = Non
         if rc >= 0:
             _check(rc, "gemm2cta_tcgen05")
             _count("gemm2cta_tcgen05")
-            return out
+            return out if gaps is None else _without_gaps(out)
     rc = _gemm_fused(a.data_ptr(), b.data_ptr(), out_ptr, M, N, K, batch, a_mn, b_mn, lda, ldb, ldc, sa, sb, stride_c,
                      int(a.dtype == torch.float16), _CODE[out.dtype], bias.data_ptr() if bias is not None else None,
                      _CODE[bias.dtype] if bias is not None else 0, act, accumulate,
@@ -635,7 +689,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, bias: Optional[torch.Tensor] = Non
         return NotImplemented
     _check(rc, "gemm_tcgen05")
     _count("gemm_tcgen05")
-    return out
+    return out if gaps is None else _without_gaps(out)
 
 
 def gemm_all_reduce_pull(pairs, comm, partial: torch.Tensor, result: torch.Tensor, flags_ptrs: torch.Tensor,
@@ -1005,7 +1059,10 @@ def ce_with_grad_cuda(logits, labels, loss_grad, ignore_index, reduction):
         lab = lab.to(torch.int32)
     ii = -100 if ignore_index is None else int(ignore_index)
     loss_row = torch.empty(rows, dtype=torch.float32, device=logits.device)
-    dlogits = torch.empty_like(logits)
+    # rows of an odd number of classes are written with aligned starts: what reads this gradient are matrix products
+    n = 16 // logits.element_size()
+    ldd = V if rows == 1 else (V + n - 1) // n * n
+    dlogits = torch.empty((*logits.shape[:-1], ldd), dtype=logits.dtype, device=logits.device)[..., :V]
     lg = loss_grad.float().reshape(())
     if reduction == "mean":
         count = (lab != ii).sum().clamp(min=1).float()
@@ -1013,7 +1070,7 @@ def ce_with_grad_cuda(logits, labels, loss_grad, ignore_index, reduction):
     else:
         count = None
         scale_t = lg.reshape(1)
-    rc = _ce(logits.data_ptr(), lab.data_ptr(), loss_row.data_ptr(), dlogits.data_ptr(), rows, V, ii,
+    rc = _ce(logits.data_ptr(), lab.data_ptr(), loss_row.data_ptr(), dlogits.data_ptr(), rows, V, ldd, ii,
              scale_t.data_ptr(), 1.0, _CODE[logits.dtype], _stream())
     if rc == -1:
         return NotImplemented

@@ -1,8 +1,13 @@
-"""Greedy choice at sizes whose rows do not start on 16-byte boundaries, with ties and without a finite maximum."""
+"""Products, cross-entropy, column sums and greedy choice at sizes whose rows do not start on 16-byte boundaries, against the
+plain operations in 64 bits. Bounds: operands are 16-bit and exact in the reference, sums are fp32, so what differs is the
+rounding of the result (half a unit of its last place, 2^-9 for bf16 and 2^-12 for fp16) and fp32 summation: the tensor cores cut
+the running sum to 24 bits at least every eight terms, at most one unit of 2^-23 each time."""
 import pytest
 import torch
 
 pytestmark = pytest.mark.gpu
+
+ROUND = {torch.bfloat16: 2.0 ** -8, torch.float16: 2.0 ** -11, torch.float32: 2.0 ** -20}
 
 
 @pytest.fixture(scope="module")
@@ -10,6 +15,66 @@ def nat():
     from popxl_addons_b200.ops import native
 
     return native
+
+
+def _near(got, want, dtype, scale=None, terms=0):
+    scale = want.abs().max() if scale is None else scale
+    assert float((got.double() - want).abs().max() / scale) <= ROUND[dtype] + terms / 8 * 2.0 ** -23
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("M,K,N", [(1, 8, 1), (3, 9, 7), (129, 65, 255), (256, 64, 257), (300, 257, 1021), (64, 1021, 129),
+                                   (513, 40, 33), (100, 33, 300)])
+def test_products(nat, M, K, N, dtype):
+    g = torch.Generator(device="cuda").manual_seed(M + K + N)
+
+    def n(*s):
+        return torch.randn(*s, device="cuda", generator=g).to(dtype)
+
+    a, b, bias = n(M, K), n(K, N), n(N)
+    at, bt = n(K, M), n(N, K)
+    for x, y in ((a, b), (at.t(), b), (a, bt.t()), (at.t(), bt.t())):
+        want = x.double() @ y.double()
+        y1 = nat.gemm(x, y)
+        assert y1.is_contiguous()
+        _near(y1, want, dtype)
+        _near(nat.gemm(x, y, out_dtype=torch.float32), want, torch.float32, scale=want.abs().max() + 1, terms=K)
+    want = torch.relu(a.double() @ b.double() + bias.double())
+    _near(nat.gemm(a, b, bias=bias, act=3), want, dtype, scale=want.max() + 1)
+    step = torch.tensor(3.0, device="cuda")
+    acc = torch.randn(M, N, device="cuda", generator=g)
+    want = acc.double() * 0.75 + (a.double() @ b.double()) * 0.25
+    assert nat.gemm(a, b, out=acc, accumulate=2, step=step) is acc
+    _near(acc, want, torch.float32, scale=want.abs().max() + 1, terms=K)
+    # an operand that starts in the middle of an allocation
+    x = n(M * K + 3)[3:].view(M, K)
+    _near(nat.gemm(x, b), x.double() @ b.double(), dtype)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("rows,V", [(1, 5), (3, 7), (2, 8), (65, 4099), (66, 1001), (70, 8193), (4, 50257)])
+def test_cross_entropy_and_its_column_sums(nat, rows, V, dtype):
+    g = torch.Generator(device="cuda").manual_seed(V)
+    x = (torch.randn(rows, V, device="cuda", generator=g) * 3).to(dtype)
+    x[:, : V // 2: 3] = float("-inf")  # masked classes
+    lab = torch.randint(V // 2, V, (rows,), device="cuda", generator=g, dtype=torch.int32)
+    one = torch.ones((), device="cuda")
+    loss, d = nat.ce_with_grad_cuda(x, lab, one, None, "none")
+    xd = x.double().requires_grad_()
+    want = torch.nn.functional.cross_entropy(xd, lab.long(), reduction="none")
+    want.sum().backward()
+    torch.testing.assert_close(loss.double(), want.detach(), rtol=2 * ROUND[dtype], atol=2e-4)
+    # exp of __expf: 2 units in the last place and a relative 2^-22 per unit of the argument (up to 30)
+    _near(d, xd.grad, dtype, scale=max(1.0, ROUND[torch.float32] / ROUND[dtype] * 8))
+    assert d.shape == x.shape
+    s = nat.sum_cuda(d, (0,), False)
+    if rows >= 64:
+        assert s is not NotImplemented and s.shape == (V,)
+        _near(s, d.double().sum(0), dtype, scale=d.double().abs().sum(0).max())
+    b = torch.randn(V, 40, device="cuda", generator=g).to(dtype)
+    if dtype != torch.float32:
+        want = d.double() @ b.double()
+        _near(nat.matmul_cuda(d, b), want, dtype, scale=want.abs().max() + 1, terms=V)
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
