@@ -162,7 +162,14 @@ __device__ __forceinline__ void tile_coords(int tile, int tiles_m, int tiles_n, 
   nb = in_group / rows;
 }
 
-template <int PN>
+// How C leaves the kernel. One instance each: with all three in one kernel the registers of the slowest form were spilled in the
+// others' loops (60 bytes a thread), which cost the weight gradients 4 % of a training step.
+//   EPI_16   16-bit C, overwritten, rows on 16-byte boundaries
+//   EPI_F32  fp32 C (overwritten or accumulated into), rows on 16-byte boundaries
+//   EPI_ANY  the rest: fp32 rows of any alignment, 16-bit C that is accumulated into or not aligned
+enum EpiKind : int { EPI_16 = 0, EPI_F32 = 1, EPI_ANY = 2 };
+
+template <int PN, int EPI>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
     gemm2cta_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                             const Gemm2Params p) {
@@ -314,45 +321,63 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
     for (int tile = pair; tile < num_tiles && ok; tile += npairs) {
       int b, mb, nb;
       tile_coords(tile, tiles_m, tiles_n, b, mb, nb);
-      const int row = mb * PAIR_M + (int)rank * CTA_M + q * 32 + lane;
+      const int row_base = mb * PAIR_M + (int)rank * CTA_M + q * 32;
+      const int row = row_base + lane;
       const bool row_ok = row < p.M;
       uint8_t* crow = (uint8_t*)p.C + ((long long)b * p.batch_stride_c + (long long)row * p.ldc) * esz;
+      float4* stage = (float4*)(staging + (warp - 2) * (32 * 32 * 4));
+      const int c_begin = col_half * COLS_PER_WARP, c_end = c_begin + COLS_PER_WARP;
+      // fp32 C: a thread holds 32 columns of ONE row, so storing from the registers would touch 32 lines per instruction (and so
+      // would reading the old contents when accumulating). Chunks of 32 x 32 go through shared memory instead and leave as whole
+      // 128-byte row pieces, four rows per instruction: lane -> row (lane / 8) of each group of four, 16 bytes.
+      const int sub_row = lane >> 3, sub_col = (lane & 7) * 4;
+      float* cbase = (float*)p.C + (long long)b * p.batch_stride_c + (long long)nb * PAIR_N + sub_col;
+      float4 old[8];
+      auto request_old = [&](int c) {
+        if (nb * PAIR_N + c + 32 > p.N) return;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const int rr = row_base + i * 4 + sub_row;
+          old[i] = rr < p.M ? __ldcs((const float4*)(cbase + (long long)rr * p.ldc + c)) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+      };
+      if (EPI == EPI_F32 && p.epi.accumulate) {
+        // The old contents are on their way while the tensor core still works on the tile: the first chunk into registers, the
+        // others into L2. Requested chunk by chunk after the accumulator was complete, their latency (an HBM round trip for each
+        // of the four chunks) was longer than the main loop over 2048 tokens.
+        request_old(c_begin);
+        if (row_ok) {
+#pragma unroll
+          for (int c = 32; c < COLS_PER_WARP; c += 32) {
+            if (nb * PAIR_N + c_begin + c < p.N)
+              asm volatile("prefetch.global.L2 [%0];" ::"l"(crow + (long long)(nb * PAIR_N + c_begin + c) * 4));
+          }
+        }
+      }
       ok = mbar_wait_pair(&tmem_full_bar[acc], acc_phase, abort_flag, peer_abort_addr, p.err, ERR2_TMEM_FULL_WAIT);
       if (!ok) break;
       tcgen05_fence_after();
       const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + acc * PAIR_N;
-      // fp32 C whose rows are 16-byte aligned: a thread holds 32 columns of ONE row, so storing from the registers would
-      // touch 32 lines per instruction (and so would reading the old contents when accumulating). The chunk goes through
-      // shared memory instead and leaves as whole 128-byte row pieces, four rows per instruction.
-      const bool staged = p.epi.c_dtype == XL_F32 && (p.ldc % 4) == 0 && ((((uintptr_t)p.C) | ((uintptr_t)(p.batch_stride_c * 4))) & 15) == 0;
-      const bool staged16 = p.epi.c_dtype != XL_F32 && !p.epi.accumulate && (p.ldc % 8) == 0 &&
-                            ((((uintptr_t)p.C) | ((uintptr_t)(p.batch_stride_c * 2))) & 15) == 0;
-      float4* stage = (float4*)(staging + (warp - 2) * (32 * 32 * 4));
-      const int row_base = mb * PAIR_M + (int)rank * CTA_M + q * 32;
 #pragma unroll 1
-      for (int c = col_half * COLS_PER_WARP; c < (col_half + 1) * COLS_PER_WARP; c += 32) {
+      for (int c = c_begin; c < c_end; c += 32) {
+        const int col0 = nb * PAIR_N + c;
+        if (col0 >= p.N) break;  // uniform over the warp
         uint32_t r[32];
         tmem_ld_32x32b_x32(taddr + c, r);
         tmem_ld_wait();
-        const int col0 = nb * PAIR_N + c;
-        if (col0 >= p.N) continue;  // uniform over the warp
-        if (staged16 && col0 + 32 <= p.N) {
+        if (EPI == EPI_16 && col0 + 32 <= p.N) {
           // 16-bit C, no accumulation: the thread's 32 columns (64 bytes) go to shared memory, 16-byte pieces rotated by
           // the row pair so that neither phase has bank conflicts; then 4 lanes store one row's 64 bytes, 8 rows per
           // instruction
           uint4* stage16 = (uint4*)stage;
+          const float bv = p.epi.bias ? epilogue_bias(p.epi, col0 + lane) : 0.f;  // column col0 + lane, handed out below
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
             float v[8];
 #pragma unroll
             for (int e = 0; e < 8; ++e) {
               float x = __uint_as_float(r[j * 8 + e]) * p.alpha;
-              if (p.epi.bias) {
-                const int col = col0 + j * 8 + e;
-                x += p.epi.bias_dtype == XL_F32 ? ((const float*)p.epi.bias)[col]
-                     : p.epi.bias_dtype == XL_BF16 ? __bfloat162float(((const __nv_bfloat16*)p.epi.bias)[col])
-                                                   : __half2float(((const __half*)p.epi.bias)[col]);
-              }
+              if (p.epi.bias) x += __shfl_sync(0xffffffffu, bv, j * 8 + e);
               v[e] = apply_act(x, p.epi.act);
             }
             stage16[lane * 4 + ((j + (lane >> 1)) & 3)] = pack8_16bit(v, p.epi.c_dtype == XL_F16);
@@ -366,9 +391,41 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
             if (rr < p.M) *(uint4*)(cbase16 + (long long)rr * p.ldc) = o;
           }
           __syncwarp();
-          continue;
-        }
-        if (p.epi.c_dtype == XL_F32 && !staged) {
+        } else if (EPI == EPI_F32 && col0 + 32 <= p.N) {
+          // this thread's row -> shared memory, 16-byte pieces swizzled by the row so that both phases are conflict-free
+          const float bv = p.epi.bias ? epilogue_bias(p.epi, col0 + lane) : 0.f;
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            float v[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              float x = __uint_as_float(r[j * 4 + e]) * p.alpha;
+              if (p.epi.bias) x += __shfl_sync(0xffffffffu, bv, j * 4 + e);
+              v[e] = apply_act(x, p.epi.act);
+            }
+            stage[lane * 8 + (j ^ (lane & 7))] = make_float4(v[0], v[1], v[2], v[3]);
+          }
+          __syncwarp();
+          float4 out[8];
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const int lr = i * 4 + sub_row;
+            float4 o = stage[lr * 8 + ((lane & 7) ^ (lr & 7))];
+            if (p.epi.accumulate == 1) { o.x += old[i].x; o.y += old[i].y; o.z += old[i].z; o.w += old[i].w; }
+            else if (p.epi.accumulate == 2) {
+              o.x = old[i].x * mean_a + o.x * mean_b; o.y = old[i].y * mean_a + o.y * mean_b;
+              o.z = old[i].z * mean_a + o.z * mean_b; o.w = old[i].w * mean_a + o.w * mean_b;
+            }
+            out[i] = o;
+          }
+          if (p.epi.accumulate && c + 32 < c_end) request_old(c + 32);  // ahead of this chunk's stores
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const int rr = row_base + i * 4 + sub_row;
+            if (rr < p.M) *(float4*)(cbase + (long long)rr * p.ldc + c) = out[i];
+          }
+          __syncwarp();  // the buffer is rewritten by the next chunk
+        } else if (EPI == EPI_ANY && p.epi.c_dtype == XL_F32) {
           // Rows that do not start on 16-byte boundaries (an odd number of columns): still whole row pieces, one column per
           // lane and one row per instruction, the old contents requested ahead of all stores. From the registers every
           // instruction touched 32 rows: the running mean of a 768 x 50257 gradient over 4096 tokens took 0.61 ms even with one
@@ -400,53 +457,9 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
             }
           }
           __syncwarp();
-          continue;
+        } else if (row_ok) {
+          epilogue_store_32cols(p.epi, r, crow, col0, p.alpha, mean_a, mean_b);
         }
-        if (!(staged && col0 + 32 <= p.N)) {
-          if (row_ok) epilogue_store_32cols(p.epi, r, crow, col0, p.alpha, mean_a, mean_b);
-          continue;
-        }
-        // old contents first (their latency overlaps the staging): lane -> row (lane / 8) of each group of four, 16 bytes
-        const int sub_row = lane >> 3, sub_col = (lane & 7) * 4;
-        float* cbase = (float*)p.C + (long long)b * p.batch_stride_c + col0 + sub_col;
-        float4 old[8];
-        if (p.epi.accumulate) {
-#pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            const int rr = row_base + i * 4 + sub_row;
-            old[i] = rr < p.M ? *(const float4*)(cbase + (long long)rr * p.ldc) : make_float4(0.f, 0.f, 0.f, 0.f);
-          }
-        }
-        // this thread's row -> shared memory, 16-byte pieces swizzled by the row so that both phases are conflict-free
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          float v[4];
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            float x = __uint_as_float(r[j * 4 + e]) * p.alpha;
-            if (p.epi.bias) {
-              const int col = col0 + j * 4 + e;
-              x += p.epi.bias_dtype == XL_F32 ? ((const float*)p.epi.bias)[col]
-                   : p.epi.bias_dtype == XL_BF16 ? __bfloat162float(((const __nv_bfloat16*)p.epi.bias)[col])
-                                                 : __half2float(((const __half*)p.epi.bias)[col]);
-            }
-            v[e] = apply_act(x, p.epi.act);
-          }
-          stage[lane * 8 + (j ^ (lane & 7))] = make_float4(v[0], v[1], v[2], v[3]);
-        }
-        __syncwarp();
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          const int lr = i * 4 + sub_row, rr = row_base + lr;
-          float4 o = stage[lr * 8 + ((lane & 7) ^ (lr & 7))];
-          if (p.epi.accumulate == 1) { o.x += old[i].x; o.y += old[i].y; o.z += old[i].z; o.w += old[i].w; }
-          else if (p.epi.accumulate == 2) {
-            o.x = old[i].x * mean_a + o.x * mean_b; o.y = old[i].y * mean_a + o.y * mean_b;
-            o.z = old[i].z * mean_a + o.z * mean_b; o.w = old[i].w * mean_a + o.w * mean_b;
-          }
-          if (rr < p.M) *(float4*)(cbase + (long long)rr * p.ldc) = o;
-        }
-        __syncwarp();  // the buffer is rewritten by the next chunk
       }
       // all TMEM reads of this warp are complete (wait::ld above): hand the accumulator back to the leader's MMA thread
       tcgen05_fence_before();
@@ -487,12 +500,12 @@ int make_map(CUtensorMap* map, const void* ptr, int is_fp16, long long rows, lon
 }
 
 // number of CTA pairs that can be resident at once on this device (0 if the query fails); looked up once
-template <int PN>
+template <int PN, int EPI>
 int max_resident_pairs() {
   constexpr int SMEM_TOTAL = PairCfg<PN>::SMEM_TOTAL;
   static int cached = -1;
   if (cached >= 0) return cached;
-  if (cudaFuncSetAttribute(gemm2cta_tcgen05_kernel<PN>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_TOTAL) != cudaSuccess) {
+  if (cudaFuncSetAttribute(gemm2cta_tcgen05_kernel<PN, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_TOTAL) != cudaSuccess) {
     cached = 0;
     return 0;
   }
@@ -508,7 +521,7 @@ int max_resident_pairs() {
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   int n = 0;
-  if (cudaOccupancyMaxActiveClusters(&n, gemm2cta_tcgen05_kernel<PN>, &cfg) != cudaSuccess) {
+  if (cudaOccupancyMaxActiveClusters(&n, gemm2cta_tcgen05_kernel<PN, EPI>, &cfg) != cudaSuccess) {
     cudaGetLastError();
     n = 0;
   }
@@ -516,9 +529,9 @@ int max_resident_pairs() {
   return n;
 }
 
-template <int PN>
+template <int PN, int EPI>
 int launch_pairs(const CUtensorMap& ma, const CUtensorMap& mb, const Gemm2Params& p, int max_pairs, cudaStream_t s) {
-  int pairs = max_resident_pairs<PN>();
+  int pairs = max_resident_pairs<PN, EPI>();
   if (pairs <= 0) return -4;
   if (max_pairs > 0 && max_pairs < pairs) pairs = max_pairs;
   const long long tiles = (long long)((p.M + PAIR_M - 1) / PAIR_M) * ((p.N + PN - 1) / PN) * p.batch;
@@ -535,7 +548,7 @@ int launch_pairs(const CUtensorMap& ma, const CUtensorMap& mb, const Gemm2Params
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  cudaError_t e = cudaLaunchKernelEx(&cfg, gemm2cta_tcgen05_kernel<PN>, ma, mb, p);
+  cudaError_t e = cudaLaunchKernelEx(&cfg, gemm2cta_tcgen05_kernel<PN, EPI>, ma, mb, p);
   return e != cudaSuccess ? (int)e : (int)cudaGetLastError();
 }
 
@@ -568,7 +581,7 @@ XL_API int xl_gemm2cta_tcgen05(const void* a, const void* b, void* c, int M, int
   if (batch > 1 && ((stride_a % 8) || (stride_b % 8))) return -1;
   if (accumulate < 0 || accumulate > 2 || (accumulate == 2 && step == nullptr)) return -1;
   if (tile_n != 0 && tile_n != 128 && tile_n != 256) return -1;
-  const int pair_n = tile_n ? tile_n : choose_pair_n(M, N, batch, max_pairs > 0 ? max_pairs : max_resident_pairs<256>());
+  const int pair_n = tile_n ? tile_n : choose_pair_n(M, N, batch, max_pairs > 0 ? max_pairs : max_resident_pairs<256, EPI_16>());
   CUtensorMap ma, mb;
   int r;
   if (!a_mn) r = make_map(&ma, a, ab_is_fp16, M, K, lda, batch, stride_a, BLOCK_K, CTA_M);
@@ -584,6 +597,15 @@ XL_API int xl_gemm2cta_tcgen05(const void* a, const void* b, void* c, int M, int
   p.epi.N = N; p.epi.c_dtype = c_dtype; p.epi.bias = bias; p.epi.bias_dtype = bias_dtype; p.epi.act = act;
   p.epi.accumulate = accumulate;
   p.step = step; p.alpha = alpha; p.is_fp16 = ab_is_fp16; p.err = err;
-  if (pair_n == 128) return launch_pairs<128>(ma, mb, p, max_pairs, s);
-  return launch_pairs<256>(ma, mb, p, max_pairs, s);
+  const int align = c_dtype == XL_F32 ? 4 : 8;  // elements of 16 bytes
+  const bool aligned = (ldc % align) == 0 && (batch == 1 || (stride_c % align) == 0) && (((uintptr_t)c) & 15) == 0;
+  const int kind = !aligned ? EPI_ANY : c_dtype == XL_F32 ? EPI_F32 : accumulate ? EPI_ANY : EPI_16;
+  if (pair_n == 128) {
+    if (kind == EPI_16) return launch_pairs<128, EPI_16>(ma, mb, p, max_pairs, s);
+    if (kind == EPI_F32) return launch_pairs<128, EPI_F32>(ma, mb, p, max_pairs, s);
+    return launch_pairs<128, EPI_ANY>(ma, mb, p, max_pairs, s);
+  }
+  if (kind == EPI_16) return launch_pairs<256, EPI_16>(ma, mb, p, max_pairs, s);
+  if (kind == EPI_F32) return launch_pairs<256, EPI_F32>(ma, mb, p, max_pairs, s);
+  return launch_pairs<256, EPI_ANY>(ma, mb, p, max_pairs, s);
 }
