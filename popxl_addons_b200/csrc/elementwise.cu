@@ -542,39 +542,103 @@ struct AdamArgs {
 
 __global__ void step_increment_kernel(float* step) { *step += 1.f; }
 
-template <typename TW, typename TG, typename TM>
+// V consecutive elements as one access: 16 bytes of fp32, 8 of 16-bit types. Every value of an optimizer step is touched once per
+// step, so the accesses are marked as not worth keeping in L2.
+template <typename T, int V> __device__ __forceinline__ void xl_stream_load(const T* p, float (&out)[V]) {
+  if constexpr (V == 1) {
+    out[0] = xl_to_float(*p);
+  } else if constexpr (sizeof(T) == 4) {
+    const float4 r = __ldcs(reinterpret_cast<const float4*>(p));
+    out[0] = r.x; out[1] = r.y; out[2] = r.z; out[3] = r.w;
+  } else {
+    const uint2 r = __ldcs(reinterpret_cast<const uint2*>(p));
+    const T* e = reinterpret_cast<const T*>(&r);
+#pragma unroll
+    for (int i = 0; i < V; ++i) out[i] = xl_to_float(e[i]);
+  }
+}
+template <typename T, int V> __device__ __forceinline__ void xl_stream_store(T* p, const float (&in)[V]) {
+  if constexpr (V == 1) {
+    *p = xl_from_float<T>(in[0]);
+  } else if constexpr (sizeof(T) == 4) {
+    __stcs(reinterpret_cast<float4*>(p), make_float4(in[0], in[1], in[2], in[3]));
+  } else {
+    uint2 r;
+    T* e = reinterpret_cast<T*>(&r);
+#pragma unroll
+    for (int i = 0; i < V; ++i) e[i] = xl_from_float<T>(in[i]);
+    __stcs(reinterpret_cast<uint2*>(p), r);
+  }
+}
+
+// Bound by HBM: 30 bytes per parameter with 16-bit weights (master and both moments read and written, the gradient read, the weight
+// written). Four elements per thread and access, all loads of two groups ahead of the first store.
+template <typename TW, typename TG, typename TM, int V>
 __global__ void __launch_bounds__(256)
     adam_kernel(TW* __restrict__ w, const TG* __restrict__ g, TM* __restrict__ m, float* __restrict__ v,
                 float* __restrict__ master, const float* __restrict__ step, AdamArgs a, long long n) {
+  constexpr int U = V == 1 ? 1 : 2;
   float c1 = 1.f, c2 = 1.f;
   if (step != nullptr && a.bias_correction) {
     const float t = *step;
     c1 = 1.f / (1.f - powf(a.beta1, t));
     c2 = 1.f / (1.f - powf(a.beta2, t));
   }
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-    const float gf = xl_to_float(g[i]) * a.grad_scale;
-    const float mf = xl_to_float(m[i]) * a.beta1 + gf * (1.f - a.beta1);
-    const float vf = v[i] * a.beta2 + gf * gf * (1.f - a.beta2);
-    const TM mq = xl_from_float<TM>(mf);
-    m[i] = mq;
-    v[i] = vf;
-    const float wf = master ? master[i] : xl_to_float(w[i]);
-    const float upd = (xl_to_float(mq) * c1) / (sqrtf(vf * c2) + a.eps) + wf * a.weight_decay;
-    const float wn = wf - a.lr * upd;
-    if (master) master[i] = wn;
-    w[i] = xl_from_float<TW>(wn);
+  const long long groups = n / V;
+  for (long long i0 = blockIdx.x * (256LL * U) + threadIdx.x; i0 < groups; i0 += gridDim.x * (256LL * U)) {
+    float gr[U][V], mo[U][V], ve[U][V], we[U][V];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const long long i = i0 + u * 256;
+      if (i < groups) {
+        xl_stream_load<TG, V>(g + i * V, gr[u]);
+        xl_stream_load<TM, V>(m + i * V, mo[u]);
+        xl_stream_load<float, V>(v + i * V, ve[u]);
+        if (master) xl_stream_load<float, V>(master + i * V, we[u]);
+        else xl_stream_load<TW, V>(w + i * V, we[u]);
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const long long i = i0 + u * 256;
+      if (i < groups) {
+#pragma unroll
+        for (int e = 0; e < V; ++e) {
+          const float gf = gr[u][e] * a.grad_scale;
+          mo[u][e] = mo[u][e] * a.beta1 + gf * (1.f - a.beta1);
+          ve[u][e] = ve[u][e] * a.beta2 + gf * gf * (1.f - a.beta2);
+          const float mq = xl_to_float(xl_from_float<TM>(mo[u][e]));  // the stored value enters the update
+          const float upd = (mq * c1) / (sqrtf(ve[u][e] * c2) + a.eps) + we[u][e] * a.weight_decay;
+          we[u][e] = we[u][e] - a.lr * upd;
+        }
+        xl_stream_store<TM, V>(m + i * V, mo[u]);
+        xl_stream_store<float, V>(v + i * V, ve[u]);
+        if (master) xl_stream_store<float, V>(master + i * V, we[u]);
+        xl_stream_store<TW, V>(w + i * V, we[u]);
+      }
+    }
   }
 }
 
+template <typename TW, typename TG, typename TM>
+static void adam_launch(void* w, const void* g, void* m, float* v, float* master, float* step, AdamArgs a, long long n, cudaStream_t s) {
+  // groups of four need 16-byte alignment (8 bytes for 16-bit types); up to three elements remain
+  const auto off = [](const void* p, size_t esz) { return ((uintptr_t)p) & (4 * esz - 1); };
+  const bool wide = !(off(w, sizeof(TW)) | off(g, sizeof(TG)) | off(m, sizeof(TM)) | off(v, 4) | off(master, 4));
+  const long long whole = wide ? n / 4 * 4 : 0;
+  if (whole)
+    adam_kernel<TW, TG, TM, 4><<<xl_grid_for(whole, 256 * 8), 256, 0, s>>>((TW*)w, (const TG*)g, (TM*)m, v, master, step, a, whole);
+  if (whole < n)
+    adam_kernel<TW, TG, TM, 1><<<xl_grid_for(n - whole, 256 * 4), 256, 0, s>>>(
+        (TW*)w + whole, (const TG*)g + whole, (TM*)m + whole, v + whole, master ? master + whole : nullptr, step, a, n - whole);
+}
 template <typename TW, typename TG>
 static int adam_launch_m(void* w, const void* g, void* m, int m_dtype, float* v, float* master, float* step,
                          AdamArgs a, long long n, cudaStream_t s) {
-  const int grid = xl_grid_for(n, 256 * 4);
   switch (m_dtype) {
-    case XL_F32: adam_kernel<TW, TG, float><<<grid, 256, 0, s>>>((TW*)w, (const TG*)g, (float*)m, v, master, step, a, n); break;
-    case XL_F16: adam_kernel<TW, TG, __half><<<grid, 256, 0, s>>>((TW*)w, (const TG*)g, (__half*)m, v, master, step, a, n); break;
-    case XL_BF16: adam_kernel<TW, TG, __nv_bfloat16><<<grid, 256, 0, s>>>((TW*)w, (const TG*)g, (__nv_bfloat16*)m, v, master, step, a, n); break;
+    case XL_F32: adam_launch<TW, TG, float>(w, g, m, v, master, step, a, n, s); break;
+    case XL_F16: adam_launch<TW, TG, __half>(w, g, m, v, master, step, a, n, s); break;
+    case XL_BF16: adam_launch<TW, TG, __nv_bfloat16>(w, g, m, v, master, step, a, n, s); break;
     default: return (int)cudaErrorInvalidValue;
   }
   return (int)cudaGetLastError();
@@ -617,23 +681,38 @@ XL_API int xl_sgd_step(void* w, int w_dtype, const void* g, int g_dtype, float* 
   return (int)cudaGetLastError();
 }
 
-// acc = acc * step/(step+1) + x/(step+1), `step` read on the device.
-template <typename TA, typename TX>
+// acc = acc * step/(step+1) + x/(step+1), `step` read on the device. Bound by HBM; four elements per thread and access.
+template <typename TA, typename TX, int V>
 __global__ void __launch_bounds__(256)
     accumulate_mean_kernel(TA* __restrict__ acc, const TX* __restrict__ x, const float* __restrict__ step, long long n) {
   const float t = *step;
   const float a = t / (t + 1.f), b = 1.f / (t + 1.f);
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-    acc[i] = xl_from_float<TA>(xl_to_float(acc[i]) * a + xl_to_float(x[i]) * b);
+  const long long groups = n / V;
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < groups; i += (long long)gridDim.x * blockDim.x) {
+    float o[V], xv[V];
+    xl_stream_load<TA, V>(acc + i * V, o);
+    xl_stream_load<TX, V>(x + i * V, xv);
+#pragma unroll
+    for (int e = 0; e < V; ++e) o[e] = o[e] * a + xv[e] * b;
+    xl_stream_store<TA, V>(acc + i * V, o);
+  }
+}
+template <typename TA, typename TX>
+static void accumulate_mean_launch(void* acc, const void* x, const float* step, long long n, cudaStream_t s) {
+  const bool wide = !((((uintptr_t)acc) & (4 * sizeof(TA) - 1)) | (((uintptr_t)x) & (4 * sizeof(TX) - 1)));
+  const long long whole = wide ? n / 4 * 4 : 0;
+  if (whole) accumulate_mean_kernel<TA, TX, 4><<<xl_grid_for(whole, 256 * 4), 256, 0, s>>>((TA*)acc, (const TX*)x, step, whole);
+  if (whole < n)
+    accumulate_mean_kernel<TA, TX, 1><<<xl_grid_for(n - whole, 256 * 4), 256, 0, s>>>((TA*)acc + whole, (const TX*)x + whole, step,
+                                                                                      n - whole);
 }
 XL_API int xl_accumulate_mean(void* acc, int acc_dtype, const void* x, int x_dtype, const float* step, long long n,
                               cudaStream_t s) {
-  const int grid = xl_grid_for(n, 256 * 4);
   XL_DISPATCH_DTYPE(acc_dtype, TA, {
-    if (x_dtype == acc_dtype) accumulate_mean_kernel<TA, TA><<<grid, 256, 0, s>>>((TA*)acc, (const TA*)x, step, n);
-    else if (x_dtype == XL_BF16) accumulate_mean_kernel<TA, __nv_bfloat16><<<grid, 256, 0, s>>>((TA*)acc, (const __nv_bfloat16*)x, step, n);
-    else if (x_dtype == XL_F16) accumulate_mean_kernel<TA, __half><<<grid, 256, 0, s>>>((TA*)acc, (const __half*)x, step, n);
-    else accumulate_mean_kernel<TA, float><<<grid, 256, 0, s>>>((TA*)acc, (const float*)x, step, n);
+    if (x_dtype == acc_dtype) accumulate_mean_launch<TA, TA>(acc, x, step, n, s);
+    else if (x_dtype == XL_BF16) accumulate_mean_launch<TA, __nv_bfloat16>(acc, x, step, n, s);
+    else if (x_dtype == XL_F16) accumulate_mean_launch<TA, __half>(acc, x, step, n, s);
+    else accumulate_mean_launch<TA, float>(acc, x, step, n, s);
   });
   return (int)cudaGetLastError();
 }

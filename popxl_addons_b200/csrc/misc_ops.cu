@@ -216,6 +216,65 @@ XL_API int xl_scatter_add_rows(const void* grad_out, int dtype, const int* idx, 
   return (int)cudaGetLastError();
 }
 
+// Running mean of an embedding table's gradient, without the dense gradient: acc = acc * t/(t+1), then the rows that the tokens
+// picked += grad_out / (t+1), t = *step. Bound by the first part, one read and write of the table; the second adds four fp32 values
+// per instruction (`red.v4`) where rows are aligned. 50400 x 4096 and 2048 tokens: zero fill, scatter, cast to 16 bits and dense
+// running mean took 0.85 ms.
+__global__ void __launch_bounds__(256) mean_decay_kernel(float* __restrict__ acc, const float* __restrict__ step, long long n) {
+  const float t = *step;
+  const float a = t / (t + 1.f);
+  const long long groups = n / 4;
+  float4* acc4 = reinterpret_cast<float4*>(acc);
+  const long long stride = (long long)gridDim.x * blockDim.x, first = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  for (long long i = first; i < groups; i += 2 * stride) {
+    const bool two = i + stride < groups;
+    float4 p = __ldcs(acc4 + i), q = two ? __ldcs(acc4 + i + stride) : make_float4(0.f, 0.f, 0.f, 0.f);
+    p.x *= a; p.y *= a; p.z *= a; p.w *= a;
+    q.x *= a; q.y *= a; q.z *= a; q.w *= a;
+    __stcs(acc4 + i, p);
+    if (two) __stcs(acc4 + i + stride, q);
+  }
+  if (first < n - groups * 4) acc[groups * 4 + first] *= a;
+}
+template <typename G, bool WIDE>
+__global__ void __launch_bounds__(256)
+    scatter_mean_rows_kernel(const G* __restrict__ grad_out, const int* __restrict__ idx, float* __restrict__ acc,
+                             const float* __restrict__ step, int rows, int cols) {
+  const long long i = blockIdx.x;
+  const int r = idx[i];
+  if (r < 0 || r >= rows) return;
+  const float b = 1.f / (*step + 1.f);
+  const G* src = grad_out + i * cols;
+  float* dst = acc + (long long)r * cols;
+  if (WIDE) {
+    for (int c = threadIdx.x * 4; c < cols; c += blockDim.x * 4) {
+      float v[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) v[e] = xl_to_float(src[c + e]) * b;
+      asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst + c), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]) : "memory");
+    }
+  } else {
+    for (int c = threadIdx.x; c < cols; c += blockDim.x) atomicAdd(dst + c, xl_to_float(src[c]) * b);
+  }
+}
+// acc: fp32 (rows, cols), contiguous and 16-byte aligned; grad_out: (n_idx, cols) of dtype.
+XL_API int xl_scatter_mean_rows(const void* grad_out, int dtype, const int* idx, float* acc, const float* step, long long n_idx,
+                                int rows, int cols, cudaStream_t s) {
+  const long long n = (long long)rows * cols;
+  if (n < 1) return 0;
+  if (((uintptr_t)acc) & 15) return -1;
+  mean_decay_kernel<<<xl_grid_for(n, 256 * 8), 256, 0, s>>>(acc, step, n);
+  if (n_idx > 0) {
+    XL_DISPATCH_DTYPE(dtype, G, {
+      if (cols % 4 == 0)
+        scatter_mean_rows_kernel<G, true><<<(unsigned)n_idx, 256, 0, s>>>((const G*)grad_out, idx, acc, step, rows, cols);
+      else
+        scatter_mean_rows_kernel<G, false><<<(unsigned)n_idx, 256, 0, s>>>((const G*)grad_out, idx, acc, step, rows, cols);
+    });
+  }
+  return (int)cudaGetLastError();
+}
+
 // ------------------------------------------------------------------------------------------------------------------
 // Row statistics for ops whose rows are sharded over ranks: per row (sum, sum of squares) for the hidden-sharded
 // LayerNorm's forward pass (its backward pass and the vocabulary-sharded cross-entropy are in sharded_ops.cu). The tiny

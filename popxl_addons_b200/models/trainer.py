@@ -93,18 +93,24 @@ def build_optimizer(ir, cfg, par, groups, hp, state_dtype, shard_optimizer, fuse
                     if cfg.dp > 1:
                         g = ops.collectives.replicated_all_reduce(g, "mean", par.dp_group)
                     master = xl.variable(host32, xl.float32, f"master.{full}", replica_grouping=rg)
-                    key = ("full", tuple(w.shape), decay)
+                    key = ("full", tuple(w.shape), w.dtype, decay)
                 masters[full] = master
+                # an update that is not sharded writes the 16-bit weight in the kernel that updates the master
+                direct = not shardable and w.dtype in (xl.bfloat16, xl.float16)
                 if key not in opt_graphs:
                     with xl.ipu(None):  # the graph is shared by parameters on different slots
                         ofacts, ograph = AdamOptimizerStep().create_graph(
-                            master, g, rg, lr=hp["lr"], beta1=hp["beta1"], beta2=hp["beta2"], eps=hp["eps"],
-                            weight_decay=decay, first_order_dtype=state_dtype, bias_correction=True)
+                            w if direct else master, g, rg, lr=hp["lr"], beta1=hp["beta1"], beta2=hp["beta2"], eps=hp["eps"],
+                            weight_decay=decay, first_order_dtype=state_dtype, bias_correction=True,
+                            **({"master": master} if direct else {}))
                     opt_graphs[key] = (ofacts, ograph)
                 ofacts, ograph = opt_graphs[key]
                 ostate = ofacts.init(f"adam.{full}")
-                ograph.bind(ostate).call(master, g)
                 opt_state[full] = ostate
+                if direct:
+                    ograph.bind(ostate).call(w, g, master)
+                    continue
+                ograph.bind(ostate).call(master, g)
                 new_w = ops.cast(master, w.dtype)
                 if shardable:
                     new_w = ops.collectives.replicated_all_gather(new_w, par.dp_group, output_shape=w.shape)

@@ -39,7 +39,7 @@ class AdamOptimizerStep(Module):
               lr: Scalar, beta1: Scalar = 0.9, beta2: Scalar = 0.999, eps: Scalar = 1e-5,
               weight_decay: Scalar = 1e-2, first_order_dtype: xl.dtype = xl.float16, bias_correction: bool = True,
               loss_scaling: Scalar = 1, global_norm: Optional[xl.Tensor] = None,
-              global_norm_max: Optional[Scalar] = None, master: Optional[xl.Tensor] = None):
+              global_norm_max: Optional[Scalar] = None, master: Optional[xl.TensorByRef] = None):
         """Update `var` in place with gradient `grad`. `loss_scaling` divides the gradient; with `global_norm` and
         `global_norm_max` it is additionally scaled by `max_norm / max(global_norm, max_norm)` (norm clipping).
         `master` is an optional fp32 copy of `var` that receives the update at full precision."""

@@ -43,7 +43,8 @@ def autodiff_with_accumulation(graph: GraphWithNamedArgs, tensors_to_accumulate_
     `mean_accum_counter` (zero it to start a new mean). Other `grads_required` remain graph outputs.
     Accumulators have the dtype of their tensor unless `accum_dtype` is given (e.g. fp32 sums for bf16 weights).
     With `fuse_matmul`, a gradient that is the direct result of a matmul and is used for nothing else is never written
-    out: the matmul and the accumulation become one `matmul_accumulate_mean_` op (GEMM with accumulating epilogue).
+    out: the matmul and the accumulation become one `matmul_accumulate_mean_` op (GEMM with accumulating epilogue). The
+    same goes for the gradient of a table that is looked up (`gather_grad_accumulate_mean_`).
 
     Returns the factories for the accumulators/counter and the gradient graph (its `args` name them)."""
     accumulate = list(tensors_to_accumulate_grads)
@@ -78,7 +79,7 @@ def autodiff_with_accumulation(graph: GraphWithNamedArgs, tensors_to_accumulate_
             named[f"accum.{key}"] = accum
             if t not in required:
                 drop.append(idx)
-            if fuse_matmul and t not in required and _fuse_matmul_into_accumulator(g, grad_t, accum, counter):
+            if fuse_matmul and t not in required and _fuse_into_accumulator(g, grad_t, accum, counter):
                 continue
             ops.var_updates.accumulate_mean_(accum, grad_t, counter)
         ops.add_(counter, xl.constant(1.0, xl.float32))
@@ -89,19 +90,27 @@ def autodiff_with_accumulation(graph: GraphWithNamedArgs, tensors_to_accumulate_
     return NamedVariableFactories.from_dict(factories), grad
 
 
-def _fuse_matmul_into_accumulator(g: xl.Graph, grad_t: xl.Tensor, accum: xl.Tensor, counter: xl.Tensor) -> bool:
-    """If `grad_t` comes straight out of a 2-D matmul and has no other consumer, replace that matmul by a
-    `matmul_accumulate_mean_` emitted now (current graph must be `g`). Returns whether the rewrite happened."""
+def _fuse_into_accumulator(g: xl.Graph, grad_t: xl.Tensor, accum: xl.Tensor, counter: xl.Tensor) -> bool:
+    """If `grad_t` comes straight out of a 2-D matmul, or out of the lookup gradient of a 2-D table with an fp32 accumulator,
+    and has no other consumer, replace that op by a `matmul_accumulate_mean_` or `gather_grad_accumulate_mean_` emitted
+    now (current graph must be `g`). Returns whether the rewrite happened."""
     op = grad_t.producer
-    if op is None or op.opdef.name != "matmul" or op.graph is not g:
+    if op is None or op.opdef.name not in ("matmul", "gather_grad") or op.graph is not g:
         return False
     a, b = op.inputs
-    if a.rank != 2 or b.rank != 2 or tuple(grad_t.shape) != tuple(accum.shape):
+    if accum.rank != 2 or tuple(grad_t.shape) != tuple(accum.shape):
+        return False
+    if op.opdef.name == "matmul" and (a.rank != 2 or b.rank != 2):
+        return False
+    if op.opdef.name == "gather_grad" and (op.attrs["axis"] != 0 or accum.dtype != xl.float32):
         return False
     if any(grad_t in other.inputs for other in g.ops) or g._outputs.count(grad_t) > 1:
         return False
     g.ops.remove(op)
-    ops.var_updates.matmul_accumulate_mean_(accum, a, b, counter)
+    if op.opdef.name == "matmul":
+        ops.var_updates.matmul_accumulate_mean_(accum, a, b, counter)
+    else:
+        ops.var_updates.gather_grad_accumulate_mean_(accum, a, b, counter, op.attrs["axis"], op.attrs["zero_OOR"])
     return True
 
 

@@ -12,7 +12,7 @@ import torch
 
 from ..core import Tensor
 from .. import dtypes as _dt
-from ..opdef import OpDef, emit, emit1
+from ..opdef import OPS, OpDef, emit, emit1
 
 Scalar = Union[float, Tensor]
 
@@ -368,3 +368,23 @@ def matmul_accumulate_mean_(acc: Tensor, lhs: Tensor, rhs: Tensor, step: Tensor)
     """`acc = acc * step/(step+1) + (lhs @ rhs)/(step+1)`: the product never exists in memory, the GEMM epilogue
     folds each output tile into the accumulator (weight gradients under gradient accumulation)."""
     return emit1("matmul_accumulate_mean_", [acc, lhs, rhs, step])
+
+
+# ---- embedding gradient folded into the running mean --------------------------------------------------------------
+
+
+def _gather_grad_acc_mean_ref(acc, g, idx, step, axis, zero_OOR):
+    if acc.device.type == "meta":
+        return acc
+    dense = OPS["gather_grad"].impl(g, idx, axis=axis, zero_OOR=zero_OOR, w_shape=tuple(acc.shape))
+    return _accumulate_mean_ref(acc, dense, step, _tensor_scalars=("step",), step=None)
+
+
+OpDef("gather_grad_accumulate_mean_", impl=_gather_grad_acc_mean_ref, inplace=True, keeps_meta=True)
+
+
+def gather_grad_accumulate_mean_(acc: Tensor, grad: Tensor, indices: Tensor, step: Tensor, axis: int = 0,
+                                 zero_OOR: bool = False) -> Tensor:
+    """`acc = acc * step/(step+1) + G/(step+1)`, where G is the gradient of the table of a `gather`: zeros with the rows of
+    `grad` added at `indices`. On the device G never exists in memory."""
+    return emit1("gather_grad_accumulate_mean_", [acc, grad, indices, step], {"axis": axis, "zero_OOR": zero_OOR})

@@ -92,3 +92,52 @@ def test_greedy_choice(nat, rows, V, valid, dtype):
     want[-1] = 0
     torch.testing.assert_close(m.cpu(), seen.max(1).values)
     assert torch.equal(i.cpu().long() - 7, want)
+
+
+@pytest.mark.parametrize("n", [1, 3, 4, 7, 1024, 2049, 4 * 256 * 2 * 3 + 5])
+@pytest.mark.parametrize("offset", [0, 1])
+@pytest.mark.parametrize("moment", [torch.float32, torch.bfloat16])
+def test_adam_writes_the_master_and_the_16_bit_weight(nat, n, offset, moment):
+    """Groups of four, the elements behind the last one and buffers that are not aligned; master and weight from one kernel.
+    Against the op's torch reference: a few fp32 roundings apart (1e-6), one bf16 step for the 16-bit outputs."""
+    from popxl_addons_b200.xl.opdef import OPS
+
+    g = torch.Generator().manual_seed(n + offset)
+    base = [torch.randn(n + offset, generator=g) for _ in range(3)] + [torch.rand(n + offset, generator=g)]
+    kw = dict(has_step=True, has_master=True, bias_correction=True, _tensor_scalars=(), lr=1e-2, beta1=0.9, beta2=0.95,
+              epsilon=1e-5, weight_decay=0.01, grad_scale=0.5)
+    got = []
+    for dev in ("cpu", "cuda"):
+        master, grad, m, v = (b.to(dev).clone()[offset:] for b in base)
+        w = base[0].to(dev).bfloat16()[offset:].clone() if offset == 0 else base[0].to(dev).bfloat16()[offset:]
+        m = m.to(moment)
+        step = torch.tensor(2.0, device=dev)
+        if dev == "cpu":
+            OPS["adam_fused_"].impl(w, grad, m, v, step, master, **kw)
+        else:
+            rc = nat._adam(w.data_ptr(), nat._CODE[w.dtype], grad.data_ptr(), nat._CODE[grad.dtype], m.data_ptr(),
+                              nat._CODE[m.dtype], v.data_ptr(), master.data_ptr(), step.data_ptr(), 1e-2, 0.9, 0.95, 1e-5,
+                              0.01, 0.5, 1, n, nat._stream())
+            assert rc == 0
+        got.append([t.float().cpu() for t in (w, m, v, master, step)])
+    for a, b, tol in zip(*got, (2 ** -8, 1e-6 if moment == torch.float32 else 2 ** -8, 1e-6, 1e-6, 0)):
+        assert torch.allclose(a, b, rtol=tol, atol=tol), (a - b).abs().max()
+
+
+@pytest.mark.parametrize("rows,cols,n", [(1, 4, 1), (5, 3, 9), (33, 130, 64), (100, 768, 257), (7, 8, 0)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("t", [0.0, 3.0])
+def test_embedding_gradient_into_the_running_mean(nat, rows, cols, n, dtype, t):
+    """Rows of a table gradient added straight into the running mean, against 64 bits: indices repeat and some are out of
+    range. fp32 sums of up to n terms: 1e-6 * n relative to the largest."""
+    g = torch.Generator().manual_seed(rows * cols + n)
+    acc = torch.randn(rows, cols, generator=g)
+    grad = torch.randn(n, cols, generator=g).to(dtype)
+    idx = torch.randint(-1, rows + 1, (n,), generator=g, dtype=torch.int32)
+    ok = (idx >= 0) & (idx < rows)
+    dense = torch.zeros(rows, cols, dtype=torch.float64).index_add_(0, idx[ok].long(), grad[ok].double())
+    want = acc.double() * (t / (t + 1)) + dense / (t + 1)
+    dev = acc.cuda()
+    out = nat.gather_grad_accumulate_mean_cuda(dev, grad.cuda(), idx.cuda(), torch.tensor(t, device="cuda"), 0, True)
+    assert out is dev
+    assert (dev.cpu().double() - want).abs().max() <= 1e-6 * max(1, n)
