@@ -118,6 +118,32 @@ static inline int xl_grid_for(long long n_items, int per_block, int max_blocks =
   return (int)b;
 }
 
+// Contiguous ranges of items for the CTAs of a grid: the first `rem` CTAs take per + 1 items, the others per.
+struct XlRanges {
+  int per, rem;
+  __device__ __forceinline__ int begin(int cta) const { return cta * per + min(cta, rem); }
+  __device__ __forceinline__ int owner(int item) const {
+    const int head = rem * (per + 1);
+    return item < head ? item / (per + 1) : rem + (item - head) / per;
+  }
+};
+
+__device__ __forceinline__ void xl_cp_async16(void* smem_dst, const void* src, bool on) {
+  const int bytes = on ? 16 : 0;  // 0: the destination is zero-filled
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(smem_dst)), "l"(src),
+               "r"(bytes)
+               : "memory");
+}
+
+// two packed 16-bit numbers of type T, low half first
+template <typename T> __device__ __forceinline__ float2 xl_pair_to_float2(uint32_t w);
+template <> __device__ __forceinline__ float2 xl_pair_to_float2<__half>(uint32_t w) {
+  return __half22float2(*reinterpret_cast<const __half2*>(&w));
+}
+template <> __device__ __forceinline__ float2 xl_pair_to_float2<__nv_bfloat16>(uint32_t w) {
+  return make_float2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u));
+}
+
 // Programmatic dependent launch: the kernel may start while its predecessor on the stream drains. It must call
 // xl_grid_dependency_wait() before it touches anything the predecessor reads or writes; what it does before (loading weights,
 // which nothing in flight writes) overlaps the predecessor's tail. xl_grid_launch_dependents() after that wait lets the

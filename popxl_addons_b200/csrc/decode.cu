@@ -1,6 +1,6 @@
 // Kernels of the token-by-token decoding path (batch of a few sequences, one new token each):
 //   xl_gq_gemm_small_m   y[M<=16, N] = x[M, K] * dequant(Wq)[K, N] (+ bias): 4-bit group-quantised weights are streamed
-//                        once, de-quantised in registers and fed to the tensor cores; no 16-bit copy of W ever exists
+//                        once and fed to the tensor cores as codes; scales and zero points meet the fp32 sums
 //   xl_rotary_at         rotary embedding of the new tokens at a position read from device memory
 //   xl_kv_append         write the new keys / values into the KV cache at that position
 //   xl_attn_decode       attention of the new query against the cache (split over the sequence + combine)
@@ -8,10 +8,10 @@
 // Everything that depends on the current position reads it from a device word, so one decoding step has no
 // launch-time argument that changes between steps and can be replayed as a CUDA graph.
 //
-// The de-quantising GEMM is bandwidth-bound by construction (M <= 16: two FLOPs per weight nibble and row), so it uses
-// the register-operand `mma.sync.m16n8k16` form: its operands come straight from the registers that hold the freshly
-// de-quantised values, which is exactly what a streaming kernel wants. (tcgen05 needs its B operand in shared memory;
-// for prefill-sized M the weights are de-quantised once and the tcgen05 GEMM is used.)
+// The int4 GEMM is bandwidth-bound by construction (M <= 16), so it uses the register-operand `mma.sync.m16n8k16` form: its
+// operands come straight from the registers that hold the freshly unpacked codes, which is exactly what a streaming kernel wants.
+// (tcgen05 needs its operands in shared memory or TMEM; for prefill-sized M the weights are de-quantised once and the tcgen05 GEMM
+// is used.)
 #include "common.cuh"
 
 #include <cooperative_groups.h>
@@ -22,306 +22,403 @@
 // ------------------------------------------------------------------------------------------------------------------
 // int4 group-quantised GEMM, M <= 16
 // ------------------------------------------------------------------------------------------------------------------
-constexpr int GQ_NT = 8;         // n-tiles of 8 columns per warp -> a CTA covers 64 output columns
-constexpr int GQ_WARPS = 8;      // warps of a CTA split K between them
-constexpr int GQ_KCHUNK = 128;   // k values per warp iteration (32 per lane quad member)
+// y[m, n] = sum over blocks b of s[n, b] * (sum_k x[m, k] * q[n, k]) + z[n, b] * (sum_k x[m, k]), q the 4-bit codes: scale and zero
+// point are applied to fp32 sums, so the weights themselves are never rounded to 16 bits, and a code costs less than one
+// instruction: a nibble moved into the mantissa of a 16-bit float with a suitable exponent IS the number BASE + n (bf16:
+// 0x4300 | n = 128 + n; fp16: 0x5400 | n << 4 = 64 + n), two at a time, and the base goes with the zero point.
+// (De-quantising every weight to 16 bits took 5.5 instructions per weight, 46 % of the issue slots at a fifth of the bandwidth.
+// Both halves of the sum are of the size of BASE * |x|: activations above 2^120 overflow, and an infinite one gives NaN.)
+//
+// The channels are the rows of the `mma.sync.m16n8k16` tiles and the tokens their columns, so up to 8 tokens take one MMA per 256
+// weights and 9 to 16 tokens two. Lane (quad g, j) holds rows g and g + 8; of every block of 64 (or 32) k values lane j of a quad
+// feeds 16 (8) consecutive ones. Any assignment of k values to the k slots of an MMA is valid as long as both operands agree: the
+// codes k and k + 4 of eight consecutive ones lie 16 bits apart, so x is permuted to (0, 4), (1, 5), ... once per chunk. An MMA
+// whose weights are all ones gives the sums of x in the layout of the accumulators.
+//
+// Work = (tiles of CT * 16 channels) x (K chunks of 128), tile-major, cut into equal contiguous ranges, one per CTA (one CTA per
+// SM): the grid is sized to the machine, not to the problem. Warps take the chunks of a tile segment in turn; weights, scales and
+// zero points reach them through per-warp double buffers filled with cp.async. A tile shared by several CTAs is finished by the one
+// that arrives last: every CTA leaves its sums in a slot of its own and the finisher adds the slots in CTA order, so results do
+// not depend on timing. A launch requests its first weights while its predecessor drains.
+constexpr int GQ_KCHUNK = 128;
 
-__device__ __forceinline__ void mma_m16n8k16(float (&c)[4], const uint32_t (&a)[4], const uint32_t (&b)[2], bool bf16) {
-  if (bf16) {
+template <typename T> __device__ __forceinline__ void mma_m16n8k16(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  if constexpr (std::is_same<T, __nv_bfloat16>::value) {
     asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
+        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
   } else {
     asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
+        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
   }
 }
 
-// ---- de-quantisation without integer->float conversions ------------------------------------------------------------
-// A nibble n placed in the mantissa of a 16-bit float with a suitable exponent IS the number base + n
-// (bf16: 0x4180 | n << 3 = 16 + n; fp16: 0x5400 | n << 4 = 64 + n). A packed subtraction of the base (exact) and one
-// packed FMA per two weights give n * s + z, rounded once like the reference. The byte shuffles below turn one 32-bit
-// load (two packed words = 8 nibbles, first element of a word in its top nibble) into four registers of two
-// consecutive weights each, low half first.
 template <typename T> struct GqFmt;
 template <> struct GqFmt<__nv_bfloat16> {
-  using T2 = __nv_bfloat162;
-  static constexpr uint32_t MASK = 0x78787878u, MAGIC = 0x41804180u;
-  static constexpr float BASE = 16.f;
-  static __device__ __forceinline__ uint32_t lo(uint32_t w) { return (w << 3) & MASK; }
-  static __device__ __forceinline__ uint32_t hi(uint32_t w) { return (w >> 1) & MASK; }
-  static __device__ __forceinline__ T2 pair(float a) { return __float2bfloat162_rn(a); }
+  static constexpr uint32_t MASK = 0x000F000Fu, MAGIC = 0x43004300u, ONES = 0x3F803F80u;
+  static constexpr float BASE = 128.f;
 };
 template <> struct GqFmt<__half> {
-  using T2 = __half2;
-  static constexpr uint32_t MASK = 0xF0F0F0F0u, MAGIC = 0x54005400u;
+  static constexpr uint32_t MASK = 0x00F000F0u, MAGIC = 0x54005400u, ONES = 0x3C003C00u;
   static constexpr float BASE = 64.f;
-  static __device__ __forceinline__ uint32_t lo(uint32_t w) { return (w << 4) & MASK; }
-  static __device__ __forceinline__ uint32_t hi(uint32_t w) { return w & MASK; }
-  static __device__ __forceinline__ T2 pair(float a) { return __float2half2_rn(a); }
 };
-
-// w: two packed words (word 0 in the low half). out[0..1]: weights 0-1, 2-3 of word 0; out[2..3]: the same of word 1.
-template <typename T>
-__device__ __forceinline__ void gq_dequant8(uint32_t w, typename GqFmt<T>::T2 s2, typename GqFmt<T>::T2 z2, uint32_t (&out)[4]) {
+// w: eight codes, two packed words (the first code of a word in its top nibble). out[i]: codes i and i + 4.
+template <typename T> __device__ __forceinline__ void gq_codes8(uint32_t w, uint32_t (&out)[4]) {
   using F = GqFmt<T>;
-  using T2 = typename F::T2;
-  const uint32_t lo = F::lo(w), hi = F::hi(w);  // low / high nibble of every byte, moved into the mantissa position
-  const uint32_t sel[4] = {0x0501u, 0x0400u, 0x0703u, 0x0602u};
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    uint32_t v = (__byte_perm(hi, lo, sel[i]) & 0x00FF00FFu) | F::MAGIC;
-    T2 r = __hfma2(__hsub2(*reinterpret_cast<T2*>(&v), F::pair(F::BASE)), s2, z2);
-    out[i] = *reinterpret_cast<uint32_t*>(&r);
+  if constexpr (std::is_same<T, __nv_bfloat16>::value) {
+    out[0] = ((w >> 12) & F::MASK) | F::MAGIC;
+    out[1] = ((w >> 8) & F::MASK) | F::MAGIC;
+    out[2] = ((w >> 4) & F::MASK) | F::MAGIC;
+    out[3] = (w & F::MASK) | F::MAGIC;
+  } else {
+    out[0] = ((w >> 8) & F::MASK) | F::MAGIC;
+    out[1] = ((w >> 4) & F::MASK) | F::MAGIC;
+    out[2] = (w & F::MASK) | F::MAGIC;
+    out[3] = ((w << 4) & F::MASK) | F::MAGIC;
   }
 }
 
-// packed: (N, K/gs, gs/4) u16, first element of a word in its top nibble; scale / zero: (N, K/gs).
-// Any assignment of actual k indices to the 16 k-slots of an MMA is valid as long as A and B agree, so each lane
-// keeps the 32 consecutive k values of its 16-byte weight load and feeds them to 8 MMAs, 4 values at a time.
-//
-// Work = (column tiles of 64) x (K chunks of 128), tile-major, cut into equal contiguous ranges, one per CTA
-// ("stream-K": the grid is sized to the machine, not to the problem, so there is no partial last wave). A CTA walks
-// its range tile by tile; its warps split the chunks of the current tile segment and reduce through shared memory.
-// A segment that covers a whole tile is finished by its CTA; otherwise the CTAs sharing the tile add their partial
-// sums into an fp32 workspace tile and the one that completes the tile's chunk count applies the epilogue and leaves
-// workspace and counter zeroed for the next launch. Epilogue: + bias, GELU on the columns >= act_from_col. x and y are
-// windows of wider matrices (ldx, ldy).
-template <typename T, typename S>
-__global__ void __launch_bounds__(GQ_WARPS * 32, 2)
-    gq_gemm_small_m_kernel(const T* __restrict__ x, const uint16_t* __restrict__ packed, const S* __restrict__ scale,
-                           const S* __restrict__ zero, const T* __restrict__ bias, T* __restrict__ y, int M, int N, int K,
-                           int group_size, long long ldx, long long ldy, int act_from_col, float* __restrict__ ws,
-                           unsigned int* __restrict__ counters, int sz_transposed) {
+struct GqParams {
+  const void* x;
+  long long ldx;
+  const uint16_t* packed;  // (N, K/gs, gs/4), first code of a word in its top nibble
+  const void *scale, *zero;  // sz_pairs: scale holds (scale, zero) pairs (K/gs, N, 2); else both (N, K/gs)
+  int sz_pairs;
+  const void* bias;
+  void* y;
+  long long ldy;
+  int M, N, K, group_size, act_from_col;
+  float* slots;            // [grid][2][16 * COLS]
+  unsigned int* counters;  // one per tile, zero between launches
+};
+
+// NT: tiles of 8 tokens; WPB: 32-bit words of codes per lane and block (2: blocks of 64 k values, 1: of 32)
+template <int NT, int WPB> struct GqCfg {
+  static constexpr int WARPS = NT == 1 ? 16 : 8;  // as many as the registers allow
+  static constexpr int CT = NT == 1 ? 4 : 8;      // with more tokens wider tiles, so that x is read less often
+  static constexpr int COLS = CT * 16;
+  static constexpr int BLOCKS = GQ_KCHUNK / (32 * WPB);
+  static constexpr int CODE_UNITS = CT * 64;                 // 16-byte units of codes per stage
+  static constexpr int SZ_UNITS = BLOCKS * COLS / 4;         // (scale, zero) pairs of 16-bit numbers, four channels per unit
+  static constexpr int STAGE_UNITS = CODE_UNITS + SZ_UNITS;
+  static constexpr int RED_LD = COLS + 4;
+  static constexpr int RED_FLOATS = WARPS * NT * 8 * RED_LD;
+  static constexpr int SMEM = WARPS * 2 * STAGE_UNITS * 16 + RED_FLOATS * 4;
+};
+
+template <typename T, typename S, int NT, int WPB>
+__global__ void __launch_bounds__(GqCfg<NT, WPB>::WARPS * 32, 1) gq_gemm_small_m_kernel(const GqParams p) {
   using F = GqFmt<T>;
-  using T2 = typename F::T2;
-  __shared__ float red[GQ_WARPS][16][8 * GQ_NT + 1];
+  using C = GqCfg<NT, WPB>;
+  constexpr int CT = C::CT, COLS = C::COLS, BLOCKS = C::BLOCKS, SB = 32 * WPB, WARPS = C::WARPS;
+  extern __shared__ uint4 gq_smem[];
   __shared__ unsigned int finish;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int quad = lane >> 2, j = lane & 3;  // quad: row of A / column of B inside a tile; j: k sub-slot
-  const int groups = K / group_size;
-  constexpr bool BF = std::is_same<T, __nv_bfloat16>::value;
-  constexpr int TILE = 16 * 8 * GQ_NT;
-  const int chunks = K / GQ_KCHUNK;
-  const int n_tiles = (N + 8 * GQ_NT - 1) / (8 * GQ_NT);
-  const long long total = (long long)n_tiles * chunks;
-  long long item = total * blockIdx.x / gridDim.x;
-  const long long item_end = total * (blockIdx.x + 1) / gridDim.x;
-  const bool row_lo = quad < M, row_hi = quad + 8 < M;
-  // Weights reach the MMAs through a per-warp double buffer in shared memory filled with cp.async: while a warp works on
-  // one chunk (8 tiles x 512 B) the next one, possibly of the next tile segment, is already in flight, so DRAM latency
-  // is hidden without spending registers. Every lane reads back exactly the 16-byte pieces it copied itself.
-  extern __shared__ uint4 wbuf_all[];
-  uint4* wbuf = wbuf_all + warp * (2 * GQ_NT * 32);
-  auto prefetch = [&](int tile_, int ch_, int buf_) {
-    const int k_lane_ = ch_ * GQ_KCHUNK + j * 32;
-#pragma unroll
-    for (int t = 0; t < GQ_NT; ++t) {
-      const int n = tile_ * (8 * GQ_NT) + t * 8 + quad;
-      uint4* dst = wbuf + (buf_ * GQ_NT + t) * 32 + lane;
-      if (n < N) {
-        const uint16_t* src = packed + (long long)n * (K / 4) + k_lane_ / 4;
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
-                     : "memory");
-      } else {
-        *dst = make_uint4(0, 0, 0, 0);
-      }
+  const int g = lane >> 2, j = lane & 3;
+  uint4* ring = gq_smem + warp * (2 * C::STAGE_UNITS);
+  float* red = reinterpret_cast<float*>(gq_smem + WARPS * 2 * C::STAGE_UNITS);
+  const int chunks = p.K / GQ_KCHUNK, n_tiles = (p.N + COLS - 1) / COLS, groups = p.K / p.group_size;
+  const int total = n_tiles * chunks;
+  const XlRanges ranges{total / (int)gridDim.x, total % (int)gridDim.x};
+  int item = ranges.begin(blockIdx.x);
+  const int item_end = ranges.begin(blockIdx.x + 1);
+  const int first_tile = item / chunks;
+  const bool pairs16 = p.sz_pairs && p.N % 4 == 0;  // scales and zero points can be copied 16 bytes at a time
+  const T* x = (const T*)p.x;
+
+  // The chunks of this warp over the whole range, tile after tile.
+  struct Cursor { int item, c1, ch, tile; };  // first item of the current tile segment, its end chunk, current chunk, tile
+  auto segment = [&](Cursor& c) {
+    while (c.item < item_end) {
+      c.tile = c.item / chunks;
+      const int c0 = c.item - c.tile * chunks;
+      c.c1 = min(chunks, c0 + (item_end - c.item));
+      c.ch = c0 + warp;
+      if (c.ch < c.c1) return;
+      c.item += c.c1 - c0;
     }
-    asm volatile("cp.async.commit_group;" ::: "memory");
   };
-  int buf = 0;
-  bool have = false;  // wbuf[buf] already holds (or is receiving) this warp's first chunk of the current segment
-  while (item < item_end) {
-    const int tile = (int)(item / chunks);
-    const int c0 = (int)(item - (long long)tile * chunks);
-    const int c1 = (int)min((long long)chunks, c0 + (item_end - item));
-    const int n_base = tile * (8 * GQ_NT);
-    float c[GQ_NT][4];
+  auto advance = [&](Cursor& c) {
+    if (c.item >= item_end) return;
+    c.ch += WARPS;
+    if (c.ch >= c.c1) {
+      c.item = c.tile * chunks + c.c1;
+      segment(c);
+    }
+  };
+  // Codes of a tile of 16 channels: piece q (32 codes) of row r at unit q * 16 + (r ^ 4 * (q & 1)), so that the eight-byte reads
+  // below touch every bank once.
+  auto request = [&](const Cursor& c, int buf) {
+    if (c.item < item_end) {
+      uint4* dst = ring + buf * C::STAGE_UNITS;
 #pragma unroll
-    for (int t = 0; t < GQ_NT; ++t)
-#pragma unroll
-      for (int e = 0; e < 4; ++e) c[t][e] = 0.f;
-    if (!have && c0 + warp < c1) prefetch(tile, c0 + warp, buf);
-    have = false;
-    for (int ch = c0 + warp; ch < c1; ch += GQ_WARPS) {
-      // start the copy of the chunk after this one: the next of this segment, or this warp's first of the next segment
-      bool next_issued = false;
-      if (ch + GQ_WARPS < c1) {
-        prefetch(tile, ch + GQ_WARPS, buf ^ 1);
-        next_issued = true;
-      } else {
-        const long long nit = item + (c1 - c0);
-        if (nit < item_end) {
-          const int ntile = (int)(nit / chunks);
-          const int nc0 = (int)(nit - (long long)ntile * chunks);
-          const int nc1 = (int)min((long long)chunks, nc0 + (item_end - nit));
-          if (nc0 + warp < nc1) {
-            prefetch(ntile, nc0 + warp, buf ^ 1);
-            next_issued = have = true;
-          }
-        }
+      for (int i = 0; i < CT * 2; ++i) {
+        const int row = i * 8 + g, n = c.tile * COLS + row, r = row & 15;
+        const bool on = n < p.N;
+        const uint16_t* src = p.packed + (long long)(on ? n : 0) * (p.K / 4) + c.ch * (GQ_KCHUNK / 4) + j * 8;
+        xl_cp_async16(dst + (row >> 4) * 64 + j * 16 + (r ^ ((j & 1) * 4)), src, on);
       }
-      const int k_lane = ch * GQ_KCHUNK + j * 32;  // this lane's 32 consecutive k values
-      uint32_t sz[GQ_NT];  // (scale, zero) of this lane's group, two S values
-      const int g = k_lane / group_size;
+      uint4* sz = dst + C::CODE_UNITS;
 #pragma unroll
-      for (int t = 0; t < GQ_NT; ++t) {
-        const int n = n_base + t * 8 + quad;
-        sz[t] = 0;
-        if (n < N) {
-          if (sz_transposed) {
-            // scale holds (groups, N, 2): 8 consecutive columns of one group are one 32-byte segment
-            sz[t] = reinterpret_cast<const uint32_t*>(scale)[(long long)g * N + n];
+      for (int i = 0; i < (C::SZ_UNITS + 31) / 32; ++i) {
+        const int u = i * 32 + lane, b = u / (COLS / 4), n = c.tile * COLS + (u % (COLS / 4)) * 4;
+        const int grp = (c.ch * GQ_KCHUNK + b * SB) / p.group_size;
+        if (u < C::SZ_UNITS) {
+          if (pairs16) {
+            const bool on = n < p.N;
+            xl_cp_async16(sz + u, (const uint32_t*)p.scale + (on ? (long long)grp * p.N + n : 0), on);
           } else {
-            const S sv = scale[(long long)n * groups + g], zv = zero[(long long)n * groups + g];
-            sz[t] = (uint32_t)(*reinterpret_cast<const uint16_t*>(&sv)) |
-                    ((uint32_t)(*reinterpret_cast<const uint16_t*>(&zv)) << 16);
+            uint32_t v[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              v[e] = 0;
+              if (n + e < p.N) {
+                if (p.sz_pairs) {
+                  v[e] = ((const uint32_t*)p.scale)[(long long)grp * p.N + n + e];
+                } else {
+                  const long long at = (long long)(n + e) * groups + grp;
+                  v[e] = ((const uint16_t*)p.scale)[at] | ((uint32_t)((const uint16_t*)p.zero)[at] << 16);
+                }
+              }
+            }
+            sz[u] = make_uint4(v[0], v[1], v[2], v[3]);
           }
         }
       }
-      if (next_issued) asm volatile("cp.async.wait_group 1;" ::: "memory");
-      else asm volatile("cp.async.wait_group 0;" ::: "memory");
-      uint4 wq[GQ_NT];
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");  // possibly empty: one group per chunk slot
+  };
+  auto load_x = [&](const Cursor& c, int b, uint4 (&v)[NT][WPB]) {
 #pragma unroll
-      for (int t = 0; t < GQ_NT; ++t) wq[t] = wbuf[(buf * GQ_NT + t) * 32 + lane];
+    for (int t = 0; t < NT; ++t)
+#pragma unroll
+      for (int q = 0; q < WPB; ++q)
+        v[t][q] = c.item < item_end && t * 8 + g < p.M
+                      ? *reinterpret_cast<const uint4*>(x + (t * 8 + g) * p.ldx + c.ch * GQ_KCHUNK + b * SB + (j * WPB + q) * 8)
+                      : make_uint4(0, 0, 0, 0);
+  };
+
+  Cursor ahead{item, 0, 0, 0};
+  segment(ahead);
+  Cursor cur = ahead;
+  request(ahead, 0);
+  advance(ahead);
+  request(ahead, 1);
+  advance(ahead);
+  xl_grid_dependency_wait();  // the first weights are on their way; everything else may come from the previous kernel
+  xl_grid_launch_dependents();
+  uint4 xn[NT][WPB];
+  load_x(cur, 0, xn);
+  int buf = 0;
+  while (item < item_end) {
+    const int tile = item / chunks, n_base = tile * COLS;
+    const int c0 = item - tile * chunks;
+    const int c1 = min(chunks, c0 + (item_end - item));
+    float acc[CT][NT][4];
+#pragma unroll
+    for (int i = 0; i < CT; ++i)
+#pragma unroll
+      for (int t = 0; t < NT; ++t)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) acc[i][t][e] = 0.f;
+    for (int ch = c0 + warp; ch < c1; ch += WARPS) {
+      Cursor next = cur;
+      advance(next);
+      asm volatile("cp.async.wait_group 1;" ::: "memory");
+      __syncwarp();  // lanes read pieces that other lanes of the warp copied
+      const uint32_t* codes = reinterpret_cast<const uint32_t*>(ring + buf * C::STAGE_UNITS);
+      const uint32_t* sz = codes + C::CODE_UNITS * 4;
+#pragma unroll
+      for (int b = 0; b < BLOCKS; ++b) {
+        uint32_t xb[NT][WPB][4];  // the B operand: x of codes (0, 4), (1, 5), (2, 6), (3, 7)
+#pragma unroll
+        for (int t = 0; t < NT; ++t)
+#pragma unroll
+          for (int q = 0; q < WPB; ++q) {
+            const uint4 v = xn[t][q];
+            xb[t][q][0] = __byte_perm(v.x, v.z, 0x5410);
+            xb[t][q][1] = __byte_perm(v.x, v.z, 0x7632);
+            xb[t][q][2] = __byte_perm(v.y, v.w, 0x5410);
+            xb[t][q][3] = __byte_perm(v.y, v.w, 0x7632);
+          }
+        load_x(b + 1 < BLOCKS ? cur : next, b + 1 < BLOCKS ? b + 1 : 0, xn);  // one block ahead
+        float xs[NT][4];  // [0], [1]: sums of x of tokens 2j, 2j + 1
+#pragma unroll
+        for (int t = 0; t < NT; ++t) {
+          const uint32_t ones[4] = {F::ONES, F::ONES, F::ONES, F::ONES};
+#pragma unroll
+          for (int e = 0; e < 4; ++e) xs[t][e] = 0.f;
+#pragma unroll
+          for (int q = 0; q < WPB; ++q) {
+            mma_m16n8k16<T>(xs[t], ones, xb[t][q][0], xb[t][q][1]);
+            mma_m16n8k16<T>(xs[t], ones, xb[t][q][2], xb[t][q][3]);
+          }
+        }
+#pragma unroll
+        for (int i = 0; i < CT; ++i) {
+          uint32_t lo[WPB], hi[WPB];  // rows g and g + 8
+          if constexpr (WPB == 2) {
+            const int piece = b * 2 + (j >> 1), sw = (piece & 1) * 4;
+            const uint2 a = *reinterpret_cast<const uint2*>(codes + (i * 64 + piece * 16 + (g ^ sw)) * 4 + (j & 1) * 2);
+            const uint2 c = *reinterpret_cast<const uint2*>(codes + (i * 64 + piece * 16 + ((g + 8) ^ sw)) * 4 + (j & 1) * 2);
+            lo[0] = a.x; lo[1] = a.y; hi[0] = c.x; hi[1] = c.y;
+          } else {
+            const int sw = (b & 1) * 4;
+            lo[0] = codes[(i * 64 + b * 16 + (g ^ sw)) * 4 + j];
+            hi[0] = codes[(i * 64 + b * 16 + ((g + 8) ^ sw)) * 4 + j];
+          }
+          const uint32_t sz_lo = sz[b * COLS + i * 16 + g], sz_hi = sz[b * COLS + i * 16 + g + 8];
+          float part[NT][4];
+#pragma unroll
+          for (int t = 0; t < NT; ++t)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) part[t][e] = 0.f;
+#pragma unroll
+          for (int q = 0; q < WPB; ++q) {
+            uint32_t cl[4], chh[4];
+            gq_codes8<T>(lo[q], cl);
+            gq_codes8<T>(hi[q], chh);
+            const uint32_t a0[4] = {cl[0], chh[0], cl[1], chh[1]}, a1[4] = {cl[2], chh[2], cl[3], chh[3]};
+#pragma unroll
+            for (int t = 0; t < NT; ++t) {
+              mma_m16n8k16<T>(part[t], a0, xb[t][q][0], xb[t][q][1]);
+              mma_m16n8k16<T>(part[t], a1, xb[t][q][2], xb[t][q][3]);
+            }
+          }
+          const float2 wl = xl_pair_to_float2<S>(sz_lo), wh = xl_pair_to_float2<S>(sz_hi);
+          const float zl = fmaf(-F::BASE, wl.x, wl.y), zh = fmaf(-F::BASE, wh.x, wh.y);
+#pragma unroll
+          for (int t = 0; t < NT; ++t) {
+            acc[i][t][0] += wl.x * part[t][0] + zl * xs[t][0];
+            acc[i][t][1] += wl.x * part[t][1] + zl * xs[t][1];
+            acc[i][t][2] += wh.x * part[t][2] + zh * xs[t][0];
+            acc[i][t][3] += wh.x * part[t][3] + zh * xs[t][1];
+          }
+        }
+      }
+      __syncwarp();  // all lanes have read this stage
+      request(ahead, buf);
+      advance(ahead);
+      cur = next;
       buf ^= 1;
-      T2 s2[GQ_NT], z2[GQ_NT];
-#pragma unroll
-      for (int t = 0; t < GQ_NT; ++t) {
-        const uint16_t s16 = (uint16_t)(sz[t] & 0xFFFFu), z16 = (uint16_t)(sz[t] >> 16);
-        s2[t] = F::pair(xl_to_float(*reinterpret_cast<const S*>(&s16)));
-        z2[t] = F::pair(xl_to_float(*reinterpret_cast<const S*>(&z16)));
-      }
-#pragma unroll
-      for (int half = 0; half < 2; ++half) {
-        uint4 xa[2], xb[2];
-        const uint4 zero4 = make_uint4(0, 0, 0, 0);
-#pragma unroll
-        for (int v = 0; v < 2; ++v) {
-          const long long off = k_lane + (2 * half + v) * 8;
-          xa[v] = row_lo ? *reinterpret_cast<const uint4*>(x + (long long)quad * ldx + off) : zero4;
-          xb[v] = row_hi ? *reinterpret_cast<const uint4*>(x + (long long)(quad + 8) * ldx + off) : zero4;
-        }
-        const uint32_t* xa32 = reinterpret_cast<const uint32_t*>(xa);
-        const uint32_t* xb32 = reinterpret_cast<const uint32_t*>(xb);
-        // k-step outermost: consecutive MMAs go to different accumulators, so none waits for its predecessor
-#pragma unroll
-        for (int mm = 0; mm < 2; ++mm) {
-          const uint32_t a0[4] = {xa32[4 * mm], xb32[4 * mm], xa32[4 * mm + 1], xb32[4 * mm + 1]};
-          const uint32_t a1[4] = {xa32[4 * mm + 2], xb32[4 * mm + 2], xa32[4 * mm + 3], xb32[4 * mm + 3]};
-#pragma unroll
-          for (int t = 0; t < GQ_NT; ++t) {
-            // 32-bit word m of a lane's 16 bytes holds packed words 2m and 2m+1, i.e. k_lane + 8m .. 8m+7
-            const uint32_t w = reinterpret_cast<const uint32_t*>(&wq[t])[2 * half + mm];
-            uint32_t b[4];
-            gq_dequant8<T>(w, s2[t], z2[t], b);
-            const uint32_t b0[2] = {b[0], b[1]}, b1[2] = {b[2], b[3]};
-            mma_m16n8k16(c[t], a0, b0, BF);
-            mma_m16n8k16(c[t], a1, b1, BF);
-          }
-        }
-      }
     }
-    // reduce the K slices of the warps through shared memory
-    __syncthreads();  // the previous segment's readers are done with `red`
+    // add the K slices of the warps up in shared memory
+    __syncthreads();  // readers of the previous segment are done with `red`
 #pragma unroll
-    for (int t = 0; t < GQ_NT; ++t) {
-      red[warp][quad][t * 8 + 2 * j] = c[t][0];
-      red[warp][quad][t * 8 + 2 * j + 1] = c[t][1];
-      red[warp][quad + 8][t * 8 + 2 * j] = c[t][2];
-      red[warp][quad + 8][t * 8 + 2 * j + 1] = c[t][3];
-    }
+    for (int i = 0; i < CT; ++i)
+#pragma unroll
+      for (int t = 0; t < NT; ++t)
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+          red[(warp * NT * 8 + t * 8 + 2 * j + (e & 1)) * C::RED_LD + i * 16 + g + (e >> 1) * 8] = acc[i][t][e];
     __syncthreads();
-    const bool whole = (c1 - c0) == chunks;
-    float* wtile = ws + (long long)tile * TILE;
+    const bool whole = c1 - c0 == chunks;
     bool finishing = whole;
     if (!whole) {
-      for (int idx = threadIdx.x; idx < TILE; idx += blockDim.x) {
-        const int r = idx / (8 * GQ_NT), col = idx % (8 * GQ_NT);
-        if (r < M && n_base + col < N) {
-          float acc = 0.f;
+      float* slot = p.slots + ((long long)blockIdx.x * 2 + (tile == first_tile ? 0 : 1)) * (16 * COLS);
+      for (int i = threadIdx.x; i < p.M * (COLS / 4); i += blockDim.x) {
+        const int r = i / (COLS / 4), col = i % (COLS / 4) * 4;
+        float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-          for (int w = 0; w < GQ_WARPS; ++w) acc += red[w][r][col];
-          atomicAdd(wtile + idx, acc);
+        for (int w = 0; w < WARPS; ++w) {
+          const float4 o = *reinterpret_cast<const float4*>(red + (w * NT * 8 + r) * C::RED_LD + col);
+          s.x += o.x; s.y += o.y; s.z += o.z; s.w += o.w;
         }
+        __stcg(reinterpret_cast<float4*>(slot + r * COLS + col), s);
       }
       __threadfence();
       __syncthreads();
       if (threadIdx.x == 0)
-        finish = atomicAdd(counters + tile, (unsigned int)(c1 - c0)) + (unsigned int)(c1 - c0) == (unsigned int)chunks;
+        finish = atomicAdd(p.counters + tile, (unsigned int)(c1 - c0)) + (unsigned int)(c1 - c0) == (unsigned int)chunks;
       __syncthreads();
       finishing = finish != 0;
       if (finishing) __threadfence();
     }
     if (finishing) {
-      for (int idx = threadIdx.x; idx < TILE; idx += blockDim.x) {
-        const int r = idx / (8 * GQ_NT), col = idx % (8 * GQ_NT);
-        const int n = n_base + col;
-        if (r < M && n < N) {
-          float acc = 0.f;
-          if (!whole) {
-            acc = __ldcg(wtile + idx);
-            wtile[idx] = 0.f;
-          } else {
+      // CTAs that share the tile, in order: all but the first begin inside it (slot 0), the first may hold an earlier tile too
+      int cta0 = blockIdx.x, cta1 = blockIdx.x, slot0 = 0;
+      if (!whole) {
+        cta0 = ranges.owner(tile * chunks);
+        cta1 = ranges.owner(tile * chunks + chunks - 1);
+        slot0 = ranges.begin(cta0) < tile * chunks ? 1 : 0;
+      }
+      for (int i = threadIdx.x; i < p.M * (COLS / 4); i += blockDim.x) {
+        const int r = i / (COLS / 4), col = i % (COLS / 4) * 4, n = n_base + col;
+        if (n >= p.N) continue;
+        float v[4] = {0.f, 0.f, 0.f, 0.f};
+        if (whole) {
 #pragma unroll
-            for (int w = 0; w < GQ_WARPS; ++w) acc += red[w][r][col];
+          for (int w = 0; w < WARPS; ++w) {
+            const float4 o = *reinterpret_cast<const float4*>(red + (w * NT * 8 + r) * C::RED_LD + col);
+            v[0] += o.x; v[1] += o.y; v[2] += o.z; v[3] += o.w;
           }
-          if (bias) acc += xl_to_float(bias[n]);
-          if (n >= act_from_col) acc = 0.5f * acc * (1.f + erff(acc * 0.70710678118654752f));
-          y[(long long)r * ldy + n] = xl_from_float<T>(acc);
+        } else {
+          const float* base = p.slots + r * COLS + col;
+#pragma unroll 4
+          for (int k = cta0; k <= cta1; ++k) {
+            const float4 o = __ldcg(reinterpret_cast<const float4*>(base + ((long long)k * 2 + (k == cta0 ? slot0 : 0)) * (16 * COLS)));
+            v[0] += o.x; v[1] += o.y; v[2] += o.z; v[3] += o.w;
+          }
+        }
+        T* yr = (T*)p.y + (long long)r * p.ldy + n;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          if (n + e < p.N) {
+            float o = v[e] + (p.bias ? xl_to_float(((const T*)p.bias)[n + e]) : 0.f);
+            if (n + e >= p.act_from_col) o = 0.5f * o * (1.f + erff(o * 0.70710678118654752f));
+            yr[e] = xl_from_float<T>(o);
+          }
         }
       }
-      if (!whole && threadIdx.x == 0) counters[tile] = 0;
+      if (!whole && threadIdx.x == 0) p.counters[tile] = 0;
     }
     item += c1 - c0;
   }
 }
 
-// Requirements: M <= 16, K % 128 == 0, group_size % 32 == 0, 16-byte aligned x rows and weight rows. `ws` / `counters`:
-// zero-initialised scratch of ceil(N/64)*1024 floats / ceil(N/64) words (the kernel leaves them zeroed). `ctas`: size of
-// the grid (0: two per SM of a 148-SM part). sz_transposed: `scale` holds (scale, zero) pairs laid out (K/gs, N, 2)
-// and `zero` is unused: the layout in which the eight columns of an MMA tile are one contiguous 32-byte read. act_from_col: first column that gets GELU (>= N: none). Returns -1 for
-// unsupported arguments.
-template <typename T>
-static void gq_small_launch(const void* x, const void* packed, const void* scale, const void* zero, const void* bias, void* y,
-                            int M, int N, int K, int group_size, long long ldx, long long ldy, int act_from_col,
-                            float* ws, unsigned int* counters, int scale_dtype, int sz_transposed, int grid,
-                            cudaStream_t s) {
-  constexpr int WBUF_BYTES = GQ_WARPS * 2 * GQ_NT * 32 * 16;  // per-warp double buffer of weight chunks
+template <typename T, typename S, int NT, int WPB> static int gq_small_launch(const GqParams& p, int ctas, cudaStream_t s) {
+  using C = GqCfg<NT, WPB>;
   static bool configured = false;
   if (!configured) {
-    cudaFuncSetAttribute(gq_gemm_small_m_kernel<T, __half>, cudaFuncAttributeMaxDynamicSharedMemorySize, WBUF_BYTES);
-    cudaFuncSetAttribute(gq_gemm_small_m_kernel<T, __nv_bfloat16>, cudaFuncAttributeMaxDynamicSharedMemorySize, WBUF_BYTES);
+    const cudaError_t e =
+        cudaFuncSetAttribute(gq_gemm_small_m_kernel<T, S, NT, WPB>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM);
+    if (e != cudaSuccess) return (int)e;
     configured = true;
   }
-  if (scale_dtype == XL_F16)
-    gq_gemm_small_m_kernel<T, __half><<<grid, GQ_WARPS * 32, WBUF_BYTES, s>>>(
-        (const T*)x, (const uint16_t*)packed, (const __half*)scale, (const __half*)zero, (const T*)bias, (T*)y, M, N, K,
-        group_size, ldx, ldy, act_from_col, ws, counters, sz_transposed);
-  else
-    gq_gemm_small_m_kernel<T, __nv_bfloat16><<<grid, GQ_WARPS * 32, WBUF_BYTES, s>>>(
-        (const T*)x, (const uint16_t*)packed, (const __nv_bfloat16*)scale, (const __nv_bfloat16*)zero, (const T*)bias,
-        (T*)y, M, N, K, group_size, ldx, ldy, act_from_col, ws, counters, sz_transposed);
+  const long long total = (long long)((p.N + C::COLS - 1) / C::COLS) * (p.K / GQ_KCHUNK);
+  if (total > (1 << 30)) return -1;
+  const int grid = (int)(total < ctas ? total : ctas);
+  const cudaError_t e = xl_launch_overlapped(gq_gemm_small_m_kernel<T, S, NT, WPB>, dim3((unsigned)grid), dim3(C::WARPS * 32),
+                                             (size_t)C::SMEM, s, p);
+  return e != cudaSuccess ? (int)e : (int)cudaGetLastError();
 }
-// `dtype`: type of x, bias and y (fp16 or bf16); `scale_dtype`: type of the per-group scale and zero point (fp16 / bf16).
+template <typename T, typename S> static int gq_small_pick(const GqParams& p, int ctas, cudaStream_t s) {
+  // a scale per 64 k values and more: blocks of 64, half as many scales to apply; up to 8 tokens: half the MMAs
+  if (p.group_size % 64 == 0)
+    return p.M <= 8 ? gq_small_launch<T, S, 1, 2>(p, ctas, s) : gq_small_launch<T, S, 2, 2>(p, ctas, s);
+  return p.M <= 8 ? gq_small_launch<T, S, 1, 1>(p, ctas, s) : gq_small_launch<T, S, 2, 1>(p, ctas, s);
+}
+
+// Floats of `slots` for a grid of `ctas`; `counters` needs ceil(N / 64) zero-initialised words (left zeroed).
+XL_API int xl_gq_gemm_small_m_slots(int ctas) { return ctas * 2 * 16 * 128; }
+
+// Requirements: M <= 16, K % 128 == 0, group_size % 32 == 0, 16-byte aligned x rows and weight rows. `ctas`: size of the grid (one
+// per SM). sz_pairs: `scale` holds (scale, zero) pairs laid out (K/gs, N, 2) and `zero` is unused. act_from_col: first column that
+// gets GELU (>= N: none). `dtype`: type of x, bias and y (fp16 or bf16); `scale_dtype`: type of the per-group scale and zero
+// point (fp16 / bf16). Returns -1 for unsupported arguments.
 XL_API int xl_gq_gemm_small_m(const void* x, const void* packed, const void* scale, const void* zero, const void* bias,
                               void* y, int M, int N, int K, int group_size, long long ldx, long long ldy, int act_from_col,
-                              int ctas, float* ws, unsigned int* counters, int dtype, int scale_dtype, int sz_transposed,
+                              int ctas, float* slots, unsigned int* counters, int dtype, int scale_dtype, int sz_pairs,
                               cudaStream_t s) {
-  if (M < 1 || M > 16 || K % GQ_KCHUNK || group_size % 32 || K % group_size || dtype == XL_F32 || scale_dtype == XL_F32)
+  if (M < 1 || M > 16 || N < 1 || K < GQ_KCHUNK || K % GQ_KCHUNK || group_size < 32 || group_size % 32 || K % group_size ||
+      dtype == XL_F32 || scale_dtype == XL_F32)
     return -1;
-  if ((ldx % 8) || ws == nullptr || counters == nullptr) return -1;
-  const long long total = (long long)((N + 8 * GQ_NT - 1) / (8 * GQ_NT)) * (K / GQ_KCHUNK);
-  long long grid = ctas > 0 ? ctas : 2 * 148;
-  if (grid > total) grid = total;
+  if ((ldx % 8) || ctas < 1 || slots == nullptr || counters == nullptr || (((uintptr_t)x | (uintptr_t)packed | (uintptr_t)scale) & 15)) return -1;
+  const GqParams p{x, ldx, (const uint16_t*)packed, scale, zero, sz_pairs, bias, y, ldy, M, N, K, group_size, act_from_col, slots, counters};
   if (dtype == XL_BF16)
-    gq_small_launch<__nv_bfloat16>(x, packed, scale, zero, bias, y, M, N, K, group_size, ldx, ldy, act_from_col, ws,
-                                   counters, scale_dtype, sz_transposed, (int)grid, s);
-  else
-    gq_small_launch<__half>(x, packed, scale, zero, bias, y, M, N, K, group_size, ldx, ldy, act_from_col, ws, counters,
-                            scale_dtype, sz_transposed, (int)grid, s);
-  return (int)cudaGetLastError();
+    return scale_dtype == XL_F16 ? gq_small_pick<__nv_bfloat16, __half>(p, ctas, s) : gq_small_pick<__nv_bfloat16, __nv_bfloat16>(p, ctas, s);
+  return scale_dtype == XL_F16 ? gq_small_pick<__half, __half>(p, ctas, s) : gq_small_pick<__half, __nv_bfloat16>(p, ctas, s);
 }
 
 // ------------------------------------------------------------------------------------------------------------------

@@ -78,12 +78,6 @@ struct SmParams {
   unsigned int* counters;  // one per tile, zero between launches
 };
 
-__device__ __forceinline__ void cp_async16(uint4* dst, const void* src, bool on) {
-  const int bytes = on ? 16 : 0;  // 0: the destination is zero-filled
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src),
-               "r"(bytes)
-               : "memory");
-}
 __device__ __forceinline__ void mma_bf16(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
                                          uint32_t b1) {
   asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
@@ -168,16 +162,6 @@ __device__ __forceinline__ float sm_epilogue(const SmParams& p, int r, int c, co
   return sq;
 }
 
-// Contiguous ranges of items: the first `rem` CTAs take per + 1 items, the others per.
-struct SmRanges {
-  int per, rem;
-  __device__ __forceinline__ int begin(int cta) const { return cta * per + min(cta, rem); }
-  __device__ __forceinline__ int owner(int item) const {
-    const int head = rem * (per + 1);
-    return item < head ? item / (per + 1) : rem + (item - head) / per;
-  }
-};
-
 template <int MODE>
 __global__ void __launch_bounds__(SM_WARPS * 32, SM_CTAS_PER_SM) linear_small_m_kernel(const SmParams p) {
   using L = SmTile<MODE>;
@@ -194,7 +178,7 @@ __global__ void __launch_bounds__(SM_WARPS * 32, SM_CTAS_PER_SM) linear_small_m_
   const int channels = MODE == SM_SPLIT_GLU ? (p.N - p.cols) / PARTS : p.N / PARTS;
   const int n_tiles = plain + (channels + CH - 1) / CH;
   const int total = n_tiles * chunks;
-  const SmRanges ranges{total / (int)gridDim.x, total % (int)gridDim.x};
+  const XlRanges ranges{total / (int)gridDim.x, total % (int)gridDim.x};
   int item = ranges.begin(blockIdx.x);
   const int item_end = ranges.begin(blockIdx.x + 1);
   const int first_tile = item / chunks;
@@ -241,7 +225,7 @@ __global__ void __launch_bounds__(SM_WARPS * 32, SM_CTAS_PER_SM) linear_small_m_
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
           const bool on = row_on && k0 + e * 32 < p.K;
-          cp_async16(dst + (t * 2 + e) * 32, src + (on ? k0 + e * 32 : 0), on);
+          xl_cp_async16(dst + (t * 2 + e) * 32, src + (on ? k0 + e * 32 : 0), on);
         }
       }
     }

@@ -94,6 +94,7 @@ _gemm_ar_pull = _sig("xl_gemm_tcgen05_ar_pull", _c_p, _c_p, _c_p, _c_p, _c_p, _c
                      _c_int, _c_int, _c_ll, _c_ll, _c_ll, _c_ll, _c_ll, _c_int, _c_int, _c_f, _c_p, _c_int, _c_p, _c_int,
                      _c_int, _c_p, _c_p, _c_int, _c_int, _c_p, _c_p)
 _symm_all_gather_mc = _sig("xl_symm_all_gather_mc", _c_p, _c_p, _c_ll, _c_p, _c_p, _c_int, _c_int, _c_int, _c_p, _c_p)
+_gq_small_slots = _sig("xl_gq_gemm_small_m_slots", _c_int)
 _gq_small = _sig("xl_gq_gemm_small_m", _c_p, _c_p, _c_p, _c_p, _c_p, _c_p, _c_int, _c_int, _c_int, _c_int, _c_ll, _c_ll,
                  _c_int, _c_int, _c_p, _c_p, _c_int, _c_int, _c_int, _c_p)
 _rot_append = _sig("xl_rotary_append", _c_p, _c_ll, _c_p, _c_p, _c_p, _c_p, _c_p, _c_int, _c_int, _c_int, _c_int, _c_int,
@@ -1215,13 +1216,14 @@ def store_row_cuda(buf, pos, vals, base):
 _GQ_SCRATCH: Dict[int, Tuple[torch.Tensor, torch.Tensor]] = {}
 
 
-def _gq_scratch(device, n_tiles: int):
-    """Zero-initialised split-K scratch of the small-M GEMM (the kernel hands it back zeroed after every launch)."""
+def _gq_scratch(device, n_tiles: int, ctas: int):
+    """Split-K scratch of the small-M int4 GEMM: slots for partial sums, and counters that every launch leaves at zero."""
     idx = device.index or 0
     cur = _GQ_SCRATCH.get(idx)
-    if cur is None or cur[1].numel() < n_tiles:
-        n = max(n_tiles, 2048)
-        cur = (torch.zeros(n * 512, dtype=torch.float32, device=device), torch.zeros(n, dtype=torch.int32, device=device))
+    slots = _gq_small_slots(ctas)
+    if cur is None or cur[1].numel() < n_tiles or cur[0].numel() < slots:
+        cur = (torch.empty(max(slots, cur[0].numel() if cur else 0), dtype=torch.float32, device=device),
+               torch.zeros(max(n_tiles, 2048, cur[1].numel() if cur else 0), dtype=torch.int32, device=device))
         _GQ_SCRATCH[idx] = cur
     return cur
 
@@ -1248,11 +1250,11 @@ def gq_gemm_small_m(x, packed, scale, zero, bias, out=None, act_from_col=None, c
     y = out if out is not None else torch.empty((M, N), dtype=x.dtype, device=x.device)
     if y.shape != (M, N) or y.dtype != x.dtype or y.stride(1) != 1:
         return NotImplemented
-    n_tiles = (N + 31) // 32
-    ws, counters = _gq_scratch(x.device, n_tiles)
+    ctas = int(ctas or _sms(x.device))
+    ws, counters = _gq_scratch(x.device, (N + 63) // 64, ctas)
     rc = _gq_small(x.data_ptr(), packed.data_ptr(), scale.data_ptr(), zero.data_ptr(),
                    bias.data_ptr() if bias is not None else None, y.data_ptr(), M, N, K, gs, x.stride(0), y.stride(0),
-                   N if act_from_col is None else int(act_from_col), int(ctas or 2 * _sms(x.device)),
+                   N if act_from_col is None else int(act_from_col), ctas,
                    ws.data_ptr(), counters.data_ptr(), _CODE[x.dtype], _CODE[scale.dtype], int(transposed), _stream())
     if rc == -1:
         return NotImplemented

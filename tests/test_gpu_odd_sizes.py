@@ -141,3 +141,26 @@ def test_embedding_gradient_into_the_running_mean(nat, rows, cols, n, dtype, t):
     out = nat.gather_grad_accumulate_mean_cuda(dev, grad.cuda(), idx.cuda(), torch.tensor(t, device="cuda"), 0, True)
     assert out is dev
     assert (dev.cpu().double() - want).abs().max() <= 1e-6 * max(1, n)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("pairs", [False, True])
+@pytest.mark.parametrize("M,N,K,gs", [(1, 1, 128, 32), (8, 63, 256, 64), (9, 130, 384, 96), (16, 257, 1024, 128), (3, 640, 2048, 64),
+                                      (16, 2052, 2304, 64), (1, 14336, 2048, 64)])
+def test_int4_product_at_the_edges_of_its_tiles(nat, dtype, pairs, M, N, K, gs):
+    """Ragged channels, each block size, both token tiles, both layouts of the scales, tiles that CTAs share, against 64 bits.
+    Sums of x times (base + code) are at most (128 + 15) / 4.6 of the result's size each, cut to 24 bits every eight terms."""
+    from popxl_addons_b200.layers.linear_gq import interleave_scale_zero
+
+    g = torch.Generator(device="cuda").manual_seed(M * N + K)
+    x = torch.randn(M, K, generator=g, device="cuda").to(dtype)
+    codes = torch.randint(0, 16, (N, K // gs, gs // 4, 4), generator=g, device="cuda")
+    word = (codes[..., 0] << 12) | (codes[..., 1] << 8) | (codes[..., 2] << 4) | codes[..., 3]
+    packed = torch.where(word > 32767, word - 65536, word).to(torch.int16).view(torch.uint16)
+    scale = (0.02 + 0.02 * torch.rand(N, K // gs, 1, generator=g, device="cuda")).half()
+    zero = (-0.3 + 0.1 * torch.rand(N, K // gs, 1, generator=g, device="cuda")).half()
+    w = codes.reshape(N, K // gs, gs).double() * scale.double() + zero.double()
+    want = x.double() @ w.reshape(N, K).t()
+    y = nat.gq_gemm_small_m(x, packed, *((interleave_scale_zero(scale, zero), None) if pairs else (scale, zero)), None)
+    assert y is not NotImplemented
+    _near(y, want, dtype, terms=31 * K)
