@@ -166,8 +166,9 @@ __device__ __forceinline__ void tile_coords(int tile, int tiles_m, int tiles_n, 
 // others' loops (60 bytes a thread), which cost the weight gradients 4 % of a training step.
 //   EPI_16   16-bit C, overwritten, rows on 16-byte boundaries
 //   EPI_F32  fp32 C (overwritten or accumulated into), rows on 16-byte boundaries
-//   EPI_ANY  the rest: fp32 rows of any alignment, 16-bit C that is accumulated into or not aligned
-enum EpiKind : int { EPI_16 = 0, EPI_F32 = 1, EPI_ANY = 2 };
+//   EPI_16A  16-bit C that is accumulated into (the second of two summed products), rows on 16-byte boundaries
+//   EPI_ANY  the rest: fp32 rows of any alignment, 16-bit C that is not aligned
+enum EpiKind : int { EPI_16 = 0, EPI_F32 = 1, EPI_ANY = 2, EPI_16A = 3 };
 
 template <int PN, int EPI>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
@@ -341,6 +342,18 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
           old[i] = rr < p.M ? __ldcs((const float4*)(cbase + (long long)rr * p.ldc + c)) : make_float4(0.f, 0.f, 0.f, 0.f);
         }
       };
+      // 16-bit C that is accumulated into takes the same way: 4 lanes per row, 8 columns each, 8 rows per instruction
+      uint16_t* cbase16 = (uint16_t*)p.C + (long long)b * p.batch_stride_c + (long long)nb * PAIR_N + (lane & 3) * 8;
+      uint4 old16[4];
+      auto request_old16 = [&](int c) {
+        if (nb * PAIR_N + c + 32 > p.N) return;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const int rr = row_base + i * 8 + (lane >> 2);
+          old16[i] = rr < p.M ? *(const uint4*)(cbase16 + (long long)rr * p.ldc + c) : make_uint4(0, 0, 0, 0);
+        }
+      };
+      if (EPI == EPI_16A) request_old16(c_begin);
       if (EPI == EPI_F32 && p.epi.accumulate) {
         // The old contents are on their way while the tensor core still works on the tile: the first chunk into registers, the
         // others into L2. Requested chunk by chunk after the accumulator was complete, their latency (an HBM round trip for each
@@ -383,15 +396,14 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
             stage16[lane * 4 + ((j + (lane >> 1)) & 3)] = pack8_16bit(v, p.epi.c_dtype == XL_F16);
           }
           __syncwarp();
-          uint16_t* cbase16 = (uint16_t*)p.C + (long long)b * p.batch_stride_c + col0 + (lane & 3) * 8;
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
             const int lr = i * 8 + (lane >> 2), rr = row_base + lr;
             const uint4 o = stage16[lr * 4 + (((lane & 3) + (lr >> 1)) & 3)];
-            if (rr < p.M) *(uint4*)(cbase16 + (long long)rr * p.ldc) = o;
+            if (rr < p.M) *(uint4*)(cbase16 + (long long)rr * p.ldc + c) = o;
           }
           __syncwarp();
-        } else if (EPI == EPI_F32 && col0 + 32 <= p.N) {
+        } else if ((EPI == EPI_F32 || EPI == EPI_16A) && col0 + 32 <= p.N) {
           // this thread's row -> shared memory, 16-byte pieces swizzled by the row so that both phases are conflict-free
           const float bv = p.epi.bias ? epilogue_bias(p.epi, col0 + lane) : 0.f;
 #pragma unroll
@@ -406,6 +418,31 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
             stage[lane * 8 + (j ^ (lane & 7))] = make_float4(v[0], v[1], v[2], v[3]);
           }
           __syncwarp();
+          if (EPI == EPI_16A) {  // the sum is fp32, rounded once
+            uint4 out16[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              const int lr = i * 8 + (lane >> 2);
+              const float4 lo = stage[lr * 8 + (((lane & 3) * 2) ^ (lr & 7))], hi = stage[lr * 8 + (((lane & 3) * 2 + 1) ^ (lr & 7))];
+              float v[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+              const uint32_t w[4] = {old16[i].x, old16[i].y, old16[i].z, old16[i].w};
+#pragma unroll
+              for (int e = 0; e < 8; ++e) {
+                const uint16_t u = (uint16_t)(e & 1 ? w[e >> 1] >> 16 : w[e >> 1] & 0xffffu);
+                const float prev = p.epi.c_dtype == XL_F16 ? __half2float(__ushort_as_half(u)) : __bfloat162float(__ushort_as_bfloat16(u));
+                v[e] = p.epi.accumulate == 1 ? prev + v[e] : prev * mean_a + v[e] * mean_b;
+              }
+              out16[i] = pack8_16bit(v, p.epi.c_dtype == XL_F16);
+            }
+            if (c + 32 < c_end) request_old16(c + 32);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              const int rr = row_base + i * 8 + (lane >> 2);
+              if (rr < p.M) *(uint4*)(cbase16 + (long long)rr * p.ldc + c) = out16[i];
+            }
+            __syncwarp();
+            continue;
+          }
           float4 out[8];
 #pragma unroll
           for (int i = 0; i < 8; ++i) {
@@ -599,13 +636,15 @@ XL_API int xl_gemm2cta_tcgen05(const void* a, const void* b, void* c, int M, int
   p.step = step; p.alpha = alpha; p.is_fp16 = ab_is_fp16; p.err = err;
   const int align = c_dtype == XL_F32 ? 4 : 8;  // elements of 16 bytes
   const bool aligned = (ldc % align) == 0 && (batch == 1 || (stride_c % align) == 0) && (((uintptr_t)c) & 15) == 0;
-  const int kind = !aligned ? EPI_ANY : c_dtype == XL_F32 ? EPI_F32 : accumulate ? EPI_ANY : EPI_16;
+  const int kind = !aligned ? EPI_ANY : c_dtype == XL_F32 ? EPI_F32 : accumulate ? EPI_16A : EPI_16;
   if (pair_n == 128) {
     if (kind == EPI_16) return launch_pairs<128, EPI_16>(ma, mb, p, max_pairs, s);
     if (kind == EPI_F32) return launch_pairs<128, EPI_F32>(ma, mb, p, max_pairs, s);
+    if (kind == EPI_16A) return launch_pairs<128, EPI_16A>(ma, mb, p, max_pairs, s);
     return launch_pairs<128, EPI_ANY>(ma, mb, p, max_pairs, s);
   }
   if (kind == EPI_16) return launch_pairs<256, EPI_16>(ma, mb, p, max_pairs, s);
   if (kind == EPI_F32) return launch_pairs<256, EPI_F32>(ma, mb, p, max_pairs, s);
+  if (kind == EPI_16A) return launch_pairs<256, EPI_16A>(ma, mb, p, max_pairs, s);
   return launch_pairs<256, EPI_ANY>(ma, mb, p, max_pairs, s);
 }
