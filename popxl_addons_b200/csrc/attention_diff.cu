@@ -109,26 +109,32 @@ __global__ void __launch_bounds__(256)
 }
 
 // ---- general kernel --------------------------------------------------------------------------------------------------
-constexpr int DG_WARPS = 4;
 constexpr int DG_MAX_DIM = 512;   // query / key features per map; value features: 32 per DG_VPL, at most 512
 
-template <typename T, int DG_VPL>
-__global__ void __launch_bounds__(DG_WARPS * 32)
+// SPLIT 1: a warp per query row, four of them per CTA. SPLIT 8: a CTA per query row whose warps take its blocks of 32 keys in turn
+// and merge their parts of the softmax in shared memory. One token of each of 4 sequences with 8 heads is 32 rows: a warp each
+// walked 7 blocks of keys one after another on 32 SMs.
+template <typename T, int DG_VPL, int SPLIT>
+__global__ void __launch_bounds__(SPLIT == 1 ? 128 : SPLIT * 32)
     diff_attn_general_kernel(const T* __restrict__ q, long long ldq, const T* __restrict__ kc, const T* __restrict__ vc,
                              T* __restrict__ out, long long ldo, const int* __restrict__ pos, const int* __restrict__ count,
                              const float* __restrict__ lam, int T_len, int H, int G, int dim, int vdim, int Smax, int chunk,
                              float scale, float eps, float out_scale) {
-  __shared__ float sq[DG_WARPS][2][DG_MAX_DIM];
+  constexpr int ROWS = SPLIT == 1 ? 4 : 1;
+  __shared__ __align__(16) float sq[ROWS][2][DG_MAX_DIM];
+  __shared__ float so[SPLIT == 1 ? 1 : SPLIT][2][SPLIT == 1 ? 1 : 32 * DG_VPL], sm[SPLIT][2], sl[SPLIT][2];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int slot = SPLIT == 1 ? warp : 0, part = SPLIT == 1 ? 0 : warp;
   const int h = blockIdx.y, b = blockIdx.z, g = h / (H / G);
-  const int t = blockIdx.x * DG_WARPS + warp;
-  if (t >= min(count[b], T_len)) return;
+  const int t = blockIdx.x * ROWS + slot;
+  if (t >= min(count[b], T_len)) return;  // whole warps, and with SPLIT > 1 whole CTAs
   const int p = pos[b] + t;
   if (p < 0 || p >= Smax) return;
   const long long row = (long long)b * T_len + t;
   for (int m = 0; m < 2; ++m)
-    for (int d = lane; d < dim; d += 32) sq[warp][m][d] = xl_to_float(q[row * ldq + ((long long)h * 2 + m) * dim + d]);
-  __syncwarp();
+    for (int d = part * 32 + lane; d < dim; d += 32 * SPLIT) sq[slot][m][d] = xl_to_float(q[row * ldq + ((long long)h * 2 + m) * dim + d]);
+  if (SPLIT == 1) __syncwarp();
+  else __syncthreads();
   const int first = chunk > 0 ? (p / chunk) * chunk : 0;
   float o[2][DG_VPL], mx[2], l[2];
 #pragma unroll
@@ -139,18 +145,13 @@ __global__ void __launch_bounds__(DG_WARPS * 32)
     for (int e = 0; e < DG_VPL; ++e) o[m][e] = 0.f;
   }
   const T* vb = vc + ((long long)b * G + g) * Smax * vdim;
-  for (int j0 = first; j0 <= p; j0 += 32) {
+  for (int j0 = first + part * 32; j0 <= p; j0 += 32 * SPLIT) {
     const int j = j0 + lane;
     float w[2];
 #pragma unroll
     for (int m = 0; m < 2; ++m) {
       float s = -INFINITY;
-      if (j <= p) {
-        const T* kr = kc + ((((long long)b * G + g) * 2 + m) * Smax + j) * dim;
-        s = 0.f;
-        for (int d = 0; d < dim; ++d) s = fmaf(sq[warp][m][d], xl_to_float(kr[d]), s);
-        s *= scale;
-      }
+      if (j <= p) s = xl_row_dot(sq[slot][m], kc + ((((long long)b * G + g) * 2 + m) * Smax + j) * dim, dim) * scale;
       const float m_new = fmaxf(mx[m], xl_warp_max(s));  // finite: key j0 is visible
       const float corr = expf(mx[m] - m_new);
       w[m] = expf(s - m_new);
@@ -160,6 +161,7 @@ __global__ void __launch_bounds__(DG_WARPS * 32)
       for (int e = 0; e < DG_VPL; ++e) o[m][e] *= corr;
     }
     const int n = min(32, p - j0 + 1);
+#pragma unroll 4
     for (int k = 0; k < n; ++k) {
       const float w0 = __shfl_sync(0xffffffffu, w[0], k), w1 = __shfl_sync(0xffffffffu, w[1], k);
       const T* vr = vb + (long long)(j0 + k) * vdim;
@@ -170,6 +172,30 @@ __global__ void __launch_bounds__(DG_WARPS * 32)
           o[0][e] = fmaf(w0, v, o[0][e]);
           o[1][e] = fmaf(w1, v, o[1][e]);
         }
+      }
+    }
+  }
+  if (SPLIT > 1) {
+#pragma unroll
+    for (int m = 0; m < 2; ++m) {
+      if (lane == 0) { sm[warp][m] = mx[m]; sl[warp][m] = l[m]; }
+#pragma unroll
+      for (int e = 0; e < DG_VPL; ++e) so[warp][m][lane + 32 * e] = o[m][e];
+    }
+    __syncthreads();
+    if (warp != 0) return;
+#pragma unroll
+    for (int m = 0; m < 2; ++m) {
+      float all = sm[0][m];  // finite: warp 0 holds the first visible key
+      for (int i = 1; i < SPLIT; ++i) all = fmaxf(all, sm[i][m]);
+      l[m] = 0.f;
+#pragma unroll
+      for (int e = 0; e < DG_VPL; ++e) o[m][e] = 0.f;
+      for (int i = 0; i < SPLIT; ++i) {
+        const float f = expf(sm[i][m] - all);  // 0 for a warp without keys
+        l[m] += sl[i][m] * f;
+#pragma unroll
+        for (int e = 0; e < DG_VPL; ++e) o[m][e] += so[i][m][lane + 32 * e] * f;
       }
     }
   }
@@ -559,17 +585,22 @@ XL_API int xl_diff_attn_general(const void* q, long long ldq, const void* kc, co
   if (B < 1 || B > 65535 || H < 1 || H > 65535 || T_len < 1 || G < 1 || H % G || dim < 1 || dim > DG_MAX_DIM || vdim < 1 ||
       vdim > 512 || Smax < 1 || chunk < 0)
     return -1;
-  const dim3 grid((T_len + DG_WARPS - 1) / DG_WARPS, H, B);
+  // a CTA per row while that is no more than about two CTAs of eight warps per SM; longer portions fill the SMs with a warp per row
+  const bool split = (long long)T_len * H * B <= 2 * 148;
+  const dim3 grid(split ? T_len : (T_len + 3) / 4, H, B);
+#define XL_DG(VPL)                                                                                                               \
+  if (split)                                                                                                                     \
+    diff_attn_general_kernel<T, VPL, 8><<<grid, 256, 0, s>>>((const T*)q, ldq, (const T*)kc, (const T*)vc, (T*)out, ldo, pos,    \
+                                                             count, lam, T_len, H, G, dim, vdim, Smax, chunk, scale, eps, out_scale); \
+  else                                                                                                                           \
+    diff_attn_general_kernel<T, VPL, 1><<<grid, 128, 0, s>>>((const T*)q, ldq, (const T*)kc, (const T*)vc, (T*)out, ldo, pos,    \
+                                                             count, lam, T_len, H, G, dim, vdim, Smax, chunk, scale, eps, out_scale)
   XL_DISPATCH_DTYPE(dtype, T, {
-    if (vdim <= 256)
-      diff_attn_general_kernel<T, 8><<<grid, DG_WARPS * 32, 0, s>>>((const T*)q, ldq, (const T*)kc, (const T*)vc, (T*)out, ldo,
-                                                                   pos, count, lam, T_len, H, G, dim, vdim, Smax, chunk, scale,
-                                                                   eps, out_scale);
-    else
-      diff_attn_general_kernel<T, 16><<<grid, DG_WARPS * 32, 0, s>>>((const T*)q, ldq, (const T*)kc, (const T*)vc, (T*)out, ldo,
-                                                                    pos, count, lam, T_len, H, G, dim, vdim, Smax, chunk, scale,
-                                                                    eps, out_scale);
+    if (vdim <= 128) { XL_DG(4); }
+    else if (vdim <= 256) { XL_DG(8); }
+    else { XL_DG(16); }
   });
+#undef XL_DG
   return (int)cudaGetLastError();
 }
 

@@ -95,40 +95,40 @@ int launch_append(const void* proj, long long ld, const float* wq, const float* 
 }
 
 // ---- general kernel --------------------------------------------------------------------------------------------------
-constexpr int WG_WARPS = 4;
 
-template <typename T, int VPL>  // VPL: value features per lane
-__global__ void __launch_bounds__(WG_WARPS * 32)
+// SPLIT 1: a warp per query row, four of them per CTA. SPLIT 8: a CTA per query row whose warps take its blocks of 32 keys in turn
+// and merge their parts of the softmax in shared memory, for the few rows of a decoding step.
+template <typename T, int VPL, int SPLIT>  // VPL: value features per lane
+__global__ void __launch_bounds__(SPLIT == 1 ? 128 : SPLIT * 32)
     window_attn_general_kernel(const T* __restrict__ qn, const T* __restrict__ kc, const T* __restrict__ vc,
                                const T* __restrict__ gate, long long ldg, T* __restrict__ out, long long ldo,
                                const int* __restrict__ pos, const int* __restrict__ count, int T_len, int H, int G, int dim,
                                int vdim, int Smax, int window, int keep_first, float scale, float sink) {
-  __shared__ float sq[WG_WARPS][WA_MAX_DIM];
+  constexpr int ROWS = SPLIT == 1 ? 4 : 1;
+  __shared__ __align__(16) float sq[ROWS][WA_MAX_DIM];
+  __shared__ float so[SPLIT == 1 ? 1 : SPLIT][SPLIT == 1 ? 1 : 32 * VPL], sm[SPLIT], sl[SPLIT];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int slot = SPLIT == 1 ? warp : 0, part = SPLIT == 1 ? 0 : warp;
   const int h = blockIdx.y, b = blockIdx.z, R = H / G, g = h / R;
-  const int t = blockIdx.x * WG_WARPS + warp;
-  if (t >= min(count[b], T_len)) return;
+  const int t = blockIdx.x * ROWS + slot;
+  if (t >= min(count[b], T_len)) return;  // whole warps, and with SPLIT > 1 whole CTAs
   const int p = pos[b] + t;
   if (p < 0 || p >= Smax) return;
   const T* q = qn + ((((long long)b * G + g) * T_len + t) * R + h % R) * dim;
-  for (int d = lane; d < dim; d += 32) sq[warp][d] = xl_to_float(q[d]);
-  __syncwarp();
+  for (int d = part * 32 + lane; d < dim; d += 32 * SPLIT) sq[slot][d] = xl_to_float(q[d]);
+  if (SPLIT == 1) __syncwarp();
+  else __syncthreads();
   const WindowRange seen = window_range(p, window, keep_first);
   const T* kb = kc + ((long long)b * G + g) * Smax * dim;
   const T* vb = vc + ((long long)b * G + g) * Smax * vdim;
-  float o[VPL], mx = sink, l = sink == -INFINITY ? 0.f : 1.f;
+  float o[VPL], mx = part ? -INFINITY : sink, l = part || sink == -INFINITY ? 0.f : 1.f;  // the sink is the first part's
 #pragma unroll
   for (int e = 0; e < VPL; ++e) o[e] = 0.f;
   auto walk = [&](int begin, int end) {
-    for (int j0 = begin; j0 < end; j0 += 32) {
+    for (int j0 = begin + part * 32; j0 < end; j0 += 32 * SPLIT) {
       const int j = j0 + lane;
       float s = -INFINITY;
-      if (j < end) {
-        const T* kr = kb + (long long)j * dim;
-        s = 0.f;
-        for (int d = 0; d < dim; ++d) s = fmaf(sq[warp][d], xl_to_float(kr[d]), s);
-        s *= scale;
-      }
+      if (j < end) s = xl_row_dot(sq[slot], kb + (long long)j * dim, dim) * scale;
       const float m_new = fmaxf(mx, xl_warp_max(s));  // finite: key j0 is visible
       const float corr = expf(mx - m_new), w = expf(s - m_new);
       l = l * corr + xl_warp_sum(w);
@@ -136,6 +136,7 @@ __global__ void __launch_bounds__(WG_WARPS * 32)
 #pragma unroll
       for (int e = 0; e < VPL; ++e) o[e] *= corr;
       const int n = min(32, end - j0);
+#pragma unroll 4
       for (int k = 0; k < n; ++k) {
         const float wk = __shfl_sync(0xffffffffu, w, k);
         const T* vr = vb + (long long)(j0 + k) * vdim;
@@ -147,6 +148,24 @@ __global__ void __launch_bounds__(WG_WARPS * 32)
   };
   walk(0, seen.kept);
   walk(seen.first, p + 1);
+  if (SPLIT > 1) {
+    if (lane == 0) { sm[warp] = mx; sl[warp] = l; }
+#pragma unroll
+    for (int e = 0; e < VPL; ++e) so[warp][lane + 32 * e] = o[e];
+    __syncthreads();
+    if (warp != 0) return;
+    mx = sm[0];
+    for (int i = 1; i < SPLIT; ++i) mx = fmaxf(mx, sm[i]);  // finite: the new key is visible to one of them
+    l = 0.f;
+#pragma unroll
+    for (int e = 0; e < VPL; ++e) o[e] = 0.f;
+    for (int i = 0; i < SPLIT; ++i) {
+      const float f = expf(sm[i] - mx);  // 0 for a warp without keys
+      l += sl[i] * f;
+#pragma unroll
+      for (int e = 0; e < VPL; ++e) o[e] += so[i][lane + 32 * e] * f;
+    }
+  }
   const long long row = (long long)b * T_len + t;
   const T* gr = gate ? gate + row * ldg + (long long)h * vdim : nullptr;
 #pragma unroll
@@ -579,14 +598,21 @@ XL_API int xl_window_attn_general(const void* qn, const void* kc, const void* vc
   if (B < 1 || B > 65535 || H < 1 || H > 65535 || T_len < 1 || G < 1 || H % G || dim < 1 || dim > WA_MAX_DIM || vdim < 1 ||
       vdim > 512 || Smax < 1 || window < 0 || keep_first < 0)
     return -1;
-  const dim3 grid((T_len + WG_WARPS - 1) / WG_WARPS, H, B);
-#define XL_WG(VPL)                                                                                                            \
-  window_attn_general_kernel<T, VPL><<<grid, WG_WARPS * 32, 0, s>>>((const T*)qn, (const T*)kc, (const T*)vc, (const T*)gate,    \
-                                                                    ldg, (T*)out, ldo, pos, count, T_len, H, G, dim, vdim, Smax, \
-                                                                    window, keep_first, scale, sink)
+  // a CTA per row while that is no more than about two CTAs of eight warps per SM; longer portions fill the SMs with a warp per row
+  const bool split = (long long)T_len * H * B <= 2 * 148;
+  const dim3 grid(split ? T_len : (T_len + 3) / 4, H, B);
+#define XL_WG(VPL)                                                                                                                 \
+  if (split)                                                                                                                       \
+    window_attn_general_kernel<T, VPL, 8><<<grid, 256, 0, s>>>((const T*)qn, (const T*)kc, (const T*)vc, (const T*)gate, ldg,      \
+                                                               (T*)out, ldo, pos, count, T_len, H, G, dim, vdim, Smax, window,     \
+                                                               keep_first, scale, sink);                                          \
+  else                                                                                                                             \
+    window_attn_general_kernel<T, VPL, 1><<<grid, 128, 0, s>>>((const T*)qn, (const T*)kc, (const T*)vc, (const T*)gate, ldg,      \
+                                                               (T*)out, ldo, pos, count, T_len, H, G, dim, vdim, Smax, window,     \
+                                                               keep_first, scale, sink)
   XL_DISPATCH_DTYPE(dtype, T, {
-    if (vdim <= 128) XL_WG(4);
-    else XL_WG(16);
+    if (vdim <= 128) { XL_WG(4); }
+    else { XL_WG(16); }
   });
 #undef XL_WG
   return (int)cudaGetLastError();

@@ -118,6 +118,25 @@ static inline int xl_grid_for(long long n_items, int per_block, int max_blocks =
   return (int)b;
 }
 
+// Dot product of n values in shared memory (16-byte aligned) with a row in global memory, added in order; rows of whole 16-byte
+// pieces are read as such, several ahead.
+template <typename T> __device__ __forceinline__ float xl_row_dot(const float* a, const T* row, int n) {
+  constexpr int V = 16 / sizeof(T);
+  float s = 0.f;
+  if (n % V == 0 && (((uintptr_t)row) & 15) == 0) {
+#pragma unroll 8
+    for (int d = 0; d < n; d += V) {
+      const uint4 raw = *reinterpret_cast<const uint4*>(row + d);
+      const T* e = reinterpret_cast<const T*>(&raw);
+#pragma unroll
+      for (int i = 0; i < V; ++i) s = fmaf(a[d + i], xl_to_float(e[i]), s);
+    }
+  } else {
+    for (int d = 0; d < n; ++d) s = fmaf(a[d], xl_to_float(row[d]), s);
+  }
+  return s;
+}
+
 // Contiguous ranges of items for the CTAs of a grid: the first `rem` CTAs take per + 1 items, the others per.
 struct XlRanges {
   int per, rem;

@@ -32,6 +32,7 @@ _window_general = _sig("xl_window_attn_general", *_WINDOW_ARGS, _c_int, _c_p)
 _window_tcgen05 = _sig("xl_window_attn_tcgen05", *_WINDOW_ARGS, _c_p, _c_p)
 _window_decode = _sig("xl_window_attn_decode", _c_p, _c_ll, _c_p, _c_p, _c_p, _c_p, _c_p, _c_ll, _c_p, _c_p, _c_int, _c_int, _c_int,
                       _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_f, _c_f, _c_f, _c_int, _c_p, _c_p, _c_p)
+_linear_f32 = _sig("xl_linear_f32", _c_p, _c_ll, _c_p, _c_p, _c_ll, _c_int, _c_int, _c_int, _c_p)
 _small_m_slots = _sig("xl_linear_small_m_slots", _c_int)
 _SMALL_TAIL = (_c_int, _c_int, _c_int, _c_p, _c_p, _c_int, _c_int, _c_p)
 _SUMSQ = (_c_p, _c_int, _c_f)  # sums of squares of a deferred norm, parts per row, eps
@@ -117,6 +118,12 @@ def product(a, weight, out_dtype=None, sumsq=None, eps=0.0):
         return NotImplemented
     if torch.backends.cuda.matmul.allow_tf32:
         raise RuntimeError("32-bit models need true fp32 matrix products: set torch.backends.cuda.matmul.allow_tf32 = False")
+    if (a.is_cuda and weight.dtype == torch.float32 and out_dtype == torch.float32 and a.shape[0] <= 16 and a.stride(1) == 1
+            and weight.is_contiguous()):
+        y = torch.empty((a.shape[0], weight.shape[0]), dtype=out_dtype, device=a.device)
+        if _small_ok(_linear_f32(a.data_ptr(), a.stride(0), weight.data_ptr(), y.data_ptr(), y.stride(0), a.shape[0],
+                                 weight.shape[0], a.shape[1], _stream()), "linear_f32"):
+            return y
     return torch.mm(a, weight.t()).to(out_dtype)
 
 

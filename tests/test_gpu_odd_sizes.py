@@ -164,3 +164,53 @@ def test_int4_product_at_the_edges_of_its_tiles(nat, dtype, pairs, M, N, K, gs):
     y = nat.gq_gemm_small_m(x, packed, *((interleave_scale_zero(scale, zero), None) if pairs else (scale, zero)), None)
     assert y is not NotImplemented
     _near(y, want, dtype, terms=31 * K)
+
+
+@pytest.mark.parametrize("rows,N,K", [(1, 1, 4), (2, 7, 132), (3, 2367, 1028), (4, 32000, 1024), (5, 30, 2816), (8, 2369, 68), (11, 513, 2048),
+                                      (16, 1024, 1020)])
+def test_few_rows_product_in_32_bits(nat, rows, N, K):
+    """Ragged weight rows and K, each number of rows a CTA takes, a slice of a wider matrix. fp32 sums of K terms whose sizes add
+    up to about sqrt(K) times the result: a few units of 2^-24 * sqrt(K)."""
+    from popxl_addons_b200.ops.native_sequence import product
+
+    g = torch.Generator(device="cuda").manual_seed(rows * N + K)
+    a = torch.randn(rows, K + 4, generator=g, device="cuda")[:, :K]
+    w = torch.randn(N, K, generator=g, device="cuda")
+    before = nat.LAUNCHES["by_kernel"].get("linear_f32", 0)
+    y = product(a, w)
+    assert nat.LAUNCHES["by_kernel"]["linear_f32"] == before + 1
+    want = a.double() @ w.double().t()
+    assert float((y.double() - want).abs().max() / want.abs().max()) <= 2.0 ** -22 * K ** 0.5
+
+
+@pytest.mark.parametrize("T", [1, 2, 70])
+@pytest.mark.parametrize("dim,vdim", [(64, 128), (20, 36), (6, 300)])
+@pytest.mark.parametrize("kind", ["diff", "window"])
+def test_general_attention_of_few_rows_equals_that_of_many(nat, kind, T, dim, vdim):
+    """A row's keys split over the warps of a CTA (few rows) against one warp per row (the same rows among many sequences): fp32 sums
+    in another order, 1e-5. 70 tokens at position 150 see blocks that some warps do not have."""
+    from popxl_addons_b200.ops import native_sequence as ns
+
+    H, G, S, B = 4, 2, 260, 80
+    g = torch.Generator(device="cuda").manual_seed(dim + T)
+    one = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    many = lambda t: t.expand(B, *t.shape[1:]).contiguous()
+    pos, s = torch.full((B,), 150, dtype=torch.int32, device="cuda"), nat._stream()
+    count = torch.full((B,), T, dtype=torch.int32, device="cuda")
+    lam = torch.tensor(0.3, device="cuda")
+    vc = one(1, G, S, vdim)
+    q, kc = (one(1, T, H * 2 * dim), one(1, G, 2, S, dim)) if kind == "diff" else (one(1, G, T, H // G, dim), one(1, G, S, dim))
+    out = []
+    for n in (1, B):
+        y = torch.zeros(n * T, H * vdim, device="cuda")
+        qn, kn, vn = (t if n == 1 else many(t) for t in (q, kc, vc))
+        if kind == "diff":
+            rc = ns._diff_general(qn.data_ptr(), H * 2 * dim, kn.data_ptr(), vn.data_ptr(), y.data_ptr(), H * vdim, pos.data_ptr(),
+                                  count.data_ptr(), lam.data_ptr(), n, T, H, G, dim, vdim, S, 128, 0.2, 1e-5, 0.7, 0, s)
+        else:
+            rc = ns._window_general(qn.data_ptr(), kn.data_ptr(), vn.data_ptr(), None, 0, y.data_ptr(), H * vdim, pos.data_ptr(),
+                                    count.data_ptr(), n, T, H, G, dim, vdim, S, 90, 3, 0.2, 0.0, 0, s)
+        assert rc == 0
+        out.append(y.view(n, T, H * vdim))
+    assert out[1].abs().max() > 0
+    assert (out[0] - out[1]).abs().max() <= 1e-5 * out[1].abs().max()
