@@ -1,8 +1,8 @@
-// Linear layers of the decoding path, bf16 weights, M <= 16 rows: C[M, N] = a[M, K] * w[N, K]^T, the weights streamed once.
-// What follows the product in a layer happens in the epilogue, on the fp32 sums:
+// Linear layers of the decoding path, bf16 weights, few rows: C[M, N] = a[M, K] * w[N, K]^T, the weights streamed once.
+// What follows the product in a layer happens in the epilogue, on the fp32 sums (M <= 16; `store` up to 128 rows):
 //   store      C as bf16 or fp32
 //   residual   x += mult * C (+ table[token]) on the fp32 residual stream; for the next layer h = DyT(x), or the first half of
-//              an RMS norm: h = x * w and the sums of squares of x over blocks of 64 columns (one column tile each)
+//              an RMS norm: h = x * w and the sums of squares of x over blocks of 64 columns
 //   swiglu     weight rows [gate | up]: y = silu(gate) * up
 //   split_glu  weight rows [plain | gate | up]: plain results stored, a clamped gated unit of the others beside them
 //   min_gru    weight rows [z | u | g], one row per sequence: one step of the recurrence on the fp32 state
@@ -10,37 +10,56 @@
 // store and split_glu may take rows of such a half-done norm: their results are multiplied by 1 / sqrt(mean(x^2) + eps), summed
 // up from the blocks' sums of squares while the weights arrive.
 //
-// The product is bandwidth-bound (at most 16 multiply-adds per weight), so it uses `mma.sync.m16n8k16` with operands from
-// registers: each lane copies two 16-byte pieces of a weight row (four lanes: 64 contiguous bytes each time) through a per-warp
-// cp.async ring and feeds them to four MMAs; the activations it needs for them are loaded one chunk ahead into registers. (Any assignment of k indices to the k slots of an MMA is valid as long as both operands agree.)
+// The product is bandwidth-bound. The weight rows are the M = 128 operand of `tcgen05.mma` and the tokens (padded to 16, 32, 64 or
+// 128) its N, so that one thread keeps the tensor core ahead of HBM: four instructions per 16 KB of weights, about 65 clocks each,
+// are twice the rate at which an SM's share of the bandwidth arrives. TMA loads 128 x 64 blocks of weights, and the tokens' 64
+// columns beside them, into a ring of about 90 KB per CTA; one CTA per SM works on a product while one of the next product already
+// fills its ring (programmatic dependent launch: weights are requested while the previous kernel drains).
 //
-// Work = (column tiles) x (K chunks of 64), tile-major, cut into equal contiguous ranges, one per CTA, so the grid fits the
-// machine and not the problem. A tile shared by several CTAs is finished by the one that arrives last: every CTA leaves its
-// partial sums in a slot of its own and the finisher adds the slots in CTA order, so results do not depend on timing.
-// No CTA waits for another. Consecutive kernels overlap: a launch requests its first weights while its predecessor drains. An epilogue that combines several weight rows per output channel (swiglu, min_gru) takes them
+// A tile of 128 weight rows belongs to a cluster of KS CTAs (1 to 8), each with an equal range of K blocks; KS is what the SMs have
+// room for. The CTAs leave their sums in shared memory, meet, and each finishes its share of the tile's results from the partial sums
+// of all of them, added in CTA order, so results do not depend on timing. (Equal ranges of tiles x K blocks, one per CTA, with
+// partial sums through global memory and the last arrival finishing a tile, took 2 to 10 us per launch more.) An epilogue
+// that combines several weight rows per output channel (swiglu, min_gru) takes them
 // into one tile: a tile is PARTS groups of CH channels, group p starting at weight row p * N / PARTS.
+//
+// Chains of launches on one B200, us (`mma.sync` with weights in registers and split K through global memory before -> now): 1 token
+// 4096 x 4096 12.4 -> 8.4, 22016 x 4096 with swiglu 39.0 -> 32.3; 16 tokens 4096 x 11008 26.9 -> 18.0, 32000 x 4096 58.0 -> 43.0
+// (6.1 TB/s); 40 tokens (tiles of 256 rows of the pair GEMM before) 2048 x 7680 30.5 -> 11.1, 12288 x 4096 29.6 -> 21.1,
+// 32000 x 4096 57.0 -> 47.2.
+//
+// Roles per CTA: warp 0 loads, warp 1 allocates TMEM and issues the MMAs, warps 2-5 drain the accumulator. Every wait is bounded; a role
+// that gives up records a code in `*err`, all threads meet at the cluster's barriers and TMEM is freed.
 #include "common.cuh"
+#include "tcgen05.cuh"
 
 #include <math.h>
 
 namespace {
 
-constexpr int SM_WARPS = 4;
-constexpr int SM_KC = 64;       // k values per chunk (16 per lane)
-constexpr int SM_STAGES = 3;
-constexpr int SM_CTAS_PER_SM = 2;
+using namespace xl_tc;
+
+constexpr int SM_KC = 64;            // k values per block: one 128-byte swizzle row
+constexpr int SM_EPI = 128;          // threads of the epilogue, one per TMEM lane
+constexpr int SM_THREADS = 64 + SM_EPI;
 
 enum SmMode : int { SM_STORE = 0, SM_RESIDUAL = 1, SM_SWIGLU = 2, SM_MINGRU = 3, SM_SPLIT_GLU = 4 };
 
-// split_glu has two kinds of tiles: first those of the plain rows (one part of 64 channels), then those of the gated unit.
+// split_glu has two kinds of tiles: first those of the plain rows (one part of 128 channels), then those of the gated unit.
 template <int MODE> struct SmTile {
   static constexpr int PARTS = MODE == SM_SWIGLU || MODE == SM_SPLIT_GLU ? 2 : (MODE == SM_MINGRU ? 3 : 1);
-  static constexpr int CH = PARTS == 2 ? 32 : (MODE == SM_MINGRU ? 16 : 64);  // channels per tile
-  static constexpr int COLS = PARTS * CH;
-  static constexpr int NT = COLS / 8;
-  static constexpr int STAGE = NT * 2 * 32;  // uint4: two pieces of NT weight rows per lane
-  static constexpr int RING_BYTES = SM_WARPS * SM_STAGES * STAGE * 16;
+  static constexpr int CH = PARTS == 2 ? 64 : (MODE == SM_MINGRU ? 40 : 128);  // channels per tile
+  static constexpr int COLS = PARTS * CH;  // rows of the MMA that hold weights (120 of 128 for min_gru)
 };
+// NTOK: columns of the MMA, the tokens padded
+template <int NTOK> struct SmRing {
+  static constexpr int W_BYTES = 128 * SM_KC * 2, A_BYTES = NTOK * SM_KC * 2, STAGE = W_BYTES + A_BYTES;
+  static constexpr int STAGES = NTOK <= 32 ? 5 : (NTOK == 64 ? 4 : 3);
+  static constexpr int SMEM = STAGES * STAGE + 1024 /*alignment slack*/;
+  static constexpr uint32_t TMEM_COLS = NTOK < 32 ? 32 : NTOK;
+  static_assert(NTOK * 132 * 4 <= STAGES * STAGE, "the partial sums take the ring's place");
+};
+enum { ERR_SM_FULL = 31, ERR_SM_EMPTY = 32, ERR_SM_ACC_FULL = 33 };
 
 struct SmParams {
   const __nv_bfloat16* a;
@@ -73,17 +92,10 @@ struct SmParams {
   const float *bz, *bu;
   float* state;
   const int *pos, *count;
-  // split-K scratch
-  float* slots;            // [grid][2][16 * COLS]
-  unsigned int* counters;  // one per tile, zero between launches
+  int ksplit;  // CTAs of a cluster
+  int* err;
 };
 
-__device__ __forceinline__ void mma_bf16(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
-                                         uint32_t b1) {
-  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-               : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
 __device__ __forceinline__ float sigmoid_f(float v) { return 1.f / (1.f + expf(-v)); }
 __device__ __forceinline__ float silu_f(float v) { return v / (1.f + expf(-v)); }
 
@@ -162,331 +174,316 @@ __device__ __forceinline__ float sm_epilogue(const SmParams& p, int r, int c, co
   return sq;
 }
 
-template <int MODE>
-__global__ void __launch_bounds__(SM_WARPS * 32, SM_CTAS_PER_SM) linear_small_m_kernel(const SmParams p) {
-  using L = SmTile<MODE>;
-  constexpr int NT = L::NT, COLS = L::COLS, CH = L::CH, PARTS = L::PARTS;
-  extern __shared__ uint4 ring_all[];
-  __shared__ float red[SM_WARPS][16][COLS + 1];
-  __shared__ unsigned int finish;
-  __shared__ float row_scale[16];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int quad = lane >> 2, j = lane & 3;
-  const int chunks = (p.K + SM_KC - 1) / SM_KC;
-  // tiles [0, plain) have one part of COLS channels (split_glu only), the others PARTS parts of CH
-  const int plain = MODE == SM_SPLIT_GLU ? (p.cols + COLS - 1) / COLS : 0;
-  const int channels = MODE == SM_SPLIT_GLU ? (p.N - p.cols) / PARTS : p.N / PARTS;
-  const int n_tiles = plain + (channels + CH - 1) / CH;
-  const int total = n_tiles * chunks;
-  const XlRanges ranges{total / (int)gridDim.x, total % (int)gridDim.x};
-  int item = ranges.begin(blockIdx.x);
-  const int item_end = ranges.begin(blockIdx.x + 1);
-  const int first_tile = item / chunks;
-  uint4* ring = ring_all + warp * (SM_STAGES * L::STAGE);
+__device__ __forceinline__ float4 ld_cluster_v4(uint32_t cluster_addr) {
+  float4 v;
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(cluster_addr) : "memory");
+  return v;
+}
 
-  // The chunks of this warp over the whole range, tile after tile: (tile, chunk) of the next one to request and of the next to
-  // multiply advance by the same rule.
-  struct Cursor { int item, c1, ch, tile; };  // first item of the current tile segment, its end chunk, current chunk
-  auto segment = [&](Cursor& c) {  // enter the segment that starts at c.item (or stop at the end of the range)
-    while (c.item < item_end) {
-      c.tile = c.item / chunks;
-      const int c0 = c.item - c.tile * chunks;
-      c.c1 = min(chunks, c0 + (item_end - c.item));
-      c.ch = c0 + warp;
-      if (c.ch < c.c1) return;
-      c.item += c.c1 - c0;
+template <int MODE, int NTOK>
+__global__ void __launch_bounds__(SM_THREADS, 1)
+    linear_small_m_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_a, const SmParams p) {
+  using L = SmTile<MODE>;
+  using R = SmRing<NTOK>;
+  constexpr int COLS = L::COLS, CH = L::CH, PARTS = L::PARTS, STAGES = R::STAGES;
+  constexpr int RED_LD = 132;
+  extern __shared__ uint8_t smem_raw[];
+  __shared__ float row_scale[NTOK];
+  __shared__ uint64_t full_bar[STAGES], empty_bar[STAGES], acc_full;
+  __shared__ uint32_t tmem_slot;
+  __shared__ int abort_word;
+  uint8_t* ring = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);  // the same offset in every CTA of the cluster
+  volatile int* abort_flag = &abort_word;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int chunks = (p.K + SM_KC - 1) / SM_KC;
+  // tiles [0, plain) have one part of 128 channels (split_glu only), the others PARTS parts of CH
+  const int plain = MODE == SM_SPLIT_GLU ? (p.cols + 127) / 128 : 0;
+  const int channels = MODE == SM_SPLIT_GLU ? (p.N - p.cols) / PARTS : p.N / PARTS;
+  const int tile = blockIdx.x / p.ksplit, rank = blockIdx.x - tile * p.ksplit;  // clusters are consecutive CTAs
+  const int kb0 = chunks * rank / p.ksplit, blocks = chunks * (rank + 1) / p.ksplit - kb0;  // at least one
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < STAGES; ++s) {
+      mbar_init(&full_bar[s], 1);
+      mbar_init(&empty_bar[s], 1);
     }
-  };
-  auto advance = [&](Cursor& c) {
-    c.ch += SM_WARPS;
-    if (c.ch >= c.c1) {
-      c.item = c.tile * chunks + c.c1;
-      segment(c);
-    }
-  };
-  auto request = [&](const Cursor& c, int buf) {
-    if (c.item < item_end) {
-      const int k0 = c.ch * SM_KC + j * 8;
-      uint4* dst = ring + buf * L::STAGE + lane;
-#pragma unroll
-      for (int t = 0; t < NT; ++t) {
-        const int col = t * 8 + quad;
-        bool row_on;
-        long long w_row;
-        if (MODE == SM_SPLIT_GLU && c.tile < plain) {
-          w_row = c.tile * COLS + col;
-          row_on = w_row < p.cols;
-        } else {
-          const int n = (c.tile - plain) * CH + col % CH;
-          row_on = n < channels;
-          w_row = (MODE == SM_SPLIT_GLU ? p.cols : 0) + (long long)(col / CH) * channels + n;
-        }
-        const __nv_bfloat16* src = p.w + (row_on ? w_row : 0) * p.K;
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          const bool on = row_on && k0 + e * 32 < p.K;
-          xl_cp_async16(dst + (t * 2 + e) * 32, src + (on ? k0 + e * 32 : 0), on);
-        }
-      }
-    }
-    asm volatile("cp.async.commit_group;" ::: "memory");  // possibly empty: one group per chunk slot
-  };
-  auto load_a = [&](const Cursor& c, uint4 (&lo)[2], uint4 (&hi)[2]) {
-#pragma unroll
-    for (int e = 0; e < 2; ++e) {
-      const int k = c.ch * SM_KC + j * 8 + e * 32;
-      const bool on = c.item < item_end && k < p.K;
-      lo[e] = on && quad < p.M ? *reinterpret_cast<const uint4*>(p.a + (long long)quad * p.lda + k) : make_uint4(0, 0, 0, 0);
-      hi[e] = on && quad + 8 < p.M ? *reinterpret_cast<const uint4*>(p.a + (long long)(quad + 8) * p.lda + k) : make_uint4(0, 0, 0, 0);
-    }
-  };
-  Cursor ahead{item, 0, 0, 0};
-  segment(ahead);
-  Cursor cur = ahead;
-#pragma unroll
-  for (int n = 0; n < SM_STAGES - 1; ++n) {
-    request(ahead, n);
-    if (ahead.item < item_end) advance(ahead);
+    mbar_init(&acc_full, 1);
+    abort_word = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  xl_grid_dependency_wait();  // the first weights are on their way; everything else may come from the previous kernel
-  xl_grid_launch_dependents();
-  uint4 a_lo[2], a_hi[2];
-  load_a(cur, a_lo, a_hi);
-  if ((MODE == SM_STORE || MODE == SM_SPLIT_GLU) && p.sumsq) {  // read after the barriers of the first tile
-    for (int r = warp; r < p.M; r += SM_WARPS) {
-      float sq = 0.f;
-      for (int i = lane; i < p.sumsq_parts; i += 32) sq += p.sumsq[(long long)r * p.sumsq_parts + i];
-      sq = xl_warp_sum(sq);
-      if (lane == 0) row_scale[r] = 1.f / sqrtf(sq / p.K + p.eps);
-    }
+  if (warp == 1) {
+    tmem_alloc(&tmem_slot, R::TMEM_COLS);
+    tmem_relinquish();
   }
-  int buf = 0;
-  while (item < item_end) {
-    const int tile = item / chunks;
-    const int c0 = item - tile * chunks;
-    const int c1 = min(chunks, c0 + (item_end - item));
-    float acc[NT][4];
+  tcgen05_fence_before();
+  __syncthreads();
+  tcgen05_fence_after();
+  const uint32_t tmem_base = tmem_slot;
+
+  if (warp == 0) {
+    // ------------------------------------------------ loads --------------------------------------------------------
+    if (elect_one()) {
+      const bool one = MODE == SM_SPLIT_GLU && tile < plain;
+      const int n0 = MODE == SM_SPLIT_GLU ? (one ? tile * 128 : p.cols + (tile - plain) * CH) : tile * CH;
+      auto load_w = [&](int i, int s) {
 #pragma unroll
-    for (int t = 0; t < NT; ++t)
-#pragma unroll
-      for (int e = 0; e < 4; ++e) acc[t][e] = 0.f;
-    for (int ch = c0 + warp; ch < c1; ch += SM_WARPS) {
-      request(ahead, (buf + SM_STAGES - 1) % SM_STAGES);
-      if (ahead.item < item_end) advance(ahead);
-      uint4 lo[2] = {a_lo[0], a_lo[1]}, hi[2] = {a_hi[0], a_hi[1]};
-      advance(cur);
-      load_a(cur, a_lo, a_hi);
-      asm volatile("cp.async.wait_group %0;" ::"n"(SM_STAGES - 1) : "memory");
-      const uint4* src = ring + buf * L::STAGE + lane;  // every lane reads back the pieces it copied itself
-      buf = (buf + 1) % SM_STAGES;
-#pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        uint4 w[NT];
-#pragma unroll
-        for (int t = 0; t < NT; ++t) w[t] = src[(t * 2 + e) * 32];
-#pragma unroll
-        for (int t = 0; t < NT; ++t) mma_bf16(acc[t], lo[e].x, hi[e].x, lo[e].y, hi[e].y, w[t].x, w[t].y);
-#pragma unroll
-        for (int t = 0; t < NT; ++t) mma_bf16(acc[t], lo[e].z, hi[e].z, lo[e].w, hi[e].w, w[t].z, w[t].w);
+        for (int q = 0; q < PARTS; ++q)  // boxes of CH rows; a plain tile's are consecutive
+          tma_load_2d(ring + s * R::STAGE + q * CH * 128, &map_w, &full_bar[s], (kb0 + i) * SM_KC, n0 + q * (one ? CH : channels));
+      };
+      auto load_a = [&](int i, int s) { tma_load_2d(ring + s * R::STAGE + R::W_BYTES, &map_a, &full_bar[s], (kb0 + i) * SM_KC, 0); };
+      constexpr uint32_t BYTES = COLS * 128 + R::A_BYTES;
+      const int ahead = min(STAGES, blocks);
+      for (int i = 0; i < ahead; ++i) {
+        mbar_expect_tx(&full_bar[i], BYTES);
+        load_w(i, i);
+      }
+      xl_grid_dependency_wait();  // the first weights are on their way; everything else may come from the previous kernel
+      xl_grid_launch_dependents();
+      for (int i = 0; i < ahead; ++i) load_a(i, i);
+      uint32_t stage = 0, phase = 0;
+      for (int i = ahead; i < blocks; ++i) {
+        if (!mbar_wait(&empty_bar[stage], phase, abort_flag, p.err, ERR_SM_EMPTY)) break;
+        mbar_expect_tx(&full_bar[stage], BYTES);
+        load_w(i, stage);
+        load_a(i, stage);
+        if (++stage == STAGES) { stage = 0; phase ^= 1; }
       }
     }
-    __syncthreads();  // readers of the previous tile are done with `red`
+    __syncwarp();
+  } else if (warp == 1) {
+    // ------------------------------------------------ MMAs ---------------------------------------------------------
+    xl_grid_dependency_wait();  // the tokens arrive after it: no bounded wait runs while the predecessor still does
+    if (elect_one()) {
+      constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(NTOK >> 3) << 17) | (8u << 24);
+      uint32_t stage = 0, phase = 0;
+      bool ok = true;
+      for (int i = 0; i < blocks; ++i) {
+        ok = mbar_wait(&full_bar[stage], phase, abort_flag, p.err, ERR_SM_FULL);
+        if (!ok) break;
+        tcgen05_fence_after();
+        const uint32_t sw = smem_u32(ring + stage * R::STAGE), sa = sw + R::W_BYTES;
 #pragma unroll
-    for (int t = 0; t < NT; ++t) {
-      red[warp][quad][t * 8 + 2 * j] = acc[t][0];
-      red[warp][quad][t * 8 + 2 * j + 1] = acc[t][1];
-      red[warp][quad + 8][t * 8 + 2 * j] = acc[t][2];
-      red[warp][quad + 8][t * 8 + 2 * j + 1] = acc[t][3];
-    }
-    __syncthreads();
-    const bool whole = c1 - c0 == chunks;
-    bool finishing = whole;
-    if (!whole) {
-      float* slot = p.slots + ((long long)blockIdx.x * 2 + (tile == first_tile ? 0 : 1)) * (16 * COLS);
-      for (int i = threadIdx.x; i < p.M * COLS; i += blockDim.x) {
-        const int r = i / COLS, col = i % COLS;
-        float s = 0.f;
-#pragma unroll
-        for (int w = 0; w < SM_WARPS; ++w) s += red[w][r][col];
-        __stcg(slot + i, s);
+        for (int k = 0; k < SM_KC / 16; ++k)
+          tcgen05_mma_f16(tmem_base, make_smem_desc(sw + k * 32, 16), make_smem_desc(sa + k * 32, 16), idesc, (i | k) != 0 ? 1u : 0u);
+        tcgen05_commit(&empty_bar[stage]);
+        if (++stage == STAGES) { stage = 0; phase ^= 1; }
       }
-      __threadfence();
-      __syncthreads();
-      if (threadIdx.x == 0)
-        finish = atomicAdd(p.counters + tile, (unsigned int)(c1 - c0)) + (unsigned int)(c1 - c0) == (unsigned int)chunks;
-      __syncthreads();
-      finishing = finish != 0;
-      if (finishing) __threadfence();
+      if (ok) tcgen05_commit(&acc_full);
     }
-    if (finishing) {
-      // CTAs that share the tile, in order. All but the first begin inside it: it is their first tile (slot 0). It is the
-      // last tile of the first one, and its first only if that one begins exactly with it.
-      int cta0 = blockIdx.x, cta1 = blockIdx.x, slot0 = 0;
-      if (!whole) {
-        cta0 = ranges.owner(tile * chunks);
-        cta1 = ranges.owner(tile * chunks + chunks - 1);
-        slot0 = ranges.begin(cta0) < tile * chunks ? 1 : 0;
-      }
-      const bool unit = tile >= plain;  // one part of COLS channels, or PARTS parts of CH
-      const int ch = MODE == SM_SPLIT_GLU && !unit ? COLS : CH, parts = MODE == SM_SPLIT_GLU && !unit ? 1 : PARTS;
-      const int end = MODE == SM_SPLIT_GLU && !unit ? p.cols : channels, per_row = ch / 4;
-      for (int i = threadIdx.x; i < p.M * per_row; i += blockDim.x) {
-        const int r = i / per_row, cc = (i % per_row) * 4, c = (unit ? tile - plain : tile) * ch + cc;
+    __syncwarp();
+  } else {
+    // ------------------------------------------------ partial sums -> shared memory --------------------------------
+    xl_grid_dependency_wait();
+    xl_grid_launch_dependents();
+    const int q4 = warp & 3, row = q4 * 32 + lane;  // TMEM lane = weight row of the tile
+    float* red = reinterpret_cast<float*>(ring);    // [token][weight row]: every load of the ring has been read by an MMA by then
+    if ((MODE == SM_STORE || MODE == SM_SPLIT_GLU) && p.sumsq) {  // while the weights arrive
+      for (int r = warp - 2; r < p.M; r += 4) {
         float sq = 0.f;
-        if (c < end) {
-          float v[PARTS][4];
-#pragma unroll
-          for (int q = 0; q < PARTS; ++q) {
-            const int col = q * CH + cc;
-            if (MODE == SM_SPLIT_GLU && q >= parts) {
-#pragma unroll
-              for (int e = 0; e < 4; ++e) v[q][e] = 0.f;
-            } else if (whole) {
-#pragma unroll
-              for (int e = 0; e < 4; ++e) {
-                v[q][e] = 0.f;
-#pragma unroll
-                for (int w = 0; w < SM_WARPS; ++w) v[q][e] += red[w][r][col + e];
-              }
-            } else {
-              const float* base = p.slots + r * COLS + col;
-              float4 t = __ldcg(reinterpret_cast<const float4*>(base + ((long long)cta0 * 2 + slot0) * (16 * COLS)));
-#pragma unroll 8
-              for (int k = cta0 + 1; k <= cta1; ++k) {
-                const float4 o = __ldcg(reinterpret_cast<const float4*>(base + (long long)k * 2 * (16 * COLS)));
-                t.x += o.x; t.y += o.y; t.z += o.z; t.w += o.w;
-              }
-              v[q][0] = t.x; v[q][1] = t.y; v[q][2] = t.z; v[q][3] = t.w;
-            }
-            if ((MODE == SM_STORE || MODE == SM_SPLIT_GLU) && p.sumsq) {
-#pragma unroll
-              for (int e = 0; e < 4; ++e) v[q][e] *= row_scale[r];
-            }
-          }
-          sq = sm_epilogue<MODE>(p, r, c, v, end, unit);
-        }
-        if (MODE == SM_RESIDUAL && p.sumsq_out) {
-          // the 16 lanes of a half-warp hold one row; either all or none of them are here
-          const unsigned int half = 0xffffu << (lane & 16);
-#pragma unroll
-          for (int o = 8; o > 0; o >>= 1) sq += __shfl_xor_sync(half, sq, o);
-          if ((lane & 15) == 0) p.sumsq_out[(long long)r * n_tiles + tile] = sq;
-        }
+        for (int i = lane; i < p.sumsq_parts; i += 32) sq += p.sumsq[(long long)r * p.sumsq_parts + i];
+        sq = xl_warp_sum(sq);
+        if (lane == 0) row_scale[r] = 1.f / sqrtf(sq / p.K + p.eps);
       }
-      if (!whole && threadIdx.x == 0) p.counters[tile] = 0;
     }
-    item += c1 - c0;
+    if (mbar_wait(&acc_full, 0, abort_flag, p.err, ERR_SM_ACC_FULL)) {
+      tcgen05_fence_after();
+#pragma unroll 1
+      for (int t0 = 0; t0 < NTOK && t0 < p.M; t0 += 16) {
+        uint32_t r[16];
+        tmem_ld_32x32b_x16(tmem_base + ((uint32_t)(q4 * 32) << 16) + t0, r);
+        tmem_ld_wait();
+#pragma unroll
+        for (int t = 0; t < 16; ++t) red[(t0 + t) * RED_LD + row] = __uint_as_float(r[t]);
+      }
+    }
+    tcgen05_fence_before();
+  }
+  __syncthreads();
+  if (p.ksplit > 1) {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  }
+  if (warp >= 2 && !*abort_flag) {
+    // ------------------------------------------------ results ------------------------------------------------------
+    const int et = threadIdx.x - 64;
+    const bool unit = tile >= plain;  // one part of 128 channels, or PARTS parts of CH
+    const int ch = MODE == SM_SPLIT_GLU && !unit ? 128 : CH, parts = MODE == SM_SPLIT_GLU && !unit ? 1 : PARTS;
+    const int end = MODE == SM_SPLIT_GLU && !unit ? p.cols : channels, per_row = ch / 4;
+    uint32_t red_at[8];  // this CTA's and its peers' partial sums
+#pragma unroll
+    for (int k = 0; k < 8; ++k)
+      if (k < p.ksplit) asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(red_at[k]) : "r"(smem_u32(ring)), "r"(k));
+    for (int i = rank * SM_EPI + et; i < p.M * per_row; i += p.ksplit * SM_EPI) {
+      const int r = i / per_row, cc = (i - r * per_row) * 4, c = (unit ? tile - plain : tile) * ch + cc;
+      float sq = 0.f;
+      if (c < end) {
+        float v[PARTS][4];
+#pragma unroll
+        for (int q = 0; q < PARTS; ++q) {
+          float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
+          if (MODE != SM_SPLIT_GLU || q < parts) {
+            const uint32_t off = (uint32_t)(r * RED_LD + q * CH + cc) * 4;
+            float4 part[8];
+#pragma unroll
+            for (int k = 0; k < 8; ++k)
+              if (k < p.ksplit) part[k] = ld_cluster_v4(red_at[k] + off);
+            t = part[0];
+#pragma unroll
+            for (int k = 1; k < 8; ++k)
+              if (k < p.ksplit) { t.x += part[k].x; t.y += part[k].y; t.z += part[k].z; t.w += part[k].w; }
+          }
+          v[q][0] = t.x; v[q][1] = t.y; v[q][2] = t.z; v[q][3] = t.w;
+          if ((MODE == SM_STORE || MODE == SM_SPLIT_GLU) && p.sumsq) {
+#pragma unroll
+            for (int e = 0; e < 4; ++e) v[q][e] *= row_scale[r];
+          }
+        }
+        sq = sm_epilogue<MODE>(p, r, c, v, end, unit);
+      }
+      if (MODE == SM_RESIDUAL && p.sumsq_out) {
+        // a half-warp holds 64 columns of one row, the warp two such blocks; all lanes are here
+#pragma unroll
+        for (int o = 8; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
+        if ((lane & 15) == 0 && c < end) p.sumsq_out[(long long)r * ((p.N + 63) / 64) + c / 64] = sq;
+      }
+    }
+  }
+  __syncwarp();
+  if (p.ksplit > 1) {  // the peers may still read this CTA's sums
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  }
+  if (warp == 1) {
+    tcgen05_fence_after();
+    tmem_dealloc(tmem_base, R::TMEM_COLS);
   }
 }
 
-template <int MODE> int sm_launch(const SmParams& p, int sms, int max_tiles, cudaStream_t s) {
+template <int MODE, int NTOK> int sm_launch_tokens(SmParams p, int sms, cudaStream_t s) {
   using L = SmTile<MODE>;
+  using R = SmRing<NTOK>;
   const int paired = MODE == SM_SPLIT_GLU ? p.N - p.cols : p.N;
   if (paired % L::PARTS) return -1;
-  const int plain = MODE == SM_SPLIT_GLU ? (p.cols + L::COLS - 1) / L::COLS : 0;
+  const int plain = MODE == SM_SPLIT_GLU ? (p.cols + 127) / 128 : 0;
   const int channels = paired / L::PARTS, chunks = (p.K + SM_KC - 1) / SM_KC, n_tiles = plain + (channels + L::CH - 1) / L::CH;
-  if (n_tiles > max_tiles) return -1;
   static bool configured = false;
   if (!configured) {
     const cudaError_t e =
-        cudaFuncSetAttribute(linear_small_m_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::RING_BYTES);
+        cudaFuncSetAttribute(linear_small_m_kernel<MODE, NTOK>, cudaFuncAttributeMaxDynamicSharedMemorySize, R::SMEM);
     if (e != cudaSuccess) return (int)e;
     configured = true;
   }
-  long long grid = (long long)SM_CTAS_PER_SM * sms;
-  const long long total = (long long)n_tiles * chunks;
-  if (total > (1 << 30)) return -1;
-  if (grid > total) grid = total;
-  const cudaError_t e = xl_launch_overlapped(linear_small_m_kernel<MODE>, dim3((unsigned)grid), dim3(SM_WARPS * 32),
-                                             L::RING_BYTES, s, p);
+  // A power of two that two CTAs per SM have room for, at most eight. Room for one CTA per SM only was slower (16 tokens, 4096 x
+  // 11008: 20.6 us with 4 CTAs per cluster, 18.0 with 8; 12288 x 4096: 22.5 with 1, 19.6 with 2), and so were clusters of 6 and 3
+  // (6144 x 4096: 15.9 us with 6, 11.9 with 4; 12288 x 4096: 25.3 with 3).
+  p.ksplit = 1;
+  while (p.ksplit < 8 && 2 * p.ksplit * n_tiles <= 2 * sms && 4 * p.ksplit <= chunks) p.ksplit *= 2;
+  CUtensorMap mw, ma;
+  int rc = make_map_bf16(&mw, p.w, p.N, p.K, p.K, L::CH);
+  if (rc == 0) rc = make_map_bf16(&ma, p.a, p.M, p.K, p.lda, NTOK);
+  if (rc) return rc == -2 ? (int)cudaErrorNotSupported : (int)cudaErrorInvalidValue;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(n_tiles * p.ksplit));
+  cfg.blockDim = dim3(SM_THREADS);
+  cfg.dynamicSmemBytes = R::SMEM;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = (unsigned)p.ksplit;
+  attr[1].val.clusterDim.y = 1;
+  attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 2;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, linear_small_m_kernel<MODE, NTOK>, mw, ma, p);
   return e != cudaSuccess ? (int)e : (int)cudaGetLastError();
 }
+template <int MODE> int sm_launch(const SmParams& p, int sms, cudaStream_t s) {
+  if (MODE == SM_STORE && p.M > 16) {
+    if (p.M <= 32) return sm_launch_tokens<SM_STORE, 32>(p, sms, s);
+    if (p.M <= 64) return sm_launch_tokens<SM_STORE, 64>(p, sms, s);
+    return sm_launch_tokens<SM_STORE, 128>(p, sms, s);
+  }
+  return sm_launch_tokens<MODE, 16>(p, sms, s);
+}
 
-int sm_check(const void* a, long long lda, const void* w, int M, int N, int K, const float* slots, const unsigned int* counters) {
-  if (M < 1 || M > 16 || N < 1 || K < 8 || (K % 8) || (lda % 8) || lda < K) return -1;
-  if (((uintptr_t)a & 15) || ((uintptr_t)w & 15) || !slots || !counters) return -1;
+int sm_check(const void* a, long long lda, const void* w, int M, int N, int K, int max_m = 16) {
+  if (M < 1 || M > max_m || N < 1 || K < 8 || (K % 8) || (lda % 8) || lda < K) return -1;
+  if (((uintptr_t)a & 15) || ((uintptr_t)w & 15)) return -1;
   return 0;
 }
 
 }  // namespace
 
-// Floats of `slots` for a device with `sms` SMs; `counters` needs `max_tiles` zero-initialised words (left zeroed).
-XL_API int xl_linear_small_m_slots(int sms) { return SM_CTAS_PER_SM * sms * 2 * 16 * 64; }
-
-// All: a (M, K) bf16 with row stride lda (a multiple of 8), w (N, K) bf16 contiguous, M <= 16, K a multiple of 8; returns -1
+// All: a (M, K) bf16 with row stride lda (a multiple of 8), w (N, K) bf16 contiguous, M <= 16 (xl_linear_small_m: 128), K a multiple of 8; returns -1
 // for arguments the kernel does not take. y (M, N) with row stride ldy, bf16 or fp32. sumsq (M, sumsq_parts), or null: the rows
 // of y are multiplied by 1 / sqrt(sum of the row's sumsq / K + eps).
 XL_API int xl_linear_small_m(const void* a, long long lda, const void* w, void* y, long long ldy, int y_f32, const float* sumsq,
-                             int sumsq_parts, float eps, int M, int N, int K, float* slots, unsigned int* counters, int max_tiles,
-                             int sms, cudaStream_t s) {
-  if (sm_check(a, lda, w, M, N, K, slots, counters) || !y || (sumsq && sumsq_parts < 1)) return -1;
+                             int sumsq_parts, float eps, int M, int N, int K, int sms, int* err, cudaStream_t s) {
+  if (sm_check(a, lda, w, M, N, K, 128) || !y || (sumsq && sumsq_parts < 1)) return -1;
   SmParams p = {};
   p.a = (const __nv_bfloat16*)a; p.lda = lda; p.w = (const __nv_bfloat16*)w; p.M = M; p.N = N; p.K = K;
   p.y = y; p.ldy = ldy; p.y_f32 = y_f32; p.sumsq = sumsq; p.sumsq_parts = sumsq_parts; p.eps = eps;
-  p.slots = slots; p.counters = counters;
-  return sm_launch<SM_STORE>(p, sms, max_tiles, s);
+  p.err = err;
+  return sm_launch<SM_STORE>(p, sms, s);
 }
 
 // w rows [cols plain | F gate | F up], N = cols + 2F: y (M, cols) with row stride ldy and z (M, F) with row stride ldz, bf16;
 // sumsq as in xl_linear_small_m.
 XL_API int xl_linear_small_m_split_glu(const void* a, long long lda, const void* w, void* y, long long ldy, int cols, void* z,
                                        long long ldz, float limit, float slope, float shift, const float* sumsq, int sumsq_parts,
-                                       float eps, int M, int N, int K, float* slots, unsigned int* counters, int max_tiles,
-                                       int sms, cudaStream_t s) {
-  if (sm_check(a, lda, w, M, N, K, slots, counters) || cols < 0 || cols > N || (cols && !y) || (cols < N && !z) ||
+                                       float eps, int M, int N, int K, int sms, int* err, cudaStream_t s) {
+  if (sm_check(a, lda, w, M, N, K) || cols < 0 || cols > N || (cols && !y) || (cols < N && !z) ||
       (sumsq && sumsq_parts < 1))
     return -1;
   SmParams p = {};
   p.a = (const __nv_bfloat16*)a; p.lda = lda; p.w = (const __nv_bfloat16*)w; p.M = M; p.N = N; p.K = K;
   p.y = y; p.ldy = ldy; p.cols = cols; p.z = (__nv_bfloat16*)z; p.ldz = ldz; p.limit = limit; p.slope = slope; p.shift = shift;
-  p.sumsq = sumsq; p.sumsq_parts = sumsq_parts; p.eps = eps; p.slots = slots; p.counters = counters;
-  return sm_launch<SM_SPLIT_GLU>(p, sms, max_tiles, s);
+  p.sumsq = sumsq; p.sumsq_parts = sumsq_parts; p.eps = eps; p.err = err;
+  return sm_launch<SM_SPLIT_GLU>(p, sms, s);
 }
 
 // x (M, N) fp32 += mult * a w^T; with nw, h (M, N) bf16 = x * nw and sumsq (M, ceil(N / 64)) = sums of x^2 over 64 columns.
 XL_API int xl_linear_small_m_residual_rms(const void* a, long long lda, const void* w, float* x, float mult, const float* nw,
-                                          void* h, float* sumsq, int M, int N, int K, float* slots, unsigned int* counters,
-                                          int max_tiles, int sms, cudaStream_t s) {
-  if (sm_check(a, lda, w, M, N, K, slots, counters) || !x || (nw && (!h || !sumsq))) return -1;
+                                          void* h, float* sumsq, int M, int N, int K, int sms, int* err, cudaStream_t s) {
+  if (sm_check(a, lda, w, M, N, K) || !x || (nw && (!h || !sumsq))) return -1;
   SmParams p = {};
   p.a = (const __nv_bfloat16*)a; p.lda = lda; p.w = (const __nv_bfloat16*)w; p.M = M; p.N = N; p.K = K;
   p.x = x; p.mult = mult; p.nw = nw; p.h = (__nv_bfloat16*)h; p.sumsq_out = nw ? sumsq : nullptr;
-  p.slots = slots; p.counters = counters;
-  return sm_launch<SM_RESIDUAL>(p, sms, max_tiles, s);
+  p.err = err;
+  return sm_launch<SM_RESIDUAL>(p, sms, s);
 }
 
 // x (M, N) fp32 += mult * a w^T (+ table[tokens]); with alpha, h (M, N) bf16 = tanh(alpha x) nw + nb.
 XL_API int xl_linear_small_m_residual(const void* a, long long lda, const void* w, float* x, float mult, const int* tokens,
                                       const void* table, int vocab, const float* alpha, const float* nw, const float* nb,
-                                      void* h, int M, int N, int K, float* slots, unsigned int* counters, int max_tiles, int sms,
-                                      cudaStream_t s) {
-  if (sm_check(a, lda, w, M, N, K, slots, counters) || !x || (table && (!tokens || vocab < 1)) || (alpha && (!nw || !nb || !h)))
+                                      void* h, int M, int N, int K, int sms, int* err, cudaStream_t s) {
+  if (sm_check(a, lda, w, M, N, K) || !x || (table && (!tokens || vocab < 1)) || (alpha && (!nw || !nb || !h)))
     return -1;
   SmParams p = {};
   p.a = (const __nv_bfloat16*)a; p.lda = lda; p.w = (const __nv_bfloat16*)w; p.M = M; p.N = N; p.K = K;
   p.x = x; p.mult = mult; p.tokens = tokens; p.table = (const __nv_bfloat16*)table; p.vocab = vocab;
-  p.alpha = alpha; p.nw = nw; p.nb = nb; p.h = (__nv_bfloat16*)h; p.slots = slots; p.counters = counters;
-  return sm_launch<SM_RESIDUAL>(p, sms, max_tiles, s);
+  p.alpha = alpha; p.nw = nw; p.nb = nb; p.h = (__nv_bfloat16*)h; p.err = err;
+  return sm_launch<SM_RESIDUAL>(p, sms, s);
 }
 
 // w rows [gate | up] (2F, K); y (M, F) bf16 contiguous.
-XL_API int xl_linear_small_m_swiglu(const void* a, long long lda, const void* w, void* y, int M, int F, int K, float* slots,
-                                    unsigned int* counters, int max_tiles, int sms, cudaStream_t s) {
-  if (sm_check(a, lda, w, M, 2 * F, K, slots, counters) || !y) return -1;
+XL_API int xl_linear_small_m_swiglu(const void* a, long long lda, const void* w, void* y, int M, int F, int K, int sms, int* err, cudaStream_t s) {
+  if (sm_check(a, lda, w, M, 2 * F, K) || !y) return -1;
   SmParams p = {};
   p.a = (const __nv_bfloat16*)a; p.lda = lda; p.w = (const __nv_bfloat16*)w; p.M = M; p.N = 2 * F; p.K = K;
-  p.y = y; p.ldy = F; p.slots = slots; p.counters = counters;
-  return sm_launch<SM_SWIGLU>(p, sms, max_tiles, s);
+  p.y = y; p.ldy = F; p.err = err;
+  return sm_launch<SM_SWIGLU>(p, sms, s);
 }
 
 // w rows [z | u | g] (3W, K); row r is the next token of sequence r: state (M, W) fp32 advances where count[r] > 0 and starts
 // from zero at pos[r] == 0; y (M, W) bf16 contiguous.
 XL_API int xl_linear_small_m_min_gru(const void* a, long long lda, const void* w, const float* bz, const float* bu, float* state,
-                                     const int* pos, const int* count, void* y, int M, int W, int K, float* slots,
-                                     unsigned int* counters, int max_tiles, int sms, cudaStream_t s) {
-  if (sm_check(a, lda, w, M, 3 * W, K, slots, counters) || !y || !state || !bz || !bu || !pos || !count) return -1;
+                                     const int* pos, const int* count, void* y, int M, int W, int K, int sms, int* err, cudaStream_t s) {
+  if (sm_check(a, lda, w, M, 3 * W, K) || !y || !state || !bz || !bu || !pos || !count) return -1;
   SmParams p = {};
   p.a = (const __nv_bfloat16*)a; p.lda = lda; p.w = (const __nv_bfloat16*)w; p.M = M; p.N = 3 * W; p.K = K;
-  p.y = y; p.ldy = W; p.bz = bz; p.bu = bu; p.state = state; p.pos = pos; p.count = count; p.slots = slots; p.counters = counters;
-  return sm_launch<SM_MINGRU>(p, sms, max_tiles, s);
+  p.y = y; p.ldy = W; p.bz = bz; p.bu = bu; p.state = state; p.pos = pos; p.count = count; p.err = err;
+  return sm_launch<SM_MINGRU>(p, sms, s);
 }

@@ -213,6 +213,9 @@ def check_gemm_errors():
                      13: "attention: key / value stage was never released", 14: "attention: scores never completed",
                      15: "attention: score buffer was never drained", 16: "attention: probabilities never arrived",
                      17: "attention: output accumulation never completed",
+                     31: "few-rows linear: operand tiles never arrived (TMA)",
+                     32: "few-rows linear: shared-memory stage was never released",
+                     33: "few-rows linear: accumulator never completed",
                      21: "CTA-pair GEMM: operand tiles never arrived (TMA)",
                      22: "CTA-pair GEMM: shared-memory stage was never released",
                      23: "CTA-pair GEMM: accumulator never completed",

@@ -33,8 +33,7 @@ _window_tcgen05 = _sig("xl_window_attn_tcgen05", *_WINDOW_ARGS, _c_p, _c_p)
 _window_decode = _sig("xl_window_attn_decode", _c_p, _c_ll, _c_p, _c_p, _c_p, _c_p, _c_p, _c_ll, _c_p, _c_p, _c_int, _c_int, _c_int,
                       _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_f, _c_f, _c_f, _c_int, _c_p, _c_p, _c_p)
 _linear_f32 = _sig("xl_linear_f32", _c_p, _c_ll, _c_p, _c_p, _c_ll, _c_int, _c_int, _c_int, _c_p)
-_small_m_slots = _sig("xl_linear_small_m_slots", _c_int)
-_SMALL_TAIL = (_c_int, _c_int, _c_int, _c_p, _c_p, _c_int, _c_int, _c_p)
+_SMALL_TAIL = (_c_int, _c_int, _c_int, _c_int, _c_p, _c_p)
 _SUMSQ = (_c_p, _c_int, _c_f)  # sums of squares of a deferred norm, parts per row, eps
 _small_store = _sig("xl_linear_small_m", _c_p, _c_ll, _c_p, _c_p, _c_ll, _c_int, *_SUMSQ, *_SMALL_TAIL)
 _small_split_glu = _sig("xl_linear_small_m_split_glu", _c_p, _c_ll, _c_p, _c_p, _c_ll, _c_int, _c_p, _c_ll, _c_f, _c_f, _c_f, *_SUMSQ,
@@ -45,30 +44,26 @@ _small_residual = _sig("xl_linear_small_m_residual", _c_p, _c_ll, _c_p, _c_p, _c
 _small_swiglu = _sig("xl_linear_small_m_swiglu", _c_p, _c_ll, _c_p, _c_p, *_SMALL_TAIL)
 _small_min_gru = _sig("xl_linear_small_m_min_gru", _c_p, _c_ll, _c_p, _c_p, _c_p, _c_p, _c_p, _c_p, _c_p, *_SMALL_TAIL)
 
-_MAX_TILES = 1 << 14  # column tiles the split-K counters of the small-M kernel cover
 _SCRATCH = {}
 
 
-def _scratch(device):
-    """Per-device scratch of the decoding kernels: partial sums, and counters that every launch leaves at zero. Allocated
-    once at its final size, since captured graphs keep the addresses."""
+def _counters(device):
+    """Counters of the decoding attention kernels, which every launch leaves at zero. Allocated once at their final size, since
+    captured graphs keep the address."""
     idx = device.index or 0
     if idx not in _SCRATCH:
-        _SCRATCH[idx] = (torch.empty(_small_m_slots(_sms(device)), dtype=torch.float32, device=device),
-                         torch.zeros(_MAX_TILES, dtype=torch.int32, device=device),
-                         torch.zeros(1 << 16, dtype=torch.int32, device=device))
+        _SCRATCH[idx] = torch.zeros(1 << 16, dtype=torch.int32, device=device)
     return _SCRATCH[idx]
 
 
-def _small(a, weight) -> bool:
+def _small(a, weight, rows=16) -> bool:
     """Whether the small-M kernels take this product."""
-    return (a.dtype == torch.bfloat16 and weight.dtype == torch.bfloat16 and a.shape[0] <= 16 and a.is_cuda
+    return (a.dtype == torch.bfloat16 and weight.dtype == torch.bfloat16 and a.shape[0] <= rows and a.is_cuda
             and a.stride(1) == 1 and weight.is_contiguous() and a.shape[1] % 8 == 0)
 
 
 def _small_tail(a, rows, weight):
-    slots, counters, _ = _scratch(a.device)
-    return (a.shape[0], rows, weight.shape[1], slots.data_ptr(), counters.data_ptr(), _MAX_TILES, _sms(a.device), _stream())
+    return a.shape[0], rows, weight.shape[1], _sms(a.device), gemm_error_flag(a.device).data_ptr(), _stream()
 
 
 def _small_ok(rc, name) -> bool:
@@ -101,7 +96,9 @@ def product(a, weight, out_dtype=None, sumsq=None, eps=0.0):
     NotImplemented)."""
     out_dtype = out_dtype or a.dtype
     if a.dtype != torch.float32:
-        if _small(a, weight) and out_dtype in (torch.bfloat16, torch.float32):
+        # Up to 128 rows the product is bound by reading the weights. The GEMM multiplies tiles of 256 rows and does not
+        # split K: a weight of 2048 x 7680 keeps 16 of 74 CTA pairs busy (40 rows: 30.5 us, 11.1 here).
+        if _small(a, weight, 128) and out_dtype in (torch.bfloat16, torch.float32):
             y = torch.empty((a.shape[0], weight.shape[0]), dtype=out_dtype, device=a.device)
             if _small_ok(_small_store(a.data_ptr(), a.stride(0), weight.data_ptr(), y.data_ptr(), y.stride(0),
                                       int(out_dtype == torch.float32), *_sumsq_args(sumsq, eps),
@@ -240,7 +237,7 @@ def diff_attention_cuda(qkv, cos, sin, kc, vc, pos, count, lam, T, heads, rotary
         units = B * G * ((heads // G + 7) // 8)
         longest = min(smax, chunk) if chunk else smax
         splits = max(1, min(2 * _sms(qkv.device) // units, (longest + 63) // 64, 64))  # one wave, two CTAs per SM
-        counters = _scratch(qkv.device)[2]
+        counters = _counters(qkv.device)
         part = torch.empty(units * splits * 16 * (vdim + 2), dtype=torch.float32, device=qkv.device) if splits > 1 else None
         if units <= counters.numel():
             rc = _diff_decode(qkv.data_ptr(), qkv.stride(0), _ptr(cos), _ptr(sin), kc.data_ptr(), vc.data_ptr(), out.data_ptr(),
@@ -362,7 +359,7 @@ def window_attention_cuda(proj, q_norm, k_norm, kc, vc, pos, count, joint, T, he
         longest = min(smax, window + keep_first) if window else smax
         # one wave, two CTAs per SM; a slice of fewer keys costs more in the merge than it saves
         splits = max(1, min(2 * _sms(proj.device) // units, (longest + 383) // 384, 64))
-        counters = _scratch(proj.device)[2]
+        counters = _counters(proj.device)
         part = torch.empty(units * splits * 16 * (vdim + 2), dtype=torch.float32, device=proj.device) if splits > 1 else None
         if units <= counters.numel():
             rc = _window_decode(proj.data_ptr(), ld, q_norm.data_ptr(), k_norm.data_ptr(), kc.data_ptr(), vc.data_ptr(),

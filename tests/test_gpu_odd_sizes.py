@@ -214,3 +214,24 @@ def test_general_attention_of_few_rows_equals_that_of_many(nat, kind, T, dim, vd
         out.append(y.view(n, T, H * vdim))
     assert out[1].abs().max() > 0
     assert (out[0] - out[1]).abs().max() <= 1e-5 * out[1].abs().max()
+
+
+@pytest.mark.parametrize("out", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("rows,N,K", [(17, 128, 64), (32, 129, 72), (33, 2048, 7680), (64, 300, 4096), (65, 40, 8), (128, 1000, 520),
+                                      (40, 32000, 2048)])
+def test_few_rows_product_at_the_edges_of_its_tiles(nat, out, rows, N, K):
+    """Each token tile, ragged weight rows and K, tiles that many CTAs share; twice, since the second launch finds the counters
+    as the first one left them. The activations are a slice of a wider matrix."""
+    from popxl_addons_b200.ops.native_sequence import product
+
+    g = torch.Generator(device="cuda").manual_seed(rows * N + K)
+    a = torch.randn(rows, K + 8, generator=g, device="cuda").bfloat16()[:, :K]
+    w = torch.randn(N, K, generator=g, device="cuda").bfloat16()
+    want = a.double() @ w.double().t()
+    before = nat.LAUNCHES["by_kernel"].get("linear_small_m", 0)
+    first = product(a, w, out)
+    y = product(a, w, out)
+    assert nat.LAUNCHES["by_kernel"]["linear_small_m"] == before + 2
+    assert y.dtype == out and torch.equal(first, y)
+    _near(y, want, out, terms=K)
+    nat.check_gemm_errors()
