@@ -170,6 +170,12 @@ template <> __device__ __forceinline__ float2 xl_pair_to_float2<__nv_bfloat16>(u
 __device__ __forceinline__ void xl_grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void xl_grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
+// returns from a launcher whose launch failed
+#define XL_TRY(call)                          \
+  do {                                        \
+    const cudaError_t xl_e = (call);          \
+    if (xl_e != cudaSuccess) return (int)xl_e; \
+  } while (0)
 template <typename... P, typename... A>
 static inline cudaError_t xl_launch_overlapped(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A... args) {
   cudaLaunchConfig_t cfg = {};

@@ -54,6 +54,18 @@ template <typename T> __device__ __forceinline__ void mma_m16n8k16(float (&c)[4]
   }
 }
 
+// the first product of a sum: no accumulator registers to clear
+template <typename T> __device__ __forceinline__ void mma_m16n8k16_first(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  if constexpr (std::is_same<T, __nv_bfloat16>::value) {
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+        : "=f"(c[0]), "=f"(c[1]), "=f"(c[2]), "=f"(c[3])
+        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.f));
+  } else {
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+        : "=f"(c[0]), "=f"(c[1]), "=f"(c[2]), "=f"(c[3])
+        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.f));
+  }
+}
 template <typename T> struct GqFmt;
 template <> struct GqFmt<__nv_bfloat16> {
   static constexpr uint32_t MASK = 0x000F000Fu, MAGIC = 0x43004300u, ONES = 0x3F803F80u;
@@ -63,19 +75,24 @@ template <> struct GqFmt<__half> {
   static constexpr uint32_t MASK = 0x00F000F0u, MAGIC = 0x54005400u, ONES = 0x3C003C00u;
   static constexpr float BASE = 64.f;
 };
+// (w & MASK) | MAGIC in one instruction
+template <typename T> __device__ __forceinline__ uint32_t gq_place(uint32_t w) {
+  uint32_t o;
+  asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(o) : "r"(w), "r"(GqFmt<T>::MASK), "r"(GqFmt<T>::MAGIC));
+  return o;
+}
 // w: eight codes, two packed words (the first code of a word in its top nibble). out[i]: codes i and i + 4.
 template <typename T> __device__ __forceinline__ void gq_codes8(uint32_t w, uint32_t (&out)[4]) {
-  using F = GqFmt<T>;
   if constexpr (std::is_same<T, __nv_bfloat16>::value) {
-    out[0] = ((w >> 12) & F::MASK) | F::MAGIC;
-    out[1] = ((w >> 8) & F::MASK) | F::MAGIC;
-    out[2] = ((w >> 4) & F::MASK) | F::MAGIC;
-    out[3] = (w & F::MASK) | F::MAGIC;
+    out[0] = gq_place<T>(w >> 12);
+    out[1] = gq_place<T>(w >> 8);
+    out[2] = gq_place<T>(w >> 4);
+    out[3] = gq_place<T>(w);
   } else {
-    out[0] = ((w >> 8) & F::MASK) | F::MAGIC;
-    out[1] = ((w >> 4) & F::MASK) | F::MAGIC;
-    out[2] = (w & F::MASK) | F::MAGIC;
-    out[3] = ((w << 4) & F::MASK) | F::MAGIC;
+    out[0] = gq_place<T>(w >> 8);
+    out[1] = gq_place<T>(w >> 4);
+    out[2] = gq_place<T>(w);
+    out[3] = gq_place<T>(w << 4);
   }
 }
 
@@ -127,8 +144,13 @@ __global__ void __launch_bounds__(GqCfg<NT, WPB>::WARPS * 32, 1) gq_gemm_small_m
   const bool pairs16 = p.sz_pairs && p.N % 4 == 0;  // scales and zero points can be copied 16 bytes at a time
   const T* x = (const T*)p.x;
 
-  // The chunks of this warp over the whole range, tile after tile.
+  // The chunks of this warp over the whole range, tile after tile. What a request needs of a tile is worked out once per tile: this
+  // lane's first row of codes, which of its rows exist, and its first unit of scales and zero points.
   struct Cursor { int item, c1, ch, tile; };  // first item of the current tile segment, its end chunk, current chunk, tile
+  const int bpg = p.group_size / SB;          // blocks per group
+  const long long row_step = 8LL * (p.K / 4);
+  const int sz_b = lane / (COLS / 4), sz_n = (lane % (COLS / 4)) * 4;  // unit `lane`; unit 32 i + lane lies i * SZ_STEP blocks on
+  constexpr int SZ_STEP = 32 / (COLS / 4);
   auto segment = [&](Cursor& c) {
     while (c.item < item_end) {
       c.tile = c.item / chunks;
@@ -139,32 +161,42 @@ __global__ void __launch_bounds__(GqCfg<NT, WPB>::WARPS * 32, 1) gq_gemm_small_m
       c.item += c.c1 - c0;
     }
   };
-  auto advance = [&](Cursor& c) {
-    if (c.item >= item_end) return;
+  auto advance = [&](Cursor& c) -> bool {  // whether the tile changed
+    if (c.item >= item_end) return false;
     c.ch += WARPS;
-    if (c.ch >= c.c1) {
-      c.item = c.tile * chunks + c.c1;
-      segment(c);
-    }
+    if (c.ch < c.c1) return false;
+    c.item = c.tile * chunks + c.c1;
+    segment(c);
+    return true;
+  };
+  const uint16_t* row0 = p.packed;  // of the tile that is requested next
+  int rows_on = 0;                  // its rows 8 i + g below N
+  auto enter = [&](const Cursor& c) {
+    if (c.item >= item_end) return;
+    const int n = c.tile * COLS + g;
+    row0 = p.packed + (long long)n * (p.K / 4) + j * 8;
+    rows_on = (p.N - n + 7) / 8;
   };
   // Codes of a tile of 16 channels: piece q (32 codes) of row r at unit q * 16 + (r ^ 4 * (q & 1)), so that the eight-byte reads
   // below touch every bank once.
+  uint4* const code_dst = ring + j * 16 + (g ^ ((j & 1) * 4));
   auto request = [&](const Cursor& c, int buf) {
     if (c.item < item_end) {
-      uint4* dst = ring + buf * C::STAGE_UNITS;
+      uint4* dst = code_dst + buf * C::STAGE_UNITS;
+      const uint16_t* src = row0 + c.ch * (GQ_KCHUNK / 4);
 #pragma unroll
       for (int i = 0; i < CT * 2; ++i) {
-        const int row = i * 8 + g, n = c.tile * COLS + row, r = row & 15;
-        const bool on = n < p.N;
-        const uint16_t* src = p.packed + (long long)(on ? n : 0) * (p.K / 4) + c.ch * (GQ_KCHUNK / 4) + j * 8;
-        xl_cp_async16(dst + (row >> 4) * 64 + j * 16 + (r ^ ((j & 1) * 4)), src, on);
+        const bool on = i < rows_on;
+        xl_cp_async16(dst + (i >> 1) * 64 + (i & 1) * 8, on ? src : p.packed, on);
+        src += row_step;
       }
-      uint4* sz = dst + C::CODE_UNITS;
+      uint4* sz = ring + buf * C::STAGE_UNITS + C::CODE_UNITS;
+      const int n = c.tile * COLS + sz_n;
 #pragma unroll
       for (int i = 0; i < (C::SZ_UNITS + 31) / 32; ++i) {
-        const int u = i * 32 + lane, b = u / (COLS / 4), n = c.tile * COLS + (u % (COLS / 4)) * 4;
-        const int grp = (c.ch * GQ_KCHUNK + b * SB) / p.group_size;
-        if (u < C::SZ_UNITS) {
+        const int u = i * 32 + lane, block = c.ch * BLOCKS + sz_b + i * SZ_STEP;
+        const int grp = bpg == 1 ? block : block / bpg;
+        if (C::SZ_UNITS % 32 == 0 || u < C::SZ_UNITS) {
           if (pairs16) {
             const bool on = n < p.N;
             xl_cp_async16(sz + u, (const uint32_t*)p.scale + (on ? (long long)grp * p.N + n : 0), on);
@@ -202,10 +234,11 @@ __global__ void __launch_bounds__(GqCfg<NT, WPB>::WARPS * 32, 1) gq_gemm_small_m
   Cursor ahead{item, 0, 0, 0};
   segment(ahead);
   Cursor cur = ahead;
+  enter(ahead);
   request(ahead, 0);
-  advance(ahead);
+  if (advance(ahead)) enter(ahead);
   request(ahead, 1);
-  advance(ahead);
+  if (advance(ahead)) enter(ahead);
   xl_grid_dependency_wait();  // the first weights are on their way; everything else may come from the previous kernel
   xl_grid_launch_dependents();
   uint4 xn[NT][WPB];
@@ -248,10 +281,9 @@ __global__ void __launch_bounds__(GqCfg<NT, WPB>::WARPS * 32, 1) gq_gemm_small_m
         for (int t = 0; t < NT; ++t) {
           const uint32_t ones[4] = {F::ONES, F::ONES, F::ONES, F::ONES};
 #pragma unroll
-          for (int e = 0; e < 4; ++e) xs[t][e] = 0.f;
-#pragma unroll
           for (int q = 0; q < WPB; ++q) {
-            mma_m16n8k16<T>(xs[t], ones, xb[t][q][0], xb[t][q][1]);
+            if (q == 0) mma_m16n8k16_first<T>(xs[t], ones, xb[t][q][0], xb[t][q][1]);
+            else mma_m16n8k16<T>(xs[t], ones, xb[t][q][0], xb[t][q][1]);
             mma_m16n8k16<T>(xs[t], ones, xb[t][q][2], xb[t][q][3]);
           }
         }
@@ -271,10 +303,6 @@ __global__ void __launch_bounds__(GqCfg<NT, WPB>::WARPS * 32, 1) gq_gemm_small_m
           const uint32_t sz_lo = sz[b * COLS + i * 16 + g], sz_hi = sz[b * COLS + i * 16 + g + 8];
           float part[NT][4];
 #pragma unroll
-          for (int t = 0; t < NT; ++t)
-#pragma unroll
-            for (int e = 0; e < 4; ++e) part[t][e] = 0.f;
-#pragma unroll
           for (int q = 0; q < WPB; ++q) {
             uint32_t cl[4], chh[4];
             gq_codes8<T>(lo[q], cl);
@@ -282,7 +310,8 @@ __global__ void __launch_bounds__(GqCfg<NT, WPB>::WARPS * 32, 1) gq_gemm_small_m
             const uint32_t a0[4] = {cl[0], chh[0], cl[1], chh[1]}, a1[4] = {cl[2], chh[2], cl[3], chh[3]};
 #pragma unroll
             for (int t = 0; t < NT; ++t) {
-              mma_m16n8k16<T>(part[t], a0, xb[t][q][0], xb[t][q][1]);
+              if (q == 0) mma_m16n8k16_first<T>(part[t], a0, xb[t][q][0], xb[t][q][1]);
+              else mma_m16n8k16<T>(part[t], a0, xb[t][q][0], xb[t][q][1]);
               mma_m16n8k16<T>(part[t], a1, xb[t][q][2], xb[t][q][3]);
             }
           }
@@ -290,16 +319,16 @@ __global__ void __launch_bounds__(GqCfg<NT, WPB>::WARPS * 32, 1) gq_gemm_small_m
           const float zl = fmaf(-F::BASE, wl.x, wl.y), zh = fmaf(-F::BASE, wh.x, wh.y);
 #pragma unroll
           for (int t = 0; t < NT; ++t) {
-            acc[i][t][0] += wl.x * part[t][0] + zl * xs[t][0];
-            acc[i][t][1] += wl.x * part[t][1] + zl * xs[t][1];
-            acc[i][t][2] += wh.x * part[t][2] + zh * xs[t][0];
-            acc[i][t][3] += wh.x * part[t][3] + zh * xs[t][1];
+            acc[i][t][0] = fmaf(wl.x, part[t][0], fmaf(zl, xs[t][0], acc[i][t][0]));
+            acc[i][t][1] = fmaf(wl.x, part[t][1], fmaf(zl, xs[t][1], acc[i][t][1]));
+            acc[i][t][2] = fmaf(wh.x, part[t][2], fmaf(zh, xs[t][0], acc[i][t][2]));
+            acc[i][t][3] = fmaf(wh.x, part[t][3], fmaf(zh, xs[t][1], acc[i][t][3]));
           }
         }
       }
       __syncwarp();  // all lanes have read this stage
       request(ahead, buf);
-      advance(ahead);
+      if (advance(ahead)) enter(ahead);
       cur = next;
       buf ^= 1;
     }
@@ -429,9 +458,10 @@ XL_API int xl_gq_gemm_small_m(const void* x, const void* packed, const void* sca
 // ------------------------------------------------------------------------------------------------------------------
 template <typename T>
 __global__ void __launch_bounds__(256)
-    rotary_append_kernel(T* __restrict__ qkv, long long ld, const T* __restrict__ sin_t, const T* __restrict__ cos_t,
-                         T* __restrict__ k_cache, T* __restrict__ v_cache, const int* __restrict__ pos_ptr, int B, int H,
-                         int D, int R, int Smax) {
+    rotary_append_kernel(T* qkv, long long ld, const T* __restrict__ sin_t, const T* __restrict__ cos_t, T* k_cache, T* v_cache,
+                         const int* pos_ptr, int B, int H, int D, int R, int Smax) {
+  xl_grid_dependency_wait();
+  xl_grid_launch_dependents();
   const int pos = *pos_ptr;
   if (pos < 0 || pos >= Smax) return;
   const int hd = H * D, half = D / 2;
@@ -470,8 +500,9 @@ XL_API int xl_rotary_append(void* qkv, long long ld, const void* sin_t, const vo
   const long long total = (long long)B * H * (D / 2);
   const int grid = xl_grid_for(total, 256);
   XL_DISPATCH_DTYPE(dtype, T, {
-    rotary_append_kernel<T><<<grid, 256, 0, s>>>((T*)qkv, ld, (const T*)sin_t, (const T*)cos_t, (T*)k_cache, (T*)v_cache,
-                                                 pos_ptr, B, H, D, R, Smax);
+    const cudaError_t e = xl_launch_overlapped(rotary_append_kernel<T>, dim3(grid), dim3(256), (size_t)0, s, (T*)qkv, ld, (const T*)sin_t,
+                                               (const T*)cos_t, (T*)k_cache, (T*)v_cache, pos_ptr, B, H, D, R, Smax);
+    if (e != cudaSuccess) return (int)e;
   });
   return (int)cudaGetLastError();
 }
@@ -494,17 +525,33 @@ struct alignas(VPL * 2 >= 16 ? 16 : (VPL == 4 ? 8 : (VPL == 2 ? 4 : 2))) AdVec {
 
 template <typename T, int VPL>
 __global__ void __launch_bounds__(AD_WARPS * 32)
-    attn_decode_kernel(const T* __restrict__ qkv, long long ldq, const T* __restrict__ k_cache,
-                       const T* __restrict__ v_cache, T* __restrict__ out, long long ldo, float* __restrict__ part,
-                       unsigned int* __restrict__ counters, const int* __restrict__ pos_ptr, int H, int Smax, float scale) {
+    attn_decode_kernel(const T* qkv, long long ldq, const T* k_cache, const T* v_cache, T* out, long long ldo, float* part,
+                       unsigned int* counters, const int* pos_ptr, int H, int Smax, float scale) {
   constexpr int D = VPL * 32;
   using Vec = AdVec<T, VPL>;
+  xl_grid_dependency_wait();
+  xl_grid_launch_dependents();
   const int bh = blockIdx.x, split = blockIdx.y, splits = gridDim.y;
   const int b = bh / H, h = bh % H;
   const int len = min(*pos_ptr + 1, Smax);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int per = (len + splits - 1) / splits;
   const int s_begin = split * per, s_end = min(len, s_begin + per);
+  const T* kb = k_cache + ((long long)bh * Smax) * D + lane * VPL;
+  const T* vb = v_cache + ((long long)bh * Smax) * D + lane * VPL;
+  // The next group of positions is requested before this one is used: with the loads of one group at a time, 5 warps per scheduler
+  // hid about half of their latency.
+  Vec kk[AD_UNROLL], vv[AD_UNROLL], kn[AD_UNROLL], vn[AD_UNROLL];
+  auto request = [&](int s0) {
+#pragma unroll
+    for (int u = 0; u < AD_UNROLL; ++u) {
+      const int sidx = min(s0 + u, s_end - 1);  // clamped: the duplicates are masked out below
+      kn[u] = *reinterpret_cast<const Vec*>(kb + (long long)sidx * D);
+      vn[u] = *reinterpret_cast<const Vec*>(vb + (long long)sidx * D);
+    }
+  };
+  int s0 = s_begin + warp * AD_UNROLL;
+  if (s0 < s_end) request(s0);
   float q[VPL], o[VPL];
   {
     const Vec qv = *reinterpret_cast<const Vec*>(qkv + (long long)b * ldq + h * D + lane * VPL);
@@ -515,16 +562,10 @@ __global__ void __launch_bounds__(AD_WARPS * 32)
     }
   }
   float m = -INFINITY, l = 0.f;
-  const T* kb = k_cache + ((long long)bh * Smax) * D + lane * VPL;
-  const T* vb = v_cache + ((long long)bh * Smax) * D + lane * VPL;
-  for (int s0 = s_begin + warp * AD_UNROLL; s0 < s_end; s0 += AD_WARPS * AD_UNROLL) {
-    Vec kk[AD_UNROLL], vv[AD_UNROLL];
+  for (; s0 < s_end; s0 += AD_WARPS * AD_UNROLL) {
 #pragma unroll
-    for (int u = 0; u < AD_UNROLL; ++u) {
-      const int sidx = min(s0 + u, s_end - 1);  // clamped: the duplicates are masked out below
-      kk[u] = *reinterpret_cast<const Vec*>(kb + (long long)sidx * D);
-      vv[u] = *reinterpret_cast<const Vec*>(vb + (long long)sidx * D);
-    }
+    for (int u = 0; u < AD_UNROLL; ++u) { kk[u] = kn[u]; vv[u] = vn[u]; }
+    if (s0 + AD_WARPS * AD_UNROLL < s_end) request(s0 + AD_WARPS * AD_UNROLL);
     float dot[AD_UNROLL];
 #pragma unroll
     for (int u = 0; u < AD_UNROLL; ++u) {
@@ -533,14 +574,17 @@ __global__ void __launch_bounds__(AD_WARPS * 32)
       for (int e = 0; e < VPL; ++e) d += q[e] * xl_to_float(kk[u].v[e]);
       dot[u] = d;
     }
+    // four sums over 32 lanes by halving: lanes with bits 16 and 8 (a, b) end up with the sum of dot[2 a + b]
+    const bool hi16 = lane & 16, hi8 = lane & 8;
+    float d0 = (hi16 ? dot[2] : dot[0]) + __shfl_xor_sync(0xffffffffu, hi16 ? dot[0] : dot[2], 16);
+    float d1 = (hi16 ? dot[3] : dot[1]) + __shfl_xor_sync(0xffffffffu, hi16 ? dot[1] : dot[3], 16);
+    d0 = (hi8 ? d1 : d0) + __shfl_xor_sync(0xffffffffu, hi8 ? d0 : d1, 8);
 #pragma unroll
-    for (int off = 16; off > 0; off >>= 1) {
-#pragma unroll
-      for (int u = 0; u < AD_UNROLL; ++u) dot[u] += __shfl_xor_sync(0xffffffffu, dot[u], off);
-    }
+    for (int off = 4; off > 0; off >>= 1) d0 += __shfl_xor_sync(0xffffffffu, d0, off);
     float m_new = m;
 #pragma unroll
     for (int u = 0; u < AD_UNROLL; ++u) {
+      dot[u] = __shfl_sync(0xffffffffu, d0, u * 8);
       if (s0 + u >= s_end) dot[u] = -INFINITY;
       m_new = fmaxf(m_new, dot[u]);
     }
@@ -626,8 +670,12 @@ XL_API int xl_attn_decode(const void* qkv, long long ldq, const void* k_cache, c
   if (splits > 1 && (scratch == nullptr || counters == nullptr)) return -1;
   dim3 grid(B * H, splits);
 #define XL_AD_LAUNCH(T, VPL)                                                                                          \
-  attn_decode_kernel<T, VPL><<<grid, AD_WARPS * 32, 0, s>>>((const T*)qkv, ldq, (const T*)k_cache, (const T*)v_cache, \
-                                                            (T*)out, ldo, scratch, counters, pos_ptr, H, Smax, scale)
+  do {                                                                                                                \
+    const cudaError_t e = xl_launch_overlapped(attn_decode_kernel<T, VPL>, grid, dim3(AD_WARPS * 32), (size_t)0, s,   \
+                                               (const T*)qkv, ldq, (const T*)k_cache, (const T*)v_cache, (T*)out, ldo, scratch, \
+                                               counters, pos_ptr, H, Smax, scale);                                    \
+    if (e != cudaSuccess) return (int)e;                                                                              \
+  } while (0)
   if (dtype == XL_BF16) {
     if (D == 256) XL_AD_LAUNCH(__nv_bfloat16, 8);
     else if (D == 128) XL_AD_LAUNCH(__nv_bfloat16, 4);
@@ -669,8 +717,10 @@ template <typename T, int N> __device__ __forceinline__ void xl_store_vec(T* __r
 // ------------------------------------------------------------------------------------------------------------------
 template <typename T>
 __global__ void __launch_bounds__(256)
-    add_layer_norm_kernel(T* __restrict__ x, const T* __restrict__ delta, const T* __restrict__ bias,
-                          const T* __restrict__ w, const T* __restrict__ b, T* __restrict__ h, int cols, float eps) {
+    add_layer_norm_kernel(T* x, const T* delta, const T* __restrict__ bias, const T* __restrict__ w, const T* __restrict__ b, T* h, int cols,
+                          float eps) {
+  xl_grid_dependency_wait();
+  xl_grid_launch_dependents();
   constexpr int MAX_VEC = 4;  // vectors of 8 elements per thread: cols <= 256 * 8 * 4
   const int row = blockIdx.x;
   T* xr = x + (long long)row * cols;
@@ -753,8 +803,9 @@ XL_API int xl_add_layer_norm(void* x, const void* delta, const void* bias, const
                              int rows, int cols, float eps, int dtype, cudaStream_t s) {
   if (cols > 256 * 32 || (cols % 8) || rows < 1 || w == nullptr || b == nullptr) return -1;
   XL_DISPATCH_DTYPE(dtype, T, {
-    add_layer_norm_kernel<T><<<rows, 256, 0, s>>>((T*)x, (const T*)delta, (const T*)bias, (const T*)w, (const T*)b, (T*)h,
-                                                 cols, eps);
+    const cudaError_t e = xl_launch_overlapped(add_layer_norm_kernel<T>, dim3(rows), dim3(256), (size_t)0, s, (T*)x, (const T*)delta,
+                                               (const T*)bias, (const T*)w, (const T*)b, (T*)h, cols, eps);
+    if (e != cudaSuccess) return (int)e;
   });
   return (int)cudaGetLastError();
 }
@@ -821,7 +872,11 @@ __global__ void __launch_bounds__(256)
     idx_out[row] = best.i + index_offset;
   }
 }
-__global__ void advance_position_kernel(int* pos) { *pos += 1; }
+__global__ void advance_position_kernel(int* pos) {
+  xl_grid_dependency_wait();
+  xl_grid_launch_dependents();
+  *pos += 1;
+}
 
 XL_API int xl_argmax_rows(const void* logits, float* max_out, int* idx_out, long long rows, int V, int valid,
                           int index_offset, int dtype, cudaStream_t s) {
@@ -853,18 +908,22 @@ XL_API int xl_argmax_rows(const void* logits, float* max_out, int* idx_out, long
   return (int)cudaGetLastError();
 }
 XL_API int xl_advance_position(int* pos, cudaStream_t s) {
-  advance_position_kernel<<<1, 1, 0, s>>>(pos);
+  const cudaError_t e = xl_launch_overlapped(advance_position_kernel, dim3(1), dim3(1), (size_t)0, s, pos);
+  if (e != cudaSuccess) return (int)e;
   return (int)cudaGetLastError();
 }
 
 // buf: (rows, B) int32; writes vals (B) into row (*pos_ptr - base).
-__global__ void store_row_kernel(int* __restrict__ buf, const int* __restrict__ pos_ptr, int base, const int* __restrict__ vals,
+__global__ void store_row_kernel(int* buf, const int* pos_ptr, int base, const int* vals,
                                  int B, int rows) {
+  xl_grid_dependency_wait();
+  xl_grid_launch_dependents();
   const int r = *pos_ptr - base;
   if (r < 0 || r >= rows) return;
   for (int i = threadIdx.x; i < B; i += blockDim.x) buf[(long long)r * B + i] = vals[i];
 }
 XL_API int xl_store_row(int* buf, const int* pos_ptr, int base, const int* vals, int B, int rows, cudaStream_t s) {
-  store_row_kernel<<<1, 128, 0, s>>>(buf, pos_ptr, base, vals, B, rows);
+  const cudaError_t e = xl_launch_overlapped(store_row_kernel, dim3(1), dim3(128), (size_t)0, s, buf, pos_ptr, base, vals, B, rows);
+  if (e != cudaSuccess) return (int)e;
   return (int)cudaGetLastError();
 }

@@ -172,15 +172,22 @@ XL_API int xl_dense_csr_matmul(const void* x, int dtype, const int* indptr, cons
 // ------------------------------------------------------------------------------------------------------------------
 template <typename T>
 __global__ void __launch_bounds__(256)
-    gather_rows_kernel(const T* __restrict__ table, const int* __restrict__ idx, T* __restrict__ out, long long n_idx,
-                       int rows, int cols) {
+    gather_rows_kernel(const T* __restrict__ table, const int* idx, T* __restrict__ out, long long n_idx, int rows, int cols) {
+  xl_grid_dependency_wait();
+  xl_grid_launch_dependents();
   const long long i = blockIdx.x;
   if (i >= n_idx) return;
   const int r = idx[i];
   const bool ok = r >= 0 && r < rows;
   const T* src = table + (long long)(ok ? r : 0) * cols;
   T* dst = out + i * cols;
-  for (int c = threadIdx.x; c < cols; c += blockDim.x) dst[c] = ok ? src[c] : xl_from_float<T>(0.f);
+  constexpr int V = 16 / sizeof(T);
+  if (cols % V == 0 && ((((uintptr_t)table) | ((uintptr_t)out)) & 15) == 0) {
+    for (int c = threadIdx.x * V; c < cols; c += blockDim.x * V)
+      *reinterpret_cast<uint4*>(dst + c) = ok ? *reinterpret_cast<const uint4*>(src + c) : make_uint4(0, 0, 0, 0);
+  } else {
+    for (int c = threadIdx.x; c < cols; c += blockDim.x) dst[c] = ok ? src[c] : xl_from_float<T>(0.f);
+  }
 }
 
 template <typename T, typename G>
@@ -200,7 +207,9 @@ XL_API int xl_gather_rows(const void* table, int dtype, const int* idx, void* ou
                           cudaStream_t s) {
   if (n_idx < 1) return 0;
   XL_DISPATCH_DTYPE(dtype, T, {
-    gather_rows_kernel<T><<<(unsigned)n_idx, 256, 0, s>>>((const T*)table, idx, (T*)out, n_idx, rows, cols);
+    const cudaError_t e = xl_launch_overlapped(gather_rows_kernel<T>, dim3((unsigned)n_idx), dim3(256), (size_t)0, s, (const T*)table, idx,
+                                               (T*)out, n_idx, rows, cols);
+    if (e != cudaSuccess) return (int)e;
   });
   return (int)cudaGetLastError();
 }

@@ -52,8 +52,10 @@ __device__ __forceinline__ void dyt_pack(const float (&x)[V], float alpha, const
 // the table row (embedding).
 template <typename T, int V>
 __global__ void __launch_bounds__(256)
-    stream_dyt_kernel(float* __restrict__ x, const T* __restrict__ y, float mult, const int* __restrict__ tokens,
-                      const T* __restrict__ table, int vocab, DytParams n, T* __restrict__ h, long long rows, int cols) {
+    stream_dyt_kernel(float* x, const T* y, float mult, const int* tokens, const T* __restrict__ table, int vocab, DytParams n, T* h,
+                      long long rows, int cols) {
+  xl_grid_dependency_wait();
+  xl_grid_launch_dependents();
   const float alpha = n.alpha ? *n.alpha : 0.f;
   const int per_row = cols / V;
   const long long total = rows * per_row;
@@ -91,8 +93,9 @@ __global__ void __launch_bounds__(256)
 // h[r] = DyT(x[r * stride + idx[r] - offset])
 template <typename T>
 __global__ void __launch_bounds__(256)
-    select_dyt_kernel(const float* __restrict__ x, const int* __restrict__ idx, int stride, int offset, long long x_rows,
-                      DytParams n, T* __restrict__ h, int cols) {
+    select_dyt_kernel(const float* x, const int* idx, int stride, int offset, long long x_rows, DytParams n, T* h, int cols) {
+  xl_grid_dependency_wait();
+  xl_grid_launch_dependents();
   const float alpha = *n.alpha;
   const long long r = blockIdx.x;
   long long src = r * stride + idx[r] - offset;
@@ -108,9 +111,11 @@ constexpr int RMS_THREADS = 256;
 // NP packs of V columns per thread stay in registers; the columns of longer rows are read again.
 template <typename T, int V, int NP>
 __global__ void __launch_bounds__(RMS_THREADS)
-    stream_rms_kernel(float* __restrict__ x, const T* __restrict__ y, float mult, const int* __restrict__ tokens,
-                      const T* __restrict__ table, int vocab, const float* __restrict__ w, float eps, T* __restrict__ h, int cols) {
+    stream_rms_kernel(float* x, const T* y, float mult, const int* tokens, const T* __restrict__ table, int vocab,
+                      const float* __restrict__ w, float eps, T* h, int cols) {
   __shared__ float red[32];
+  xl_grid_dependency_wait();
+  xl_grid_launch_dependents();
   const long long row = blockIdx.x;
   float* xr = x + row * cols;
   const T* src = y ? y + row * cols : table + (long long)min(max(tokens[row], 0), vocab - 1) * cols;
@@ -169,9 +174,11 @@ __global__ void __launch_bounds__(RMS_THREADS)
 // h[r] = RMS norm of x[r * stride + idx[r] - offset]
 template <typename T>
 __global__ void __launch_bounds__(RMS_THREADS)
-    select_rms_kernel(const float* __restrict__ x, const int* __restrict__ idx, int stride, int offset, long long x_rows,
-                      const float* __restrict__ w, float eps, T* __restrict__ h, int cols) {
+    select_rms_kernel(const float* x, const int* idx, int stride, int offset, long long x_rows, const float* __restrict__ w, float eps,
+                      T* h, int cols) {
   __shared__ float red[32];
+  xl_grid_dependency_wait();
+  xl_grid_launch_dependents();
   const long long r = blockIdx.x;
   long long src = r * stride + idx[r] - offset;
   src = src < 0 ? 0 : (src >= x_rows ? x_rows - 1 : src);
@@ -185,8 +192,9 @@ __global__ void __launch_bounds__(RMS_THREADS)
 // gate: columns [0, F) of rows of stride ldg, up: the F columns after them; y: F columns of rows of stride ldy.
 template <typename T, int V>
 __global__ void __launch_bounds__(256)
-    clamped_glu_kernel(const T* __restrict__ gate, long long ldg, T* __restrict__ y, long long ldy, long long rows, int F,
-                       float limit, float slope, float shift) {
+    clamped_glu_kernel(const T* gate, long long ldg, T* y, long long ldy, long long rows, int F, float limit, float slope, float shift) {
+  xl_grid_dependency_wait();
+  xl_grid_launch_dependents();
   const int per_row = F / V;
   const long long total = rows * per_row;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
@@ -202,7 +210,9 @@ __global__ void __launch_bounds__(256)
 }
 
 template <typename T, int V>
-__global__ void __launch_bounds__(256) swiglu_packed_kernel(const T* __restrict__ gu, T* __restrict__ y, long long rows, int F) {
+__global__ void __launch_bounds__(256) swiglu_packed_kernel(const T* gu, T* y, long long rows, int F) {
+  xl_grid_dependency_wait();
+  xl_grid_launch_dependents();
   const int per_row = F / V;
   const long long total = rows * per_row;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
@@ -218,6 +228,8 @@ __global__ void __launch_bounds__(256) swiglu_packed_kernel(const T* __restrict_
 }
 
 __global__ void advance_by_kernel(int* pos, const int* count, int n) {
+  xl_grid_dependency_wait();
+  xl_grid_launch_dependents();
   for (int i = threadIdx.x; i < n; i += blockDim.x) pos[i] += count[i];
 }
 
@@ -354,11 +366,11 @@ template <typename T>
 int launch_stream(float* x, const void* y, float mult, const int* tokens, const void* table, int vocab, DytParams n, void* h,
                   long long rows, int cols, cudaStream_t s) {
   if (cols % 4 == 0) {
-    stream_dyt_kernel<T, 4><<<xl_grid_for(rows * (cols / 4), 256), 256, 0, s>>>(x, (const T*)y, mult, tokens, (const T*)table,
-                                                                               vocab, n, (T*)h, rows, cols);
+    XL_TRY(xl_launch_overlapped(stream_dyt_kernel<T, 4>, dim3(xl_grid_for(rows * (cols / 4), 256)), dim3(256), (size_t)0, s, x, (const T*)y, mult, tokens, (const T*)table,
+                                                                               vocab, n, (T*)h, rows, cols));
   } else {
-    stream_dyt_kernel<T, 1><<<xl_grid_for(rows * cols, 256), 256, 0, s>>>(x, (const T*)y, mult, tokens, (const T*)table, vocab,
-                                                                         n, (T*)h, rows, cols);
+    XL_TRY(xl_launch_overlapped(stream_dyt_kernel<T, 1>, dim3(xl_grid_for(rows * cols, 256)), dim3(256), (size_t)0, s, x, (const T*)y, mult, tokens, (const T*)table, vocab,
+                                                                         n, (T*)h, rows, cols));
   }
   return (int)cudaGetLastError();
 }
@@ -369,8 +381,8 @@ int launch_rms(float* x, const void* y, float mult, const int* tokens, const voi
   const int packs = (cols + V - 1) / V;
   const int threads = packs >= RMS_THREADS ? RMS_THREADS : (packs + 31) / 32 * 32;
 #define XL_RMS(NP)                                                                                                         \
-  stream_rms_kernel<T, V, NP><<<(unsigned)rows, threads, 0, s>>>(x, (const T*)y, mult, tokens, (const T*)table, vocab, w,    \
-                                                                 eps, (T*)h, cols)
+  XL_TRY(xl_launch_overlapped(stream_rms_kernel<T, V, NP>, dim3((unsigned)rows), dim3(threads), (size_t)0, s, x, (const T*)y, mult, tokens, (const T*)table, vocab, w,    \
+                                                                 eps, (T*)h, cols))
   if (packs <= RMS_THREADS) XL_RMS(1);
   else if (packs <= 4 * RMS_THREADS) XL_RMS(4);
   else XL_RMS(8);
@@ -396,7 +408,7 @@ XL_API int xl_select_rms(const float* x, const int* idx, int stride, int offset,
                          void* h, int rows, int cols, int dtype, cudaStream_t s) {
   if (rows < 1 || cols < 1 || x_rows < 1 || !w) return -1;
   XL_DISPATCH_DTYPE(dtype, T, {
-    select_rms_kernel<T><<<rows, RMS_THREADS, 0, s>>>(x, idx, stride, offset, x_rows, w, eps, (T*)h, cols);
+    XL_TRY(xl_launch_overlapped(select_rms_kernel<T>, dim3(rows), dim3(RMS_THREADS), (size_t)0, s, x, idx, stride, offset, x_rows, w, eps, (T*)h, cols));
   });
   return (int)cudaGetLastError();
 }
@@ -408,11 +420,11 @@ XL_API int xl_clamped_glu(const void* gate, long long ldg, void* y, long long ld
   XL_DISPATCH_DTYPE(dtype, T, {
     constexpr int V = 16 / sizeof(T);
     if (F % V == 0 && ldg % V == 0 && ldy % V == 0 && (((uintptr_t)gate | (uintptr_t)y) & 15) == 0)
-      clamped_glu_kernel<T, V><<<xl_grid_for(rows * (F / V), 256), 256, 0, s>>>((const T*)gate, ldg, (T*)y, ldy, rows, F, limit,
-                                                                               slope, shift);
+      XL_TRY(xl_launch_overlapped(clamped_glu_kernel<T, V>, dim3(xl_grid_for(rows * (F / V), 256)), dim3(256), (size_t)0, s, (const T*)gate, ldg, (T*)y, ldy, rows, F, limit,
+                                                                               slope, shift));
     else
-      clamped_glu_kernel<T, 1><<<xl_grid_for(rows * F, 256), 256, 0, s>>>((const T*)gate, ldg, (T*)y, ldy, rows, F, limit,
-                                                                         slope, shift);
+      XL_TRY(xl_launch_overlapped(clamped_glu_kernel<T, 1>, dim3(xl_grid_for(rows * F, 256)), dim3(256), (size_t)0, s, (const T*)gate, ldg, (T*)y, ldy, rows, F, limit,
+                                                                         slope, shift));
   });
   return (int)cudaGetLastError();
 }
@@ -433,7 +445,7 @@ XL_API int xl_select_dyt(const float* x, const int* idx, int stride, int offset,
   if (rows < 1 || cols < 1 || x_rows < 1 || !alpha || !w || !b) return -1;
   const DytParams n{alpha, w, b};
   XL_DISPATCH_DTYPE(dtype, T, {
-    select_dyt_kernel<T><<<rows, 256, 0, s>>>(x, idx, stride, offset, x_rows, n, (T*)h, cols);
+    XL_TRY(xl_launch_overlapped(select_dyt_kernel<T>, dim3(rows), dim3(256), (size_t)0, s, x, idx, stride, offset, x_rows, n, (T*)h, cols));
   });
   return (int)cudaGetLastError();
 }
@@ -444,15 +456,15 @@ XL_API int xl_swiglu_packed(const void* gu, void* y, long long rows, int F, int 
   XL_DISPATCH_DTYPE(dtype, T, {
     constexpr int V = 16 / sizeof(T);
     if (F % V == 0)
-      swiglu_packed_kernel<T, V><<<xl_grid_for(rows * (F / V), 256), 256, 0, s>>>((const T*)gu, (T*)y, rows, F);
+      XL_TRY(xl_launch_overlapped(swiglu_packed_kernel<T, V>, dim3(xl_grid_for(rows * (F / V), 256)), dim3(256), (size_t)0, s, (const T*)gu, (T*)y, rows, F));
     else
-      swiglu_packed_kernel<T, 1><<<xl_grid_for(rows * F, 256), 256, 0, s>>>((const T*)gu, (T*)y, rows, F);
+      XL_TRY(xl_launch_overlapped(swiglu_packed_kernel<T, 1>, dim3(xl_grid_for(rows * F, 256)), dim3(256), (size_t)0, s, (const T*)gu, (T*)y, rows, F));
   });
   return (int)cudaGetLastError();
 }
 
 XL_API int xl_advance_by(int* pos, const int* count, int n, cudaStream_t s) {
-  advance_by_kernel<<<1, 128, 0, s>>>(pos, count, n);
+  XL_TRY(xl_launch_overlapped(advance_by_kernel, dim3(1), dim3(128), (size_t)0, s, pos, count, n));
   return (int)cudaGetLastError();
 }
 
