@@ -508,6 +508,32 @@ XL_API int xl_rotary_append(void* qkv, long long ld, const void* sin_t, const vo
 }
 
 // ------------------------------------------------------------------------------------------------------------------
+// Keys and values of whole prompts into the caches: rows (b, s) of qkv hold [q | k | v], each heads x D; caches (B, H, Smax, D). Bound by
+// HBM: 16-byte pieces, read in the order of the rows. (Two strided copies of 8192 x 4096 took 79 us each, both 40 us this way.)
+// ------------------------------------------------------------------------------------------------------------------
+__global__ void __launch_bounds__(256)
+    kv_fill_kernel(const uint4* __restrict__ qkv, uint32_t ld, uint4* __restrict__ k_cache, uint4* __restrict__ v_cache, uint32_t total,
+                   uint32_t S, uint32_t H, uint32_t D, uint32_t Smax) {  // ld, D: in 16-byte pieces
+  const uint32_t hd = H * D;
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
+    const uint32_t row = i / (2 * hd), c = i - row * 2 * hd;  // c: piece of [k | v]
+    const uint32_t b = row / S, pos = row - b * S, f = c < hd ? c : c - hd, h = f / D;
+    const uint4 v = qkv[(long long)row * ld + hd + c];
+    (c < hd ? k_cache : v_cache)[(((long long)b * H + h) * Smax + pos) * D + (f - h * D)] = v;
+  }
+}
+XL_API int xl_kv_fill(const void* qkv, long long ld, void* k_cache, void* v_cache, int B, int S, int H, int D, int Smax, int dtype,
+                      cudaStream_t s) {
+  const int n = dtype == XL_F32 ? 4 : 8;  // values per piece
+  const long long total = (long long)B * S * 2 * H * D / n;
+  if (B < 1 || S < 1 || S > Smax || H < 1 || D < n || D % n || ld % n || total > 0x7fffffffLL || ld / n > 0x7fffffffLL) return -1;
+  if ((((uintptr_t)qkv) | ((uintptr_t)k_cache) | ((uintptr_t)v_cache)) & 15) return -1;
+  kv_fill_kernel<<<xl_grid_for(total, 256 * 4), 256, 0, s>>>((const uint4*)qkv, (uint32_t)(ld / n), (uint4*)k_cache, (uint4*)v_cache,
+                                                            (uint32_t)total, (uint32_t)S, (uint32_t)H, (uint32_t)(D / n), (uint32_t)Smax);
+  return (int)cudaGetLastError();
+}
+
+// ------------------------------------------------------------------------------------------------------------------
 // Decode attention: one query per (b, h) against cache positions [0, len), len = *pos_ptr + 1, one launch.
 // Grid (B*H, splits): each CTA covers a slice of the positions with an online softmax. A warp takes four positions per
 // iteration (lanes over the head dimension, one vector load of D/32 values per lane, position and tensor), so eight

@@ -94,6 +94,7 @@ _gemm_ar_pull = _sig("xl_gemm_tcgen05_ar_pull", _c_p, _c_p, _c_p, _c_p, _c_p, _c
                      _c_int, _c_int, _c_ll, _c_ll, _c_ll, _c_ll, _c_ll, _c_int, _c_int, _c_f, _c_p, _c_int, _c_p, _c_int,
                      _c_int, _c_p, _c_p, _c_int, _c_int, _c_p, _c_p)
 _symm_all_gather_mc = _sig("xl_symm_all_gather_mc", _c_p, _c_p, _c_ll, _c_p, _c_p, _c_int, _c_int, _c_int, _c_p, _c_p)
+_kv_fill = _sig("xl_kv_fill", _c_p, _c_ll, _c_p, _c_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_p)
 _gq_small_slots = _sig("xl_gq_gemm_small_m_slots", _c_int)
 _gq_small = _sig("xl_gq_gemm_small_m", _c_p, _c_p, _c_p, _c_p, _c_p, _c_p, _c_int, _c_int, _c_int, _c_int, _c_ll, _c_ll,
                  _c_int, _c_int, _c_p, _c_p, _c_int, _c_int, _c_int, _c_p)
@@ -1204,6 +1205,21 @@ def advance_position_cuda(pos):
     _check(_advance(pos.data_ptr(), _stream()), "advance_position")
     _count("advance_position")
     return pos
+
+
+@native("kv_cache_fill_")
+def kv_cache_fill_cuda(qkv, kc, vc, seq_len, n_heads, head_dim):
+    if not _ok(qkv, kc, vc) or not (qkv.dtype == kc.dtype == vc.dtype) or qkv.dim() != 2 or kc.shape != vc.shape:
+        return NotImplemented
+    B, H, smax, D = kc.shape
+    if (H, D) != (n_heads, head_dim) or qkv.shape[0] != B * seq_len or qkv.shape[1] < 3 * H * D:
+        return NotImplemented
+    rc = _kv_fill(qkv.data_ptr(), qkv.stride(0), kc.data_ptr(), vc.data_ptr(), B, seq_len, H, D, smax, _CODE[qkv.dtype], _stream())
+    if rc == -1:
+        return NotImplemented
+    _check(rc, "kv_fill")
+    _count("kv_fill")
+    return kc
 
 
 @native("store_row_")

@@ -235,3 +235,43 @@ def test_few_rows_product_at_the_edges_of_its_tiles(nat, out, rows, N, K):
     assert y.dtype == out and torch.equal(first, y)
     _near(y, want, out, terms=K)
     nat.check_gemm_errors()
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("B,S,H,D,smax", [(1, 1, 1, 8, 1), (2, 5, 3, 16, 9), (3, 67, 4, 256, 70), (2, 3, 2, 12, 4)])
+def test_prompt_into_the_caches(nat, dtype, B, S, H, D, smax):
+    """Every element moved, none besides; 12 bf16 features are refused (the plain copies take them)."""
+    from popxl_addons_b200.xl.opdef import OPS
+
+    qkv = torch.randn(B * S, 3 * H * D, generator=torch.Generator().manual_seed(D)).to(dtype)
+    got = [torch.full((B, H, smax, D), 7.0, dtype=dtype, device="cuda") for _ in range(2)]
+    want = [g.cpu().clone() for g in got]
+    res = nat.kv_cache_fill_cuda(qkv.cuda(), *got, seq_len=S, n_heads=H, head_dim=D)
+    assert (res is NotImplemented) == (D * dtype.itemsize % 16 != 0)
+    if res is not NotImplemented:
+        OPS["kv_cache_fill_"].impl(qkv, *want, seq_len=S, n_heads=H, head_dim=D)
+        assert all(torch.equal(g.cpu(), w) for g, w in zip(got, want))
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("B,H,S,D,R,packed", [(2, 3, 5, 16, 8, True), (1, 2, 67, 128, 128, True), (2, 2, 9, 20, 12, True),
+                                              (2, 3, 7, 24, 6, False), (1, 4, 33, 64, 16, False)])
+@pytest.mark.parametrize("inplace", [False, True])
+def test_rotary_in_pieces_and_in_pairs(nat, dtype, B, H, S, D, R, packed, inplace):
+    """Vectors of pairs (sizes and strides that allow them) and single pairs, per-batch tables, both directions, against 64 bits: one
+    rounding of the result."""
+    g = torch.Generator().manual_seed(D + S)
+    if packed:  # the query part of packed (tokens, 3 * H * D) rows
+        x = torch.randn(B * S, 3 * H * D, generator=g).to(dtype).cuda()[:, :H * D].view(B, S, H, D).permute(0, 2, 1, 3)
+    else:
+        x = torch.randn(B, H, S, D, generator=g).to(dtype).cuda()
+    angle = torch.rand(B, S, R // 2, generator=g) * 6
+    sin, cos = angle.sin().to(dtype).cuda(), angle.cos().to(dtype).cuda()
+    for inverse in (False, True):
+        want = x.double().clone()
+        sn, cs = sin.double()[:, None] * (-1 if inverse else 1), cos.double()[:, None]
+        a, b = want[..., 0:R:2].clone(), want[..., 1:R:2].clone()
+        want[..., 0:R:2], want[..., 1:R:2] = a * cs - b * sn, b * cs + a * sn
+        y = x if inplace else torch.empty_like(x)
+        nat.rotary_launch(x, sin, cos, y, R, inverse)
+        _near(y, want, dtype)
