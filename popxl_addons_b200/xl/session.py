@@ -359,7 +359,9 @@ class Session:
     # ------------------------------------------------------------------------------------------------------
     # host IO
     # ------------------------------------------------------------------------------------------------------
-    def _stage_inputs(self, inputs: Mapping[HostToDeviceStream, Any]):
+    def _stage_inputs(self, inputs: Mapping[HostToDeviceStream, Any], keep_on_host: bool = False):
+        """Inputs of a run, by stream: on the session's device, or with `keep_on_host` in pinned memory (a replayed program
+        copies them straight into the buffers it was captured with)."""
         T = int(self.ir.num_host_transfers)
         R = self.num_replicas
         self._inputs, self._cursor = {}, {}
@@ -387,7 +389,7 @@ class Session:
             if self.device.type == "cuda" and host.device.type == "cpu":
                 if not host.is_pinned():
                     host = host.contiguous().pin_memory()
-                dev = host.to(self.device, non_blocking=True)
+                dev = host if keep_on_host else host.to(self.device, non_blocking=True)
             else:
                 dev = host  # already resident on the session's device
             self._inputs[stream] = dev
@@ -416,7 +418,10 @@ class Session:
         T = int(self.ir.num_host_transfers)
         res = {}
         for stream, items in self._outputs.items():
-            stacked = torch.stack([torch.stack(per_replica) for per_replica in items])  # (t, R_local, *shape)
+            if len(items) == 1 and len(items[0]) == 1:
+                stacked = items[0][0][None, None]
+            else:
+                stacked = torch.stack([torch.stack(per_replica) for per_replica in items])  # (t, R_local, *shape)
             if not fetch:
                 res[stream] = stacked
                 continue
@@ -938,9 +943,9 @@ class Session:
         return {"graph": g, "static_in": static_in, "outputs": outs_rec, "kernels": kernels, "carried": carried,
                 "ptrs": tuple(v[0].data_ptr() for v in vals[n_out:])}
 
-    def _after_replay(self, state):
+    def _after_replay(self, state, copy: bool = True):
         for stream, tensors in state["outputs"]:
-            self._outputs.setdefault(stream, []).append([t.clone() for t in tensors])
+            self._outputs.setdefault(stream, []).append([t.clone() for t in tensors] if copy else list(tensors))
 
     def run(self, inputs: Optional[Mapping[HostToDeviceStream, Any]] = None,
             downcast_inputs: bool = True, fetch: bool = True) -> Dict[DeviceToHostStream, np.ndarray]:
@@ -970,19 +975,21 @@ class Session:
         """Execute a `Program` once; inputs, outputs and `fetch` as in `run`. The first run is eager (lazy
         initialisation); a capturable program is captured into a CUDA graph at its second run and replayed from then on."""
         self._outputs = {}
-        self._stage_inputs(inputs or {})
+        state = self._programs.get(program)
+        capturable = (program.capture and self.device.type == "cuda" and self.num_local == 1 and self.profile is None
+                      and self.ir.options.cuda_graphs)
+        replayed = state is not None and capturable
+        self._stage_inputs(inputs or {}, keep_on_host=replayed)
         with torch.no_grad():
-            state = self._programs.get(program)
-            capturable = (program.capture and self.device.type == "cuda" and self.num_local == 1 and self.profile is None
-                          and self.ir.options.cuda_graphs)
-            if state is not None and capturable:
+            if replayed:
                 from ..ops import native as _native
 
                 for stream, static in state["static_in"].items():
                     static.copy_(self._next_host_item(stream), non_blocking=True)
                 state["graph"].replay()
                 _native.count_replay(state["kernels"])
-                self._after_replay(state)
+                # outputs that are read before anything else can replay the program need no copy of their own
+                self._after_replay(state, copy=not fetch)
             else:
                 vals = [self._value(t, {}) for t in program.bindings.values()]
                 if capturable and program in self._programs and self._capture_safe(program.graph):
