@@ -239,6 +239,7 @@ struct DecodeParams {
   float* part;             // [B * G * head chunks][splits][16][vdim + 2]
   unsigned int* counters;  // [B * G * head chunks], zero between launches
   int stages;
+  int read_ahead;  // positions, counts and the cached keys and values were complete before the previous launch
 };
 
 // bytes of one ring stage of one warp: 16 keys x 2 maps x KD pieces of 64 B, then 16 value rows of vdim + 8 elements
@@ -257,6 +258,7 @@ __global__ void __launch_bounds__(DD_WARPS * 32) diff_attn_decode_kernel(const D
   const int split = blockIdx.x, splits = gridDim.x, g = blockIdx.y / hchunks, b = blockIdx.z;
   const int h0 = g * per_g + (blockIdx.y % hchunks) * DD_HEADS;  // first query head of this CTA
   const int nh = min(DD_HEADS, (g + 1) * per_g - h0);
+  if (!p.read_ahead) xl_grid_dependency_wait();
   const int pos = p.pos[b];
   if (p.count[b] <= 0 || pos < 0 || pos >= p.Smax) {
     xl_grid_dependency_wait();  // no kernel of a chain ends before its predecessor
@@ -303,7 +305,7 @@ __global__ void __launch_bounds__(DD_WARPS * 32) diff_attn_decode_kernel(const D
   const bool appends = split == splits - 1;
   if (!appends)
     for (int n = 0; n < p.stages - 1; ++n) prefetch(n);
-  xl_grid_dependency_wait();  // the new projections; positions and older keys were there before the previous kernel started
+  xl_grid_dependency_wait();  // the new projections
   xl_grid_launch_dependents();
   // ---- rotated queries to shared memory; the CTAs with the last keys append the new key and value (the same data each) ----
   const int half = p.dim / 2;  // dim is even
@@ -610,7 +612,7 @@ XL_API int xl_diff_attn_general(const void* q, long long ldq, const void* kc, co
 XL_API int xl_diff_attn_decode(const void* qkv, long long ld, const float* cos_t, const float* sin_t, void* kc, void* vc,
                                void* out, long long ldo, const int* pos, const int* count, const float* lam, int B, int H, int G,
                                int dim, int vdim, int R, int Smax, int chunk, float scale, float eps, float out_scale,
-                               int splits, float* part, unsigned int* counters, cudaStream_t s) {
+                               int splits, float* part, unsigned int* counters, int read_ahead, cudaStream_t s) {
   if (B < 1 || B > 65535 || G < 1 || H % G || H > 4096 || dim < 8 || dim > 128 || dim % 8 || vdim < 8 || vdim > 256 || vdim % 8 ||
       R < 0 || R > dim || (R & 1) || Smax < 1 || chunk < 0 || splits < 1 || splits > DD_MAX_SPLITS || (ld % 8))
     return -1;
@@ -621,6 +623,7 @@ XL_API int xl_diff_attn_decode(const void* qkv, long long ld, const float* cos_t
   p.kc = (__nv_bfloat16*)kc; p.vc = (__nv_bfloat16*)vc; p.out = (__nv_bfloat16*)out; p.ldo = ldo;
   p.pos = pos; p.count = count; p.lam = lam; p.H = H; p.G = G; p.dim = dim; p.vdim = vdim; p.R = R; p.Smax = Smax;
   p.chunk = chunk; p.scale = scale; p.eps = eps; p.out_scale = out_scale; p.part = part; p.counters = counters;
+  p.read_ahead = read_ahead;
 #define XL_DD(KD)                                       \
   if (vdim <= 64) return dd_launch<KD, 8>(p, B, splits, s);   \
   if (vdim <= 128) return dd_launch<KD, 16>(p, B, splits, s); \

@@ -204,6 +204,7 @@ struct WindowDecodeParams {
   float* part;             // [B * G * head chunks][splits][heads per CTA][vdim + 2]
   unsigned int* counters;  // [B * G * head chunks], zero between launches
   int stages;
+  int read_ahead;  // positions, counts and the cached keys and values were complete before the previous launch
 };
 
 // keys per block: more of them where their rows are short, so that the work per block stays about the same
@@ -238,6 +239,7 @@ __global__ void __launch_bounds__(WD_WARPS * 32) window_attn_decode_kernel(const
   const int split = blockIdx.x, splits = gridDim.x, g = blockIdx.y / hchunks, b = blockIdx.z;
   const int h0 = g * per_g + (blockIdx.y % hchunks) * HEADS;  // first query head of this CTA
   const int nh = min(HEADS, (g + 1) * per_g - h0);
+  if (!p.read_ahead) xl_grid_dependency_wait();
   const int pos = p.pos[b];
   if (p.count[b] <= 0 || pos < 0 || pos >= p.Smax) {
     xl_grid_dependency_wait();  // no kernel of a chain ends before its predecessor
@@ -289,7 +291,7 @@ __global__ void __launch_bounds__(WD_WARPS * 32) window_attn_decode_kernel(const
     asm volatile("cp.async.commit_group;" ::: "memory");  // possibly empty: keeps the group count per block fixed
   };
   for (int n = 0; n < p.stages - 1; ++n) prefetch(n);
-  xl_grid_dependency_wait();  // the new projections; positions and older keys were there before the previous kernel started
+  xl_grid_dependency_wait();  // the new projections
   xl_grid_launch_dependents();
   // ---- normalised queries and new key to shared memory; the CTAs with the last keys append (the same data each) ---------------
   const bool appends = split == splits - 1;
@@ -625,7 +627,7 @@ XL_API int xl_window_attn_general(const void* qn, const void* kc, const void* vc
 XL_API int xl_window_attn_decode(const void* proj, long long ld, const float* wq, const float* wk, void* kc, void* vc, void* out,
                                  long long ldo, const int* pos, const int* count, int B, int H, int G, int dim, int vdim, int Smax,
                                  int window, int keep_first, int gated, float scale, float sink, float eps, int splits,
-                                 float* part, unsigned int* counters, cudaStream_t s) {
+                                 float* part, unsigned int* counters, int read_ahead, cudaStream_t s) {
   if (B < 1 || B > 65535 || G < 1 || H < 1 || H % G || H > 4096 || dim < 8 || dim > 128 || dim % 8 || vdim < 8 || vdim > 256 ||
       vdim % 8 || Smax < 1 || window < 0 || keep_first < 0 || splits < 1 || splits > WD_MAX_SPLITS || (ld % 8) || !wq || !wk ||
       ld < (long long)(H + G) * dim + (long long)G * vdim + (gated ? (long long)H * vdim : 0) || ldo < (long long)H * vdim)
@@ -637,6 +639,7 @@ XL_API int xl_window_attn_decode(const void* proj, long long ld, const float* wq
   p.kc = (__nv_bfloat16*)kc; p.vc = (__nv_bfloat16*)vc; p.out = (__nv_bfloat16*)out; p.ldo = ldo;
   p.pos = pos; p.count = count; p.H = H; p.G = G; p.dim = dim; p.vdim = vdim; p.Smax = Smax; p.window = window;
   p.keep_first = keep_first; p.gated = gated; p.scale = scale; p.sink = sink; p.eps = eps; p.part = part; p.counters = counters;
+  p.read_ahead = read_ahead;
 #define XL_WD(KD)                                             \
   if (vdim <= 64) return wd_launch<KD, 8>(p, B, splits, s);   \
   if (vdim <= 128) return wd_launch<KD, 16>(p, B, splits, s); \

@@ -39,7 +39,7 @@
 // SM): the grid is sized to the machine, not to the problem. Warps take the chunks of a tile segment in turn; weights, scales and
 // zero points reach them through per-warp double buffers filled with cp.async. A tile shared by several CTAs is finished by the one
 // that arrives last: every CTA leaves its sums in a slot of its own and the finisher adds the slots in CTA order, so results do
-// not depend on timing. A launch requests its first weights while its predecessor drains.
+// not depend on timing. A launch requests its first weights while its predecessor drains, if that does not write them.
 constexpr int GQ_KCHUNK = 128;
 
 template <typename T> __device__ __forceinline__ void mma_m16n8k16(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
@@ -108,6 +108,7 @@ struct GqParams {
   int M, N, K, group_size, act_from_col;
   float* slots;            // [grid][2][16 * COLS]
   unsigned int* counters;  // one per tile, zero between launches
+  int read_ahead;          // codes, scales and zero points were complete before the previous launch
 };
 
 // NT: tiles of 8 tokens; WPB: 32-bit words of codes per lane and block (2: blocks of 64 k values, 1: of 32)
@@ -235,6 +236,7 @@ __global__ void __launch_bounds__(GqCfg<NT, WPB>::WARPS * 32, 1) gq_gemm_small_m
   segment(ahead);
   Cursor cur = ahead;
   enter(ahead);
+  if (!p.read_ahead) xl_grid_dependency_wait();
   request(ahead, 0);
   if (advance(ahead)) enter(ahead);
   request(ahead, 1);
@@ -435,16 +437,16 @@ XL_API int xl_gq_gemm_small_m_slots(int ctas) { return ctas * 2 * 16 * 128; }
 // Requirements: M <= 16, K % 128 == 0, group_size % 32 == 0, 16-byte aligned x rows and weight rows. `ctas`: size of the grid (one
 // per SM). sz_pairs: `scale` holds (scale, zero) pairs laid out (K/gs, N, 2) and `zero` is unused. act_from_col: first column that
 // gets GELU (>= N: none). `dtype`: type of x, bias and y (fp16 or bf16); `scale_dtype`: type of the per-group scale and zero
-// point (fp16 / bf16). Returns -1 for unsupported arguments.
+// point (fp16 / bf16). read_ahead: packed, scale and zero were complete before the previous launch on the stream. Returns -1 for unsupported arguments.
 XL_API int xl_gq_gemm_small_m(const void* x, const void* packed, const void* scale, const void* zero, const void* bias,
                               void* y, int M, int N, int K, int group_size, long long ldx, long long ldy, int act_from_col,
                               int ctas, float* slots, unsigned int* counters, int dtype, int scale_dtype, int sz_pairs,
-                              cudaStream_t s) {
+                              int read_ahead, cudaStream_t s) {
   if (M < 1 || M > 16 || N < 1 || K < GQ_KCHUNK || K % GQ_KCHUNK || group_size < 32 || group_size % 32 || K % group_size ||
       dtype == XL_F32 || scale_dtype == XL_F32)
     return -1;
   if ((ldx % 8) || ctas < 1 || slots == nullptr || counters == nullptr || (((uintptr_t)x | (uintptr_t)packed | (uintptr_t)scale) & 15)) return -1;
-  const GqParams p{x, ldx, (const uint16_t*)packed, scale, zero, sz_pairs, bias, y, ldy, M, N, K, group_size, act_from_col, slots, counters};
+  const GqParams p{x, ldx, (const uint16_t*)packed, scale, zero, sz_pairs, bias, y, ldy, M, N, K, group_size, act_from_col, slots, counters, read_ahead};
   if (dtype == XL_BF16)
     return scale_dtype == XL_F16 ? gq_small_pick<__nv_bfloat16, __half>(p, ctas, s) : gq_small_pick<__nv_bfloat16, __nv_bfloat16>(p, ctas, s);
   return scale_dtype == XL_F16 ? gq_small_pick<__half, __half>(p, ctas, s) : gq_small_pick<__half, __nv_bfloat16>(p, ctas, s);
@@ -458,7 +460,7 @@ XL_API int xl_gq_gemm_small_m(const void* x, const void* packed, const void* sca
 // ------------------------------------------------------------------------------------------------------------------
 template <typename T>
 __global__ void __launch_bounds__(256)
-    rotary_append_kernel(T* qkv, long long ld, const T* __restrict__ sin_t, const T* __restrict__ cos_t, T* k_cache, T* v_cache,
+    rotary_append_kernel(T* qkv, long long ld, const T* sin_t, const T* cos_t, T* k_cache, T* v_cache,
                          const int* pos_ptr, int B, int H, int D, int R, int Smax) {
   xl_grid_dependency_wait();
   xl_grid_launch_dependents();
@@ -736,8 +738,7 @@ template <typename T, int N> __device__ __forceinline__ void xl_store_vec(T* __r
 // ------------------------------------------------------------------------------------------------------------------
 template <typename T>
 __global__ void __launch_bounds__(256)
-    add_layer_norm_kernel(T* x, const T* delta, const T* __restrict__ bias, const T* __restrict__ w, const T* __restrict__ b, T* h, int cols,
-                          float eps) {
+    add_layer_norm_kernel(T* x, const T* delta, const T* bias, const T* w, const T* b, T* h, int cols, float eps) {
   xl_grid_dependency_wait();
   xl_grid_launch_dependents();
   constexpr int MAX_VEC = 4;  // vectors of 8 elements per thread: cols <= 256 * 8 * 4
@@ -843,8 +844,7 @@ __device__ __forceinline__ void arg_take(ArgBest& b, float v, int i) {
 }
 template <typename T>
 __global__ void __launch_bounds__(256)
-    argmax_rows_kernel(const T* __restrict__ logits, float* __restrict__ max_out, int* __restrict__ idx_out, int V,
-                       int valid, int index_offset) {
+    argmax_rows_kernel(const T* logits, float* max_out, int* idx_out, int V, int valid, int index_offset) {
   constexpr int N = XlVec<T>::N;
   namespace cg = cooperative_groups;
   cg::cluster_group cluster = cg::this_cluster();

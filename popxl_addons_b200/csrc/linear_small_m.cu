@@ -14,7 +14,7 @@
 // 128) its N, so that one thread keeps the tensor core ahead of HBM: four instructions per 16 KB of weights, about 65 clocks each,
 // are twice the rate at which an SM's share of the bandwidth arrives. TMA loads 128 x 64 blocks of weights, and the tokens' 64
 // columns beside them, into a ring of about 90 KB per CTA; one CTA per SM works on a product while one of the next product already
-// fills its ring (programmatic dependent launch: weights are requested while the previous kernel drains).
+// fills its ring (programmatic dependent launch: weights that the previous kernel does not write are requested while it drains).
 //
 // A tile of 128 weight rows belongs to a cluster of KS CTAs (1 to 8), each with an equal range of K blocks; KS is what the SMs have
 // room for. The CTAs leave their sums in shared memory, meet, and each finishes its share of the tile's results from the partial sums
@@ -93,6 +93,7 @@ struct SmParams {
   float* state;
   const int *pos, *count;
   int ksplit;  // CTAs of a cluster
+  int read_ahead;  // the weights were complete before the previous launch
   int* err;
 };
 
@@ -233,6 +234,7 @@ __global__ void __launch_bounds__(SM_THREADS, 1)
       auto load_a = [&](int i, int s) { tma_load_2d(ring + s * R::STAGE + R::W_BYTES, &map_a, &full_bar[s], (kb0 + i) * SM_KC, 0); };
       constexpr uint32_t BYTES = COLS * 128 + R::A_BYTES;
       const int ahead = min(STAGES, blocks);
+      if (!p.read_ahead) xl_grid_dependency_wait();
       for (int i = 0; i < ahead; ++i) {
         mbar_expect_tx(&full_bar[i], BYTES);
         load_w(i, i);
@@ -417,15 +419,17 @@ int sm_check(const void* a, long long lda, const void* w, int M, int N, int K, i
 }  // namespace
 
 // All: a (M, K) bf16 with row stride lda (a multiple of 8), w (N, K) bf16 contiguous, M <= 16 (xl_linear_small_m: 128), K a multiple of 8; returns -1
-// for arguments the kernel does not take. y (M, N) with row stride ldy, bf16 or fp32. sumsq (M, sumsq_parts), or null: the rows
+// for arguments the kernel does not take. read_ahead: w was complete before the previous launch on the stream. y (M, N) with row
+// stride ldy, bf16 or fp32. sumsq (M, sumsq_parts), or null: the rows
 // of y are multiplied by 1 / sqrt(sum of the row's sumsq / K + eps).
 XL_API int xl_linear_small_m(const void* a, long long lda, const void* w, void* y, long long ldy, int y_f32, const float* sumsq,
-                             int sumsq_parts, float eps, int M, int N, int K, int sms, int* err, cudaStream_t s) {
+                             int sumsq_parts, float eps, int M, int N, int K, int sms, int read_ahead, int* err,
+                             cudaStream_t s) {
   if (sm_check(a, lda, w, M, N, K, 128) || !y || (sumsq && sumsq_parts < 1)) return -1;
   SmParams p = {};
   p.a = (const __nv_bfloat16*)a; p.lda = lda; p.w = (const __nv_bfloat16*)w; p.M = M; p.N = N; p.K = K;
   p.y = y; p.ldy = ldy; p.y_f32 = y_f32; p.sumsq = sumsq; p.sumsq_parts = sumsq_parts; p.eps = eps;
-  p.err = err;
+  p.read_ahead = read_ahead; p.err = err;
   return sm_launch<SM_STORE>(p, sms, s);
 }
 
@@ -433,57 +437,62 @@ XL_API int xl_linear_small_m(const void* a, long long lda, const void* w, void* 
 // sumsq as in xl_linear_small_m.
 XL_API int xl_linear_small_m_split_glu(const void* a, long long lda, const void* w, void* y, long long ldy, int cols, void* z,
                                        long long ldz, float limit, float slope, float shift, const float* sumsq, int sumsq_parts,
-                                       float eps, int M, int N, int K, int sms, int* err, cudaStream_t s) {
+                                       float eps, int M, int N, int K, int sms, int read_ahead, int* err,
+                                       cudaStream_t s) {
   if (sm_check(a, lda, w, M, N, K) || cols < 0 || cols > N || (cols && !y) || (cols < N && !z) ||
       (sumsq && sumsq_parts < 1))
     return -1;
   SmParams p = {};
   p.a = (const __nv_bfloat16*)a; p.lda = lda; p.w = (const __nv_bfloat16*)w; p.M = M; p.N = N; p.K = K;
   p.y = y; p.ldy = ldy; p.cols = cols; p.z = (__nv_bfloat16*)z; p.ldz = ldz; p.limit = limit; p.slope = slope; p.shift = shift;
-  p.sumsq = sumsq; p.sumsq_parts = sumsq_parts; p.eps = eps; p.err = err;
+  p.sumsq = sumsq; p.sumsq_parts = sumsq_parts; p.eps = eps; p.read_ahead = read_ahead; p.err = err;
   return sm_launch<SM_SPLIT_GLU>(p, sms, s);
 }
 
 // x (M, N) fp32 += mult * a w^T; with nw, h (M, N) bf16 = x * nw and sumsq (M, ceil(N / 64)) = sums of x^2 over 64 columns.
 XL_API int xl_linear_small_m_residual_rms(const void* a, long long lda, const void* w, float* x, float mult, const float* nw,
-                                          void* h, float* sumsq, int M, int N, int K, int sms, int* err, cudaStream_t s) {
+                                          void* h, float* sumsq, int M, int N, int K, int sms, int read_ahead, int* err,
+                                          cudaStream_t s) {
   if (sm_check(a, lda, w, M, N, K) || !x || (nw && (!h || !sumsq))) return -1;
   SmParams p = {};
   p.a = (const __nv_bfloat16*)a; p.lda = lda; p.w = (const __nv_bfloat16*)w; p.M = M; p.N = N; p.K = K;
   p.x = x; p.mult = mult; p.nw = nw; p.h = (__nv_bfloat16*)h; p.sumsq_out = nw ? sumsq : nullptr;
-  p.err = err;
+  p.read_ahead = read_ahead; p.err = err;
   return sm_launch<SM_RESIDUAL>(p, sms, s);
 }
 
 // x (M, N) fp32 += mult * a w^T (+ table[tokens]); with alpha, h (M, N) bf16 = tanh(alpha x) nw + nb.
 XL_API int xl_linear_small_m_residual(const void* a, long long lda, const void* w, float* x, float mult, const int* tokens,
                                       const void* table, int vocab, const float* alpha, const float* nw, const float* nb,
-                                      void* h, int M, int N, int K, int sms, int* err, cudaStream_t s) {
+                                      void* h, int M, int N, int K, int sms, int read_ahead, int* err,
+                                      cudaStream_t s) {
   if (sm_check(a, lda, w, M, N, K) || !x || (table && (!tokens || vocab < 1)) || (alpha && (!nw || !nb || !h)))
     return -1;
   SmParams p = {};
   p.a = (const __nv_bfloat16*)a; p.lda = lda; p.w = (const __nv_bfloat16*)w; p.M = M; p.N = N; p.K = K;
   p.x = x; p.mult = mult; p.tokens = tokens; p.table = (const __nv_bfloat16*)table; p.vocab = vocab;
-  p.alpha = alpha; p.nw = nw; p.nb = nb; p.h = (__nv_bfloat16*)h; p.err = err;
+  p.alpha = alpha; p.nw = nw; p.nb = nb; p.h = (__nv_bfloat16*)h; p.read_ahead = read_ahead; p.err = err;
   return sm_launch<SM_RESIDUAL>(p, sms, s);
 }
 
 // w rows [gate | up] (2F, K); y (M, F) bf16 contiguous.
-XL_API int xl_linear_small_m_swiglu(const void* a, long long lda, const void* w, void* y, int M, int F, int K, int sms, int* err, cudaStream_t s) {
+XL_API int xl_linear_small_m_swiglu(const void* a, long long lda, const void* w, void* y, int M, int F, int K, int sms, int read_ahead, int* err,
+                                    cudaStream_t s) {
   if (sm_check(a, lda, w, M, 2 * F, K) || !y) return -1;
   SmParams p = {};
   p.a = (const __nv_bfloat16*)a; p.lda = lda; p.w = (const __nv_bfloat16*)w; p.M = M; p.N = 2 * F; p.K = K;
-  p.y = y; p.ldy = F; p.err = err;
+  p.y = y; p.ldy = F; p.read_ahead = read_ahead; p.err = err;
   return sm_launch<SM_SWIGLU>(p, sms, s);
 }
 
 // w rows [z | u | g] (3W, K); row r is the next token of sequence r: state (M, W) fp32 advances where count[r] > 0 and starts
 // from zero at pos[r] == 0; y (M, W) bf16 contiguous.
 XL_API int xl_linear_small_m_min_gru(const void* a, long long lda, const void* w, const float* bz, const float* bu, float* state,
-                                     const int* pos, const int* count, void* y, int M, int W, int K, int sms, int* err, cudaStream_t s) {
+                                     const int* pos, const int* count, void* y, int M, int W, int K, int sms, int read_ahead, int* err,
+                                     cudaStream_t s) {
   if (sm_check(a, lda, w, M, 3 * W, K) || !y || !state || !bz || !bu || !pos || !count) return -1;
   SmParams p = {};
   p.a = (const __nv_bfloat16*)a; p.lda = lda; p.w = (const __nv_bfloat16*)w; p.M = M; p.N = 3 * W; p.K = K;
-  p.y = y; p.ldy = W; p.bz = bz; p.bu = bu; p.state = state; p.pos = pos; p.count = count; p.err = err;
+  p.y = y; p.ldy = W; p.bz = bz; p.bu = bu; p.state = state; p.pos = pos; p.count = count; p.read_ahead = read_ahead; p.err = err;
   return sm_launch<SM_MINGRU>(p, sms, s);
 }

@@ -172,7 +172,7 @@ XL_API int xl_dense_csr_matmul(const void* x, int dtype, const int* indptr, cons
 // ------------------------------------------------------------------------------------------------------------------
 template <typename T>
 __global__ void __launch_bounds__(256)
-    gather_rows_kernel(const T* __restrict__ table, const int* idx, T* __restrict__ out, long long n_idx, int rows, int cols) {
+    gather_rows_kernel(const T* table, const int* idx, T* out, long long n_idx, int rows, int cols) {
   xl_grid_dependency_wait();
   xl_grid_launch_dependents();
   const long long i = blockIdx.x;

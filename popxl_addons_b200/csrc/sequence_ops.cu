@@ -52,7 +52,7 @@ __device__ __forceinline__ void dyt_pack(const float (&x)[V], float alpha, const
 // the table row (embedding).
 template <typename T, int V>
 __global__ void __launch_bounds__(256)
-    stream_dyt_kernel(float* x, const T* y, float mult, const int* tokens, const T* __restrict__ table, int vocab, DytParams n, T* h,
+    stream_dyt_kernel(float* x, const T* y, float mult, const int* tokens, const T* table, int vocab, DytParams n, T* h,
                       long long rows, int cols) {
   xl_grid_dependency_wait();
   xl_grid_launch_dependents();
@@ -111,8 +111,8 @@ constexpr int RMS_THREADS = 256;
 // NP packs of V columns per thread stay in registers; the columns of longer rows are read again.
 template <typename T, int V, int NP>
 __global__ void __launch_bounds__(RMS_THREADS)
-    stream_rms_kernel(float* x, const T* y, float mult, const int* tokens, const T* __restrict__ table, int vocab,
-                      const float* __restrict__ w, float eps, T* h, int cols) {
+    stream_rms_kernel(float* x, const T* y, float mult, const int* tokens, const T* table, int vocab, const float* w,
+                      float eps, T* h, int cols) {
   __shared__ float red[32];
   xl_grid_dependency_wait();
   xl_grid_launch_dependents();
@@ -174,8 +174,8 @@ __global__ void __launch_bounds__(RMS_THREADS)
 // h[r] = RMS norm of x[r * stride + idx[r] - offset]
 template <typename T>
 __global__ void __launch_bounds__(RMS_THREADS)
-    select_rms_kernel(const float* x, const int* idx, int stride, int offset, long long x_rows, const float* __restrict__ w, float eps,
-                      T* h, int cols) {
+    select_rms_kernel(const float* x, const int* idx, int stride, int offset, long long x_rows, const float* w, float eps, T* h,
+                      int cols) {
   __shared__ float red[32];
   xl_grid_dependency_wait();
   xl_grid_launch_dependents();

@@ -11,6 +11,7 @@ from typing import Dict, Optional, Tuple
 
 import torch
 
+from ..xl import read_ahead
 from ..xl.opdef import FALLBACKS, OPS, STRICT, NativeFallback, native, note_fallback  # noqa: F401  (re-exported)
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
@@ -97,7 +98,7 @@ _symm_all_gather_mc = _sig("xl_symm_all_gather_mc", _c_p, _c_p, _c_ll, _c_p, _c_
 _kv_fill = _sig("xl_kv_fill", _c_p, _c_ll, _c_p, _c_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_p)
 _gq_small_slots = _sig("xl_gq_gemm_small_m_slots", _c_int)
 _gq_small = _sig("xl_gq_gemm_small_m", _c_p, _c_p, _c_p, _c_p, _c_p, _c_p, _c_int, _c_int, _c_int, _c_int, _c_ll, _c_ll,
-                 _c_int, _c_int, _c_p, _c_p, _c_int, _c_int, _c_int, _c_p)
+                 _c_int, _c_int, _c_p, _c_p, _c_int, _c_int, _c_int, _c_int, _c_p)
 _rot_append = _sig("xl_rotary_append", _c_p, _c_ll, _c_p, _c_p, _c_p, _c_p, _c_p, _c_int, _c_int, _c_int, _c_int, _c_int,
                    _c_int, _c_p)
 _attn_dec = _sig("xl_attn_decode", _c_p, _c_ll, _c_p, _c_p, _c_p, _c_ll, _c_p, _c_p, _c_p, _c_int, _c_int, _c_int, _c_int,
@@ -141,13 +142,17 @@ _rts_adam = _sig("xl_rts_adam", _c_p, _c_p, _c_int, _c_p, _c_p, _c_int, _c_p, _c
 
 
 def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    # the handle of torch.cuda.current_stream(), without the objects around it (1 us of every launch)
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 _RECORDING = []  # stack of lists: kernels launched while a CUDA graph is being captured
 
 
 def _count(name: str):
+    order = read_ahead.current()
+    if order is not None:
+        order.launched(_stream())
     LAUNCHES["count"] += 1
     LAUNCHES["by_kernel"][name] = LAUNCHES["by_kernel"].get(name, 0) + 1
     if _RECORDING:
@@ -1274,7 +1279,8 @@ def gq_gemm_small_m(x, packed, scale, zero, bias, out=None, act_from_col=None, c
     rc = _gq_small(x.data_ptr(), packed.data_ptr(), scale.data_ptr(), zero.data_ptr(),
                    bias.data_ptr() if bias is not None else None, y.data_ptr(), M, N, K, gs, x.stride(0), y.stride(0),
                    N if act_from_col is None else int(act_from_col), ctas,
-                   ws.data_ptr(), counters.data_ptr(), _CODE[x.dtype], _CODE[scale.dtype], int(transposed), _stream())
+                   ws.data_ptr(), counters.data_ptr(), _CODE[x.dtype], _CODE[scale.dtype], int(transposed),
+                   int(read_ahead.allowed(packed, scale, zero)), _stream())
     if rc == -1:
         return NotImplemented
     _check(rc, "gq_gemm_small_m")

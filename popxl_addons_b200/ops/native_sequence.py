@@ -2,6 +2,7 @@
 32-bit models use plain fp32 matrix products (never a reduced-precision matrix mode) and the same kernels for the rest."""
 import torch
 
+from ..xl import read_ahead
 from ..xl.opdef import native
 from ..xl.ops.sequence import SUMSQ_BLOCK
 from .native import (_CODE, _c_f, _c_int, _c_ll, _c_p, _check, _count, _ok, _sig, _sms, _stream, gemm,
@@ -18,7 +19,8 @@ _rope_append = _sig("xl_diff_rope_append", _c_p, _c_ll, _c_p, _c_p, _c_p, _c_p, 
 _diff_general = _sig("xl_diff_attn_general", _c_p, _c_ll, _c_p, _c_p, _c_p, _c_ll, _c_p, _c_p, _c_p, _c_int, _c_int, _c_int,
                      _c_int, _c_int, _c_int, _c_int, _c_int, _c_f, _c_f, _c_f, _c_int, _c_p)
 _diff_decode = _sig("xl_diff_attn_decode", _c_p, _c_ll, _c_p, _c_p, _c_p, _c_p, _c_p, _c_ll, _c_p, _c_p, _c_p, _c_int, _c_int,
-                    _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_f, _c_f, _c_f, _c_int, _c_p, _c_p, _c_p)
+                    _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_f, _c_f, _c_f, _c_int, _c_p, _c_p, _c_int,
+                    _c_p)
 _diff_tcgen05 = _sig("xl_diff_attn_tcgen05", _c_p, _c_ll, _c_p, _c_p, _c_p, _c_ll, _c_p, _c_p, _c_p, _c_int, _c_int, _c_int, _c_int,
                      _c_int, _c_int, _c_int, _c_int, _c_f, _c_f, _c_f, _c_p, _c_p)
 _stream_rms = _sig("xl_stream_rms", _c_p, _c_p, _c_f, _c_p, _c_p, _c_int, _c_p, _c_f, _c_p, _c_ll, _c_int, _c_int, _c_p)
@@ -31,9 +33,10 @@ _WINDOW_ARGS = (_c_p, _c_p, _c_p, _c_p, _c_ll, _c_p, _c_ll, _c_p, _c_p, _c_int, 
 _window_general = _sig("xl_window_attn_general", *_WINDOW_ARGS, _c_int, _c_p)
 _window_tcgen05 = _sig("xl_window_attn_tcgen05", *_WINDOW_ARGS, _c_p, _c_p)
 _window_decode = _sig("xl_window_attn_decode", _c_p, _c_ll, _c_p, _c_p, _c_p, _c_p, _c_p, _c_ll, _c_p, _c_p, _c_int, _c_int, _c_int,
-                      _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_f, _c_f, _c_f, _c_int, _c_p, _c_p, _c_p)
-_linear_f32 = _sig("xl_linear_f32", _c_p, _c_ll, _c_p, _c_p, _c_ll, _c_int, _c_int, _c_int, _c_p)
-_SMALL_TAIL = (_c_int, _c_int, _c_int, _c_int, _c_p, _c_p)
+                      _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_f, _c_f, _c_f, _c_int, _c_p, _c_p, _c_int,
+                      _c_p)
+_linear_f32 = _sig("xl_linear_f32", _c_p, _c_ll, _c_p, _c_p, _c_ll, _c_int, _c_int, _c_int, _c_int, _c_p)
+_SMALL_TAIL = (_c_int, _c_int, _c_int, _c_int, _c_int, _c_p, _c_p)
 _SUMSQ = (_c_p, _c_int, _c_f)  # sums of squares of a deferred norm, parts per row, eps
 _small_store = _sig("xl_linear_small_m", _c_p, _c_ll, _c_p, _c_p, _c_ll, _c_int, *_SUMSQ, *_SMALL_TAIL)
 _small_split_glu = _sig("xl_linear_small_m_split_glu", _c_p, _c_ll, _c_p, _c_p, _c_ll, _c_int, _c_p, _c_ll, _c_f, _c_f, _c_f, *_SUMSQ,
@@ -63,7 +66,8 @@ def _small(a, weight, rows=16) -> bool:
 
 
 def _small_tail(a, rows, weight):
-    return a.shape[0], rows, weight.shape[1], _sms(a.device), gemm_error_flag(a.device).data_ptr(), _stream()
+    return (a.shape[0], rows, weight.shape[1], _sms(a.device), int(read_ahead.allowed(weight)), gemm_error_flag(a.device).data_ptr(),
+            _stream())
 
 
 def _small_ok(rc, name) -> bool:
@@ -119,7 +123,7 @@ def product(a, weight, out_dtype=None, sumsq=None, eps=0.0):
             and weight.is_contiguous()):
         y = torch.empty((a.shape[0], weight.shape[0]), dtype=out_dtype, device=a.device)
         if _small_ok(_linear_f32(a.data_ptr(), a.stride(0), weight.data_ptr(), y.data_ptr(), y.stride(0), a.shape[0],
-                                 weight.shape[0], a.shape[1], _stream()), "linear_f32"):
+                                 weight.shape[0], a.shape[1], int(read_ahead.allowed(weight)), _stream()), "linear_f32"):
             return y
     return torch.mm(a, weight.t()).to(out_dtype)
 
@@ -243,7 +247,7 @@ def diff_attention_cuda(qkv, cos, sin, kc, vc, pos, count, lam, T, heads, rotary
             rc = _diff_decode(qkv.data_ptr(), qkv.stride(0), _ptr(cos), _ptr(sin), kc.data_ptr(), vc.data_ptr(), out.data_ptr(),
                               out.stride(0), pos.data_ptr(), count.data_ptr(), lam.data_ptr(), B, heads, G, dim, vdim,
                               rotary_dim, smax, chunk, float(scale), float(eps), float(out_scale), splits, _ptr(part),
-                              counters.data_ptr(), s)
+                              counters.data_ptr(), int(read_ahead.allowed(pos, count, kc, vc)), s)
             if _small_ok(rc, "diff_attn_decode"):
                 return out
     rc = _rope_append(qkv.data_ptr(), qkv.stride(0), _ptr(cos), _ptr(sin), kc.data_ptr(), vc.data_ptr(), pos.data_ptr(),
@@ -364,7 +368,8 @@ def window_attention_cuda(proj, q_norm, k_norm, kc, vc, pos, count, joint, T, he
         if units <= counters.numel():
             rc = _window_decode(proj.data_ptr(), ld, q_norm.data_ptr(), k_norm.data_ptr(), kc.data_ptr(), vc.data_ptr(),
                                 joint.data_ptr(), ldo, pos.data_ptr(), count.data_ptr(), B, heads, G, dim, vdim, smax, window,
-                                keep_first, int(gated), scale, sink, eps, splits, _ptr(part), counters.data_ptr(), s)
+                                keep_first, int(gated), scale, sink, eps, splits, _ptr(part), counters.data_ptr(),
+                                int(read_ahead.allowed(pos, count, kc, vc)), s)
             if _small_ok(rc, "window_attn_decode"):
                 return joint
     qn = torch.empty((B, G, T, heads // G, dim), dtype=proj.dtype, device=proj.device)

@@ -10,6 +10,8 @@ import os
 
 import torch
 
+from ..xl import read_ahead
+
 
 def _flush():
     if not hasattr(_flush, "buf"):
@@ -38,11 +40,11 @@ def graph_time_ms(fn, reps=40, iters=5):
     """Device time of one launch of a short kernel: `reps` back-to-back launches captured in a CUDA graph and replayed
     (no host launch path in the timed region), median over `iters` replays, divided by `reps`. Caches stay warm, which
     is what a decode step replayed from a graph sees for its small activations (the weights still stream from HBM when
-    they exceed L2)."""
+    they exceed L2). Nothing is written that a later launch takes as its weights, so they may be read ahead."""
     fn()
     torch.cuda.synchronize()
     g = torch.cuda.CUDAGraph()
-    with torch.cuda.graph(g):
+    with torch.cuda.graph(g), read_ahead.following(read_ahead.LaunchOrder(torch.cuda.current_stream().cuda_stream)):
         for _ in range(reps):
             fn()
     g.replay()

@@ -18,6 +18,7 @@ import numpy as np
 import torch
 
 from . import dtypes as _dt
+from . import read_ahead as _read_ahead
 from .buffers import DeviceToHostStream, HostToDeviceStream, RemoteBuffer
 from .comm import DistComm, SimComm
 from .core import Constant, Graph, Ir, LazyInit, Tensor, Variable
@@ -79,6 +80,7 @@ class Session:
         self._buffers: Dict[RemoteBuffer, List[torch.Tensor]] = {}
         self._consts: Dict[Constant, torch.Tensor] = {}
         self._liveness: Dict[Graph, Dict[int, List[Tensor]]] = {}
+        self._reads_ahead: Dict[Graph, bool] = {}
         self._inputs: Dict[HostToDeviceStream, List[List[torch.Tensor]]] = {}
         self._cursor: Dict[HostToDeviceStream, int] = {}
         self._outputs: Dict[DeviceToHostStream, List[List[torch.Tensor]]] = {}
@@ -645,6 +647,7 @@ class Session:
         native_dev = self.device.type if self.use_native else None
         staged = self.slot is not None
         frame = self._frame_dev[-1] if self._frame_dev else None
+        order = _read_ahead.current()
         for i, op in enumerate(graph.ops):
             od = op.opdef
             if staged:
@@ -660,10 +663,14 @@ class Session:
                         od.special(self, op, env)
                     finally:
                         self._frame_dev.pop()
+                    if order is not None:
+                        order.touch(*map(env.get, op.outputs))
                     self._free_dead(frees, i, env)
                     continue
                 if name == "ipu_copy":
                     env[op.outputs[0]] = self.device_copy(env.get(op.inputs[0]), op)
+                    if order is not None:
+                        order.touch(*map(env.get, op.inputs), *map(env.get, op.outputs))
                     self._free_dead(frees, i, env)
                     continue
                 if self._effective_device(op, frame) != self.slot:
@@ -725,6 +732,14 @@ class Session:
                     outs_per_replica.append((res,) if isinstance(res, torch.Tensor) else tuple(res or ()))
                 for j, t in enumerate(op.outputs):
                     env[t] = [outs_per_replica[r][j] for r in range(self.num_local)]
+            if order is not None:
+                # (a control op's inputs were in the hands of the ops of the graphs that it ran)
+                only_read = _read_ahead.READERS.get(od.name)
+                if od.special is not None:
+                    ins = () if control else [env.get(t) for t in op.inputs]
+                elif only_read is not None:
+                    ins = [v for j, v in enumerate(ins) if j not in only_read]
+                order.touch(ins, [env.get(t) for t in op.outputs])
             if self._nvtx:
                 torch.cuda.nvtx.range_pop()
             if timed:
@@ -901,6 +916,27 @@ class Session:
                 self._host_loads_of(callee, found, seen)
         return found
 
+    def _launch_order(self, graph: Graph) -> Optional[_read_ahead.LaunchOrder]:
+        """What the kernels of a run of `graph` may read ahead of their predecessors, if any of them asks."""
+        if not self.use_native:
+            return None
+        if graph not in self._reads_ahead:
+            seen, todo, found = set(), [graph], False
+            while todo and not found:
+                g = todo.pop()
+                if id(g) in seen:
+                    continue
+                seen.add(id(g))
+                for o in g.ops:
+                    found = found or o.opdef.name in _read_ahead.READERS
+                    todo += [c for c in map(o.attrs.get, ("graph", "then_graph", "else_graph")) if hasattr(c, "ops")]
+            self._reads_ahead[graph] = found
+        return self._new_order() if self._reads_ahead[graph] else None
+
+    def _new_order(self) -> _read_ahead.LaunchOrder:
+        on_gpu = self.device.type == "cuda"
+        return _read_ahead.LaunchOrder(torch.cuda.current_stream(self.device).cuda_stream if on_gpu else 0)
+
     def _capture(self, op, graph: Graph, vals, carried):
         from ..ops import native as _native
 
@@ -920,7 +956,9 @@ class Session:
         ok = False
         self._capturing = True
         try:
-            with torch.cuda.graph(g, capture_error_mode="thread_local"):
+            # a graph starts when everything queued before it has ended: the launches before the capture do not count
+            with torch.cuda.graph(g, capture_error_mode="thread_local"), \
+                    _read_ahead.following(self._new_order() if _read_ahead.current() is not None else None):
                 outs = self.run_graph(graph, carried + list(vals[n_out:]))
                 # every stream forked inside the body joins before its results are read back and the capture ends
                 self._join_streams()
@@ -958,7 +996,7 @@ class Session:
         self._stage_inputs(inputs or {})
         main = self.ir.main_graph
         env: Dict[Tensor, List[torch.Tensor]] = {}
-        with torch.no_grad():
+        with torch.no_grad(), _read_ahead.following(self._launch_order(main)):
             self._exec_ops(main, env)
             self._join_streams()
         out = self._collect_outputs(fetch)
@@ -992,14 +1030,15 @@ class Session:
                 self._after_replay(state, copy=not fetch)
             else:
                 vals = [self._value(t, {}) for t in program.bindings.values()]
-                if capturable and program in self._programs and self._capture_safe(program.graph):
-                    state = self._capture(None, program.graph, vals, [])
-                    self._programs[program] = state
-                    self._after_replay(state)
-                else:
-                    self.run_graph(program.graph, vals)
-                    self._join_streams()
-                    self._programs.setdefault(program, None)
+                with _read_ahead.following(self._launch_order(program.graph)):
+                    if capturable and program in self._programs and self._capture_safe(program.graph):
+                        state = self._capture(None, program.graph, vals, [])
+                        self._programs[program] = state
+                        self._after_replay(state)
+                    else:
+                        self.run_graph(program.graph, vals)
+                        self._join_streams()
+                        self._programs.setdefault(program, None)
         out = self._collect_outputs(fetch)
         if self.use_native and fetch:
             from ..ops import native as _native
