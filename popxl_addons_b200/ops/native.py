@@ -7,6 +7,9 @@ missing on a machine with a GPU the import fails loudly rather than silently run
 """
 import ctypes
 import os
+import threading
+from collections import OrderedDict
+from contextlib import contextmanager
 from typing import Dict, Optional, Tuple
 
 import torch
@@ -184,19 +187,65 @@ def _ok(*ts) -> bool:
 
 
 # ---- scratch memory ------------------------------------------------------------------------------------------------
-_WORKSPACE: Dict[Tuple[int, str], torch.Tensor] = {}
+# What a launch leaves in scratch memory is for later launches on the same stream only, so every stream has its own, and so has
+# every captured graph, which may be replayed on any stream and keeps the addresses it was captured with.
+_MAX_STREAMS = 32
+_STREAM_SCRATCH: "OrderedDict[Tuple[int, int], Dict[str, torch.Tensor]]" = OrderedDict()  # the streams used last
+_CAPTURES = threading.local()  # .held: scratch of the graph that this thread is capturing
 _ERR: Dict[int, torch.Tensor] = {}
 
 
+def _stream_scratch(device) -> Dict[str, torch.Tensor]:
+    key = (device.index or 0, _stream())
+    held = _STREAM_SCRATCH.get(key)
+    if held is None:
+        held = _STREAM_SCRATCH[key] = {}
+        while len(_STREAM_SCRATCH) > _MAX_STREAMS:
+            _STREAM_SCRATCH.popitem(last=False)  # goes back to the allocator, which orders it behind its stream's work
+    elif len(_STREAM_SCRATCH) > 1:
+        _STREAM_SCRATCH.move_to_end(key)
+    return held
+
+
 def workspace(nbytes: int, device: torch.device, tag: str = "default") -> torch.Tensor:
-    """Per-device scratch buffer (fp32 view), grown on demand and reused by later launches on the same stream."""
-    key = (device.index or 0, tag)
-    buf = _WORKSPACE.get(key)
+    """Scratch buffer of the current stream (fp32 view), grown on demand and reused by later launches. In a capture a new one,
+    from the graph's own memory."""
     n = (nbytes + 3) // 4
+    if torch.cuda.is_current_stream_capturing():
+        return torch.empty(n, dtype=torch.float32, device=device)
+    held = _stream_scratch(device)
+    buf = held.get(tag)
     if buf is None or buf.numel() < n:
-        buf = torch.empty(max(n, 1 << 18), dtype=torch.float32, device=device)
-        _WORKSPACE[key] = buf
+        buf = held[tag] = torch.empty(max(n, 1 << 18), dtype=torch.float32, device=device)
     return buf
+
+
+def counters(n: int, device: torch.device, tag: str, least: int = 4096) -> torch.Tensor:
+    """At least `n` int32 zeros of the current stream, or of the graph that is being captured, which every launch leaves at
+    zero. Names of counters begin with "counters"."""
+    held = getattr(_CAPTURES, "held", None)
+    if held is None:
+        if torch.cuda.is_current_stream_capturing():  # a graph that nobody keeps scratch for: zeroed in every replay
+            return torch.zeros(n, dtype=torch.int32, device=device)
+        held = _stream_scratch(device)
+    buf = held.get(tag)
+    if buf is None or buf.numel() < n:
+        if buf is not None and held is getattr(_CAPTURES, "held", None):
+            held[f"{tag} {buf.data_ptr()}"] = buf  # launches captured so far use it
+        buf = held[tag] = torch.zeros(max(n, least), dtype=torch.int32, device=device)
+    return buf
+
+
+@contextmanager
+def capture_scratch(device):
+    """Around a capture: gives it counters of its own, already zero for those that the current stream has used. The dict it
+    yields is to be kept as long as the graph."""
+    before = getattr(_CAPTURES, "held", None)
+    _CAPTURES.held = {tag: torch.zeros_like(t) for tag, t in _stream_scratch(device).items() if tag.startswith("counters")}
+    try:
+        yield _CAPTURES.held
+    finally:
+        _CAPTURES.held = before
 
 
 def gemm_error_flag(device: torch.device) -> torch.Tensor:
@@ -1129,9 +1178,6 @@ def rotary_kv_append_cuda(qkv, sin_tab, cos_tab, k_cache, v_cache, pos, n_heads,
     return qkv
 
 
-_AD_SCRATCH: Dict[int, torch.Tensor] = {}
-
-
 def _attn_decode_launch(qkv, k_cache, v_cache, pos, n_heads, head_dim, scale, out):
     if not (_row_window_ok(qkv) and _row_window_ok(out)) or not _ok(k_cache, v_cache) or pos.dtype != torch.int32:
         return NotImplemented
@@ -1142,12 +1188,9 @@ def _attn_decode_launch(qkv, k_cache, v_cache, pos, n_heads, head_dim, scale, ou
     # enough CTAs to fill the machine, at least 32 cache positions per CTA
     splits = max(1, min((8 * _sms(qkv.device) + bh - 1) // bh, (smax + 31) // 32, 64))
     ws = workspace(bh * splits * (head_dim + 2) * 4, qkv.device, "attn_decode")
-    idx = qkv.device.index or 0
-    counters = _AD_SCRATCH.get(idx)
-    if counters is None or counters.numel() < bh:
-        counters = _AD_SCRATCH[idx] = torch.zeros(max(bh, 4096), dtype=torch.int32, device=qkv.device)
+    done = counters(bh, qkv.device, "counters attn_decode")
     rc = _attn_dec(qkv.data_ptr(), qkv.stride(0), k_cache.data_ptr(), v_cache.data_ptr(), out.data_ptr(), out.stride(0),
-                   ws.data_ptr(), counters.data_ptr(), pos.data_ptr(), B, n_heads, head_dim, smax, float(scale), splits,
+                   ws.data_ptr(), done.data_ptr(), pos.data_ptr(), B, n_heads, head_dim, smax, float(scale), splits,
                    _CODE[qkv.dtype], _stream())
     if rc == -1:
         return NotImplemented
@@ -1237,21 +1280,6 @@ def store_row_cuda(buf, pos, vals, base):
     return buf
 
 
-_GQ_SCRATCH: Dict[int, Tuple[torch.Tensor, torch.Tensor]] = {}
-
-
-def _gq_scratch(device, n_tiles: int, ctas: int):
-    """Split-K scratch of the small-M int4 GEMM: slots for partial sums, and counters that every launch leaves at zero."""
-    idx = device.index or 0
-    cur = _GQ_SCRATCH.get(idx)
-    slots = _gq_small_slots(ctas)
-    if cur is None or cur[1].numel() < n_tiles or cur[0].numel() < slots:
-        cur = (torch.empty(max(slots, cur[0].numel() if cur else 0), dtype=torch.float32, device=device),
-               torch.zeros(max(n_tiles, 2048, cur[1].numel() if cur else 0), dtype=torch.int32, device=device))
-        _GQ_SCRATCH[idx] = cur
-    return cur
-
-
 def gq_gemm_small_m(x, packed, scale, zero, bias, out=None, act_from_col=None, ctas=None):
     """`x (M<=16, K) @ dequant(packed (N, K/gs, gs/4))^T + bias` with the de-quantisation fused into the GEMM; GELU on
     the output columns `>= act_from_col` if given. `x` and `out` may be column windows of wider row-major matrices.
@@ -1275,11 +1303,12 @@ def gq_gemm_small_m(x, packed, scale, zero, bias, out=None, act_from_col=None, c
     if y.shape != (M, N) or y.dtype != x.dtype or y.stride(1) != 1:
         return NotImplemented
     ctas = int(ctas or _sms(x.device))
-    ws, counters = _gq_scratch(x.device, (N + 63) // 64, ctas)
+    ws = workspace(_gq_small_slots(ctas) * 4, x.device, "gq_slots")  # partial sums
+    done = counters((N + 63) // 64, x.device, "counters gq")
     rc = _gq_small(x.data_ptr(), packed.data_ptr(), scale.data_ptr(), zero.data_ptr(),
                    bias.data_ptr() if bias is not None else None, y.data_ptr(), M, N, K, gs, x.stride(0), y.stride(0),
                    N if act_from_col is None else int(act_from_col), ctas,
-                   ws.data_ptr(), counters.data_ptr(), _CODE[x.dtype], _CODE[scale.dtype], int(transposed),
+                   ws.data_ptr(), done.data_ptr(), _CODE[x.dtype], _CODE[scale.dtype], int(transposed),
                    int(read_ahead.allowed(packed, scale, zero)), _stream())
     if rc == -1:
         return NotImplemented
@@ -1375,9 +1404,6 @@ def matmul_pow2scaled_cuda(a, b, log2_scale, out_dt):
     return res.view(*a.shape[:-1], b.shape[-1])
 
 
-_MSE_SCRATCH: Dict[int, torch.Tensor] = {}
-
-
 def fp8_mse_scale_cuda(x, fmt_name, src_mantissa_bits):
     from .fp8_mse_scale import _format_window
     from .fp8_utils import FP8_FORMATS
@@ -1387,10 +1413,7 @@ def fp8_mse_scale_cuda(x, fmt_name, src_mantissa_bits):
     fmt = FP8_FORMATS[fmt_name]
     lo, span = _format_window(fmt)
     qerr = 2.0 ** (-2.0 * (src_mantissa_bits - fmt["mantissa_bits"]))
-    idx = x.device.index or 0
-    scratch = _MSE_SCRATCH.get(idx)
-    if scratch is None:
-        scratch = _MSE_SCRATCH[idx] = torch.zeros(256, dtype=torch.int32, device=x.device)
+    scratch = counters(256, x.device, "counters mse_scale", 256)
     out = torch.empty((), dtype=torch.int32, device=x.device)
     _check(_mse_scale(x.data_ptr(), _CODE[x.dtype], x.numel(), scratch.data_ptr(), int(lo), int(span), float(qerr),
                       out.data_ptr(), _stream()), "fp8_mse_scale")

@@ -5,7 +5,7 @@ import torch
 from ..xl import read_ahead
 from ..xl.opdef import native
 from ..xl.ops.sequence import SUMSQ_BLOCK
-from .native import (_CODE, _c_f, _c_int, _c_ll, _c_p, _check, _count, _ok, _sig, _sms, _stream, gemm,
+from .native import (_CODE, _c_f, _c_int, _c_ll, _c_p, _check, _count, _ok, _sig, _sms, _stream, counters, gemm,
                      gemm_error_flag)
 
 _stream_dyt = _sig("xl_stream_dyt", _c_p, _c_p, _c_f, _c_p, _c_p, _c_int, _c_p, _c_p, _c_p, _c_p, _c_ll, _c_int, _c_int, _c_p)
@@ -46,18 +46,6 @@ _small_residual = _sig("xl_linear_small_m_residual", _c_p, _c_ll, _c_p, _c_p, _c
                        *_SMALL_TAIL)
 _small_swiglu = _sig("xl_linear_small_m_swiglu", _c_p, _c_ll, _c_p, _c_p, *_SMALL_TAIL)
 _small_min_gru = _sig("xl_linear_small_m_min_gru", _c_p, _c_ll, _c_p, _c_p, _c_p, _c_p, _c_p, _c_p, _c_p, *_SMALL_TAIL)
-
-_SCRATCH = {}
-
-
-def _counters(device):
-    """Counters of the decoding attention kernels, which every launch leaves at zero. Allocated once at their final size, since
-    captured graphs keep the address."""
-    idx = device.index or 0
-    if idx not in _SCRATCH:
-        _SCRATCH[idx] = torch.zeros(1 << 16, dtype=torch.int32, device=device)
-    return _SCRATCH[idx]
-
 
 def _small(a, weight, rows=16) -> bool:
     """Whether the small-M kernels take this product."""
@@ -241,13 +229,13 @@ def diff_attention_cuda(qkv, cos, sin, kc, vc, pos, count, lam, T, heads, rotary
         units = B * G * ((heads // G + 7) // 8)
         longest = min(smax, chunk) if chunk else smax
         splits = max(1, min(2 * _sms(qkv.device) // units, (longest + 63) // 64, 64))  # one wave, two CTAs per SM
-        counters = _counters(qkv.device)
+        done = counters(units, qkv.device, "counters sequence", 1 << 16)
         part = torch.empty(units * splits * 16 * (vdim + 2), dtype=torch.float32, device=qkv.device) if splits > 1 else None
-        if units <= counters.numel():
+        if units <= 1 << 16:
             rc = _diff_decode(qkv.data_ptr(), qkv.stride(0), _ptr(cos), _ptr(sin), kc.data_ptr(), vc.data_ptr(), out.data_ptr(),
                               out.stride(0), pos.data_ptr(), count.data_ptr(), lam.data_ptr(), B, heads, G, dim, vdim,
                               rotary_dim, smax, chunk, float(scale), float(eps), float(out_scale), splits, _ptr(part),
-                              counters.data_ptr(), int(read_ahead.allowed(pos, count, kc, vc)), s)
+                              done.data_ptr(), int(read_ahead.allowed(pos, count, kc, vc)), s)
             if _small_ok(rc, "diff_attn_decode"):
                 return out
     rc = _rope_append(qkv.data_ptr(), qkv.stride(0), _ptr(cos), _ptr(sin), kc.data_ptr(), vc.data_ptr(), pos.data_ptr(),
@@ -363,12 +351,12 @@ def window_attention_cuda(proj, q_norm, k_norm, kc, vc, pos, count, joint, T, he
         longest = min(smax, window + keep_first) if window else smax
         # one wave, two CTAs per SM; a slice of fewer keys costs more in the merge than it saves
         splits = max(1, min(2 * _sms(proj.device) // units, (longest + 383) // 384, 64))
-        counters = _counters(proj.device)
+        done = counters(units, proj.device, "counters sequence", 1 << 16)
         part = torch.empty(units * splits * 16 * (vdim + 2), dtype=torch.float32, device=proj.device) if splits > 1 else None
-        if units <= counters.numel():
+        if units <= 1 << 16:
             rc = _window_decode(proj.data_ptr(), ld, q_norm.data_ptr(), k_norm.data_ptr(), kc.data_ptr(), vc.data_ptr(),
                                 joint.data_ptr(), ldo, pos.data_ptr(), count.data_ptr(), B, heads, G, dim, vdim, smax, window,
-                                keep_first, int(gated), scale, sink, eps, splits, _ptr(part), counters.data_ptr(),
+                                keep_first, int(gated), scale, sink, eps, splits, _ptr(part), done.data_ptr(),
                                 int(read_ahead.allowed(pos, count, kc, vc)), s)
             if _small_ok(rc, "window_attn_decode"):
                 return joint

@@ -41,10 +41,13 @@ def graph_time_ms(fn, reps=40, iters=5):
     (no host launch path in the timed region), median over `iters` replays, divided by `reps`. Caches stay warm, which
     is what a decode step replayed from a graph sees for its small activations (the weights still stream from HBM when
     they exceed L2). Nothing is written that a later launch takes as its weights, so they may be read ahead."""
+    from ..ops import native
+
     fn()
     torch.cuda.synchronize()
     g = torch.cuda.CUDAGraph()
-    with torch.cuda.graph(g), read_ahead.following(read_ahead.LaunchOrder(torch.cuda.current_stream().cuda_stream)):
+    with native.capture_scratch(torch.device("cuda", torch.cuda.current_device())) as scratch, torch.cuda.graph(g), \
+            read_ahead.following(read_ahead.LaunchOrder(torch.cuda.current_stream().cuda_stream)):
         for _ in range(reps):
             fn()
     g.replay()
@@ -57,6 +60,7 @@ def graph_time_ms(fn, reps=40, iters=5):
         e.record()
         torch.cuda.synchronize()
         times.append(s.elapsed_time(e) / reps)
+    del scratch  # the graph's until here
     times.sort()
     return times[len(times) // 2]
 

@@ -957,7 +957,7 @@ class Session:
         self._capturing = True
         try:
             # a graph starts when everything queued before it has ended: the launches before the capture do not count
-            with torch.cuda.graph(g, capture_error_mode="thread_local"), \
+            with _native.capture_scratch(self.device) as scratch, torch.cuda.graph(g, capture_error_mode="thread_local"), \
                     _read_ahead.following(self._new_order() if _read_ahead.current() is not None else None):
                 outs = self.run_graph(graph, carried + list(vals[n_out:]))
                 # every stream forked inside the body joins before its results are read back and the capture ends
@@ -978,7 +978,7 @@ class Session:
                   file=sys.stderr, flush=True)
         g.replay()  # capture records but does not execute
         _native.count_replay(kernels)
-        return {"graph": g, "static_in": static_in, "outputs": outs_rec, "kernels": kernels, "carried": carried,
+        return {"graph": g, "static_in": static_in, "outputs": outs_rec, "kernels": kernels, "carried": carried, "scratch": scratch,
                 "ptrs": tuple(v[0].data_ptr() for v in vals[n_out:])}
 
     def _after_replay(self, state, copy: bool = True):
