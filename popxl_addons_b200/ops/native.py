@@ -534,7 +534,7 @@ def accumulate_mean_cuda(acc, x, *extra, **attrs):
 
 @native("matmul_accumulate_mean_")
 def matmul_accumulate_mean_cuda(acc, a, b, step):
-    if step.dtype != torch.float32 or not acc.is_contiguous():
+    if step.dtype != torch.float32 or not acc.is_contiguous() or not gemm_pays(a, b, acc):
         return NotImplemented
     res = gemm(a, b, out=acc, accumulate=2, step=step)
     return res
@@ -616,6 +616,32 @@ def _major(t: torch.Tensor, contraction_last: bool):
     return None
 
 
+def _rows_aligned(t: torch.Tensor) -> bool:
+    """Whether the rows (transposed: columns) of a 2-D operand start on 16-byte boundaries; a single row's stride is free."""
+    rows, ld = (t.shape[0], t.stride(0)) if t.stride(1) == 1 else (t.shape[1], t.stride(1))
+    return t.data_ptr() % 16 == 0 and (rows == 1 or ld * t.element_size() % 16 == 0)
+
+
+def gemm_pays(a: torch.Tensor, b: torch.Tensor, out: Optional[torch.Tensor] = None, out_dtype: Optional[torch.dtype] = None) -> bool:
+    """Whether `gemm(a, b)`, or with `out` the accumulating `gemm(a, b, out=out)`, is worth its copies (2-D operands). It always is
+    if all rows start on 16-byte boundaries. Otherwise up to three launches move operands and result, 15 us of host time each;
+    what it saves against the library grows with the work (us on the GPU and per eager call, library -> these kernels):
+    256 x 257 x 255 6.7 -> 20.3 and 12 -> 71, 1024 x 1021 x 1025 35 -> 16.5 and 35 -> 71, 2048 x 768 x 5001 148 -> 33 and
+    150 -> 56, 4096 x 768 x 10001 443 -> 100. Few rows or columns leave the library bound by memory, which the copies only add
+    to (1 x 768 x 50257: 24 -> 59). Accumulation replaces more of the library's passes: fp32 512 x 513 x 511 33 -> 15, and
+    only its rows of 49 to 128 columns, which leave the kernel element by element, lose (128 x 129 x 127: 24.6 -> 31.9);
+    16-bit ones all do (256 x 257 x 255 30.9 -> 44.2, 1024 x 1021 x 1025 77 -> 51)."""
+    (M, K), N = a.shape, b.shape[1]
+    work = M * N * K
+    if out is not None:
+        if _rows_aligned(a) and _rows_aligned(b) and _rows_aligned(out):
+            return True
+        return N <= 48 or (N > 128 if out.dtype == torch.float32 else work >= 1 << 28)
+    if _rows_aligned(a) and _rows_aligned(b) and N * (out_dtype or a.dtype).itemsize % 16 == 0:
+        return True
+    return min(M, N, K) >= 128 and work >= 1 << 31
+
+
 def _aligned_operand(t: torch.Tensor) -> torch.Tensor:
     """A 2-D GEMM operand whose rows (or, transposed, columns) all start on 16-byte boundaries: `t`, or a copy with padded
     rows. The copy costs two passes over the operand; without it the product would leave the tcgen05 kernels."""
@@ -623,6 +649,9 @@ def _aligned_operand(t: torch.Tensor) -> torch.Tensor:
     if t.dtype not in (torch.bfloat16, torch.float16) or (src.stride(0) % 8 == 0 and t.data_ptr() % 16 == 0):
         return t
     rows, cols = src.shape
+    if rows == 1 and t.data_ptr() % 16 == 0:
+        dst = torch.as_strided(src, (1, cols), ((cols + 7) // 8 * 8, 1))  # the stride of a single row is free
+        return dst if src is t else dst.t()
     dst = torch.empty((rows, (cols + 7) // 8 * 8), dtype=t.dtype, device=t.device)
     _check(_pack_rows16(src.data_ptr(), src.stride(0), dst.data_ptr(), dst.stride(0), rows, cols, _stream()), "pack_rows")
     _count("pack_rows")
@@ -827,7 +856,7 @@ def matmul_cuda(a, b):
         return NotImplemented
     if b.dim() == 2 and a.dim() >= 2:
         a2 = a.reshape(-1, a.shape[-1]) if a.dim() > 2 else a
-        res = gemm(a2, b)
+        res = gemm(a2, b) if gemm_pays(a2, b) else NotImplemented
         if res is NotImplemented:
             return res
         return res.view(*a.shape[:-1], b.shape[-1])
@@ -849,7 +878,8 @@ _ACT = {"none": 0, "gelu": 1, "gelu_tanh": 2, "relu": 3}
 def linear_bias_act_cuda(x, w, *b, act):
     if x.dtype != w.dtype or x.dtype not in (torch.bfloat16, torch.float16) or not x.is_contiguous():
         return NotImplemented
-    res = gemm(x.reshape(-1, x.shape[-1]), w, bias=b[0] if b else None, act=_ACT[act])
+    x2 = x.reshape(-1, x.shape[-1])
+    res = gemm(x2, w, bias=b[0] if b else None, act=_ACT[act]) if gemm_pays(x2, w) else NotImplemented
     if res is NotImplemented:
         return res
     return res.view(*x.shape[:-1], w.shape[-1])
@@ -1655,7 +1685,7 @@ def _register_late():
         if w is NotImplemented:
             return NotImplemented
         wt = w if dim in (-1, 1) else w.t()
-        res = gemm(x.reshape(-1, x.shape[-1]), wt, bias=b[0] if b else None)
+        res = gemm(x2, wt, bias=b[0] if b else None) if gemm_pays(x2, wt) else NotImplemented
         if res is NotImplemented:
             return res
         return res.view(*x.shape[:-1], wt.shape[-1])

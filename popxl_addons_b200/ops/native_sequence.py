@@ -6,7 +6,7 @@ from ..xl import read_ahead
 from ..xl.opdef import native
 from ..xl.ops.sequence import SUMSQ_BLOCK
 from .native import (_CODE, _c_f, _c_int, _c_ll, _c_p, _check, _count, _ok, _sig, _sms, _stream, counters, gemm,
-                     gemm_error_flag)
+                     gemm_error_flag, gemm_pays)
 
 _stream_dyt = _sig("xl_stream_dyt", _c_p, _c_p, _c_f, _c_p, _c_p, _c_int, _c_p, _c_p, _c_p, _c_p, _c_ll, _c_int, _c_int, _c_p)
 _select_dyt = _sig("xl_select_dyt", _c_p, _c_p, _c_int, _c_int, _c_ll, _c_p, _c_p, _c_p, _c_p, _c_int, _c_int, _c_int, _c_p)
@@ -98,7 +98,7 @@ def product(a, weight, out_dtype=None, sumsq=None, eps=0.0):
                 return y
         if sumsq is not None:
             return NotImplemented
-        y = gemm(a, weight.t(), out_dtype=out_dtype)
+        y = gemm(a, weight.t(), out_dtype=out_dtype) if gemm_pays(a, weight.t(), out_dtype=out_dtype) else NotImplemented
         if y is not NotImplemented:
             return y
         y = torch.mm(a, weight.t())

@@ -107,7 +107,7 @@ def _matmul_add_cuda(c, a, w):
 
     if c.dim() != 2 or a.dim() != 2 or w.dim() != 2 or not c.is_contiguous():
         return NotImplemented
-    res = native.gemm(a, w, out=c, accumulate=1)  # c += a @ w in the GEMM epilogue (c is dead after this op)
+    res = native.gemm(a, w, out=c, accumulate=1) if native.gemm_pays(a, w, c) else NotImplemented  # c += a @ w in the GEMM epilogue (c is dead after this op)
     return res
 
 
