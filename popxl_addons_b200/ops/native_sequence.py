@@ -89,8 +89,10 @@ def product(a, weight, out_dtype=None, sumsq=None, eps=0.0):
     out_dtype = out_dtype or a.dtype
     if a.dtype != torch.float32:
         # Up to 128 rows the product is bound by reading the weights. The GEMM multiplies tiles of 256 rows and does not
-        # split K: a weight of 2048 x 7680 keeps 16 of 74 CTA pairs busy (40 rows: 30.5 us, 11.1 here).
-        if _small(a, weight, 128) and out_dtype in (torch.bfloat16, torch.float32):
+        # split K: a weight of 2048 x 7680 keeps 16 of 74 CTA pairs busy (40 rows: 30.5 us, 11.1 here). A small weight is no
+        # reading at all, and wide tiles of tokens take longer to store (64 x 64, GEMM -> here: 40 rows 5.0 -> 4.0 us, 96 rows
+        # 5.0 -> 6.9, 128 rows 5.0 -> 8.5; 256 x 256: 64 rows 7.3 -> 5.4, 128 rows 7.7 -> 8.1).
+        if _small(a, weight, 128 if weight.numel() >= 1 << 16 else 40) and out_dtype in (torch.bfloat16, torch.float32):
             y = torch.empty((a.shape[0], weight.shape[0]), dtype=out_dtype, device=a.device)
             if _small_ok(_small_store(a.data_ptr(), a.stride(0), weight.data_ptr(), y.data_ptr(), y.stride(0),
                                       int(out_dtype == torch.float32), *_sumsq_args(sumsq, eps),
@@ -107,7 +109,13 @@ def product(a, weight, out_dtype=None, sumsq=None, eps=0.0):
         return NotImplemented
     if torch.backends.cuda.matmul.allow_tf32:
         raise RuntimeError("32-bit models need true fp32 matrix products: set torch.backends.cuda.matmul.allow_tf32 = False")
-    if (a.is_cuda and weight.dtype == torch.float32 and out_dtype == torch.float32 and a.shape[0] <= 16 and a.stride(1) == 1
+    # Up to four rows the weights bound the product at every size. With more, every CTA reads more activations than weights, which
+    # the library shares better in large matrices (32000 x 1024, library -> here: 4 rows 55 -> 30 us, 6 rows 55 -> 60, 16 rows 56 ->
+    # 85; 4096 x 4096: 8 rows 49 -> 27, 16 rows 65 -> 55), and with more than eight its launch is shorter for small ones
+    # (256 x 256: 8 rows 3.4 -> 2.8, 16 rows 3.4 -> 4.6; 1024 x 1024: 16 rows 9.8 -> 5.4).
+    n, size = a.shape[0], weight.numel()
+    few = n <= 4 or (n <= 8 and size <= 1 << 24) or (n <= 16 and 1 << 18 <= size <= 1 << 24)
+    if (few and a.is_cuda and weight.dtype == torch.float32 and out_dtype == torch.float32 and a.stride(1) == 1
             and weight.is_contiguous()):
         y = torch.empty((a.shape[0], weight.shape[0]), dtype=out_dtype, device=a.device)
         if _small_ok(_linear_f32(a.data_ptr(), a.stride(0), weight.data_ptr(), y.data_ptr(), y.stride(0), a.shape[0],
