@@ -571,8 +571,19 @@ template <typename T, int V> __device__ __forceinline__ void xl_stream_store(T* 
   }
 }
 
+// One element: gradient, moments and weight in, moments and weight out.
+template <typename TM> __device__ __forceinline__ void adam_element(float g, float& m, float& v, float& w, const AdamArgs& a, float c1, float c2) {
+  const float gf = g * a.grad_scale;
+  m = m * a.beta1 + gf * (1.f - a.beta1);
+  v = v * a.beta2 + gf * gf * (1.f - a.beta2);
+  const float mq = xl_to_float(xl_from_float<TM>(m));  // the stored value enters the update
+  const float upd = (mq * c1) / (sqrtf(v * c2) + a.eps) + w * a.weight_decay;
+  w = w - a.lr * upd;
+}
+
 // Bound by HBM: 30 bytes per parameter with 16-bit weights (master and both moments read and written, the gradient read, the weight
-// written). Four elements per thread and access, all loads of two groups ahead of the first store.
+// written). Four elements per thread and access, all loads of two groups ahead of the first store; up to three elements remain for
+// single accesses of the first CTA (in a launch of their own they cost a parameter of 5 elements 2.9 of 6.4 us).
 template <typename TW, typename TG, typename TM, int V>
 __global__ void __launch_bounds__(256)
     adam_kernel(TW* __restrict__ w, const TG* __restrict__ g, TM* __restrict__ m, float* __restrict__ v,
@@ -603,14 +614,7 @@ __global__ void __launch_bounds__(256)
       const long long i = i0 + u * 256;
       if (i < groups) {
 #pragma unroll
-        for (int e = 0; e < V; ++e) {
-          const float gf = gr[u][e] * a.grad_scale;
-          mo[u][e] = mo[u][e] * a.beta1 + gf * (1.f - a.beta1);
-          ve[u][e] = ve[u][e] * a.beta2 + gf * gf * (1.f - a.beta2);
-          const float mq = xl_to_float(xl_from_float<TM>(mo[u][e]));  // the stored value enters the update
-          const float upd = (mq * c1) / (sqrtf(ve[u][e] * c2) + a.eps) + we[u][e] * a.weight_decay;
-          we[u][e] = we[u][e] - a.lr * upd;
-        }
+        for (int e = 0; e < V; ++e) adam_element<TM>(gr[u][e], mo[u][e], ve[u][e], we[u][e], a, c1, c2);
         xl_stream_store<TM, V>(m + i * V, mo[u]);
         xl_stream_store<float, V>(v + i * V, ve[u]);
         if (master) xl_stream_store<float, V>(master + i * V, we[u]);
@@ -618,19 +622,26 @@ __global__ void __launch_bounds__(256)
       }
     }
   }
+  const long long i = groups * V + threadIdx.x;
+  if (blockIdx.x == 0 && i < n) {
+    float mo = xl_to_float(m[i]), ve = v[i], we = master ? master[i] : xl_to_float(w[i]);
+    adam_element<TM>(xl_to_float(g[i]), mo, ve, we, a, c1, c2);
+    m[i] = xl_from_float<TM>(mo);
+    v[i] = ve;
+    if (master) master[i] = we;
+    w[i] = xl_from_float<TW>(we);
+  }
 }
 
 template <typename TW, typename TG, typename TM>
 static void adam_launch(void* w, const void* g, void* m, float* v, float* master, float* step, AdamArgs a, long long n, cudaStream_t s) {
-  // groups of four need 16-byte alignment (8 bytes for 16-bit types); up to three elements remain
+  // groups of four need 16-byte alignment (8 bytes for 16-bit types)
   const auto off = [](const void* p, size_t esz) { return ((uintptr_t)p) & (4 * esz - 1); };
   const bool wide = !(off(w, sizeof(TW)) | off(g, sizeof(TG)) | off(m, sizeof(TM)) | off(v, 4) | off(master, 4));
-  const long long whole = wide ? n / 4 * 4 : 0;
-  if (whole)
-    adam_kernel<TW, TG, TM, 4><<<xl_grid_for(whole, 256 * 8), 256, 0, s>>>((TW*)w, (const TG*)g, (TM*)m, v, master, step, a, whole);
-  if (whole < n)
-    adam_kernel<TW, TG, TM, 1><<<xl_grid_for(n - whole, 256 * 4), 256, 0, s>>>(
-        (TW*)w + whole, (const TG*)g + whole, (TM*)m + whole, v + whole, master ? master + whole : nullptr, step, a, n - whole);
+  if (wide)
+    adam_kernel<TW, TG, TM, 4><<<xl_grid_for(n, 256 * 8), 256, 0, s>>>((TW*)w, (const TG*)g, (TM*)m, v, master, step, a, n);
+  else
+    adam_kernel<TW, TG, TM, 1><<<xl_grid_for(n, 256 * 4), 256, 0, s>>>((TW*)w, (const TG*)g, (TM*)m, v, master, step, a, n);
 }
 template <typename TW, typename TG>
 static int adam_launch_m(void* w, const void* g, void* m, int m_dtype, float* v, float* master, float* step,
@@ -696,15 +707,14 @@ __global__ void __launch_bounds__(256)
     for (int e = 0; e < V; ++e) o[e] = o[e] * a + xv[e] * b;
     xl_stream_store<TA, V>(acc + i * V, o);
   }
+  const long long i = groups * V + threadIdx.x;  // up to three elements remain
+  if (blockIdx.x == 0 && i < n) acc[i] = xl_from_float<TA>(xl_to_float(acc[i]) * a + xl_to_float(x[i]) * b);
 }
 template <typename TA, typename TX>
 static void accumulate_mean_launch(void* acc, const void* x, const float* step, long long n, cudaStream_t s) {
   const bool wide = !((((uintptr_t)acc) & (4 * sizeof(TA) - 1)) | (((uintptr_t)x) & (4 * sizeof(TX) - 1)));
-  const long long whole = wide ? n / 4 * 4 : 0;
-  if (whole) accumulate_mean_kernel<TA, TX, 4><<<xl_grid_for(whole, 256 * 4), 256, 0, s>>>((TA*)acc, (const TX*)x, step, whole);
-  if (whole < n)
-    accumulate_mean_kernel<TA, TX, 1><<<xl_grid_for(n - whole, 256 * 4), 256, 0, s>>>((TA*)acc + whole, (const TX*)x + whole, step,
-                                                                                      n - whole);
+  if (wide) accumulate_mean_kernel<TA, TX, 4><<<xl_grid_for(n, 256 * 4), 256, 0, s>>>((TA*)acc, (const TX*)x, step, n);
+  else accumulate_mean_kernel<TA, TX, 1><<<xl_grid_for(n, 256 * 4), 256, 0, s>>>((TA*)acc, (const TX*)x, step, n);
 }
 XL_API int xl_accumulate_mean(void* acc, int acc_dtype, const void* x, int x_dtype, const float* step, long long n,
                               cudaStream_t s) {

@@ -124,6 +124,22 @@ def test_adam_writes_the_master_and_the_16_bit_weight(nat, n, offset, moment):
         assert torch.allclose(a, b, rtol=tol, atol=tol), (a - b).abs().max()
 
 
+@pytest.mark.parametrize("n", [1, 3, 5, 1023, 4099])
+@pytest.mark.parametrize("offset", [0, 1])
+@pytest.mark.parametrize("acc_dtype,dtype", [(torch.float32, torch.bfloat16), (torch.bfloat16, torch.float32), (torch.float32, torch.float32)])
+def test_running_mean_in_groups_and_the_elements_behind(nat, n, offset, acc_dtype, dtype):
+    """One launch for all of it, aligned or not, against 64 bits: three fp32 roundings of the result, and that to the accumulator's type."""
+    g = torch.Generator().manual_seed(n)
+    acc, x = torch.randn(n + 1, generator=g).to(acc_dtype)[offset:n + offset], torch.randn(n + 1, generator=g).to(dtype)[offset:n + offset]
+    bufs = [torch.empty(n + 1, dtype=t.dtype, device="cuda")[offset:n + offset].copy_(t) for t in (acc, x)]
+    step = torch.tensor(3.0, device="cuda")
+    rc = nat._acc_mean(bufs[0].data_ptr(), nat._CODE[acc_dtype], bufs[1].data_ptr(), nat._CODE[dtype], step.data_ptr(), n, nat._stream())
+    assert rc == 0
+    want = acc.double() * 0.75 + x.double() * 0.25
+    tol = 2.0 ** -22 if acc_dtype == torch.float32 else 2.0 ** -8
+    assert ((bufs[0].double().cpu() - want).abs() <= tol * (acc.double().abs() + x.double().abs())).all()
+
+
 @pytest.mark.parametrize("rows,cols,n", [(1, 4, 1), (5, 3, 9), (33, 130, 64), (100, 768, 257), (7, 8, 0)])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("t", [0.0, 3.0])
