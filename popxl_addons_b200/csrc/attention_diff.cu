@@ -541,12 +541,8 @@ template <int KD, int VT> int dd_launch(DecodeParams p, int B, int splits, cudaS
   int bytes = p.stages * stage;
   const int merge = DD_WARPS * 16 * p.vdim * 4;
   if (bytes < merge) bytes = merge;
-  static int configured = 0;
-  if (configured < bytes) {
-    const cudaError_t e = cudaFuncSetAttribute(diff_attn_decode_kernel<KD, VT>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    if (e != cudaSuccess) return (int)e;
-    configured = bytes;
-  }
+  static XlPerDevice smem;
+  XL_TRY(xl_allow_smem(diff_attn_decode_kernel<KD, VT>, bytes, smem));
   const int hchunks = (p.H / p.G + DD_HEADS - 1) / DD_HEADS;
   const cudaError_t e = xl_launch_overlapped(diff_attn_decode_kernel<KD, VT>, dim3(splits, p.G * hchunks, B), dim3(DD_WARPS * 32),
                                              (size_t)bytes, s, p);

@@ -343,13 +343,8 @@ int launch(const void* q, long long ldq, const void* kc, const void* vc, const D
   if (r) return r;
   r = make_map_bf16(&mv, vc, (long long)B * p.G * p.Smax, p.vdim, p.vdim, 64);
   if (r) return r;
-  static bool configured = false;
-  if (!configured) {
-    const cudaError_t e =
-        cudaFuncSetAttribute(diff_attn_tcgen05_kernel<DK, VD>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::TOTAL);
-    if (e != cudaSuccess) return (int)e;
-    configured = true;
-  }
+  static XlPerDevice smem;
+  XL_TRY(xl_allow_smem(diff_attn_tcgen05_kernel<DK, VD>, L::TOTAL, smem));
   const dim3 grid(p.H, (p.T + BLOCK_Q - 1) / BLOCK_Q, B);
   diff_attn_tcgen05_kernel<DK, VD><<<grid, NUM_THREADS, L::TOTAL, s>>>(mq, mk, mv, p);
   return (int)cudaGetLastError();

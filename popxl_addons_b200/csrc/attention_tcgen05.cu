@@ -487,13 +487,8 @@ int launch(const void* qkv, long long rows, long long cols, long long ld, const 
   if (r) return r;
   r = make_map(&mv, qkv, p.is_fp16, rows, cols, ld, 64);
   if (r) return r;
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(attn_fwd_tcgen05_kernel<D, BKV>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         L::TOTAL);
-    if (e != cudaSuccess) return (int)e;
-    configured = true;
-  }
+  static XlPerDevice smem;
+  XL_TRY(xl_allow_smem(attn_fwd_tcgen05_kernel<D, BKV>, L::TOTAL, smem));
   AttnParams q = p;
   q.items = attn_items(p.S, p.causal, BKV, p.chunk);
   if (q.items > 65535) return -1;

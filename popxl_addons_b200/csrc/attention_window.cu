@@ -555,13 +555,8 @@ template <int KD, int VT, int RT> int wd_launch_rows(WindowDecodeParams p, int B
   int bytes = p.stages * stage;
   const int merge = WD_WARPS * 8 * RT * p.vdim * 4;
   if (bytes < merge) bytes = merge;
-  static int configured = 0;
-  if (configured < bytes) {
-    const cudaError_t e =
-        cudaFuncSetAttribute(window_attn_decode_kernel<KD, VT, RT>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    if (e != cudaSuccess) return (int)e;
-    configured = bytes;
-  }
+  static XlPerDevice smem;
+  XL_TRY(xl_allow_smem(window_attn_decode_kernel<KD, VT, RT>, bytes, smem));
   const int hchunks = (p.H / p.G + 8 * RT - 1) / (8 * RT);
   const cudaError_t e = xl_launch_overlapped(window_attn_decode_kernel<KD, VT, RT>, dim3(splits, p.G * hchunks, B),
                                              dim3(WD_WARPS * 32), (size_t)bytes, s, p);

@@ -336,13 +336,8 @@ int launch(const void* qn, const void* kc, const void* vc, const WindowParams& p
   if (r) return r;
   r = make_map_bf16(&mv, vc, (long long)B * p.G * p.Smax, p.vdim, p.vdim, 64);
   if (r) return r;
-  static bool configured = false;
-  if (!configured) {
-    const cudaError_t e =
-        cudaFuncSetAttribute(window_attn_tcgen05_kernel<DK, VD>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::TOTAL);
-    if (e != cudaSuccess) return (int)e;
-    configured = true;
-  }
+  static XlPerDevice smem;
+  XL_TRY(xl_allow_smem(window_attn_tcgen05_kernel<DK, VD>, L::TOTAL, smem));
   const long long rows = (long long)p.T * (p.H / p.G);
   const dim3 grid(p.G, (unsigned)((rows + 2 * TILE_M - 1) / (2 * TILE_M)), B);
   window_attn_tcgen05_kernel<DK, VD><<<grid, NUM_THREADS, L::TOTAL, s>>>(mq, mk, mv, p);

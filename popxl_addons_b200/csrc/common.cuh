@@ -7,6 +7,10 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <mutex>
+
+#include "per_device.h"
+
 #define XL_API extern "C" __attribute__((visibility("default")))
 
 enum XlDtype : int { XL_F32 = 0, XL_F16 = 1, XL_BF16 = 2 };
@@ -179,6 +183,18 @@ __device__ __forceinline__ void xl_grid_launch_dependents() { asm volatile("grid
     const cudaError_t xl_e = (call);          \
     if (xl_e != cudaSuccess) return (int)xl_e; \
   } while (0)
+// Lets launches of `kernel` on the current device take `bytes` of dynamic shared memory. `granted`: what each device allows already.
+template <typename K> static inline cudaError_t xl_allow_smem(K kernel, int bytes, XlPerDevice& granted) {
+  int device = 0;
+  cudaError_t e = cudaGetDevice(&device);
+  if (e != cudaSuccess || granted.get(device) >= bytes) return e;
+  static std::mutex one_at_a_time;  // the attribute and what is known of it change together
+  const std::lock_guard<std::mutex> lock(one_at_a_time);
+  if (granted.get(device) >= bytes) return cudaSuccess;
+  e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  if (e == cudaSuccess) granted.set(device, bytes);
+  return e;
+}
 template <typename... P, typename... A>
 static inline cudaError_t xl_launch_overlapped(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A... args) {
   cudaLaunchConfig_t cfg = {};

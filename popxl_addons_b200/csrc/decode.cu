@@ -410,13 +410,8 @@ __global__ void __launch_bounds__(GqCfg<NT, WPB>::WARPS * 32, 1) gq_gemm_small_m
 
 template <typename T, typename S, int NT, int WPB> static int gq_small_launch(const GqParams& p, int ctas, cudaStream_t s) {
   using C = GqCfg<NT, WPB>;
-  static bool configured = false;
-  if (!configured) {
-    const cudaError_t e =
-        cudaFuncSetAttribute(gq_gemm_small_m_kernel<T, S, NT, WPB>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM);
-    if (e != cudaSuccess) return (int)e;
-    configured = true;
-  }
+  static XlPerDevice smem;
+  XL_TRY(xl_allow_smem(gq_gemm_small_m_kernel<T, S, NT, WPB>, C::SMEM, smem));
   const long long total = (long long)((p.N + C::COLS - 1) / C::COLS) * (p.K / GQ_KCHUNK);
   if (total > (1 << 30)) return -1;
   const int grid = (int)(total < ctas ? total : ctas);

@@ -536,14 +536,16 @@ int make_map(CUtensorMap* map, const void* ptr, int is_fp16, long long rows, lon
   return r == CUDA_SUCCESS ? 0 : -3;
 }
 
-// number of CTA pairs that can be resident at once on this device (0 if the query fails); looked up once
+// number of CTA pairs that can be resident at once on this device (0 if the query fails); looked up once per device
 template <int PN, int EPI>
 int max_resident_pairs() {
   constexpr int SMEM_TOTAL = PairCfg<PN>::SMEM_TOTAL;
-  static int cached = -1;
-  if (cached >= 0) return cached;
-  if (cudaFuncSetAttribute(gemm2cta_tcgen05_kernel<PN, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_TOTAL) != cudaSuccess) {
-    cached = 0;
+  static XlPerDevice known, smem;  // known: the number + 1
+  int device = 0;
+  if (cudaGetDevice(&device) != cudaSuccess) return 0;
+  if (known.get(device)) return known.get(device) - 1;
+  if (xl_allow_smem(gemm2cta_tcgen05_kernel<PN, EPI>, SMEM_TOTAL, smem) != cudaSuccess) {
+    known.set(device, 1);
     return 0;
   }
   cudaLaunchConfig_t cfg = {};
@@ -562,7 +564,7 @@ int max_resident_pairs() {
     cudaGetLastError();
     n = 0;
   }
-  cached = n;
+  known.set(device, n + 1);
   return n;
 }
 

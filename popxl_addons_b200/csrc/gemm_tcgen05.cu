@@ -840,14 +840,9 @@ template <int BLOCK_N>
 int launch(const CUtensorMap& ma, const CUtensorMap& mb, const GemmParams& p, int sm_count, cudaStream_t s,
            const CUtensorMap* ma2 = nullptr, const CUtensorMap* mb2 = nullptr) {
   using L = SmemLayout<BLOCK_N>;
-  static bool configured = false;
   constexpr int TOTAL_COMM = L::TOTAL + NUM_EPI_WARPS * EPI_STAGE_BYTES;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_tcgen05_kernel<BLOCK_N>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         TOTAL_COMM);
-    if (e != cudaSuccess) return (int)e;
-    configured = true;
-  }
+  static XlPerDevice smem;
+  XL_TRY(xl_allow_smem(gemm_tcgen05_kernel<BLOCK_N>, TOTAL_COMM, smem));
   const int smem_bytes = (p.accumulate == 3 || p.accumulate == 4) ? TOTAL_COMM : L::TOTAL;
   const int tiles = ((p.M + BLOCK_M - 1) / BLOCK_M) * ((p.N + BLOCK_N - 1) / BLOCK_N) * p.batch;
   // copy / reducer CTAs and GEMM CTAs wait on one another: all must be resident

@@ -368,13 +368,8 @@ template <int MODE, int NTOK> int sm_launch_tokens(SmParams p, int sms, cudaStre
   if (paired % L::PARTS) return -1;
   const int plain = MODE == SM_SPLIT_GLU ? (p.cols + 127) / 128 : 0;
   const int channels = paired / L::PARTS, chunks = (p.K + SM_KC - 1) / SM_KC, n_tiles = plain + (channels + L::CH - 1) / L::CH;
-  static bool configured = false;
-  if (!configured) {
-    const cudaError_t e =
-        cudaFuncSetAttribute(linear_small_m_kernel<MODE, NTOK>, cudaFuncAttributeMaxDynamicSharedMemorySize, R::SMEM);
-    if (e != cudaSuccess) return (int)e;
-    configured = true;
-  }
+  static XlPerDevice smem;
+  XL_TRY(xl_allow_smem(linear_small_m_kernel<MODE, NTOK>, R::SMEM, smem));
   // A power of two that two CTAs per SM have room for, at most eight. Room for one CTA per SM only was slower (16 tokens, 4096 x
   // 11008: 20.6 us with 4 CTAs per cluster, 18.0 with 8; 12288 x 4096: 22.5 with 1, 19.6 with 2), and so were clusters of 6 and 3
   // (6144 x 4096: 15.9 us with 6, 11.9 with 4; 12288 x 4096: 25.3 with 3).
