@@ -421,7 +421,7 @@ class Session:
         res = {}
         for stream, items in self._outputs.items():
             if len(items) == 1 and len(items[0]) == 1:
-                stacked = items[0][0][None, None]
+                stacked = items[0][0].contiguous()[None, None]
             else:
                 stacked = torch.stack([torch.stack(per_replica) for per_replica in items])  # (t, R_local, *shape)
             if not fetch:
