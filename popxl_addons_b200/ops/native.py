@@ -1287,6 +1287,8 @@ def advance_position_cuda(pos):
 
 @native("kv_cache_fill_")
 def kv_cache_fill_cuda(qkv, kc, vc, seq_len, n_heads, head_dim):
+    if head_dim * qkv.element_size() % 16:  # the plain copies take them, without the way through the library
+        return NotImplemented
     if not _ok(qkv, kc, vc) or not (qkv.dtype == kc.dtype == vc.dtype) or qkv.dim() != 2 or kc.shape != vc.shape:
         return NotImplemented
     B, H, smax, D = kc.shape
