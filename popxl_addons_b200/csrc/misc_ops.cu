@@ -225,16 +225,82 @@ XL_API int xl_scatter_add_rows(const void* grad_out, int dtype, const int* idx, 
   return (int)cudaGetLastError();
 }
 
+// V consecutive values of any type as fp32: single ones, or four with one access
+template <typename G, int V> __device__ __forceinline__ void xl_load_group(const G* p, float (&out)[V]) {
+  if constexpr (V == 1) {
+    out[0] = xl_to_float(*p);
+  } else if constexpr (sizeof(G) == 4) {
+    const float4 v = *reinterpret_cast<const float4*>(p);
+    out[0] = v.x; out[1] = v.y; out[2] = v.z; out[3] = v.w;
+  } else {
+    const uint2 v = *reinterpret_cast<const uint2*>(p);
+    const G* e = reinterpret_cast<const G*>(&v);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) out[i] = xl_to_float(e[i]);
+  }
+}
+
 // Running mean of an embedding table's gradient, without the dense gradient: acc = acc * t/(t+1), then the rows that the tokens
-// picked += grad_out / (t+1), t = *step. Bound by the first part, one read and write of the table; the second adds four fp32 values
-// per instruction (`red.v4`) where rows are aligned. 50400 x 4096 and 2048 tokens: zero fill, scatter, cast to 16 bits and dense
-// running mean took 0.85 ms, these two 0.27 + 0.015 ms.
-__global__ void __launch_bounds__(256) mean_decay_kernel(float* __restrict__ acc, const float* __restrict__ step, long long n) {
+// picked += (sum of their grad_out) / (t+1), t = *step. Bound by the first part, one read and write of the table. The second adds a
+// row's tokens up in an order that depends on the indices alone, so that the same inputs give the same bits (atomic additions did not:
+// a training step differed from itself by 1e-7). For that the first launch also sorts the tokens by row, in CTAs of its own beside the
+// pass over the table: a token's place is the number of tokens with a smaller row, and of earlier ones with the same.
+// 50400 x 4096, 2048 tokens: zero fill, scatter, cast and dense running mean took 783 us, a pass and atomic additions 270, this 298;
+// 50257 x 768, 4096 tokens 158, 51, 57; 1024 x 256, 256 tokens 7.2, 4.0, 5.2. 8192 tokens of a text (a frequent word has hundreds): 387.
+constexpr int EMB_TOKENS = 32768;           // tokens per pair of launches
+constexpr int EMB_SORTED = 64;              // tokens a CTA finds the places of, four threads each
+constexpr int EMB_NONE = 0x7fffffff;        // the row of a token outside the table: sorted behind all others
+__global__ void __launch_bounds__(256)
+    mean_decay_and_sort_kernel(float* __restrict__ acc, const float* __restrict__ step, long long n, const int* __restrict__ idx, int n_idx,
+                               int rows, int sort_ctas, int* __restrict__ order) {  // order: n_idx sorted rows, n_idx tokens
+  if ((int)blockIdx.x < sort_ctas) {
+    __shared__ __align__(16) int keys[1024];
+    const int first = blockIdx.x * EMB_SORTED, i = first + (threadIdx.x >> 2), q = threadIdx.x & 3;
+    auto key = [&](int j) {
+      const int r = j < n_idx ? idx[j] : -1;
+      return r >= 0 && r < rows ? r : EMB_NONE;
+    };
+    const int mine = key(i);
+    int place = 0;
+    for (int base = 0; base < n_idx; base += 1024) {
+      __syncthreads();
+#pragma unroll
+      for (int e = 0; e < 1024; e += 256) keys[e + threadIdx.x] = key(base + e + threadIdx.x);
+      __syncthreads();
+      // in fours: earlier tokens than the CTA's, the CTA's, later ones
+      const int4* k4 = reinterpret_cast<const int4*>(keys);
+      const int end = min(256, (n_idx - base + 3) / 4);
+      const int own = min(max(first - base, 0) / 4, end), later = min(max(first + EMB_SORTED - base, 0) / 4, end);
+#pragma unroll 8
+      for (int j = q; j < own; j += 4) {
+        const int4 k = k4[j];
+        place += (k.x <= mine) + (k.y <= mine) + (k.z <= mine) + (k.w <= mine);
+      }
+      for (int j = own + q; j < later; j += 4) {
+        const int4 k = k4[j];
+        const int at = base + 4 * j;
+        place += (k.x < mine || (k.x == mine && at < i)) + (k.y < mine || (k.y == mine && at + 1 < i)) +
+                 (k.z < mine || (k.z == mine && at + 2 < i)) + (k.w < mine || (k.w == mine && at + 3 < i));
+      }
+#pragma unroll 8
+      for (int j = later + q; j < end; j += 4) {
+        const int4 k = k4[j];
+        place += (k.x < mine) + (k.y < mine) + (k.z < mine) + (k.w < mine);
+      }
+    }
+    place += __shfl_xor_sync(0xffffffffu, place, 1);
+    place += __shfl_xor_sync(0xffffffffu, place, 2);
+    if (q == 0 && i < n_idx) {
+      order[place] = mine;
+      order[n_idx + place] = i;
+    }
+    return;
+  }
   const float t = *step;
   const float a = t / (t + 1.f);
   const long long groups = n / 4;
   float4* acc4 = reinterpret_cast<float4*>(acc);
-  const long long stride = (long long)gridDim.x * blockDim.x, first = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  const long long cta = blockIdx.x - sort_ctas, stride = (long long)(gridDim.x - sort_ctas) * 256, first = cta * 256 + threadIdx.x;
   for (long long i = first; i < groups; i += 2 * stride) {
     const bool two = i + stride < groups;
     float4 p = __ldcs(acc4 + i), q = two ? __ldcs(acc4 + i + stride) : make_float4(0.f, 0.f, 0.f, 0.f);
@@ -245,40 +311,133 @@ __global__ void __launch_bounds__(256) mean_decay_kernel(float* __restrict__ acc
   }
   if (first < n - groups * 4) acc[groups * 4 + first] *= a;
 }
-template <typename G, bool WIDE>
+
+// A warp takes the tokens of one row (from the place in the sorted list where they begin) and NB times 32 V columns. Rows with 32
+// tokens and more (padding, frequent words) are shared by the eight warps of the CTA, an eighth of the tokens each.
+template <typename G, int V, int NB>
 __global__ void __launch_bounds__(256)
-    scatter_mean_rows_kernel(const G* __restrict__ grad_out, const int* __restrict__ idx, float* __restrict__ acc,
-                             const float* __restrict__ step, int rows, int cols) {
-  const long long i = blockIdx.x;
-  const int r = idx[i];
-  if (r < 0 || r >= rows) return;
-  const float b = 1.f / (*step + 1.f);
-  const G* src = grad_out + i * cols;
-  float* dst = acc + (long long)r * cols;
-  if (WIDE) {
-    for (int c = threadIdx.x * 4; c < cols; c += blockDim.x * 4) {
-      float v[4];
+    add_sorted_rows_kernel(const G* __restrict__ grad_out, const int* __restrict__ order, float* __restrict__ acc,
+                           const float* __restrict__ step, int n_idx, int cols) {
+  constexpr int WIDTH = 32 * V * NB, AHEAD = 8 / NB;
+  __shared__ float part[8][WIDTH];
+  __shared__ int shared_row[8];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int place = blockIdx.x * 8 + warp, c = blockIdx.y * WIDTH + lane * V;  // and every 32 V columns on
+  const int *order_row = order, *order_token = order + n_idx;
+  float sum[NB][V], old[NB][V];
+  auto add_tokens = [&](int from, int to, int token) {  // token: of place from + lane
 #pragma unroll
-      for (int e = 0; e < 4; ++e) v[e] = xl_to_float(src[c + e]) * b;
-      asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst + c), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]) : "memory");
+    for (int q = 0; q < NB; ++q)
+#pragma unroll
+      for (int e = 0; e < V; ++e) sum[q][e] = 0.f;
+    for (int k0 = from; k0 < to; k0 += 32) {
+      const int n = min(32, to - k0);
+      if (k0 > from) token = lane < n ? order_token[k0 + lane] : 0;
+      for (int k1 = 0; k1 < n; k1 += AHEAD) {
+        float g[AHEAD][NB][V];
+#pragma unroll
+        for (int k = 0; k < AHEAD; ++k) {
+          const int tk = __shfl_sync(0xffffffffu, token, (k1 + k) & 31);
+#pragma unroll
+          for (int q = 0; q < NB; ++q)
+            if (k1 + k < n && c + q * 32 * V < cols) xl_load_group<G, V>(grad_out + (long long)tk * cols + c + q * 32 * V, g[k][q]);
+        }
+#pragma unroll
+        for (int k = 0; k < AHEAD; ++k)
+          if (k1 + k < n)
+#pragma unroll
+            for (int q = 0; q < NB; ++q)
+#pragma unroll
+              for (int e = 0; e < V; ++e) sum[q][e] += g[k][q][e];
+      }
     }
-  } else {
-    for (int c = threadIdx.x; c < cols; c += blockDim.x) atomicAdd(dst + c, xl_to_float(src[c]) * b);
+  };
+  auto load_old = [&](int row) {
+#pragma unroll
+    for (int q = 0; q < NB; ++q)
+      if (c + q * 32 * V < cols) xl_load_group<float, V>(acc + (long long)row * cols + c + q * 32 * V, old[q]);
+  };
+  const float b = 1.f / (*step + 1.f);
+  auto store = [&](int row) {
+#pragma unroll
+    for (int q = 0; q < NB; ++q) {
+      if (c + q * 32 * V >= cols) continue;
+      float* dst = acc + (long long)row * cols + c + q * 32 * V;
+#pragma unroll
+      for (int e = 0; e < V; ++e) old[q][e] += sum[q][e] * b;
+      if constexpr (V == 4) *reinterpret_cast<float4*>(dst) = make_float4(old[q][0], old[q][1], old[q][2], old[q][3]);
+      else dst[0] = old[q][0];
+    }
+  };
+  // the list around this warp's place, in one go: the row before it, its row and the 31 after, their tokens
+  const int at = place + lane;
+  const int row_at = at < n_idx ? order_row[at] : EMB_NONE, token = at < n_idx ? order_token[at] : 0;
+  const int before = place > 0 && place < n_idx ? order_row[place - 1] : EMB_NONE;
+  const int row = __shfl_sync(0xffffffffu, row_at, 0);
+  const bool begins = row != EMB_NONE && before != row;
+  const unsigned same = __ballot_sync(0xffffffffu, begins && row_at == row);
+  const bool shared = same == 0xffffffffu;
+  if (begins && !shared) {
+    load_old(row);
+    add_tokens(place, place + __popc(same), token);
+    store(row);
+  }
+  if (lane == 0) shared_row[warp] = shared ? row : EMB_NONE;
+  if (!__syncthreads_or(shared)) return;
+  for (int w = 0; w < 8; ++w) {
+    const int r = shared_row[w];
+    if (r == EMB_NONE) continue;
+    const int from = blockIdx.x * 8 + w;
+    int last = from + 31, end = n_idx;  // the row's tokens reach up to `last` at least and to before `end`
+    while (end - last > 1) {
+      const int gap = (end - last + 31) / 32, probe = last + (lane + 1) * gap;
+      const unsigned m = __ballot_sync(0xffffffffu, probe < end && order_row[min(probe, n_idx - 1)] == r);
+      last += __popc(m) * gap;
+      end = min(end, last + gap);
+    }
+    const int n = last + 1 - from, begin = from + (int)((long long)n * warp / 8), stop = from + (int)((long long)n * (warp + 1) / 8);
+    if (warp == 0) load_old(r);
+    add_tokens(begin, stop, begin + lane < stop ? order_token[begin + lane] : 0);
+#pragma unroll
+    for (int q = 0; q < NB; ++q)
+#pragma unroll
+      for (int e = 0; e < V; ++e) part[warp][(q * 32 + lane) * V + e] = sum[q][e];
+    __syncthreads();
+    if (warp == 0) {
+#pragma unroll
+      for (int q = 0; q < NB; ++q)
+#pragma unroll
+        for (int e = 0; e < V; ++e) {
+          sum[q][e] = 0.f;
+          for (int v = 0; v < 8; ++v) sum[q][e] += part[v][(q * 32 + lane) * V + e];
+        }
+      store(r);
+    }
+    __syncthreads();
   }
 }
-// acc: fp32 (rows, cols), contiguous and 16-byte aligned; grad_out: (n_idx, cols) of dtype.
+// Integers of scratch for n_idx tokens.
+XL_API long long xl_scatter_mean_scratch(long long n_idx) { return 2 * (n_idx < EMB_TOKENS ? n_idx : EMB_TOKENS); }
+// acc: fp32 (rows, cols), contiguous and 16-byte aligned; grad_out: (n_idx, cols) of dtype, aligned likewise. Indices outside the table
+// are skipped.
 XL_API int xl_scatter_mean_rows(const void* grad_out, int dtype, const int* idx, float* acc, const float* step, long long n_idx,
-                                int rows, int cols, cudaStream_t s) {
+                                int rows, int cols, int* order, cudaStream_t s) {
   const long long n = (long long)rows * cols;
   if (n < 1) return 0;
-  if (((uintptr_t)acc) & 15) return -1;
-  mean_decay_kernel<<<xl_grid_for(n, 256 * 8), 256, 0, s>>>(acc, step, n);
-  if (n_idx > 0) {
+  if ((((uintptr_t)acc) | ((uintptr_t)grad_out)) & 15 || (n_idx > 0 && !order)) return -1;
+  const int width = cols % 4 ? 32 : cols > 128 ? 256 : 128;  // columns per warp
+  if ((cols + width - 1) / width > 65535) return -1;
+  for (long long i0 = 0; i0 == 0 || i0 < n_idx; i0 += EMB_TOKENS) {
+    const int m = (int)(n_idx - i0 < EMB_TOKENS ? n_idx - i0 : EMB_TOKENS), sort_ctas = (m + EMB_SORTED - 1) / EMB_SORTED;
+    const int decay_ctas = i0 == 0 ? xl_grid_for(n, 256 * 8) : 0;  // the mean's old part once
+    mean_decay_and_sort_kernel<<<sort_ctas + decay_ctas, 256, 0, s>>>(acc, step, n, idx + i0, m, rows, sort_ctas, order);
+    if (m == 0) break;
+    const dim3 grid((m + 7) / 8, (cols + width - 1) / width);
     XL_DISPATCH_DTYPE(dtype, G, {
-      if (cols % 4 == 0)
-        scatter_mean_rows_kernel<G, true><<<(unsigned)n_idx, 256, 0, s>>>((const G*)grad_out, idx, acc, step, rows, cols);
-      else
-        scatter_mean_rows_kernel<G, false><<<(unsigned)n_idx, 256, 0, s>>>((const G*)grad_out, idx, acc, step, rows, cols);
+      const G* g = (const G*)grad_out + i0 * cols;
+      if (width == 256) add_sorted_rows_kernel<G, 4, 2><<<grid, 256, 0, s>>>(g, order, acc, step, m, cols);
+      else if (width == 128) add_sorted_rows_kernel<G, 4, 1><<<grid, 256, 0, s>>>(g, order, acc, step, m, cols);
+      else add_sorted_rows_kernel<G, 1, 1><<<grid, 256, 0, s>>>(g, order, acc, step, m, cols);
     });
   }
   return (int)cudaGetLastError();

@@ -121,7 +121,8 @@ _from_fp8 = _sig("xl_pow2_cast_from_fp8", _c_p, _c_p, _c_int, _c_p, _c_int, _c_l
 _mse_scale = _sig("xl_fp8_mse_scale", _c_p, _c_int, _c_ll, _c_p, _c_int, _c_int, ctypes.c_double, _c_p, _c_p)
 _csr_mm = _sig("xl_dense_csr_matmul", _c_p, _c_int, _c_p, _c_p, _c_p, _c_p, _c_int, _c_int, _c_int, _c_int, _c_p)
 _gather_rows = _sig("xl_gather_rows", _c_p, _c_int, _c_p, _c_p, _c_ll, _c_int, _c_int, _c_p)
-_scatter_mean_rows = _sig("xl_scatter_mean_rows", _c_p, _c_int, _c_p, _c_p, _c_p, _c_ll, _c_int, _c_int, _c_p)
+_scatter_mean_rows = _sig("xl_scatter_mean_rows", _c_p, _c_int, _c_p, _c_p, _c_p, _c_ll, _c_int, _c_int, _c_p, _c_p)
+_scatter_mean_scratch = _sig("xl_scatter_mean_scratch", _c_ll, restype=_c_ll)
 _scatter_rows = _sig("xl_scatter_add_rows", _c_p, _c_int, _c_p, _c_p, _c_ll, _c_int, _c_int, _c_p)
 _row_sum_sumsq = _sig("xl_row_sum_sumsq", _c_p, _c_int, _c_p, _c_int, _c_int, _c_p)
 _ln_apply_stats = _sig("xl_ln_apply_stats", _c_p, _c_int, _c_p, _c_p, _c_p, _c_p, _c_p, _c_p, _c_int, _c_int, _c_f, _c_f, _c_p)
@@ -1497,8 +1498,9 @@ def gather_grad_accumulate_mean_cuda(acc, g, idx, step, axis, zero_OOR):
             or not idx.is_contiguous() or step.dtype != torch.float32 or g.shape[-1] != acc.shape[1]
             or g.numel() != idx.numel() * acc.shape[1]):
         return NotImplemented
+    order = torch.empty(_scatter_mean_scratch(idx.numel()), dtype=torch.int32, device=acc.device)
     rc = _scatter_mean_rows(g.data_ptr(), _CODE[g.dtype], idx.data_ptr(), acc.data_ptr(), step.data_ptr(), idx.numel(),
-                            acc.shape[0], acc.shape[1], _stream())
+                            acc.shape[0], acc.shape[1], order.data_ptr(), _stream())
     if rc == -1:
         return NotImplemented
     _check(rc, "scatter_mean_rows")

@@ -159,6 +159,26 @@ def test_embedding_gradient_into_the_running_mean(nat, rows, cols, n, dtype, t):
     assert (dev.cpu().double() - want).abs().max() <= 1e-6 * max(1, n)
 
 
+@pytest.mark.parametrize("rows,cols,n", [(40, 256, 5000), (3000, 768, 4097), (3, 8196, 2048), (2, 2001, 33), (600, 4, 9000), (9, 132, 70),
+                                         (5, 12, 32768 + 300), (1, 64, 1024), (1000, 1, 300)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_embedding_gradient_repeats_itself(nat, rows, cols, n, dtype):
+    """Tokens with the frequencies of a text's words, so that rows get up to all of them: runs that one warp takes and runs that a CTA
+    shares, more tokens than a pair of launches sorts, ragged and single columns. The same inputs give the same bits. Each of m <=
+    n additions rounds a partial sum of about 4 sqrt(m) at most, with random signs."""
+    g = torch.Generator().manual_seed(rows * cols + n)
+    idx = (rows ** torch.rand(n, generator=g, dtype=torch.float64) - 1).int().clamp(0, rows - 1)
+    acc, grad, step = torch.randn(rows, cols, generator=g), torch.randn(n, cols, generator=g).to(dtype), torch.tensor(2.0, device="cuda")
+    dense = torch.zeros(rows, cols, dtype=torch.float64).index_add_(0, idx.long(), grad.double())
+    got = []
+    for _ in range(8):
+        dev = acc.cuda()
+        assert nat.gather_grad_accumulate_mean_cuda(dev, grad.cuda(), idx.cuda(), step, 0, False) is dev
+        got.append(dev.cpu())
+    assert all(torch.equal(got[0], y) for y in got[1:])
+    assert (got[0].double() - (acc.double() * (2 / 3) + dense / 3)).abs().max() <= 2.0 ** -24 * (4 * n + 16)
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("pairs", [False, True])
 @pytest.mark.parametrize("M,N,K,gs", [(1, 1, 128, 32), (8, 63, 256, 64), (9, 130, 384, 96), (16, 257, 1024, 128), (3, 640, 2048, 64),
