@@ -27,7 +27,8 @@
 // instruction: a nibble moved into the mantissa of a 16-bit float with a suitable exponent IS the number BASE + n (bf16:
 // 0x4300 | n = 128 + n; fp16: 0x5400 | n << 4 = 64 + n), two at a time, and the base goes with the zero point.
 // (De-quantising every weight to 16 bits took 5.5 instructions per weight, 46 % of the issue slots at a fifth of the bandwidth.
-// Both halves of the sum are of the size of BASE * |x|: activations above 2^120 overflow, and an infinite one gives NaN.)
+// Both halves of the sum are of the size of BASE * |x|: activations above 2^120 overflow, and an infinite one gives NaN. Results that
+// are not finite are therefore taken again from the weights themselves, gq_from_weights.)
 //
 // The channels are the rows of the `mma.sync.m16n8k16` tiles and the tokens their columns, so up to 8 tokens take one MMA per 256
 // weights and 9 to 16 tokens two. Lane (quad g, j) holds rows g and g + 8; of every block of 64 (or 32) k values lane j of a quad
@@ -125,8 +126,46 @@ template <int NT, int WPB> struct GqCfg {
   static constexpr int SMEM = WARPS * 2 * STAGE_UNITS * 16 + RED_FLOATS * 4;
 };
 
+template <typename T> __device__ __forceinline__ T gq_result(const GqParams& p, float sum, int n) {
+  float o = sum + (p.bias ? xl_to_float(((const T*)p.bias)[n]) : 0.f);
+  if (n >= p.act_from_col) o = 0.5f * o * (1.f + erff(o * 0.70710678118654752f));
+  return xl_from_float<T>(o);
+}
+
+// Results of a warp that are not finite, from weights that are de-quantised to T first: an infinite activation times a weight is what it
+// is elsewhere, and sums overflow only where the products do. The lanes in `mask` have stored row r, channels n .. n + 3; the warp
+// takes one result after another. Rare, so it is kept out of the registers of the kernel.
+template <typename T, typename S> __device__ __noinline__ void gq_from_weights(const GqParams& p, unsigned mask, int r, int n) {
+  const int lane = threadIdx.x & 31, groups = p.K / p.group_size;
+  __syncwarp();  // the stored results are read by all lanes
+  for (; mask; mask &= mask - 1) {
+    const int row = __shfl_sync(0xffffffffu, r, __ffs(mask) - 1), first = __shfl_sync(0xffffffffu, n, __ffs(mask) - 1);
+    for (int c = first; c < min(first + 4, p.N); ++c) {
+      T* y = (T*)p.y + (long long)row * p.ldy + c;
+      if (isfinite(xl_to_float(*y))) continue;
+      const uint16_t* codes = p.packed + (long long)c * (p.K / 4);
+      float sum = 0.f;
+      for (int k = lane * 8; k < p.K; k += 256) {
+        const int g = k / p.group_size;
+        const S* sz = p.sz_pairs ? (const S*)p.scale + 2 * ((long long)g * p.N + c) : (const S*)p.scale + (long long)c * groups + g;
+        const float s = xl_to_float(*sz), z = xl_to_float(p.sz_pairs ? sz[1] : ((const S*)p.zero)[(long long)c * groups + g]);
+        float x[8];
+        xl_load16((const T*)p.x + (long long)row * p.ldx + k, x);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+          const float w = xl_to_float(xl_from_float<T>(fmaf((float)((codes[k / 4 + e / 4] >> (12 - 4 * (e & 3))) & 15), s, z)));
+          sum = fmaf(x[e], w, sum);
+        }
+      }
+      sum = xl_warp_sum(sum);  // and all lanes have read *y
+      if (lane == 0) *y = gq_result<T>(p, sum, c);
+    }
+  }
+}
+
 template <typename T, typename S, int NT, int WPB>
-__global__ void __launch_bounds__(GqCfg<NT, WPB>::WARPS * 32, 1) gq_gemm_small_m_kernel(const GqParams p) {
+__global__ void __launch_bounds__(GqCfg<NT, WPB>::WARPS * 32, 1)
+    gq_gemm_small_m_kernel(const __grid_constant__ GqParams p) {
   using F = GqFmt<T>;
   using C = GqCfg<NT, WPB>;
   constexpr int CT = C::CT, COLS = C::COLS, BLOCKS = C::BLOCKS, SB = 32 * WPB, WARPS = C::WARPS;
@@ -374,17 +413,17 @@ __global__ void __launch_bounds__(GqCfg<NT, WPB>::WARPS * 32, 1) gq_gemm_small_m
         cta1 = ranges.owner(tile * chunks + chunks - 1);
         slot0 = ranges.begin(cta0) < tile * chunks ? 1 : 0;
       }
-      for (int i = threadIdx.x; i < p.M * (COLS / 4); i += blockDim.x) {
-        const int r = i / (COLS / 4), col = i % (COLS / 4) * 4, n = n_base + col;
-        if (n >= p.N) continue;
+      for (int i0 = warp * 32; i0 < p.M * (COLS / 4); i0 += WARPS * 32) {  // whole warps
+        const int i = i0 + lane, r = i / (COLS / 4), col = i % (COLS / 4) * 4, n = n_base + col;
+        const bool on = r < p.M && n < p.N;
         float v[4] = {0.f, 0.f, 0.f, 0.f};
-        if (whole) {
+        if (on && whole) {
 #pragma unroll
           for (int w = 0; w < WARPS; ++w) {
             const float4 o = *reinterpret_cast<const float4*>(red + (w * NT * 8 + r) * C::RED_LD + col);
             v[0] += o.x; v[1] += o.y; v[2] += o.z; v[3] += o.w;
           }
-        } else {
+        } else if (on) {
           const float* base = p.slots + r * COLS + col;
 #pragma unroll 4
           for (int k = cta0; k <= cta1; ++k) {
@@ -395,12 +434,11 @@ __global__ void __launch_bounds__(GqCfg<NT, WPB>::WARPS * 32, 1) gq_gemm_small_m
         T* yr = (T*)p.y + (long long)r * p.ldy + n;
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-          if (n + e < p.N) {
-            float o = v[e] + (p.bias ? xl_to_float(((const T*)p.bias)[n + e]) : 0.f);
-            if (n + e >= p.act_from_col) o = 0.5f * o * (1.f + erff(o * 0.70710678118654752f));
-            yr[e] = xl_from_float<T>(o);
-          }
+          if (on && n + e < p.N) yr[e] = gq_result<T>(p, v[e], n + e);
         }
+        // (a channel from N on has zero codes, scale and zero point: 0, or NaN for nothing that is stored)
+        const unsigned bad = __ballot_sync(0xffffffffu, on && !(isfinite(v[0]) && isfinite(v[1]) && isfinite(v[2]) && isfinite(v[3])));
+        if (bad) gq_from_weights<T, S>(p, bad, r, n);
       }
       if (!whole && threadIdx.x == 0) p.counters[tile] = 0;
     }

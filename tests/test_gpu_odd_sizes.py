@@ -202,6 +202,30 @@ def test_int4_product_at_the_edges_of_its_tiles(nat, dtype, pairs, M, N, K, gs):
     _near(y, want, dtype, terms=31 * K)
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("M,N,K,gs", [(5, 130, 256, 32), (16, 700, 4096, 64), (6, 64, 128, 64)])
+def test_int4_product_with_activations_that_are_not_finite(nat, dtype, M, N, K, gs):
+    """Infinite, missing and (bf16) nearly infinite activations give what they give as products with the weights: the sums of x times
+    the base of the codes, which overflow, do not show. Other rows keep their bits. Tiles of one CTA and tiles that CTAs share."""
+    g = torch.Generator(device="cuda").manual_seed(N + K)
+    x = torch.randn(M, K, generator=g, device="cuda").to(dtype)
+    codes = torch.randint(0, 16, (N, K // gs, gs // 4, 4), generator=g, device="cuda")
+    word = (codes[..., 0] << 12) | (codes[..., 1] << 8) | (codes[..., 2] << 4) | codes[..., 3]
+    packed = torch.where(word > 32767, word - 65536, word).to(torch.int16).view(torch.uint16)
+    scale, zero = (torch.full((N, K // gs, 1), v, device="cuda").half() for v in (0.02, -0.13))  # no weight is 0
+    scale[7], zero[7] = 0, 0                                                                     # but in one channel all are
+    bias = torch.randn(N, generator=g, device="cuda").to(dtype)
+    plain = nat.gq_gemm_small_m(x, packed, scale, zero, bias)
+    big = 2.0 ** 125 if dtype == torch.bfloat16 else 60000.0
+    x[0, 3], x[1, K - 1], x[2, 5], x[3, 9] = float("inf"), float("-inf"), float("nan"), big
+    y = nat.gq_gemm_small_m(x, packed, scale, zero, bias)
+    w = (codes.reshape(N, K // gs, gs).float() * scale.float() + zero.float()).to(dtype).double().reshape(N, K)
+    want = x.double() @ w.t() + bias.double()
+    torch.testing.assert_close(y[:4].double(), want[:4], rtol=2 * ROUND[dtype], atol=0.05 + 2.0 ** -8 * K ** 0.5, equal_nan=True)
+    assert y[0].isinf().sum() == N - 1 and y[3].isfinite().all()
+    assert torch.equal(y[4:], plain[4:])
+
+
 @pytest.mark.parametrize("rows,N,K", [(1, 1, 4), (2, 7, 132), (3, 2367, 1028), (4, 32000, 1024), (5, 30, 2816), (8, 2369, 68), (11, 513, 2048),
                                       (16, 1024, 1020)])
 def test_few_rows_product_in_32_bits(nat, rows, N, K):
