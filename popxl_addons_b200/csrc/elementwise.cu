@@ -1025,14 +1025,14 @@ XL_API int xl_attn_softmax_bwd(const void* p, void* dp, long long rows, int Sq, 
 template <typename T>
 __global__ void __launch_bounds__(512)
     ce_fwd_bwd_kernel(const T* __restrict__ logits, const int* __restrict__ labels, float* __restrict__ loss_row,
-                      T* __restrict__ dlogits, int V, int ldd, int ignore_index, const float* __restrict__ grad_scale_ptr,
-                      float grad_scale) {
+                      T* __restrict__ dlogits, int V, int ldd, int ignore_index, int clamp_labels,
+                      const float* __restrict__ grad_scale_ptr, float grad_scale) {
   constexpr int N = XlVec<T>::N;
   __shared__ float red[32];
   const long long row = blockIdx.x;
   const T* xr = logits + row * V;
-  const int label = labels[row];
-  const bool valid = label != ignore_index && label >= 0 && label < V;
+  const int given = labels[row], label = clamp_labels ? min(max(given, 0), V - 1) : given;
+  const bool valid = given != ignore_index && label >= 0 && label < V;
   const int nvec = V / N;
   auto load = [&](int i, float (&a)[N]) {
     const uint4 raw = xl_load16_any(xr + i * N);
@@ -1090,13 +1090,15 @@ __global__ void __launch_bounds__(512)
   for (int i = V + threadIdx.x; i < ldd; i += blockDim.x) dr[i] = xl_from_float<T>(0.f);
 }
 // logits (rows, V) contiguous; dlogits (rows, V) with row stride ldd >= V whose rows are 16-byte aligned (one row: any ldd).
+// Labels outside the classes: the nearest class with clamp_labels, else as `ignore_index`.
 XL_API int xl_ce_fwd_bwd(const void* logits, const int* labels, float* loss_row, void* dlogits, long long rows, int V, int ldd,
-                         int ignore_index, const float* grad_scale_ptr, float grad_scale, int dtype, cudaStream_t s) {
+                         int ignore_index, int clamp_labels, const float* grad_scale_ptr, float grad_scale, int dtype,
+                         cudaStream_t s) {
   const int vec = dtype == XL_F32 ? 4 : 8;
   if (rows < 1 || V < 1 || ldd < V || (((uintptr_t)dlogits) & 15) || (rows > 1 && ldd % vec != 0)) return -1;
   XL_DISPATCH_DTYPE(dtype, T, {
     ce_fwd_bwd_kernel<T><<<(unsigned)rows, 512, 0, s>>>((const T*)logits, labels, loss_row, (T*)dlogits, V, ldd, ignore_index,
-                                                       grad_scale_ptr, grad_scale);
+                                                       clamp_labels, grad_scale_ptr, grad_scale);
   });
   return (int)cudaGetLastError();
 }

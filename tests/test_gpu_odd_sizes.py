@@ -77,6 +77,27 @@ def test_cross_entropy_and_its_column_sums(nat, rows, V, dtype):
         _near(nat.matmul_cuda(d, b), want, dtype, scale=want.abs().max() + 1, terms=V)
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("V", [7, 1001, 1000])
+@pytest.mark.parametrize("reduction", ["none", "mean"])
+def test_cross_entropy_of_labels_outside_the_classes(nat, V, dtype, reduction):
+    """Rows of an odd number of classes: the nearest class, as in the op's reference. Rows of whole 16-byte pieces: masked, though
+    they count in the mean. Against 64 bits, one rounding of the result."""
+    g = torch.Generator(device="cuda").manual_seed(V)
+    x = torch.randn(6, V, device="cuda", generator=g).to(dtype)
+    lab = torch.tensor([-3, V, V + 400, 2, -100, V - 1], dtype=torch.int32, device="cuda")
+    loss, d = nat.ce_with_grad_cuda(x, lab, torch.ones((), device="cuda"), None, reduction)
+    given = lab.clamp(0, V - 1).long()
+    counts = (lab != -100) if V % 8 else (lab >= 0) & (lab < V)
+    xd = x.double().requires_grad_()
+    want = torch.nn.functional.cross_entropy(xd, given, reduction="none") * counts
+    if reduction == "mean":
+        want = want.sum() / 5
+    want.sum().backward()
+    torch.testing.assert_close(loss.double(), want.detach(), rtol=2 * ROUND[dtype], atol=2e-6)
+    torch.testing.assert_close(d.double(), xd.grad, rtol=2 * ROUND[dtype], atol=1e-6)
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
 @pytest.mark.parametrize("rows,V,valid", [(1, 1, 1), (1, 3, 2), (5, 33, 33), (16, 50400, 50257), (40, 32001, 32001), (700, 8190, 8189),
                                           (2, 70001, 70001)])
