@@ -1019,26 +1019,35 @@ XL_API int xl_attn_softmax_bwd(const void* p, void* dp, long long rows, int Sq, 
 // Cross-entropy on logits with the gradient fused: one CTA per row, two sweeps over the row. The first keeps a running maximum
 // and sum of exponentials per thread, the second (from L1 / L2: a row has at most ~100 KB) writes the gradient.
 // loss_row[r] = -log softmax(x)[label]; dlogits = (softmax - onehot) * grad_scale for valid rows, 0 for ignored rows. Mean
-// reduction and its 1/count are applied by the caller. Rows of logits may start at any element; rows of dlogits start at
-// multiples of `ldd` elements, 16-byte aligned, and their padding (V .. ldd) is written as zeros.
+// reduction and its 1/count are applied by the caller. Rows of dlogits start at multiples of `ldd` elements, 16-byte aligned, and
+// their padding (V .. ldd) is written as zeros. RAGGED: rows of logits start at any element, and for fp32 exponentials are exact: such
+// rows used to take softmax with expf, and the fast exponential's error grows with the distance from the maximum (2048 x 50257 fp32:
+// 224 -> 245 us, bound by the exponentials; softmax and its gradient step by step took 1007).
 // ------------------------------------------------------------------------------------------------------------------
-template <typename T>
+template <typename T, bool RAGGED>
 __global__ void __launch_bounds__(512)
     ce_fwd_bwd_kernel(const T* __restrict__ logits, const int* __restrict__ labels, float* __restrict__ loss_row,
-                      T* __restrict__ dlogits, int V, int ldd, int ignore_index, int clamp_labels,
-                      const float* __restrict__ grad_scale_ptr, float grad_scale) {
+                      T* __restrict__ dlogits, int V, int ldd, int ignore_index, const float* __restrict__ grad_scale_ptr,
+                      float grad_scale) {
   constexpr int N = XlVec<T>::N;
+  constexpr bool EXACT = RAGGED && sizeof(T) == 4;
   __shared__ float red[32];
   const long long row = blockIdx.x;
   const T* xr = logits + row * V;
-  const int given = labels[row], label = clamp_labels ? min(max(given, 0), V - 1) : given;
+  const int given = labels[row], label = RAGGED ? min(max(given, 0), V - 1) : given;
   const bool valid = given != ignore_index && label >= 0 && label < V;
   const int nvec = V / N;
   auto load = [&](int i, float (&a)[N]) {
-    const uint4 raw = xl_load16_any(xr + i * N);
+    uint4 raw;
+    if constexpr (RAGGED) raw = xl_load16_any(xr + i * N);
+    else raw = *reinterpret_cast<const uint4*>(xr + i * N);
     const T* e = reinterpret_cast<const T*>(&raw);
 #pragma unroll
     for (int k = 0; k < N; ++k) a[k] = xl_to_float(e[k]);
+  };
+  auto ex = [](float v) {
+    if constexpr (EXACT) return expf(v);
+    else return __expf(v);
   };
   float mx = -INFINITY, sum = 0.f;
 #pragma unroll 2
@@ -1048,26 +1057,31 @@ __global__ void __launch_bounds__(512)
     float m = mx;
 #pragma unroll
     for (int k = 0; k < N; ++k) m = fmaxf(m, a[k]);
-    if (m != mx) { sum *= __expf(mx - m); mx = m; }  // from -inf: the sum is still 0
+    if (m != mx) { sum *= ex(mx - m); mx = m; }  // from -inf: the sum is still 0
     if (mx == -INFINITY) {  // masked so far: nothing to add, but a NaN stays one
 #pragma unroll
       for (int k = 0; k < N; ++k) sum += a[k] != a[k] ? a[k] : 0.f;
       continue;
     }
 #pragma unroll
-    for (int k = 0; k < N; ++k) sum += __expf(a[k] - mx);
+    for (int k = 0; k < N; ++k) sum += ex(a[k] - mx);
   }
   for (int i = nvec * N + threadIdx.x; i < V; i += blockDim.x) {
     const float v = xl_to_float(xr[i]), m = fmaxf(mx, v);
-    if (m != mx) { sum *= __expf(mx - m); mx = m; }
-    sum += mx == -INFINITY ? (v != v ? v : 0.f) : __expf(v - mx);
+    if (m != mx) { sum *= ex(mx - m); mx = m; }
+    sum += mx == -INFINITY ? (v != v ? v : 0.f) : ex(v - mx);
   }
   const float top = xl_block_max(mx, red);
-  if (mx != top) sum *= __expf(mx - top);  // a thread without a finite value has the sum 0 (or NaN, which stays)
+  if (mx != top) sum *= ex(mx - top);  // a thread without a finite value has the sum 0 (or NaN, which stays)
   sum = xl_block_sum(sum, red);
-  const float lse = top + logf(sum);
-  if (threadIdx.x == 0) loss_row[row] = valid ? lse - xl_to_float(xr[label]) : 0.f;
+  const float log_sum = logf(sum), lse = top + log_sum;
+  // (top - x) + log_sum: top + log_sum alone is rounded to the size of the logits, the loss may be far smaller
+  if (threadIdx.x == 0) loss_row[row] = valid ? (top - xl_to_float(xr[label])) + log_sum : 0.f;
   if (dlogits == nullptr) return;
+  auto prob = [&](float v) {
+    if constexpr (EXACT) return expf(v - top) / sum;
+    else return __expf(v - lse);
+  };
   const float gs = valid ? (grad_scale_ptr ? *grad_scale_ptr * grad_scale : grad_scale) : 0.f;
   T* dr = dlogits + row * ldd;
 #pragma unroll 2
@@ -1076,29 +1090,31 @@ __global__ void __launch_bounds__(512)
     load(i, a);
 #pragma unroll
     for (int k = 0; k < N; ++k) {
-      float p = __expf(a[k] - lse);
+      float p = prob(a[k]);
       if (i * N + k == label) p -= 1.f;
       a[k] = p * gs;
     }
     xl_store16(dr + i * N, a);
   }
   for (int i = nvec * N + threadIdx.x; i < V; i += blockDim.x) {
-    float p = __expf(xl_to_float(xr[i]) - lse);
+    float p = prob(xl_to_float(xr[i]));
     if (i == label) p -= 1.f;
     dr[i] = xl_from_float<T>(p * gs);
   }
   for (int i = V + threadIdx.x; i < ldd; i += blockDim.x) dr[i] = xl_from_float<T>(0.f);
 }
 // logits (rows, V) contiguous; dlogits (rows, V) with row stride ldd >= V whose rows are 16-byte aligned (one row: any ldd).
-// Labels outside the classes: the nearest class with clamp_labels, else as `ignore_index`.
+// Labels outside the classes: the nearest class where rows of logits are ragged (several rows of no whole 16-byte pieces), else as
+// `ignore_index`.
 XL_API int xl_ce_fwd_bwd(const void* logits, const int* labels, float* loss_row, void* dlogits, long long rows, int V, int ldd,
-                         int ignore_index, int clamp_labels, const float* grad_scale_ptr, float grad_scale, int dtype,
-                         cudaStream_t s) {
+                         int ignore_index, const float* grad_scale_ptr, float grad_scale, int dtype, cudaStream_t s) {
   const int vec = dtype == XL_F32 ? 4 : 8;
   if (rows < 1 || V < 1 || ldd < V || (((uintptr_t)dlogits) & 15) || (rows > 1 && ldd % vec != 0)) return -1;
   XL_DISPATCH_DTYPE(dtype, T, {
-    ce_fwd_bwd_kernel<T><<<(unsigned)rows, 512, 0, s>>>((const T*)logits, labels, loss_row, (T*)dlogits, V, ldd, ignore_index,
-                                                       clamp_labels, grad_scale_ptr, grad_scale);
+    const bool ragged = (rows > 1 && V % vec != 0) || (((uintptr_t)logits) & 15);
+    const auto kernel = ragged ? ce_fwd_bwd_kernel<T, true> : ce_fwd_bwd_kernel<T, false>;
+    kernel<<<(unsigned)rows, 512, 0, s>>>((const T*)logits, labels, loss_row, (T*)dlogits, V, ldd, ignore_index, grad_scale_ptr,
+                                          grad_scale);
   });
   return (int)cudaGetLastError();
 }

@@ -79,7 +79,7 @@ _attn_bwd_dq = _sig("xl_attn_bwd_dq_tcgen05", _c_p, _c_ll, _c_ll, _c_p, _c_ll, _
                     _c_p)
 _attn_bwd_plan = _sig("xl_attn_bwd_plan", _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_p)
 _sm_bwd = _sig("xl_attn_softmax_bwd", _c_p, _c_p, _c_ll, _c_int, _c_int, _c_f, _c_int, _c_int, _c_p)
-_ce = _sig("xl_ce_fwd_bwd", _c_p, _c_p, _c_p, _c_p, _c_ll, _c_int, _c_int, _c_int, _c_int, _c_p, _c_f, _c_int, _c_p)
+_ce = _sig("xl_ce_fwd_bwd", _c_p, _c_p, _c_p, _c_p, _c_ll, _c_int, _c_int, _c_int, _c_p, _c_f, _c_int, _c_p)
 _pack_rows16 = _sig("xl_pack_rows16", _c_p, _c_ll, _c_p, _c_ll, _c_ll, _c_int, _c_p)
 _unpack_rows16 = _sig("xl_unpack_rows16", _c_p, _c_ll, _c_p, _c_ll, _c_int, _c_p)
 _gemm = _sig("xl_gemm_tcgen05", _c_p, _c_p, _c_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_ll, _c_ll, _c_ll,
@@ -1163,8 +1163,7 @@ def ce_with_grad_cuda(logits, labels, loss_grad, ignore_index, reduction):
         scale_t = lg.reshape(1)
     # Labels outside the classes count as the nearest class, as in the op's reference, where rows are no whole 16-byte pieces;
     # where they are, as masked.
-    clamp = rows > 1 and V % n != 0
-    rc = _ce(logits.data_ptr(), lab.data_ptr(), loss_row.data_ptr(), dlogits.data_ptr(), rows, V, ldd, ii, int(clamp),
+    rc = _ce(logits.data_ptr(), lab.data_ptr(), loss_row.data_ptr(), dlogits.data_ptr(), rows, V, ldd, ii,
              scale_t.data_ptr(), 1.0, _CODE[logits.dtype], _stream())
     if rc == -1:
         return NotImplemented

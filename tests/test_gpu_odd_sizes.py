@@ -54,19 +54,32 @@ def test_products(nat, M, K, N, dtype):
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
 @pytest.mark.parametrize("rows,V", [(1, 5), (3, 7), (2, 8), (65, 4099), (66, 1001), (70, 8193), (4, 50257)])
 def test_cross_entropy_and_its_column_sums(nat, rows, V, dtype):
+    """Element by element and relative to the element, with labels and large logits in the first piece of 16 bytes and in the
+    ragged last one, so that what a row's ends get wrong shows."""
     g = torch.Generator(device="cuda").manual_seed(V)
     x = (torch.randn(rows, V, device="cuda", generator=g) * 3).to(dtype)
-    x[:, : V // 2: 3] = float("-inf")  # masked classes
+    x[:, 2: V // 2: 3] = float("-inf")  # masked classes
     lab = torch.randint(V // 2, V, (rows,), device="cuda", generator=g, dtype=torch.int32)
+    lab[::3], lab[1::3] = 0, V - 1
+    x[::2, V - 1 - V % 3], x[1::2, 1] = 8, 9
     one = torch.ones((), device="cuda")
     loss, d = nat.ce_with_grad_cuda(x, lab, one, None, "none")
     xd = x.double().requires_grad_()
     want = torch.nn.functional.cross_entropy(xd, lab.long(), reduction="none")
     want.sum().backward()
-    torch.testing.assert_close(loss.double(), want.detach(), rtol=2 * ROUND[dtype], atol=2e-4)
-    # exp of __expf: 2 units in the last place and a relative 2^-22 per unit of the argument (up to 30)
-    _near(d, xd.grad, dtype, scale=max(1.0, ROUND[torch.float32] / ROUND[dtype] * 8))
+    torch.testing.assert_close(loss.double(), want.detach(), rtol=2 * ROUND[dtype], atol=1e-6)
+    # 16 bits: a rounding of the result, the fast exponential's relative 2^-22 per unit of its argument (up to 30) is far below it; fp16
+    # has steps of 2^-24 near 0. fp32: two units of the exponential, the rounded argument (up to 30), V / 512 additions per thread
+    # and the sums over threads and warps, a division. At the label the result is p - 1. (fp32 rows of whole 16-byte pieces and single
+    # rows: the fast exponential, 2 + 1.2 per unit of its argument.)
+    rel = ROUND[dtype] if dtype != torch.float32 else ((64 if rows > 1 and V % 4 else 128) + V / 512) * 2.0 ** -24
+    near0 = {torch.float16: 2.0 ** -24, torch.bfloat16: 0.0, torch.float32: 0.0}[dtype]
+    hit = torch.zeros_like(xd.grad).scatter_(1, lab.long()[:, None], 1.0)
+    off = (d.double() - xd.grad).abs()
+    assert (off <= rel * torch.maximum(xd.grad.abs(), hit) + near0).all()
     assert d.shape == x.shape
+    ldd = d.stride(0) if rows > 1 else V
+    assert (torch.as_strided(d, (rows, ldd), (ldd, 1))[:, V:] == 0).all()  # the padding behind every row
     s = nat.sum_cuda(d, (0,), False)
     if rows >= 64:
         assert s is not NotImplemented and s.shape == (V,)
@@ -75,6 +88,27 @@ def test_cross_entropy_and_its_column_sums(nat, rows, V, dtype):
     if dtype != torch.float32:
         want = d.double() @ b.double()
         _near(nat.matmul_cuda(d, b), want, dtype, scale=want.abs().max() + 1, terms=V)
+
+
+@pytest.mark.parametrize("V", [7, 1001, 50257])
+@pytest.mark.parametrize("shift", [0.0, 40.0])
+def test_cross_entropy_of_fp32_logits_is_as_exact_as_softmax(nat, V, shift):
+    """Rows of an odd number of classes: loss and gradient against 64 bits, no further away than from fp32 softmax with exact
+    exponentials, for logits of a trained model's spread around 0 and far from 0."""
+    g = torch.Generator(device="cuda").manual_seed(V)
+    x = torch.randn(64, V, device="cuda", generator=g) * 5 + shift
+    lab = torch.where(torch.arange(64, device="cuda") % 2 == 0, x.argmax(1), torch.randint(0, V, (64,), device="cuda", generator=g)).int()
+    x[::2] += 10 * torch.nn.functional.one_hot(lab[::2].long(), V)  # losses close to 0
+    loss, d = nat.ce_with_grad_cuda(x, lab, torch.ones((), device="cuda"), None, "none")
+    logp = torch.log_softmax(x.double(), 1)
+    hit = torch.nn.functional.one_hot(lab.long(), V)
+    want, want_loss = logp.exp() - hit, -logp.gather(1, lab.long()[:, None])[:, 0]
+    p32 = torch.softmax(x, 1)
+    loss32 = -torch.log(p32.gather(1, lab.long()[:, None])[:, 0])
+    away = lambda got: float(((got.double() - want).abs() / torch.maximum(want.abs(), hit)).square().mean().sqrt())
+    assert away(d) <= 1.25 * away(p32 - hit)
+    away = lambda got: float((got.double() - want_loss).square().mean().sqrt())
+    assert away(loss) <= 1.25 * away(loss32)
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
@@ -301,8 +335,8 @@ def test_general_attention_of_few_rows_equals_that_of_many(nat, kind, T, dim, vd
 @pytest.mark.parametrize("rows,N,K", [(17, 128, 64), (32, 129, 72), (33, 2048, 7680), (64, 300, 4096), (65, 8200, 8), (128, 1000, 520),
                                       (40, 32000, 2048)])
 def test_few_rows_product_at_the_edges_of_its_tiles(nat, out, rows, N, K):
-    """Each token tile, ragged weight rows and K, tiles that many CTAs share; twice, since the second launch finds the counters
-    as the first one left them. The activations are a slice of a wider matrix."""
+    """Each token tile, ragged weight rows and K, tiles that many CTAs share; twice, since the sums are added in a fixed order. The
+    activations are a slice of a wider matrix."""
     from popxl_addons_b200.ops.native_sequence import product
 
     g = torch.Generator(device="cuda").manual_seed(rows * N + K)
