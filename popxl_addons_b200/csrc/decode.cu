@@ -470,7 +470,8 @@ XL_API int xl_gq_gemm_small_m_slots(int ctas) { return ctas * 2 * 16 * 128; }
 // Requirements: M <= 16, K % 128 == 0, group_size % 32 == 0, 16-byte aligned x rows and weight rows. `ctas`: size of the grid (one
 // per SM). sz_pairs: `scale` holds (scale, zero) pairs laid out (K/gs, N, 2) and `zero` is unused. act_from_col: first column that
 // gets GELU (>= N: none). `dtype`: type of x, bias and y (fp16 or bf16); `scale_dtype`: type of the per-group scale and zero
-// point (fp16 / bf16). read_ahead: packed, scale and zero were complete before the previous launch on the stream. Returns -1 for unsupported arguments.
+// point (fp16 / bf16). read_ahead: packed, scale and zero were complete before the previous launch on the stream. Returns -1 for
+// unsupported arguments.
 XL_API int xl_gq_gemm_small_m(const void* x, const void* packed, const void* scale, const void* zero, const void* bias,
                               void* y, int M, int N, int K, int group_size, long long ldx, long long ldy, int act_from_col,
                               int ctas, float* slots, unsigned int* counters, int dtype, int scale_dtype, int sz_pairs,
@@ -478,8 +479,9 @@ XL_API int xl_gq_gemm_small_m(const void* x, const void* packed, const void* sca
   if (M < 1 || M > 16 || N < 1 || K < GQ_KCHUNK || K % GQ_KCHUNK || group_size < 32 || group_size % 32 || K % group_size ||
       dtype == XL_F32 || scale_dtype == XL_F32)
     return -1;
-  if ((ldx % 8) || ctas < 1 || slots == nullptr || counters == nullptr || (((uintptr_t)x | (uintptr_t)packed | (uintptr_t)scale) & 15)) return -1;
-  const GqParams p{x, ldx, (const uint16_t*)packed, scale, zero, sz_pairs, bias, y, ldy, M, N, K, group_size, act_from_col, slots, counters, read_ahead};
+  if ((ldx % 8) || ctas < 1 || !slots || !counters || (((uintptr_t)x | (uintptr_t)packed | (uintptr_t)scale) & 15)) return -1;
+  const GqParams p{x, ldx, (const uint16_t*)packed, scale, zero, sz_pairs, bias, y, ldy, M, N, K, group_size, act_from_col, slots,
+                   counters, read_ahead};
   if (dtype == XL_BF16)
     return scale_dtype == XL_F16 ? gq_small_pick<__nv_bfloat16, __half>(p, ctas, s) : gq_small_pick<__nv_bfloat16, __nv_bfloat16>(p, ctas, s);
   return scale_dtype == XL_F16 ? gq_small_pick<__half, __half>(p, ctas, s) : gq_small_pick<__half, __nv_bfloat16>(p, ctas, s);

@@ -13,8 +13,9 @@
 // The product is bandwidth-bound. The weight rows are the M = 128 operand of `tcgen05.mma` and the tokens (padded to 16, 32, 64 or
 // 128) its N, so that one thread keeps the tensor core ahead of HBM: four instructions per 16 KB of weights, about 65 clocks each,
 // are twice the rate at which an SM's share of the bandwidth arrives. TMA loads 128 x 64 blocks of weights, and the tokens' 64
-// columns beside them, into a ring of about 90 KB per CTA; one CTA per SM works on a product while one of the next product already
-// fills its ring (programmatic dependent launch: weights that the previous kernel does not write are requested while it drains).
+// columns beside them, into a ring of 90 to 100 KB per CTA, two CTAs per SM. The two are CTAs of one product (K is split until
+// both slots have one), or of a product that fills less than half of the slots and of its successor, whose ring fills while the
+// product drains (programmatic dependent launch: weights that the previous kernel does not write are requested ahead of its end).
 //
 // A tile of 128 weight rows belongs to a cluster of KS CTAs (1 to 8), each with an equal range of K blocks; KS is what the SMs have
 // room for. The CTAs leave their sums in shared memory, meet, and each finishes its share of the tile's results from the partial sums
@@ -413,10 +414,10 @@ int sm_check(const void* a, long long lda, const void* w, int M, int N, int K, i
 
 }  // namespace
 
-// All: a (M, K) bf16 with row stride lda (a multiple of 8), w (N, K) bf16 contiguous, M <= 16 (xl_linear_small_m: 128), K a multiple of 8; returns -1
-// for arguments the kernel does not take. read_ahead: w was complete before the previous launch on the stream. y (M, N) with row
-// stride ldy, bf16 or fp32. sumsq (M, sumsq_parts), or null: the rows
-// of y are multiplied by 1 / sqrt(sum of the row's sumsq / K + eps).
+// All: a (M, K) bf16 with row stride lda (a multiple of 8), w (N, K) bf16 contiguous, M <= 16 (xl_linear_small_m: 128), K a multiple
+// of 8; returns -1 for arguments the kernel does not take. read_ahead: w was complete before the previous launch on the stream. y
+// (M, N) with row stride ldy, bf16 or fp32. sumsq (M, sumsq_parts), or null: the rows of y are multiplied by
+// 1 / sqrt(sum of the row's sumsq / K + eps).
 XL_API int xl_linear_small_m(const void* a, long long lda, const void* w, void* y, long long ldy, int y_f32, const float* sumsq,
                              int sumsq_parts, float eps, int M, int N, int K, int sms, int read_ahead, int* err,
                              cudaStream_t s) {
@@ -471,8 +472,8 @@ XL_API int xl_linear_small_m_residual(const void* a, long long lda, const void* 
 }
 
 // w rows [gate | up] (2F, K); y (M, F) bf16 contiguous.
-XL_API int xl_linear_small_m_swiglu(const void* a, long long lda, const void* w, void* y, int M, int F, int K, int sms, int read_ahead, int* err,
-                                    cudaStream_t s) {
+XL_API int xl_linear_small_m_swiglu(const void* a, long long lda, const void* w, void* y, int M, int F, int K, int sms,
+                                    int read_ahead, int* err, cudaStream_t s) {
   if (sm_check(a, lda, w, M, 2 * F, K) || !y) return -1;
   SmParams p = {};
   p.a = (const __nv_bfloat16*)a; p.lda = lda; p.w = (const __nv_bfloat16*)w; p.M = M; p.N = 2 * F; p.K = K;

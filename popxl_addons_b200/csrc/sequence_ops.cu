@@ -366,11 +366,11 @@ template <typename T>
 int launch_stream(float* x, const void* y, float mult, const int* tokens, const void* table, int vocab, DytParams n, void* h,
                   long long rows, int cols, cudaStream_t s) {
   if (cols % 4 == 0) {
-    XL_TRY(xl_launch_overlapped(stream_dyt_kernel<T, 4>, dim3(xl_grid_for(rows * (cols / 4), 256)), dim3(256), (size_t)0, s, x, (const T*)y, mult, tokens, (const T*)table,
-                                                                               vocab, n, (T*)h, rows, cols));
+    XL_TRY(xl_launch_overlapped(stream_dyt_kernel<T, 4>, dim3(xl_grid_for(rows * (cols / 4), 256)), dim3(256), (size_t)0, s,
+                                x, (const T*)y, mult, tokens, (const T*)table, vocab, n, (T*)h, rows, cols));
   } else {
-    XL_TRY(xl_launch_overlapped(stream_dyt_kernel<T, 1>, dim3(xl_grid_for(rows * cols, 256)), dim3(256), (size_t)0, s, x, (const T*)y, mult, tokens, (const T*)table, vocab,
-                                                                         n, (T*)h, rows, cols));
+    XL_TRY(xl_launch_overlapped(stream_dyt_kernel<T, 1>, dim3(xl_grid_for(rows * cols, 256)), dim3(256), (size_t)0, s, x,
+                                (const T*)y, mult, tokens, (const T*)table, vocab, n, (T*)h, rows, cols));
   }
   return (int)cudaGetLastError();
 }
@@ -381,8 +381,8 @@ int launch_rms(float* x, const void* y, float mult, const int* tokens, const voi
   const int packs = (cols + V - 1) / V;
   const int threads = packs >= RMS_THREADS ? RMS_THREADS : (packs + 31) / 32 * 32;
 #define XL_RMS(NP)                                                                                                         \
-  XL_TRY(xl_launch_overlapped(stream_rms_kernel<T, V, NP>, dim3((unsigned)rows), dim3(threads), (size_t)0, s, x, (const T*)y, mult, tokens, (const T*)table, vocab, w,    \
-                                                                 eps, (T*)h, cols))
+  XL_TRY(xl_launch_overlapped(stream_rms_kernel<T, V, NP>, dim3((unsigned)rows), dim3(threads), (size_t)0, s, x, (const T*)y,  \
+                              mult, tokens, (const T*)table, vocab, w, eps, (T*)h, cols))
   if (packs <= RMS_THREADS) XL_RMS(1);
   else if (packs <= 4 * RMS_THREADS) XL_RMS(4);
   else XL_RMS(8);
@@ -408,7 +408,8 @@ XL_API int xl_select_rms(const float* x, const int* idx, int stride, int offset,
                          void* h, int rows, int cols, int dtype, cudaStream_t s) {
   if (rows < 1 || cols < 1 || x_rows < 1 || !w) return -1;
   XL_DISPATCH_DTYPE(dtype, T, {
-    XL_TRY(xl_launch_overlapped(select_rms_kernel<T>, dim3(rows), dim3(RMS_THREADS), (size_t)0, s, x, idx, stride, offset, x_rows, w, eps, (T*)h, cols));
+    XL_TRY(xl_launch_overlapped(select_rms_kernel<T>, dim3(rows), dim3(RMS_THREADS), (size_t)0, s, x, idx, stride, offset,
+                                x_rows, w, eps, (T*)h, cols));
   });
   return (int)cudaGetLastError();
 }
@@ -420,11 +421,11 @@ XL_API int xl_clamped_glu(const void* gate, long long ldg, void* y, long long ld
   XL_DISPATCH_DTYPE(dtype, T, {
     constexpr int V = 16 / sizeof(T);
     if (F % V == 0 && ldg % V == 0 && ldy % V == 0 && (((uintptr_t)gate | (uintptr_t)y) & 15) == 0)
-      XL_TRY(xl_launch_overlapped(clamped_glu_kernel<T, V>, dim3(xl_grid_for(rows * (F / V), 256)), dim3(256), (size_t)0, s, (const T*)gate, ldg, (T*)y, ldy, rows, F, limit,
-                                                                               slope, shift));
+      XL_TRY(xl_launch_overlapped(clamped_glu_kernel<T, V>, dim3(xl_grid_for(rows * (F / V), 256)), dim3(256), (size_t)0, s,
+                                  (const T*)gate, ldg, (T*)y, ldy, rows, F, limit, slope, shift));
     else
-      XL_TRY(xl_launch_overlapped(clamped_glu_kernel<T, 1>, dim3(xl_grid_for(rows * F, 256)), dim3(256), (size_t)0, s, (const T*)gate, ldg, (T*)y, ldy, rows, F, limit,
-                                                                         slope, shift));
+      XL_TRY(xl_launch_overlapped(clamped_glu_kernel<T, 1>, dim3(xl_grid_for(rows * F, 256)), dim3(256), (size_t)0, s,
+                                  (const T*)gate, ldg, (T*)y, ldy, rows, F, limit, slope, shift));
   });
   return (int)cudaGetLastError();
 }
@@ -445,7 +446,8 @@ XL_API int xl_select_dyt(const float* x, const int* idx, int stride, int offset,
   if (rows < 1 || cols < 1 || x_rows < 1 || !alpha || !w || !b) return -1;
   const DytParams n{alpha, w, b};
   XL_DISPATCH_DTYPE(dtype, T, {
-    XL_TRY(xl_launch_overlapped(select_dyt_kernel<T>, dim3(rows), dim3(256), (size_t)0, s, x, idx, stride, offset, x_rows, n, (T*)h, cols));
+    XL_TRY(xl_launch_overlapped(select_dyt_kernel<T>, dim3(rows), dim3(256), (size_t)0, s, x, idx, stride, offset, x_rows, n,
+                                (T*)h, cols));
   });
   return (int)cudaGetLastError();
 }
@@ -456,9 +458,11 @@ XL_API int xl_swiglu_packed(const void* gu, void* y, long long rows, int F, int 
   XL_DISPATCH_DTYPE(dtype, T, {
     constexpr int V = 16 / sizeof(T);
     if (F % V == 0)
-      XL_TRY(xl_launch_overlapped(swiglu_packed_kernel<T, V>, dim3(xl_grid_for(rows * (F / V), 256)), dim3(256), (size_t)0, s, (const T*)gu, (T*)y, rows, F));
+      XL_TRY(xl_launch_overlapped(swiglu_packed_kernel<T, V>, dim3(xl_grid_for(rows * (F / V), 256)), dim3(256), (size_t)0,
+                                  s, (const T*)gu, (T*)y, rows, F));
     else
-      XL_TRY(xl_launch_overlapped(swiglu_packed_kernel<T, 1>, dim3(xl_grid_for(rows * F, 256)), dim3(256), (size_t)0, s, (const T*)gu, (T*)y, rows, F));
+      XL_TRY(xl_launch_overlapped(swiglu_packed_kernel<T, 1>, dim3(xl_grid_for(rows * F, 256)), dim3(256), (size_t)0, s,
+                                  (const T*)gu, (T*)y, rows, F));
   });
   return (int)cudaGetLastError();
 }

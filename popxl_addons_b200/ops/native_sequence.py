@@ -1,5 +1,6 @@
 """CUDA implementations of the sequence-model ops (`xl/ops/sequence.py`): bf16 models run hand-written kernels throughout;
-32-bit models use plain fp32 matrix products (never a reduced-precision matrix mode) and the same kernels for the rest."""
+32-bit models use plain fp32 matrix products (an own kernel for few rows, else the vendor's, never in a reduced-precision matrix
+mode) and the same kernels for the rest."""
 import torch
 
 from ..xl import read_ahead
@@ -83,9 +84,9 @@ def _sumsq_args(sumsq, eps):
 
 
 def product(a, weight, out_dtype=None, sumsq=None, eps=0.0):
-    """`a (n, K) @ weight (N, K)^T` with 32-bit accumulation: the tcgen05 GEMM for 16-bit operands, the vendor product for
-    sizes it does not take and for 32-bit models. `sumsq`: `a` is half of a deferred norm (few rows only, else
-    NotImplemented)."""
+    """`a (n, K) @ weight (N, K)^T` with 32-bit accumulation. 16-bit operands: the few-rows kernel up to 128 rows, else the tcgen05
+    GEMM; 32-bit ones: a streaming kernel of fp32 FMAs for few rows; the vendor product for what these do not take. `sumsq`: `a`
+    is half of a deferred norm (bf16 and few rows only, else NotImplemented)."""
     out_dtype = out_dtype or a.dtype
     if a.dtype != torch.float32:
         # Up to 128 rows the product is bound by reading the weights. The GEMM multiplies tiles of 256 rows and does not
