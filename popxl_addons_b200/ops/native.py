@@ -101,7 +101,7 @@ _symm_all_gather_mc = _sig("xl_symm_all_gather_mc", _c_p, _c_p, _c_ll, _c_p, _c_
 _kv_fill = _sig("xl_kv_fill", _c_p, _c_ll, _c_p, _c_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_p)
 _gq_small_slots = _sig("xl_gq_gemm_small_m_slots", _c_int)
 _gq_small = _sig("xl_gq_gemm_small_m", _c_p, _c_p, _c_p, _c_p, _c_p, _c_p, _c_int, _c_int, _c_int, _c_int, _c_ll, _c_ll,
-                 _c_int, _c_int, _c_p, _c_p, _c_int, _c_int, _c_int, _c_int, _c_p)
+                 _c_int, _c_int, _c_p, _c_p, _c_int, _c_int, _c_int, _c_int, _c_p, _c_p)
 _rot_append = _sig("xl_rotary_append", _c_p, _c_ll, _c_p, _c_p, _c_p, _c_p, _c_p, _c_int, _c_int, _c_int, _c_int, _c_int,
                    _c_int, _c_p)
 _attn_dec = _sig("xl_attn_decode", _c_p, _c_ll, _c_p, _c_p, _c_p, _c_ll, _c_p, _c_p, _c_p, _c_int, _c_int, _c_int, _c_int,
@@ -1344,7 +1344,7 @@ def gq_gemm_small_m(x, packed, scale, zero, bias, out=None, act_from_col=None, c
                    bias.data_ptr() if bias is not None else None, y.data_ptr(), M, N, K, gs, x.stride(0), y.stride(0),
                    N if act_from_col is None else int(act_from_col), ctas,
                    ws.data_ptr(), done.data_ptr(), _CODE[x.dtype], _CODE[scale.dtype], int(transposed),
-                   int(read_ahead.allowed(packed, scale, zero)), _stream())
+                   int(read_ahead.allowed(packed, scale, zero)), gemm_error_flag(x.device).data_ptr(), _stream())
     if rc == -1:
         return NotImplemented
     _check(rc, "gq_gemm_small_m")

@@ -281,6 +281,38 @@ def test_int4_product_with_activations_that_are_not_finite(nat, dtype, M, N, K, 
     assert torch.equal(y[4:], plain[4:])
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("M,N,K,gs", [(1, 4, 128, 64), (8, 128, 256, 128), (9, 132, 384, 128), (16, 1000, 1152, 64), (16, 260, 2048, 256),
+                                      (3, 124, 1024, 512), (16, 640, 6144, 1024), (2, 20004, 512, 64), (13, 2048, 10240, 64)])
+def test_int4_product_through_the_ring(nat, dtype, M, N, K, gs):
+    """Scales as pairs: every group size the ring takes, half a chunk at the end of K, ragged channels, tiles of one CTA and of many, more
+    chunks than the ring holds; against 64 bits, against the kernel that takes the same weights with their scales apart, the same bits
+    twice, and a row that is not finite. Sums of x times (base + code) as above."""
+    from popxl_addons_b200.layers.linear_gq import interleave_scale_zero
+
+    g = torch.Generator(device="cuda").manual_seed(M * N + K)
+    x = torch.randn(M, K, generator=g, device="cuda").to(dtype)
+    codes = torch.randint(0, 16, (N, K // gs, gs // 4, 4), generator=g, device="cuda")
+    word = (codes[..., 0] << 12) | (codes[..., 1] << 8) | (codes[..., 2] << 4) | codes[..., 3]
+    packed = torch.where(word > 32767, word - 65536, word).to(torch.int16).view(torch.uint16)
+    scale = (0.02 + 0.02 * torch.rand(N, K // gs, 1, generator=g, device="cuda")).half()
+    zero = (-0.3 + 0.1 * torch.rand(N, K // gs, 1, generator=g, device="cuda")).half()
+    pairs, bias = interleave_scale_zero(scale, zero), torch.randn(N, generator=g, device="cuda").to(dtype)
+    w = codes.reshape(N, K // gs, gs).double() * scale.double() + zero.double()
+    want = x.double() @ w.reshape(N, K).t() + bias.double()
+    first = nat.gq_gemm_small_m(x, packed, pairs, None, bias)
+    for ctas in (None, 3, 1):
+        y = nat.gq_gemm_small_m(x, packed, pairs, None, bias, ctas=ctas)
+        _near(y, want, dtype, terms=31 * K)
+        assert ctas or torch.equal(y, first)
+    _near(nat.gq_gemm_small_m(x, packed, scale, zero, bias), want, dtype, terms=31 * K)
+    x[M // 2, K - 1] = float("inf")
+    y = nat.gq_gemm_small_m(x, packed, pairs, None, bias)
+    assert y[M // 2].isinf().all() or (w.reshape(N, K)[:, K - 1] == 0).any()
+    assert torch.equal(y[M // 2 + 1:], first[M // 2 + 1:]) and torch.equal(y[:M // 2], first[:M // 2])
+    nat.check_gemm_errors()
+
+
 @pytest.mark.parametrize("rows,N,K", [(1, 1, 4), (2, 7, 132), (3, 2367, 1028), (4, 32000, 1024), (5, 30, 2816), (8, 2369, 68), (11, 513, 2048),
                                       (16, 1024, 1020)])
 def test_few_rows_product_in_32_bits(nat, rows, N, K):
