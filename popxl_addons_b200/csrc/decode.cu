@@ -3,7 +3,6 @@
 //                        once and fed to the tensor cores as codes; scales and zero points meet the fp32 sums
 //   xl_rotary_at         rotary embedding of the new tokens at a position read from device memory
 //   xl_kv_append         write the new keys / values into the KV cache at that position
-//   xl_attn_decode       attention of the new query against the cache (split over the sequence + combine)
 //   xl_argmax_rows       greedy sampling: per-row (max, index) of the local logits slice
 // Everything that depends on the current position reads it from a device word, so one decoding step has no
 // launch-time argument that changes between steps and can be replayed as a CUDA graph.
@@ -462,181 +461,6 @@ XL_API int xl_kv_fill(const void* qkv, long long ld, void* k_cache, void* v_cach
   if ((((uintptr_t)qkv) | ((uintptr_t)k_cache) | ((uintptr_t)v_cache)) & 15) return -1;
   kv_fill_kernel<<<xl_grid_for(total, 256 * 4), 256, 0, s>>>((const uint4*)qkv, (uint32_t)(ld / n), (uint4*)k_cache, (uint4*)v_cache,
                                                             (uint32_t)total, (uint32_t)S, (uint32_t)H, (uint32_t)(D / n), (uint32_t)Smax);
-  return (int)cudaGetLastError();
-}
-
-// ------------------------------------------------------------------------------------------------------------------
-// Decode attention: one query per (b, h) against cache positions [0, len), len = *pos_ptr + 1, one launch.
-// Grid (B*H, splits): each CTA covers a slice of the positions with an online softmax. A warp takes four positions per
-// iteration (lanes over the head dimension, one vector load of D/32 values per lane, position and tensor), so eight
-// independent loads are in flight per lane. Each CTA writes (max, sum, unnormalised output) of its slice; the last CTA
-// of a (b, h) to finish (a counter per (b, h), left at zero again) merges the slices and writes the output row.
-// ------------------------------------------------------------------------------------------------------------------
-constexpr int AD_WARPS = 4;
-constexpr int AD_MAX_D = 256;  // head_dim <= 256 (8 values per lane)
-constexpr int AD_UNROLL = 4;
-
-template <typename T, int VPL>
-struct alignas(VPL * 2 >= 16 ? 16 : (VPL == 4 ? 8 : (VPL == 2 ? 4 : 2))) AdVec {
-  T v[VPL];
-};
-
-template <typename T, int VPL>
-__global__ void __launch_bounds__(AD_WARPS * 32)
-    attn_decode_kernel(const T* qkv, long long ldq, const T* k_cache, const T* v_cache, T* out, long long ldo, float* part,
-                       unsigned int* counters, const int* pos_ptr, int H, int Smax, float scale) {
-  constexpr int D = VPL * 32;
-  using Vec = AdVec<T, VPL>;
-  xl_grid_dependency_wait();
-  xl_grid_launch_dependents();
-  const int bh = blockIdx.x, split = blockIdx.y, splits = gridDim.y;
-  const int b = bh / H, h = bh % H;
-  const int len = min(*pos_ptr + 1, Smax);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int per = (len + splits - 1) / splits;
-  const int s_begin = split * per, s_end = min(len, s_begin + per);
-  const T* kb = k_cache + ((long long)bh * Smax) * D + lane * VPL;
-  const T* vb = v_cache + ((long long)bh * Smax) * D + lane * VPL;
-  float q[VPL], o[VPL];
-  {
-    const Vec qv = *reinterpret_cast<const Vec*>(qkv + (long long)b * ldq + h * D + lane * VPL);
-#pragma unroll
-    for (int e = 0; e < VPL; ++e) {
-      q[e] = xl_to_float(qv.v[e]) * scale;
-      o[e] = 0.f;
-    }
-  }
-  float m = -INFINITY, l = 0.f;
-  for (int s0 = s_begin + warp * AD_UNROLL; s0 < s_end; s0 += AD_WARPS * AD_UNROLL) {
-    Vec kk[AD_UNROLL], vv[AD_UNROLL];
-#pragma unroll
-    for (int u = 0; u < AD_UNROLL; ++u) {
-      const int sidx = min(s0 + u, s_end - 1);  // clamped: the duplicates are masked out below
-      kk[u] = *reinterpret_cast<const Vec*>(kb + (long long)sidx * D);
-      vv[u] = *reinterpret_cast<const Vec*>(vb + (long long)sidx * D);
-    }
-    float dot[AD_UNROLL];
-#pragma unroll
-    for (int u = 0; u < AD_UNROLL; ++u) {
-      float d = 0.f;
-#pragma unroll
-      for (int e = 0; e < VPL; ++e) d += q[e] * xl_to_float(kk[u].v[e]);
-      dot[u] = d;
-    }
-    // four sums over 32 lanes by halving: lanes with bits 16 and 8 (a, b) end up with the sum of dot[2 a + b]
-    // (Requesting the next group's keys and values ahead of this arithmetic took the registers of a fifth of the warps: 23.9 us
-    // against 18.7 for 16 sequences of 576, 16 heads of 128.)
-    const bool hi16 = lane & 16, hi8 = lane & 8;
-    float d0 = (hi16 ? dot[2] : dot[0]) + __shfl_xor_sync(0xffffffffu, hi16 ? dot[0] : dot[2], 16);
-    float d1 = (hi16 ? dot[3] : dot[1]) + __shfl_xor_sync(0xffffffffu, hi16 ? dot[1] : dot[3], 16);
-    d0 = (hi8 ? d1 : d0) + __shfl_xor_sync(0xffffffffu, hi8 ? d0 : d1, 8);
-#pragma unroll
-    for (int off = 4; off > 0; off >>= 1) d0 += __shfl_xor_sync(0xffffffffu, d0, off);
-    float m_new = m;
-#pragma unroll
-    for (int u = 0; u < AD_UNROLL; ++u) {
-      dot[u] = __shfl_sync(0xffffffffu, d0, u * 8);
-      if (s0 + u >= s_end) dot[u] = -INFINITY;
-      m_new = fmaxf(m_new, dot[u]);
-    }
-    const float corr = __expf(m - m_new);  // m_new is finite here: position s0 is valid
-    l *= corr;
-#pragma unroll
-    for (int e = 0; e < VPL; ++e) o[e] *= corr;
-#pragma unroll
-    for (int u = 0; u < AD_UNROLL; ++u) {
-      const float p = __expf(dot[u] - m_new);  // exp(-inf) = 0 for the masked duplicates
-      l += p;
-#pragma unroll
-      for (int e = 0; e < VPL; ++e) o[e] += p * xl_to_float(vv[u].v[e]);
-    }
-    m = m_new;
-  }
-  // merge the warps of this CTA
-  __shared__ float sm[AD_WARPS], sl[AD_WARPS], so[AD_WARPS][AD_MAX_D];
-  __shared__ unsigned int is_last;
-  if (lane == 0) { sm[warp] = m; sl[warp] = l; }
-#pragma unroll
-  for (int e = 0; e < VPL; ++e) so[warp][lane * VPL + e] = o[e];
-  __syncthreads();
-  float* mine = part + ((long long)bh * splits + split) * (D + 2);
-  if (warp == 0) {
-    float mm = -INFINITY;
-    for (int w = 0; w < AD_WARPS; ++w) mm = fmaxf(mm, sm[w]);
-    float ll = 0.f;
-    float acc[VPL];
-#pragma unroll
-    for (int e = 0; e < VPL; ++e) acc[e] = 0.f;
-    for (int w = 0; w < AD_WARPS; ++w) {
-      const float f = (sm[w] == -INFINITY) ? 0.f : __expf(sm[w] - mm);
-      ll += sl[w] * f;
-#pragma unroll
-      for (int e = 0; e < VPL; ++e) acc[e] += so[w][lane * VPL + e] * f;
-    }
-    if (splits == 1) {
-      const float inv = 1.f / ll;
-      Vec r;
-#pragma unroll
-      for (int e = 0; e < VPL; ++e) r.v[e] = xl_from_float<T>(acc[e] * inv);
-      *reinterpret_cast<Vec*>(out + (long long)b * ldo + h * D + lane * VPL) = r;
-    } else {
-      if (lane == 0) { mine[0] = mm; mine[1] = ll; }
-#pragma unroll
-      for (int e = 0; e < VPL; ++e) mine[2 + lane * VPL + e] = acc[e];
-    }
-  }
-  if (splits == 1) return;
-  __threadfence();
-  __syncthreads();
-  if (threadIdx.x == 0) is_last = atomicAdd(counters + bh, 1u) == (unsigned int)splits - 1;
-  __syncthreads();
-  if (!is_last) return;
-  __threadfence();
-  const float* p = part + (long long)bh * splits * (D + 2);
-  float mm = -INFINITY;
-  for (int sp = 0; sp < splits; ++sp) mm = fmaxf(mm, __ldcg(p + sp * (D + 2)));
-  float ll = 0.f;
-  for (int sp = 0; sp < splits; ++sp) {
-    const float ms = __ldcg(p + sp * (D + 2));
-    ll += (ms == -INFINITY) ? 0.f : __ldcg(p + sp * (D + 2) + 1) * __expf(ms - mm);
-  }
-  for (int d = threadIdx.x; d < D; d += blockDim.x) {
-    float acc = 0.f;
-    for (int sp = 0; sp < splits; ++sp) {
-      const float ms = __ldcg(p + sp * (D + 2));
-      if (ms != -INFINITY) acc += __ldcg(p + sp * (D + 2) + 2 + d) * __expf(ms - mm);
-    }
-    out[(long long)b * ldo + h * D + d] = xl_from_float<T>(acc / ll);
-  }
-  if (threadIdx.x == 0) counters[bh] = 0;
-}
-
-// q: rows of ldq elements (the first H*D are used); out: rows of ldo elements (H*D written). scratch: at least
-// B*H*splits*(D+2) floats; counters: B*H zero-initialised words (left zeroed). D in {64, 128, 256}; ldq, ldo and the
-// window offsets must keep every head 16-byte aligned.
-XL_API int xl_attn_decode(const void* qkv, long long ldq, const void* k_cache, const void* v_cache, void* out, long long ldo,
-                          float* scratch, unsigned int* counters, const int* pos_ptr, int B, int H, int D, int Smax,
-                          float scale, int splits, int dtype, cudaStream_t s) {
-  if ((D != 64 && D != 128 && D != 256) || splits < 1 || dtype == XL_F32 || (ldq % 8) || (ldo % 8)) return -1;
-  if (splits > 1 && (scratch == nullptr || counters == nullptr)) return -1;
-  dim3 grid(B * H, splits);
-#define XL_AD_LAUNCH(T, VPL)                                                                                          \
-  do {                                                                                                                \
-    const cudaError_t e = xl_launch_overlapped(attn_decode_kernel<T, VPL>, grid, dim3(AD_WARPS * 32), (size_t)0, s,   \
-                                               (const T*)qkv, ldq, (const T*)k_cache, (const T*)v_cache, (T*)out, ldo, scratch, \
-                                               counters, pos_ptr, H, Smax, scale);                                    \
-    if (e != cudaSuccess) return (int)e;                                                                              \
-  } while (0)
-  if (dtype == XL_BF16) {
-    if (D == 256) XL_AD_LAUNCH(__nv_bfloat16, 8);
-    else if (D == 128) XL_AD_LAUNCH(__nv_bfloat16, 4);
-    else XL_AD_LAUNCH(__nv_bfloat16, 2);
-  } else {
-    if (D == 256) XL_AD_LAUNCH(__half, 8);
-    else if (D == 128) XL_AD_LAUNCH(__half, 4);
-    else XL_AD_LAUNCH(__half, 2);
-  }
-#undef XL_AD_LAUNCH
   return (int)cudaGetLastError();
 }
 

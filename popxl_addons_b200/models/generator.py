@@ -209,15 +209,15 @@ class DecoderGenerator:
                 return ops.add_layer_norm_(x, delta, delta_bias, lnw, lnb, eps=cfg.eps)
 
             def decode_block(x, delta, delta_bias, L, pos):
-                """One token per sequence, five kernels: (all-reduce +) residual + LayerNorm; [qkv | gelu(fc_in)] in one
-                de-quantising GEMM; rotary + cache append; attention, written next to the fc_in output; [out | fc_out] in
+                """One token per sequence, four kernels: (all-reduce +) residual + LayerNorm; [qkv | gelu(fc_in)] in one
+                de-quantising GEMM; rotary, cache append and attention, written next to the fc_in output; [out | fc_out] in
                 one GEMM. Returns this rank's partial layer output; the next layer's first kernel reduces it."""
                 h = residual_norm(x, delta, delta_bias, L["ln_w"], L["ln_b"])
                 w1 = L["w1"]
                 buf = linear_gq_window_t(h, w1["weight_compressed"], w1["weight_scale_zero_t"], w1["bias"],
                                          act_from_col=3 * hd)
-                buf = ops.rotary_kv_append_(buf, sin_tab_i, cos_tab_i, L["k"], L["v"], pos, H, D, cfg.rotary_dim)
-                buf = ops.attention_decode_into_(buf, L["k"], L["v"], pos, H, D, out_col=2 * hd)
+                buf = ops.rotary_attention_decode_into_(buf, sin_tab_i, cos_tab_i, L["k"], L["v"], pos, H, D, cfg.rotary_dim,
+                                                        out_col=2 * hd)
                 w2 = L["w2"]
                 return linear_gq_window_t(buf, w2["weight_compressed"], w2["weight_scale_zero_t"], None, x_col=2 * hd,
                                           k=hd + F)

@@ -104,8 +104,8 @@ _gq_small = _sig("xl_gq_gemm_small_m", _c_p, _c_p, _c_p, _c_p, _c_p, _c_p, _c_in
                  _c_int, _c_int, _c_p, _c_p, _c_int, _c_int, _c_int, _c_int, _c_p, _c_p)
 _rot_append = _sig("xl_rotary_append", _c_p, _c_ll, _c_p, _c_p, _c_p, _c_p, _c_p, _c_int, _c_int, _c_int, _c_int, _c_int,
                    _c_int, _c_p)
-_attn_dec = _sig("xl_attn_decode", _c_p, _c_ll, _c_p, _c_p, _c_p, _c_ll, _c_p, _c_p, _c_p, _c_int, _c_int, _c_int, _c_int,
-                 _c_f, _c_int, _c_int, _c_p)
+_attn_dec = _sig("xl_attn_decode", _c_p, _c_ll, _c_p, _c_p, _c_p, _c_p, _c_p, _c_ll, _c_p, _c_p, _c_p, _c_int, _c_int, _c_int, _c_int,
+                 _c_int, _c_f, _c_int, _c_int, _c_int, _c_int, _c_p, _c_p)
 _ar_add_ln = _sig("xl_ar_add_layer_norm", _c_p, _c_p, _c_p, _c_p, _c_p, _c_p, _c_int, _c_int, _c_f, _c_int, _c_p, _c_p, _c_ll,
                   _c_p, _c_p, _c_int, _c_int, _c_int, _c_p, _c_p)
 _add_ln = _sig("xl_add_layer_norm", _c_p, _c_p, _c_p, _c_p, _c_p, _c_p, _c_int, _c_int, _c_f, _c_int, _c_p)
@@ -157,18 +157,19 @@ def _count(name: str):
     order = read_ahead.current()
     if order is not None:
         order.launched(_stream())
-    LAUNCHES["count"] += 1
-    LAUNCHES["by_kernel"][name] = LAUNCHES["by_kernel"].get(name, 0) + 1
+    count_replay([name])
     if _RECORDING:
         _RECORDING[-1].append(name)
 
 
 def count_replay(names):
-    """Account for the kernels of a captured graph each time it is replayed."""
+    """Account for the kernels of a captured graph each time it is replayed. "a+b" is one launch that does the work of the kernels a
+    and b: it counts once, and under both names."""
     LAUNCHES["count"] += len(names)
     by = LAUNCHES["by_kernel"]
-    for n in names:
-        by[n] = by.get(n, 0) + 1
+    for name in names:
+        for n in name.split("+"):
+            by[n] = by.get(n, 0) + 1
 
 
 def _check(rc: int, name: str):
@@ -1211,25 +1212,53 @@ def rotary_kv_append_cuda(qkv, sin_tab, cos_tab, k_cache, v_cache, pos, n_heads,
     return qkv
 
 
-def _attn_decode_launch(qkv, k_cache, v_cache, pos, n_heads, head_dim, scale, out):
+def _attn_decode_splits(bh: int, smax: int, head_dim: int, sms: int) -> int:
+    """CTAs that share a (sequence, head): what takes the least time for a full cache. A CTA reads up to 55 KB a us, all together 6.4
+    TB/s; starting one and merging what several leave cost about 1.5 us each (1 sequence of 2000, 16 heads of 256: 9.6 us with 8 CTAs per
+    head; 16 of 1000, 32 heads of 64: 41 us with 4, for which 1 is chosen)."""
+    bytes_each = 4 * head_dim
+
+    def us(n):
+        rate = min(55e3, 6.4e6 / min(bh * n, 2 * sms)) / bytes_each  # positions a us
+        return -(-bh * n // (2 * sms)) * (smax / n / rate + 1.5) + (1.5 if n > 1 else 0)
+
+    return min(range(1, max(1, min(smax // 64, 64)) + 1), key=lambda n: (round(us(n), 1), n))
+
+
+def _attn_decode_launch(qkv, k_cache, v_cache, pos, n_heads, head_dim, scale, out, rotary=None):
+    """`rotary`: (sin, cos, rotary_dim) to rotate and append the new keys and values first."""
     if not (_row_window_ok(qkv) and _row_window_ok(out)) or not _ok(k_cache, v_cache) or pos.dtype != torch.int32:
         return NotImplemented
     if head_dim not in (64, 128, 256) or k_cache.dtype != qkv.dtype or out.dtype != qkv.dtype:
         return NotImplemented
     B, smax = qkv.shape[0], k_cache.shape[2]
     bh = B * n_heads
-    # enough CTAs to fill the machine, at least 32 cache positions per CTA
-    splits = max(1, min((8 * _sms(qkv.device) + bh - 1) // bh, (smax + 31) // 32, 64))
-    ws = workspace(bh * splits * (head_dim + 2) * 4, qkv.device, "attn_decode")
-    done = counters(bh, qkv.device, "counters attn_decode")
-    rc = _attn_dec(qkv.data_ptr(), qkv.stride(0), k_cache.data_ptr(), v_cache.data_ptr(), out.data_ptr(), out.stride(0),
-                   ws.data_ptr(), done.data_ptr(), pos.data_ptr(), B, n_heads, head_dim, smax, float(scale), splits,
-                   _CODE[qkv.dtype], _stream())
+    splits = _attn_decode_splits(bh, smax, head_dim, _sms(qkv.device))
+    ws = done = None
+    if splits > 1:
+        ws = workspace(bh * splits * (head_dim + 2) * 4, qkv.device, "attn_decode").data_ptr()
+        done = counters(bh, qkv.device, "counters attn_decode").data_ptr()
+    sin, cos, rotary_dim = rotary or (None, None, 0)
+    rc = _attn_dec(qkv.data_ptr(), qkv.stride(0), sin.data_ptr() if rotary_dim else None, cos.data_ptr() if rotary_dim else None,
+                   k_cache.data_ptr(), v_cache.data_ptr(), out.data_ptr(), out.stride(0), ws, done, pos.data_ptr(), B, n_heads,
+                   head_dim, rotary_dim, smax, float(scale), splits, int(rotary is not None),
+                   int(rotary is not None and read_ahead.allowed(pos, k_cache, v_cache)), _CODE[qkv.dtype],
+                   gemm_error_flag(qkv.device).data_ptr(), _stream())
     if rc == -1:
         return NotImplemented
     _check(rc, "attn_decode")
-    _count("attn_decode")
+    _count("rotary_append+attn_decode" if rotary else "attn_decode")
     return out
+
+
+@native("rotary_attention_decode_into_")
+def rotary_attention_decode_into_cuda(buf, sin_tab, cos_tab, k_cache, v_cache, pos, n_heads, head_dim, rotary_dim, out_col, scale):
+    hd = n_heads * head_dim
+    if rotary_dim and not (_ok(sin_tab, cos_tab) and sin_tab.dtype == cos_tab.dtype == buf.dtype):
+        return NotImplemented
+    res = _attn_decode_launch(buf, k_cache, v_cache, pos, n_heads, head_dim, scale, buf[:, out_col:out_col + hd],
+                              (sin_tab, cos_tab, rotary_dim))
+    return buf if res is not NotImplemented else NotImplemented
 
 
 @native("attention_decode_packed")

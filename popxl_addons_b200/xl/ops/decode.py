@@ -92,6 +92,16 @@ def _attn_decode_into_ref(buf, k_cache, v_cache, pos, n_heads, head_dim, out_col
     return buf
 
 
+def _rotary_attn_decode_into_ref(buf, sin_tab, cos_tab, k_cache, v_cache, pos, n_heads, head_dim, rotary_dim, out_col, scale):
+    if buf.device.type == "meta":
+        return buf
+    qkv = _rotary_kv_append_ref(buf[:, :3 * n_heads * head_dim].clone(), sin_tab, cos_tab, k_cache, v_cache, pos, n_heads, head_dim,
+                                rotary_dim)
+    o = _attn_decode_packed_ref(qkv, k_cache, v_cache, pos, n_heads, head_dim, scale)
+    buf[:, out_col:out_col + n_heads * head_dim].copy_(o)
+    return buf
+
+
 def _add_layer_norm_ref(x, *rest, has_delta, has_bias, eps):
     if x.device.type == "meta":
         return torch.empty_like(x)
@@ -110,6 +120,7 @@ def _add_layer_norm_ref(x, *rest, has_delta, has_bias, eps):
 
 
 OpDef("attention_decode_into_", impl=_attn_decode_into_ref, inplace=True)
+OpDef("rotary_attention_decode_into_", impl=_rotary_attn_decode_into_ref, inplace=True)
 OpDef("add_layer_norm_", impl=_add_layer_norm_ref)
 OpDef("rotary_kv_append_", impl=_rotary_kv_append_ref, inplace=True)
 OpDef("attention_decode_packed", impl=_attn_decode_packed_ref)
@@ -143,6 +154,16 @@ def attention_decode_into_(buf: Tensor, k_cache: Tensor, v_cache: Tensor, pos: T
     scale = float(scale) if scale is not None else 1.0 / math.sqrt(head_dim)
     return emit1("attention_decode_into_", [buf, k_cache, v_cache, pos],
                  dict(n_heads=int(n_heads), head_dim=int(head_dim), out_col=int(out_col), scale=scale))
+
+
+def rotary_attention_decode_into_(buf: Tensor, sin_table: Tensor, cos_table: Tensor, k_cache: Tensor, v_cache: Tensor, pos: Tensor,
+                                  n_heads: int, head_dim: int, rotary_dim: int, out_col: int, scale: Optional[float] = None) -> Tensor:
+    """`rotary_kv_append_` and `attention_decode_into_` as one op: the new keys (rotated) and values of `buf (batch, [q | k | v | ...])`
+    go to the caches at `pos`, the attention of the rotated queries to `buf[:, out_col : out_col + heads*head_dim]`. The projections in
+    `buf` are not rotated in place."""
+    scale = float(scale) if scale is not None else 1.0 / math.sqrt(head_dim)
+    return emit1("rotary_attention_decode_into_", [buf, sin_table, cos_table, k_cache, v_cache, pos],
+                 dict(n_heads=int(n_heads), head_dim=int(head_dim), rotary_dim=int(rotary_dim), out_col=int(out_col), scale=scale))
 
 
 def add_layer_norm_(x: Tensor, delta: Optional[Tensor], bias: Optional[Tensor], weight: Tensor, ln_bias: Tensor,

@@ -22,7 +22,7 @@ import torch
 READERS: Dict[str, Tuple[int, ...]] = {
     "linear_rows": (1,), "linear_swiglu": (1,), "linear_split_glu": (1,), "linear_residual_dyt_": (2,), "linear_residual_rms_": (2,),
     "min_gru_": (1,), "linear_gq": (1, 2, 3), "linear_gq_window": (1, 2, 3), "linear_gq_window_t": (1, 2),
-    "diff_attention_": (), "window_attention_": (),
+    "diff_attention_": (), "window_attention_": (), "rotary_attention_decode_into_": (),
 }
 
 _THREAD = threading.local()

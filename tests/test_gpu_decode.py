@@ -132,6 +132,33 @@ def test_rotary_append_and_attention_decode(nat, dtype, B, H, D, R, S, pos):
     torch.testing.assert_close(buf[:, :2 * H * D], qkv[:, :2 * H * D])
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("B,H,D,R,S,pos", [(16, 2, 256, 64, 640, 512), (3, 4, 64, 32, 128, 0), (2, 16, 128, 0, 300, 299), (1, 3, 128, 128, 2100, 2050),
+                                           (2, 5, 64, 64, 1024, 31), (1, 2, 256, 2, 600, 32), (20, 16, 256, 256, 600, 97), (1, 1, 64, 6, 20000, 19999)])
+def test_rotation_append_and_attention_in_one_launch(nat, dtype, B, H, D, R, S, pos):
+    """One CTA and many per head, first and last position, a position on each side of a stage, partly and fully rotated heads: caches to the
+    bit of the separate kernel, result against fp32 (weights sum to 1, so a result is off by its rounding and by rounded keys' scores),
+    the rest of the buffer untouched; twice, with the split counters back at zero."""
+    from popxl_addons_b200.ops.rotary_pos_embed import trig_tables
+
+    g = torch.Generator(device="cuda").manual_seed(B + S + pos)
+    buf = torch.randn(B, 3 * H * D + 64, generator=g, device="cuda").to(dtype)
+    k, v = (torch.randn(B, H, S, D, generator=g, device="cuda").to(dtype) for _ in range(2))
+    sin, cos = (torch.tensor(t, device="cuda").to(dtype) for t in trig_tables(S, R or 2))
+    p, hd = torch.tensor(pos, dtype=torch.int32, device="cuda"), H * D
+    qkv, k_r, v_r = buf[:, :3 * hd].clone(memory_format=torch.contiguous_format), k.clone(), v.clone()
+    assert nat.rotary_kv_append_cuda(qkv, sin, cos, k_r, v_r, p, H, D, R) is not NotImplemented
+    want = _ref("attention_decode_packed")(qkv.float(), k_r.float(), v_r.float(), p, H, D, D ** -0.5)
+    assert torch.isfinite(want).all()
+    for _ in range(2):
+        out = buf.clone()
+        assert nat.rotary_attention_decode_into_cuda(out, sin, cos, k, v, p, H, D, R, 2 * hd, D ** -0.5) is out
+        assert torch.equal(k, k_r) and torch.equal(v, v_r)
+        torch.testing.assert_close(out[:, 2 * hd:3 * hd].float(), want, rtol=2.0 ** -7, atol=2.0 ** -8)
+        assert torch.equal(out[:, :2 * hd], buf[:, :2 * hd]) and torch.equal(out[:, 3 * hd:], buf[:, 3 * hd:])
+    nat.check_gemm_errors()
+
+
 def test_argmax_store_row_advance(nat):
     torch.manual_seed(2)
     logits = torch.randn(16, 6300, device="cuda").bfloat16()
