@@ -104,6 +104,7 @@ template <int D, int BKV>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
     attn_bwd_dq_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_do,
                                const __grid_constant__ CUtensorMap map_kv, const AttnBwdParams p) {
+  xl_grid_launch_dependents();
   using L = BwdSmem<D, BKV>;
   static_assert(D % 64 == 0 && D <= 256 && BKV % 32 == 0 && BKV <= 64 && D + 4 * BKV <= (int)TMEM_COLS, "unsupported tile");
   extern __shared__ uint8_t smem_raw[];
@@ -432,6 +433,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
 // delta = dO . O of every (batch, head, position): one warp per row, the lanes across the features.
 template <int D>
 __global__ void __launch_bounds__(256) attn_bwd_delta_kernel(const AttnBwdParams p) {
+  xl_grid_launch_dependents();
   const int lane = threadIdx.x & 31;
   const long long w = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (w >= (long long)p.B * p.H * p.S) return;
@@ -473,6 +475,7 @@ __global__ void __launch_bounds__(256) attn_bwd_delta_kernel(const AttnBwdParams
 // written by the main kernel already.
 template <int D>
 __global__ void __launch_bounds__(256) attn_bwd_dq_merge_kernel(const AttnBwdParams p, int bkv) {
+  xl_grid_launch_dependents();
   const int lane = threadIdx.x & 31;
   const long long w = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (w >= (long long)p.B * p.H * p.S) return;

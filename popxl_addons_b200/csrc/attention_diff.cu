@@ -26,6 +26,7 @@ __global__ void __launch_bounds__(256)
     diff_rope_append_kernel(T* __restrict__ qkv, long long ld, const float* __restrict__ cos_t, const float* __restrict__ sin_t,
                             T* __restrict__ kc, T* __restrict__ vc, const int* __restrict__ pos, const int* __restrict__ count,
                             long long rows, int T_len, int H, int G, int dim, int vdim, int R, int Smax) {
+  xl_grid_launch_dependents();
   const int half = (dim + 1) / 2, vhalf = (vdim + 1) / 2;
   const int nq = H * 2 * half, nk = G * 2 * half, nv = G * vhalf;
   const long long per_row = nq + nk + nv, total = rows * per_row;
@@ -76,6 +77,7 @@ __global__ void __launch_bounds__(256)
     diff_rope_append_vec_kernel(T* __restrict__ qkv, long long ld, const float* __restrict__ cos_t, const float* __restrict__ sin_t,
                                 T* __restrict__ kc, T* __restrict__ vc, const int* __restrict__ pos, const int* __restrict__ count,
                                 int T_len, int H, int G, int dim, int vdim, int R, int Smax) {
+  xl_grid_launch_dependents();
   constexpr int V = 16 / sizeof(T);
   const int b = blockIdx.y, t = blockIdx.x, p = pos[b] + t;
   if (t >= count[b] || p < 0 || p >= Smax) return;
@@ -120,6 +122,7 @@ __global__ void __launch_bounds__(SPLIT == 1 ? 128 : SPLIT * 32)
                              T* __restrict__ out, long long ldo, const int* __restrict__ pos, const int* __restrict__ count,
                              const float* __restrict__ lam, int T_len, int H, int G, int dim, int vdim, int Smax, int chunk,
                              float scale, float eps, float out_scale) {
+  xl_grid_launch_dependents();
   constexpr int ROWS = SPLIT == 1 ? 4 : 1;
   __shared__ __align__(16) float sq[ROWS][2][DG_MAX_DIM];
   __shared__ float so[SPLIT == 1 ? 1 : SPLIT][2][SPLIT == 1 ? 1 : 32 * DG_VPL], sm[SPLIT][2], sl[SPLIT][2];

@@ -55,6 +55,7 @@ template <int DK, int VD>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
     diff_attn_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                              const __grid_constant__ CUtensorMap map_v, const DiffParams p) {
+  xl_grid_launch_dependents();
   using L = DiffSmem<DK, VD>;
   static_assert(L::TOTAL <= 227 * 1024, "shared memory");
   extern __shared__ uint8_t smem_raw[];

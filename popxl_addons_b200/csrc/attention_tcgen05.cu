@@ -80,6 +80,7 @@ template <int D, int BKV>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
     attn_fwd_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                             const __grid_constant__ CUtensorMap map_v, const AttnParams p) {
+  xl_grid_launch_dependents();
   using L = AttnSmem<D, BKV>;
   static_assert(D % 64 == 0 && D <= 256 && BKV % 64 == 0 && D + 2 * BKV <= (int)TMEM_COLS, "unsupported tile");
   extern __shared__ uint8_t smem_raw[];
@@ -393,6 +394,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
 // were written by the main kernel already.
 template <int D>
 __global__ void __launch_bounds__(256) attn_fwd_merge_kernel(const AttnParams p, int bkv) {
+  xl_grid_launch_dependents();
   const int lane = threadIdx.x & 31;
   const long long w = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (w >= (long long)p.B * p.H * p.S) return;

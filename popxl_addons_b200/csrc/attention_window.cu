@@ -35,6 +35,7 @@ __global__ void __launch_bounds__(256)
                           T* __restrict__ qn, T* __restrict__ kc, T* __restrict__ vc, const int* __restrict__ pos,
                           const int* __restrict__ count, int T_len, int H, int G, int dim, int vdim, int Smax, float eps,
                           int group) {
+  xl_grid_launch_dependents();
   constexpr int NP = 16 / V;  // pieces per lane: 32 lanes cover WA_MAX_DIM features
   const int b = blockIdx.y, t = blockIdx.x, p = pos[b] + t;
   if (t >= count[b] || p < 0 || p >= Smax) return;
@@ -104,6 +105,7 @@ __global__ void __launch_bounds__(SPLIT == 1 ? 128 : SPLIT * 32)
                                const T* __restrict__ gate, long long ldg, T* __restrict__ out, long long ldo,
                                const int* __restrict__ pos, const int* __restrict__ count, int T_len, int H, int G, int dim,
                                int vdim, int Smax, int window, int keep_first, float scale, float sink) {
+  xl_grid_launch_dependents();
   constexpr int ROWS = SPLIT == 1 ? 4 : 1;
   __shared__ __align__(16) float sq[ROWS][WA_MAX_DIM];
   __shared__ float so[SPLIT == 1 ? 1 : SPLIT][SPLIT == 1 ? 1 : 32 * VPL], sm[SPLIT], sl[SPLIT];

@@ -12,6 +12,7 @@ constexpr int EW_UNROLL = 4;  // 16-byte vectors per thread and iteration: keeps
 
 template <typename T, typename F>
 __global__ void __launch_bounds__(256) ew_unary_kernel(const T* __restrict__ x, T* __restrict__ y, long long n, F f) {
+  xl_grid_launch_dependents();
   constexpr int N = XlVec<T>::N;
   const long long nvec = n / N;
   const long long stride = (long long)gridDim.x * blockDim.x;
@@ -41,6 +42,7 @@ __global__ void __launch_bounds__(256) ew_unary_kernel(const T* __restrict__ x, 
 template <typename T, typename F>
 __global__ void __launch_bounds__(256)
     ew_binary_kernel(const T* __restrict__ x, const T* __restrict__ g, T* __restrict__ y, long long n, F f) {
+  xl_grid_launch_dependents();
   constexpr int N = XlVec<T>::N;
   const long long nvec = n / N;
   const long long stride = (long long)gridDim.x * blockDim.x;
@@ -165,6 +167,7 @@ template <typename T>
 __global__ void __launch_bounds__(256) swiglu_bwd_kernel(const T* __restrict__ gate, const T* __restrict__ up,
                                                         const T* __restrict__ g, T* __restrict__ dgate,
                                                         T* __restrict__ dup, long long n) {
+  xl_grid_launch_dependents();
   constexpr int N = XlVec<T>::N;
   const long long nvec = n / N;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < nvec; i += (long long)gridDim.x * blockDim.x) {
@@ -207,6 +210,7 @@ template <typename T, bool RMS, int ITERS>
 __global__ void __launch_bounds__(NORM_THREADS)
     norm_fwd_kernel(const T* __restrict__ x, const T* __restrict__ w, const T* __restrict__ b, T* __restrict__ y,
                     float* __restrict__ mean_out, float* __restrict__ rstd_out, int cols, float eps) {
+  xl_grid_launch_dependents();
   constexpr int N = XlVec<T>::N;
   __shared__ float red[32];
   const long long row = blockIdx.x;
@@ -307,6 +311,7 @@ __global__ void __launch_bounds__(NORM_THREADS)
     norm_bwd_kernel(const T* __restrict__ x, const T* __restrict__ w, const float* __restrict__ mean,
                     const float* __restrict__ rstd, const T* __restrict__ g, T* __restrict__ dx,
                     float* __restrict__ partial, long long rows, int cols) {
+  xl_grid_launch_dependents();
   constexpr int N = XlVec<T>::N;
   __shared__ float red[32];
   const int nvec = cols / N;
@@ -398,6 +403,7 @@ __global__ void __launch_bounds__(NORM_THREADS)
 template <typename T>
 __global__ void __launch_bounds__(256)
     norm_bwd_finish_kernel(const float* __restrict__ partial, T* __restrict__ dw, T* __restrict__ db, int nparts, int cols) {
+  xl_grid_launch_dependents();
   __shared__ float sw[8][33], sb[8][33];
   const int lane = threadIdx.x & 31, grp = threadIdx.x >> 5;
   const int c = blockIdx.x * 32 + lane;
@@ -458,6 +464,7 @@ constexpr int COLSUM_THREADS = 256;
 template <typename T>
 __global__ void __launch_bounds__(COLSUM_THREADS)
     col_sum_kernel(const T* __restrict__ x, float* __restrict__ partial, long long rows, int cols, long long rows_per_part) {
+  xl_grid_launch_dependents();
   constexpr int N = XlVec<T>::N;
   __shared__ float red[COLSUM_THREADS / 32][32 * N + 1];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -501,6 +508,7 @@ __global__ void __launch_bounds__(COLSUM_THREADS)
 }
 template <typename T>
 __global__ void __launch_bounds__(256) col_sum_finish_kernel(const float* __restrict__ partial, T* __restrict__ out, int parts, int cols) {
+  xl_grid_launch_dependents();
   const int c = blockIdx.x * 256 + threadIdx.x;
   if (c >= cols) return;
   float t = 0.f;
@@ -588,6 +596,7 @@ template <typename TW, typename TG, typename TM, int V>
 __global__ void __launch_bounds__(256)
     adam_kernel(TW* __restrict__ w, const TG* __restrict__ g, TM* __restrict__ m, float* __restrict__ v,
                 float* __restrict__ master, const float* __restrict__ step, AdamArgs a, long long n) {
+  xl_grid_launch_dependents();
   constexpr int U = V == 1 ? 1 : 2;
   float c1 = 1.f, c2 = 1.f;
   if (step != nullptr && a.bias_correction) {
@@ -696,6 +705,7 @@ XL_API int xl_sgd_step(void* w, int w_dtype, const void* g, int g_dtype, float* 
 template <typename TA, typename TX, int V>
 __global__ void __launch_bounds__(256)
     accumulate_mean_kernel(TA* __restrict__ acc, const TX* __restrict__ x, const float* __restrict__ step, long long n) {
+  xl_grid_launch_dependents();
   const float t = *step;
   const float a = t / (t + 1.f), b = 1.f / (t + 1.f);
   const long long groups = n / V;
@@ -768,6 +778,7 @@ template <typename T, int VP>
 __global__ void __launch_bounds__(256)
     rotary_kernel(const T* x, const T* __restrict__ sin_t, const T* __restrict__ cos_t, T* y, uint32_t total, uint32_t H, uint32_t S, int D,
                   int R, int sin_batch, float sign, long long xb, long long xh, long long xs, long long yb, long long yh, long long ys) {
+  xl_grid_launch_dependents();
   // in place only the rotated pairs are touched; out of place the pass-through features are copied as well
   const uint32_t per_row = (uint32_t)((x == y) ? R / 2 : D / 2) / VP;
   struct alignas(2 * VP * sizeof(T)) Pairs { T v[2 * VP]; };
@@ -800,6 +811,7 @@ template <typename T>
 __global__ void __launch_bounds__(256)
     rotary_any_kernel(const T* x, const T* __restrict__ sin_t, const T* __restrict__ cos_t, T* y, long long total_pairs, int H, int S, int D,
                       int R, int sin_batch, float sign, long long xb, long long xh, long long xs, long long yb, long long yh, long long ys) {
+  xl_grid_launch_dependents();
   const int pairs_per_row = (x == y) ? R / 2 : D / 2;
   for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < total_pairs; p += (long long)gridDim.x * blockDim.x) {
     const int j = (int)(p % pairs_per_row);
@@ -856,6 +868,7 @@ template <typename T, typename S>
 __global__ void __launch_bounds__(256)
     gq_decompress_kernel(const uint16_t* __restrict__ packed, const S* __restrict__ scale, const S* __restrict__ bias,
                          T* __restrict__ out, long long n_pairs, uint32_t pairs_per_group) {
+  xl_grid_launch_dependents();
   const bool small = n_pairs <= 0xffffffffLL, wide = (((uintptr_t)out) & 15) == 0;
   for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < n_pairs; p += (long long)gridDim.x * blockDim.x) {
     const uint32_t two = *reinterpret_cast<const uint32_t*>(packed + 2 * p);
@@ -902,6 +915,7 @@ constexpr int SM_MAX_ITERS = 8;
 template <typename T, int ITERS>
 __global__ void __launch_bounds__(SM_THREADS)
     attn_softmax_fwd_kernel(T* __restrict__ s, float* __restrict__ lse, int Sq, int Sk, float scale, int causal) {
+  xl_grid_launch_dependents();
   constexpr int N = XlVec<T>::N;
   __shared__ float red[32];
   const long long row = blockIdx.x;
@@ -954,6 +968,7 @@ __global__ void __launch_bounds__(SM_THREADS)
 template <typename T, int ITERS>
 __global__ void __launch_bounds__(SM_THREADS)
     attn_softmax_bwd_kernel(const T* __restrict__ p, T* __restrict__ dp, int Sq, int Sk, float scale, int causal) {
+  xl_grid_launch_dependents();
   constexpr int N = XlVec<T>::N;
   __shared__ float red[32];
   const long long row = blockIdx.x;
@@ -1029,6 +1044,7 @@ __global__ void __launch_bounds__(512)
     ce_fwd_bwd_kernel(const T* __restrict__ logits, const int* __restrict__ labels, float* __restrict__ loss_row,
                       T* __restrict__ dlogits, int V, int ldd, int ignore_index, const float* __restrict__ grad_scale_ptr,
                       float grad_scale) {
+  xl_grid_launch_dependents();
   constexpr int N = XlVec<T>::N;
   constexpr bool EXACT = RAGGED && sizeof(T) == 4;
   __shared__ float red[32];

@@ -18,6 +18,13 @@
 // then leave their loops, meet at the closing cluster barrier (which every thread of both CTAs reaches), TMEM is freed
 // and the kernel returns.
 //
+// Start and end of a launch, which is all of a small product (128 x 256 x 768, a chain of launches in a graph: 7.1 us -> 4.25; 2048 x 768 x 768:
+// 9.3 -> 6.9; 128 x 256 x 768 into an fp32 mean: 8.5 -> 6.1). By clock stamps in the first form: 1500 cycles to the first cluster barrier, 1600 for the
+// TMEM allocation and a second barrier, 1800 to the first operands, 4100 for two chunks of the epilogue, 1600 for the closing
+// barrier. Now the loads start after the first barrier, their descriptors are prefetched, the launch overlaps its predecessor's end
+// (programmatic dependent launch: every role waits before it touches global memory), tile coordinates take no integer
+// divisions, and the epilogue's unrolled code holds the activations only where they are asked for (gemm_epilogue.cuh).
+//
 // Scope: plain GEMMs (any operand major-ness, batch, bias / activation / accumulate epilogue) with N > 128. Collective
 // epilogues, the all-gather prologue, causal tile skipping and 8-bit operands stay on the single-CTA kernel.
 #include "tcgen05.cuh"
@@ -146,20 +153,25 @@ __device__ __forceinline__ bool mbar_wait_pair(uint64_t* bar, uint32_t parity, v
   return false;
 }
 
+// t / d for 0 <= t, 1 <= d and quotients below 2^22, remainder in `r`: a chain of three integer divisions took some 600 cycles of a small
+// product's launch
+__device__ __forceinline__ int tile_div(int t, int d, int& r) {
+  int q = (int)((float)t * __frcp_rn((float)d));  // off by one at most
+  r = t - q * d;
+  if (r < 0) { --q; r += d; }
+  if (r >= d) { ++q; r -= d; }
+  return q;
+}
+
 // tile index -> (batch, m block, n block); m-blocks are walked in groups of 8 inside each n-column so that the tiles in
 // flight share operand panels in L2
 __device__ __forceinline__ void tile_coords(int tile, int tiles_m, int tiles_n, int& b, int& mb, int& nb) {
   constexpr int GROUP = 8;
-  const int per_batch = tiles_m * tiles_n;
-  b = tile / per_batch;
-  const int t = tile - b * per_batch;
-  const int group_size = GROUP * tiles_n;
-  const int g = t / group_size;
-  const int first_m = g * GROUP;
-  const int rows = min(GROUP, tiles_m - first_m);
-  const int in_group = t - g * group_size;
-  mb = first_m + in_group % rows;
-  nb = in_group / rows;
+  int t, in_group, m_in;
+  b = tile_div(tile, tiles_m * tiles_n, t);
+  const int g = tile_div(t, GROUP * tiles_n, in_group);
+  nb = tile_div(in_group, min(GROUP, tiles_m - g * GROUP), m_in);
+  mb = g * GROUP + m_in;
 }
 
 // How C leaves the kernel. One instance each: with all three in one kernel the registers of the slowest form were spilled in the
@@ -215,20 +227,30 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
+  if (threadIdx.x == 32) {  // the first loads would wait for the descriptors
+    asm volatile("prefetch.tensormap [%0];" ::"l"(&map_a) : "memory");
+    asm volatile("prefetch.tensormap [%0];" ::"l"(&map_b) : "memory");
+  }
   __syncthreads();
   cluster_sync_all();  // both CTAs run and their barriers are initialised before anything involves the pair
+  // From here on the loads are under way; the MMAs and the epilogue also need the TMEM of both CTAs, which a second cluster barrier
+  // says. The producer arrives at it like everyone, and waits for it when its loads are issued.
   if (warp == 1) {
     tmem_alloc_pair(tmem_base_slot, TMEM_COLS);  // one warp of each CTA: the allocation is collective over the pair
     tmem_relinquish_pair();
   }
   tcgen05_fence_before();
-  __syncthreads();
-  cluster_sync_all();
-  tcgen05_fence_after();
-  const uint32_t tmem_base = *tmem_base_slot;
+  __syncwarp();
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  if (warp != 0) {
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    tcgen05_fence_after();
+  }
 
   if (warp == 0) {
     // ------------------------------------------------ TMA producer ------------------------------------------------
+    xl_grid_dependency_wait();
+    xl_grid_launch_dependents();
     if (elect_one()) {
       uint32_t stage = 0, phase = 0;
       bool ok = true;
@@ -263,7 +285,11 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
         }
       }
     }
+    __syncwarp();
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
   } else if (warp == 1) {
+    const uint32_t tmem_base = *tmem_base_slot;
+    xl_grid_dependency_wait();  // no bounded wait runs while the previous kernel still does
     // ------------------------------------------------ MMA issuer (leader CTA only) -------------------------------
     if (leader && elect_one()) {
       const uint32_t fmt = p.is_fp16 ? 0u : 1u;
@@ -306,6 +332,8 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
       }
     }
   } else {
+    const uint32_t tmem_base = *tmem_base_slot;
+    xl_grid_dependency_wait();
     // ------------------------------------------------ epilogue ----------------------------------------------------
     const int q = warp & 3;                // TMEM lane quarter this warp may access
     const int col_half = (warp - 2) >> 2;  // which half of the accumulator columns this warp drains
@@ -383,18 +411,20 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
           // the row pair so that neither phase has bank conflicts; then 4 lanes store one row's 64 bytes, 8 rows per
           // instruction
           uint4* stage16 = (uint4*)stage;
-          const float bv = p.epi.bias ? epilogue_bias(p.epi, col0 + lane) : 0.f;  // column col0 + lane, handed out below
+          with_bias_and_act(p.epi, [&](auto bias, auto act) {
+            const float bv = decltype(bias)::value ? epilogue_bias(p.epi, col0 + lane) : 0.f;  // column col0 + lane, handed out below
 #pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            float v[8];
+            for (int j = 0; j < 4; ++j) {
+              float v[8];
 #pragma unroll
-            for (int e = 0; e < 8; ++e) {
-              float x = __uint_as_float(r[j * 8 + e]) * p.alpha;
-              if (p.epi.bias) x += __shfl_sync(0xffffffffu, bv, j * 8 + e);
-              v[e] = apply_act(x, p.epi.act);
+              for (int e = 0; e < 8; ++e) {
+                v[e] = __uint_as_float(r[j * 8 + e]) * p.alpha;
+                if (decltype(bias)::value) v[e] += __shfl_sync(0xffffffffu, bv, j * 8 + e);
+                if (decltype(act)::value) v[e] = apply_act(v[e], p.epi.act);
+              }
+              stage16[lane * 4 + ((j + (lane >> 1)) & 3)] = pack8_16bit(v, p.epi.c_dtype == XL_F16);
             }
-            stage16[lane * 4 + ((j + (lane >> 1)) & 3)] = pack8_16bit(v, p.epi.c_dtype == XL_F16);
-          }
+          });
           __syncwarp();
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
@@ -405,18 +435,20 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
           __syncwarp();
         } else if ((EPI == EPI_F32 || EPI == EPI_16A) && col0 + 32 <= p.N) {
           // this thread's row -> shared memory, 16-byte pieces swizzled by the row so that both phases are conflict-free
-          const float bv = p.epi.bias ? epilogue_bias(p.epi, col0 + lane) : 0.f;
+          with_bias_and_act(p.epi, [&](auto bias, auto act) {
+            const float bv = decltype(bias)::value ? epilogue_bias(p.epi, col0 + lane) : 0.f;
 #pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            float v[4];
+            for (int j = 0; j < 8; ++j) {
+              float v[4];
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {
-              float x = __uint_as_float(r[j * 4 + e]) * p.alpha;
-              if (p.epi.bias) x += __shfl_sync(0xffffffffu, bv, j * 4 + e);
-              v[e] = apply_act(x, p.epi.act);
+              for (int e = 0; e < 4; ++e) {
+                v[e] = __uint_as_float(r[j * 4 + e]) * p.alpha;
+                if (decltype(bias)::value) v[e] += __shfl_sync(0xffffffffu, bv, j * 4 + e);
+                if (decltype(act)::value) v[e] = apply_act(v[e], p.epi.act);
+              }
+              stage[lane * 8 + (j ^ (lane & 7))] = make_float4(v[0], v[1], v[2], v[3]);
             }
-            stage[lane * 8 + (j ^ (lane & 7))] = make_float4(v[0], v[1], v[2], v[3]);
-          }
+          });
           __syncwarp();
           if (EPI == EPI_16A) {  // the sum is fp32, rounded once
             uint4 out16[4];
@@ -480,19 +512,22 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
 #pragma unroll
           for (int j = 0; j < 32; ++j) stage32[lane * 32 + (j ^ lane)] = __uint_as_float(r[j]) * p.alpha;
           __syncwarp();
+          with_bias_and_act(p.epi, [&](auto, auto act) {
 #pragma unroll
-          for (int i0 = 0; i0 < 32; i0 += 8) {  // reads of shared memory first: the compiler keeps them behind earlier stores
-            float o[8];
+            for (int i0 = 0; i0 < 32; i0 += 8) {  // reads of shared memory first: the compiler keeps them behind earlier stores
+              float o[8];
 #pragma unroll
-            for (int i = 0; i < 8; ++i) o[i] = stage32[(i0 + i) * 32 + (lane ^ (i0 + i))];
+              for (int i = 0; i < 8; ++i) o[i] = stage32[(i0 + i) * 32 + (lane ^ (i0 + i))];
 #pragma unroll
-            for (int i = 0; i < 8; ++i) {
-              float t = apply_act(o[i] + bv, p.epi.act);
-              if (p.epi.accumulate == 1) t += before[i0 + i];
-              else if (p.epi.accumulate == 2) t = before[i0 + i] * mean_a + t * mean_b;
-              if (on && i0 + i < rows) c32[(i0 + i) * p.ldc] = t;
+              for (int i = 0; i < 8; ++i) {
+                float t = o[i] + bv;
+                if (decltype(act)::value) t = apply_act(t, p.epi.act);
+                if (p.epi.accumulate == 1) t += before[i0 + i];
+                else if (p.epi.accumulate == 2) t = before[i0 + i] * mean_a + t * mean_b;
+                if (on && i0 + i < rows) c32[(i0 + i) * p.ldc] = t;
+              }
             }
-          }
+          });
           __syncwarp();
         } else if (row_ok) {
           epilogue_store_32cols(p.epi, r, crow, col0, p.alpha, mean_a, mean_b);
@@ -516,7 +551,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
   cluster_sync_all();
   if (warp == 1) {
     tcgen05_fence_after();
-    tmem_dealloc_pair(tmem_base, TMEM_COLS);
+    tmem_dealloc_pair(*tmem_base_slot, TMEM_COLS);
   }
 }
 
@@ -580,13 +615,15 @@ int launch_pairs(const CUtensorMap& ma, const CUtensorMap& mb, const Gemm2Params
   cfg.blockDim = dim3(NUM_THREADS, 1, 1);
   cfg.dynamicSmemBytes = PairCfg<PN>::SMEM_TOTAL;
   cfg.stream = s;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = 2;
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = 2;
   cudaError_t e = cudaLaunchKernelEx(&cfg, gemm2cta_tcgen05_kernel<PN, EPI>, ma, mb, p);
   return e != cudaSuccess ? (int)e : (int)cudaGetLastError();
 }

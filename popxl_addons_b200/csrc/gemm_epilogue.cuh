@@ -3,6 +3,7 @@
 #include "common.cuh"
 
 #include <math.h>
+#include <type_traits>
 
 namespace {  // internal linkage: every kernel file that includes this gets its own copy
 
@@ -27,6 +28,20 @@ __device__ __forceinline__ float epilogue_bias(const EpilogueParams& p, int col)
   if (p.bias_dtype == XL_F32) return ((const float*)p.bias)[col];
   if (p.bias_dtype == XL_BF16) return __bfloat162float(((const __nv_bfloat16*)p.bias)[col]);
   return __half2float(((const __half*)p.bias)[col]);
+}
+
+// Calls f(bias, act) with compile-time truth values: unrolled code of an epilogue holds the activations only where they are asked for. With
+// all of them behind a branch per element, 32 elements were some 40 KB of code to jump through, and the instructions came
+// from L2: 2000 cycles per 32 columns (see gemm2cta_tcgen05.cu).
+template <typename F> __device__ __forceinline__ void with_bias_and_act(const EpilogueParams& p, const F& f) {
+  if (p.act) {
+    if (p.bias) f(std::true_type{}, std::true_type{});
+    else f(std::false_type{}, std::true_type{});
+  } else if (p.bias) {
+    f(std::true_type{}, std::false_type{});
+  } else {
+    f(std::false_type{}, std::false_type{});
+  }
 }
 
 // One thread's 32 consecutive accumulator columns (row `crow`, columns col0 .. col0 + 31) -> scale, bias, activation,

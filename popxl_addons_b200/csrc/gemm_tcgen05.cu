@@ -339,6 +339,10 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
+  if (threadIdx.x == 64) {  // the first loads would wait for the descriptors
+    asm volatile("prefetch.tensormap [%0];" ::"l"(&map_a) : "memory");
+    asm volatile("prefetch.tensormap [%0];" ::"l"(&map_b) : "memory");
+  }
   if (warp == 1) {
     tmem_alloc(tmem_base_slot, TMEM_COLS);
     tmem_relinquish();
@@ -347,6 +351,10 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
   __syncthreads();
   tcgen05_fence_after();
   const uint32_t tmem_base = *tmem_base_slot;
+  if (p.accumulate <= 2 && !p.gather_mode) {  // plain products are launched while their predecessor drains
+    xl_grid_dependency_wait();
+    xl_grid_launch_dependents();
+  }
 
   if (is_reducer) {
     // ------------------------------------------------ all-reduce reducer CTA: all ten warps reduce ----------------
@@ -850,7 +858,12 @@ int launch(const CUtensorMap& ma, const CUtensorMap& mb, const GemmParams& p, in
   const int gemm_ctas = tiles < sm_count - n_copy ? tiles : sm_count - n_copy;
   const int grid = gemm_ctas + n_copy;
   // without a second operand pair the kernel never touches the second pair of maps: pass the first pair again
-  gemm_tcgen05_kernel<BLOCK_N><<<grid, NUM_THREADS, smem_bytes, s>>>(ma, mb, ma2 ? *ma2 : ma, mb2 ? *mb2 : mb, p);
+  const CUtensorMap &m2 = ma2 ? *ma2 : ma, &n2 = mb2 ? *mb2 : mb;
+  if (p.accumulate <= 2 && !p.gather_mode) {
+    XL_TRY(xl_launch_overlapped(gemm_tcgen05_kernel<BLOCK_N>, dim3(grid), dim3(NUM_THREADS), (size_t)smem_bytes, s, ma, mb, m2, n2, p));
+  } else {
+    gemm_tcgen05_kernel<BLOCK_N><<<grid, NUM_THREADS, smem_bytes, s>>>(ma, mb, m2, n2, p);
+  }
   return (int)cudaGetLastError();
 }
 

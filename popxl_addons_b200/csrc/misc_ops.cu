@@ -253,6 +253,7 @@ constexpr int EMB_NONE = 0x7fffffff;        // the row of a token outside the ta
 __global__ void __launch_bounds__(256)
     mean_decay_and_sort_kernel(float* __restrict__ acc, const float* __restrict__ step, long long n, const int* __restrict__ idx, int n_idx,
                                int rows, int sort_ctas, int* __restrict__ order) {  // order: n_idx sorted rows, n_idx tokens
+  xl_grid_launch_dependents();
   if ((int)blockIdx.x < sort_ctas) {
     __shared__ __align__(16) int keys[1024];
     const int first = blockIdx.x * EMB_SORTED, i = first + (threadIdx.x >> 2), q = threadIdx.x & 3;
@@ -318,6 +319,7 @@ template <typename G, int V, int NB>
 __global__ void __launch_bounds__(256)
     add_sorted_rows_kernel(const G* __restrict__ grad_out, const int* __restrict__ order, float* __restrict__ acc,
                            const float* __restrict__ step, int n_idx, int cols) {
+  xl_grid_launch_dependents();
   constexpr int WIDTH = 32 * V * NB, AHEAD = 8 / NB;
   __shared__ float part[8][WIDTH];
   __shared__ int shared_row[8];
@@ -524,6 +526,7 @@ XL_API int xl_ln_apply_stats(const void* x, int dtype, const float* stats, const
 __global__ void __launch_bounds__(256)
     pack_rows_kernel(const uint16_t* __restrict__ src, long long ld_src, uint16_t* __restrict__ dst, long long ld_dst, long long rows,
                      int cols) {
+  xl_grid_launch_dependents();
   const int pieces = (int)(ld_dst / 8);
   const int c = blockIdx.x * 256 + threadIdx.x;
   if (c >= pieces) return;
@@ -545,6 +548,7 @@ __global__ void __launch_bounds__(256)
 // dst without gaps: a thread writes 8 consecutive elements, which lie in one row or go on in the next ones.
 __global__ void __launch_bounds__(256)
     unpack_rows_kernel(const uint16_t* __restrict__ src, long long ld_src, uint16_t* __restrict__ dst, long long rows, unsigned int cols) {
+  xl_grid_launch_dependents();
   const long long total = rows * cols;
 #pragma unroll 2
   for (long long i = ((long long)blockIdx.x * 256 + threadIdx.x) * 8; i < total; i += (long long)gridDim.x * 256 * 8) {

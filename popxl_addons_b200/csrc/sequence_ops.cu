@@ -271,6 +271,7 @@ __device__ __forceinline__ void gru_step(const float (&zr)[V], const float (&ur)
 
 template <typename T, int V, bool OUTPUT>
 __global__ void __launch_bounds__(GRU_THREADS) min_gru_kernel(const T* __restrict__ zxg, T* __restrict__ y, const GruParams p) {
+  xl_grid_launch_dependents();
   const int ch = (blockIdx.x * GRU_THREADS + threadIdx.x) * V;
   const int range = blockIdx.y, b = blockIdx.z;
   const int cnt = min(p.count[b], p.T);
@@ -340,6 +341,7 @@ __global__ void __launch_bounds__(GRU_THREADS) min_gru_kernel(const T* __restric
 }
 
 __global__ void __launch_bounds__(256) min_gru_commit_kernel(const GruParams p) {
+  xl_grid_launch_dependents();
   const int c = blockIdx.x * blockDim.x + threadIdx.x, b = blockIdx.y;
   if (c < p.W && min(p.count[b], p.T) > 0)
     p.state[(long long)b * p.W + c] = p.pairs[((long long)b * p.ranges + p.ranges - 1) * p.W + c].y;

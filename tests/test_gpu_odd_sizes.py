@@ -281,6 +281,42 @@ def test_int4_product_with_activations_that_are_not_finite(nat, dtype, M, N, K, 
     assert torch.equal(y[4:], plain[4:])
 
 
+@pytest.mark.parametrize("M,K,N", [(128, 64, 256), (256, 256, 768), (128, 192, 64), (4096, 64, 5000)])
+def test_products_wait_for_what_they_read(nat, M, K, N):
+    """Products start while their predecessor runs: a chain in which each reads what the launch before wrote (an element-wise kernel, another
+    product, a running mean), replayed as a graph, against the same calls with the device idle in between. The last shape has
+    320 tiles, more than a wave, in a ragged last group of rows and columns."""
+    g = torch.Generator(device="cuda").manual_seed(M + N)
+    x = torch.randn(M, K, generator=g, device="cuda").bfloat16()
+    w, back = ((torch.randn(*s, generator=g, device="cuda") * 0.1).bfloat16() for s in ((K, N), (N, K)))
+    step = torch.ones((), device="cuda")
+
+    def chain(x, between):
+        mean, held = torch.zeros(K, N, device="cuda"), []
+        for _ in range(6):
+            h = nat.gelu_cuda(x)
+            between()
+            y = nat.gemm(h, w)
+            between()
+            x = nat.gemm(y, back)
+            between()
+            nat.gemm(h.t(), y, out=mean, accumulate=2, step=step)
+            between()
+            held += [y, x]
+        return held + [mean]
+
+    want = chain(x, torch.cuda.synchronize)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got = chain(x, lambda: None)
+    for _ in range(3):
+        graph.replay()
+    torch.cuda.synchronize()
+    assert all(torch.equal(a, b) for a, b in zip(got, want))
+    h = nat.gelu_cuda(x)
+    _near(want[0], h.double() @ w.double(), torch.bfloat16, terms=K)
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("M,N,K,gs", [(1, 4, 128, 64), (8, 128, 256, 128), (9, 132, 384, 128), (16, 1000, 1152, 64), (16, 260, 2048, 256),
                                       (3, 124, 1024, 512), (16, 640, 6144, 1024), (2, 20004, 512, 64), (13, 2048, 10240, 64)])
