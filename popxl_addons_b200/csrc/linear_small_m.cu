@@ -1,5 +1,5 @@
 // Linear layers of the decoding path, bf16 weights, few rows: C[M, N] = a[M, K] * w[N, K]^T, the weights streamed once.
-// What follows the product in a layer happens in the epilogue, on the fp32 sums (M <= 16; `store` up to 128 rows):
+// What follows the product in a layer happens in the epilogue, on the fp32 sums (M <= 64; `store` up to 128 rows):
 //   store      C as bf16 or fp32
 //   residual   x += mult * C (+ table[token]) on the fp32 residual stream; for the next layer h = DyT(x), or the first half of
 //              an RMS norm: h = x * w and the sums of squares of x over blocks of 64 columns
@@ -27,9 +27,11 @@
 // Chains of launches on one B200, us (`mma.sync` with weights in registers and split K through global memory before -> now): 1 token
 // 4096 x 4096 12.4 -> 8.4, 22016 x 4096 with swiglu 39.0 -> 32.3; 16 tokens 4096 x 11008 26.9 -> 18.0, 32000 x 4096 58.0 -> 43.0
 // (6.1 TB/s); 40 tokens (tiles of 256 rows of the pair GEMM before) 2048 x 7680 30.5 -> 11.1, 12288 x 4096 29.6 -> 21.1,
-// 32000 x 4096 57.0 -> 47.2.
+// 32000 x 4096 57.0 -> 47.2. Epilogues of 17 to 64 tokens against plain products and kernels of their own: 40 tokens, width 2048
+// split_glu 17.0 -> 15.6, residual with RMS norm 11.8 -> 10.7, swiglu 14.7 -> 12.9, min_gru 14.6 -> 10.5; 64 tokens, width 4096
+// 50.3 -> 46.6, 25.9 -> 22.3, 38.6 -> 36.6, 31.1 -> 25.8.
 //
-// Roles per CTA: warp 0 loads, warp 1 allocates TMEM and issues the MMAs, warps 2-5 drain the accumulator. Every wait is bounded; a role
+// Roles per CTA: warp 0 loads, warp 1 allocates TMEM and issues the MMAs, warps 2-5 (above 32 tokens 2-9) drain the accumulator. Every wait is bounded; a role
 // that gives up records a code in `*err`, all threads meet at the cluster's barriers and TMEM is freed.
 #include "common.cuh"
 #include "tcgen05.cuh"
@@ -41,8 +43,6 @@ namespace {
 using namespace xl_tc;
 
 constexpr int SM_KC = 64;            // k values per block: one 128-byte swizzle row
-constexpr int SM_EPI = 128;          // threads of the epilogue, one per TMEM lane
-constexpr int SM_THREADS = 64 + SM_EPI;
 
 enum SmMode : int { SM_STORE = 0, SM_RESIDUAL = 1, SM_SWIGLU = 2, SM_MINGRU = 3, SM_SPLIT_GLU = 4 };
 
@@ -57,6 +57,9 @@ template <int NTOK> struct SmRing {
   static constexpr int W_BYTES = 128 * SM_KC * 2, A_BYTES = NTOK * SM_KC * 2, STAGE = W_BYTES + A_BYTES;
   static constexpr int STAGES = NTOK <= 32 ? 5 : (NTOK == 64 ? 4 : 3);
   static constexpr int SMEM = STAGES * STAGE + 1024 /*alignment slack*/;
+  // threads of the epilogue: one per TMEM lane, or two where many results are to be finished (40 tokens, 4096 x 12288 min_gru 24.7 -> 23.1
+  // us, 16384 x 2048 split_glu 16.2 -> 15.6; 24 tokens, 3072 x 1024 min_gru 7.1 -> 8.5)
+  static constexpr int EPI = NTOK > 32 ? 256 : 128;
   static constexpr uint32_t TMEM_COLS = NTOK < 32 ? 32 : NTOK;
   static_assert(NTOK * 132 * 4 <= STAGES * STAGE, "the partial sums take the ring's place");
 };
@@ -178,16 +181,16 @@ __device__ __forceinline__ float sm_epilogue(const SmParams& p, int r, int c, co
 
 __device__ __forceinline__ float4 ld_cluster_v4(uint32_t cluster_addr) {
   float4 v;
-  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(cluster_addr) : "memory");
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(cluster_addr));
   return v;
 }
 
 template <int MODE, int NTOK>
-__global__ void __launch_bounds__(SM_THREADS, 1)
+__global__ void __launch_bounds__(64 + SmRing<NTOK>::EPI, 2)
     linear_small_m_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_a, const SmParams p) {
   using L = SmTile<MODE>;
   using R = SmRing<NTOK>;
-  constexpr int COLS = L::COLS, CH = L::CH, PARTS = L::PARTS, STAGES = R::STAGES;
+  constexpr int COLS = L::COLS, CH = L::CH, PARTS = L::PARTS, STAGES = R::STAGES, SM_EPI = R::EPI;
   constexpr int RED_LD = 132;
   extern __shared__ uint8_t smem_raw[];
   __shared__ float row_scale[NTOK];
@@ -281,17 +284,23 @@ __global__ void __launch_bounds__(SM_THREADS, 1)
     const int q4 = warp & 3, row = q4 * 32 + lane;  // TMEM lane = weight row of the tile
     float* red = reinterpret_cast<float*>(ring);    // [token][weight row]: every load of the ring has been read by an MMA by then
     if ((MODE == SM_STORE || MODE == SM_SPLIT_GLU) && p.sumsq) {  // while the weights arrive
-      for (int r = warp - 2; r < p.M; r += 4) {
+      const int et = threadIdx.x - 64;
+      for (int r0 = 0; r0 < p.M; r0 += SM_EPI / 8) {  // eight lanes add a row's parts up
+        const int r = r0 + (et >> 3);
         float sq = 0.f;
-        for (int i = lane; i < p.sumsq_parts; i += 32) sq += p.sumsq[(long long)r * p.sumsq_parts + i];
-        sq = xl_warp_sum(sq);
-        if (lane == 0) row_scale[r] = 1.f / sqrtf(sq / p.K + p.eps);
+        if (r < p.M) {
+#pragma unroll 8
+          for (int i = et & 7; i < p.sumsq_parts; i += 8) sq += p.sumsq[(long long)r * p.sumsq_parts + i];
+        }
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
+        if ((et & 7) == 0 && r < p.M) row_scale[r] = 1.f / sqrtf(sq / p.K + p.eps);
       }
     }
     if (mbar_wait(&acc_full, 0, abort_flag, p.err, ERR_SM_ACC_FULL)) {
       tcgen05_fence_after();
 #pragma unroll 1
-      for (int t0 = 0; t0 < NTOK && t0 < p.M; t0 += 16) {
+      for (int t0 = (warp - 2) / 4 * 16; t0 < NTOK && t0 < p.M; t0 += SM_EPI / 8) {
         uint32_t r[16];
         tmem_ld_32x32b_x16(tmem_base + ((uint32_t)(q4 * 32) << 16) + t0, r);
         tmem_ld_wait();
@@ -382,7 +391,7 @@ template <int MODE, int NTOK> int sm_launch_tokens(SmParams p, int sms, cudaStre
   if (rc) return rc == -2 ? (int)cudaErrorNotSupported : (int)cudaErrorInvalidValue;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(n_tiles * p.ksplit));
-  cfg.blockDim = dim3(SM_THREADS);
+  cfg.blockDim = dim3(64 + R::EPI);
   cfg.dynamicSmemBytes = R::SMEM;
   cfg.stream = s;
   cudaLaunchAttribute attr[2];
@@ -398,15 +407,13 @@ template <int MODE, int NTOK> int sm_launch_tokens(SmParams p, int sms, cudaStre
   return e != cudaSuccess ? (int)e : (int)cudaGetLastError();
 }
 template <int MODE> int sm_launch(const SmParams& p, int sms, cudaStream_t s) {
-  if (MODE == SM_STORE && p.M > 16) {
-    if (p.M <= 32) return sm_launch_tokens<SM_STORE, 32>(p, sms, s);
-    if (p.M <= 64) return sm_launch_tokens<SM_STORE, 64>(p, sms, s);
-    return sm_launch_tokens<SM_STORE, 128>(p, sms, s);
-  }
-  return sm_launch_tokens<MODE, 16>(p, sms, s);
+  if (p.M <= 16) return sm_launch_tokens<MODE, 16>(p, sms, s);
+  if (p.M <= 32) return sm_launch_tokens<MODE, 32>(p, sms, s);
+  if (MODE != SM_STORE || p.M <= 64) return sm_launch_tokens<MODE, 64>(p, sms, s);
+  return sm_launch_tokens<SM_STORE, 128>(p, sms, s);
 }
 
-int sm_check(const void* a, long long lda, const void* w, int M, int N, int K, int max_m = 16) {
+int sm_check(const void* a, long long lda, const void* w, int M, int N, int K, int max_m = 64) {
   if (M < 1 || M > max_m || N < 1 || K < 8 || (K % 8) || (lda % 8) || lda < K) return -1;
   if (((uintptr_t)a & 15) || ((uintptr_t)w & 15)) return -1;
   return 0;
@@ -414,7 +421,7 @@ int sm_check(const void* a, long long lda, const void* w, int M, int N, int K, i
 
 }  // namespace
 
-// All: a (M, K) bf16 with row stride lda (a multiple of 8), w (N, K) bf16 contiguous, M <= 16 (xl_linear_small_m: 128), K a multiple
+// All: a (M, K) bf16 with row stride lda (a multiple of 8), w (N, K) bf16 contiguous, M <= 64 (xl_linear_small_m: 128), K a multiple
 // of 8; returns -1 for arguments the kernel does not take. read_ahead: w was complete before the previous launch on the stream. y
 // (M, N) with row stride ldy, bf16 or fp32. sumsq (M, sumsq_parts), or null: the rows of y are multiplied by
 // 1 / sqrt(sum of the row's sumsq / K + eps).

@@ -228,7 +228,7 @@ class Zirunex:
         """Whether the norms inside the layers are finished by the products that read them: few rows, sizes that the small-M
         kernels take."""
         c = self.cfg
-        return (rows <= 16 and self.dtype == xl.bfloat16 and c.width % 8 == 0
+        return (rows <= 64 and self.dtype == xl.bfloat16 and c.width % 8 == 0
                 and all(L.joint_cols % 8 == 0 for L in c.layers))
 
     def portion(self, T: int, t: Callable[[str], xl.Tensor], tokens: xl.Tensor, pos: xl.Tensor, count: xl.Tensor,

@@ -48,7 +48,7 @@ _small_residual = _sig("xl_linear_small_m_residual", _c_p, _c_ll, _c_p, _c_p, _c
 _small_swiglu = _sig("xl_linear_small_m_swiglu", _c_p, _c_ll, _c_p, _c_p, *_SMALL_TAIL)
 _small_min_gru = _sig("xl_linear_small_m_min_gru", _c_p, _c_ll, _c_p, _c_p, _c_p, _c_p, _c_p, _c_p, _c_p, *_SMALL_TAIL)
 
-def _small(a, weight, rows=16) -> bool:
+def _small(a, weight, rows=64) -> bool:
     """Whether the small-M kernels take this product."""
     return (a.dtype == torch.bfloat16 and weight.dtype == torch.bfloat16 and a.shape[0] <= rows and a.is_cuda
             and a.stride(1) == 1 and weight.is_contiguous() and a.shape[1] % 8 == 0)

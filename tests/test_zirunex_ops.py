@@ -85,6 +85,52 @@ def test_linear_split_glu(backend, rows, cols, F, K):  # noqa: F811
             close(joint[:, 16:], plain.clamped_glu(y[:, cols:cols + F], y[:, cols + F:], limit), backend, 2e-5, 2e-2)
 
 
+@pytest.mark.parametrize("rows,N,K", [(17, 130, 72), (32, 640, 264), (33, 130, 1032), (40, 1000, 200), (64, 260, 4096)])
+def test_epilogues_of_many_rows(backend, rows, N, K):  # noqa: F811
+    """What follows a product in its epilogue, up to the 64 rows that it takes: token tiles of 32 and 64, ragged channels in every kind of
+    tile, one CTA per tile and several; the unit of a deferred norm, the residual update with either norm, gates, the recurrence
+    with a fresh, an idle and continued sequences."""
+    if backend == ("cuda", torch.float32):
+        pytest.skip("32-bit models have these as kernels of their own")
+    eps, F = 1e-3, N // 2
+    a, a64 = rnd(backend, rows, K, seed=1)
+    m, m64 = rnd(backend, N, K, std=K ** -0.5, seed=2)
+    y = a64 @ m64.T
+    close(op("linear_swiglu", backend, a, m), y[:, :F] * torch.sigmoid(y[:, :F]) * y[:, F:], backend, 2e-5, 2e-2)
+    w, w64 = rnd(f32(backend), N, seed=4)
+    b, b64 = rnd(f32(backend), N, seed=5)
+    x0, x64 = rnd(f32(backend), rows + 1, N, seed=3)
+    want = x64[:rows] + 0.5 * y
+    x = x0.clone()
+    h, sq = op("linear_residual_rms_", backend, x, a, m, w, mult=0.5, eps=eps, deferred=True)
+    close(x[:rows], want, backend)
+    assert torch.equal(x[rows], x0[rows])
+    close(h, want * w64, backend)
+    close(sq.sum(-1), (want ** 2).sum(-1), backend, 1e-5, 1e-2)
+    x, alpha = x0.clone(), torch.tensor(0.7, device=backend[0])
+    h = op("linear_residual_dyt_", backend, x, a, m, alpha, w, b, mult=0.5, has_norm=True, has_inject=False)
+    close(x[:rows], want, backend)
+    close(h, torch.tanh(0.7 * want) * w64 + b64, backend, 2e-5, 2e-2)
+    W = N // 3
+    g, g64 = m[:3 * W].contiguous(), m64[:3 * W]
+    state, s64 = rnd(f32(backend), rows, W, seed=6)
+    keep = state.clone()
+    pos, count = i32(backend, 0, *[7] * (rows - 1)), i32(backend, *[1] * (rows - 1), 0)
+    got = op("min_gru_", backend, a, g, w[:W].contiguous(), b[:W].contiguous(), state, pos, count, T=1)
+    z, u, gate = (a64 @ g64.T).split(W, dim=-1)
+    z, u, old = torch.sigmoid(z + w64[:W]), u + b64[:W], s64.clone()
+    old[0] = 0.0
+    new = (1 - z) * old + z * torch.where(u >= 0, u + 0.5, torch.sigmoid(u))
+    close(state[:-1], new[:-1], backend, 3e-5, 2e-2)
+    close(got[:-1], (new * gate * torch.sigmoid(gate))[:-1], backend, 3e-5, 2e-2)
+    assert torch.equal(state[-1], keep[-1])
+
+
+@pytest.mark.parametrize("rows,N,K", [(17, 130, 72), (33, 260, 1032), (64, 642, 264)])
+def test_many_rows_that_finish_a_deferred_norm(backend, rows, N, K):  # noqa: F811
+    test_products_that_finish_a_deferred_norm(backend, rows, N, K)
+
+
 def attention_oracle(proj64, wq, wk, H, G, dim, vdim, scale, window, keep, sink, eps, gated):
     """All positions of one sequence from position 0."""
     n, qk = proj64.shape[0], (H + G) * dim
