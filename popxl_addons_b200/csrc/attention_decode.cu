@@ -25,7 +25,7 @@ using namespace xl_tc;
 
 constexpr int AD_WARPS = 8, AD_UNROLL = 4;
 constexpr int AD_THREADS = (AD_WARPS + 1) * 32;
-enum { ERR_AD_FULL = 51, ERR_AD_EMPTY = 52 };
+enum { ERR_AD_FULL = 64, ERR_AD_EMPTY = 65 };
 
 template <int D> struct AdCfg {
   static constexpr int LANES = D / 8, GROUPS = 32 / LANES;  // lanes of a position, positions of a warp at a time

@@ -28,7 +28,7 @@ using namespace xl_tc;
 constexpr int GS_ROWS = 128, GS_K = 256, GS_BLOCKS = GS_K / 64;
 constexpr int GS_TEAM = 8, GS_TEAMS = 1, GS_MULT = GS_TEAM * GS_TEAMS, GS_PREP = 4;  // warps
 constexpr int GS_THREADS = (GS_MULT + GS_PREP + 1) * 32;
-enum { ERR_GS_FULL = 41, ERR_GS_EMPTY = 42, ERR_GS_EMPTY_X = 43 };
+enum { ERR_GS_FULL = 61, ERR_GS_EMPTY = 62, ERR_GS_EMPTY_X = 63 };
 
 template <int NT> struct GsCfg {  // NT: tiles of 8 tokens
   static constexpr int TOK = NT * 8;

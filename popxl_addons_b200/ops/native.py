@@ -288,7 +288,11 @@ def check_gemm_errors():
                      53: "window attention: key / value stage was never released",
                      54: "window attention: scores never completed",
                      55: "window attention: probabilities never arrived",
-                     56: "window attention: output accumulation never completed"}
+                     56: "window attention: output accumulation never completed",
+                     61: "int4 product: codes or tokens never arrived", 62: "int4 product: shared-memory stage was never released (codes)",
+                     63: "int4 product: shared-memory stage was never released (tokens)",
+                     64: "decode attention: keys and values never arrived",
+                     65: "decode attention: shared-memory stage was never released"}
             raise RuntimeError(f"tcgen05 GEMM on cuda:{idx} gave up waiting: {names.get(code, code)}")
 
 
