@@ -490,7 +490,7 @@ template <typename T, int N> __device__ __forceinline__ void xl_store_vec(T* __r
 // ------------------------------------------------------------------------------------------------------------------
 // Residual update + LayerNorm for a few rows: x += delta (+ bias); h = LayerNorm(x) * w + b. One CTA per row. What bounds it is one
 // round trip to memory and the two sums over the CTA, so everything that is read is asked for at once and a sum takes one
-// barrier (each warp adds the warps' sums up itself). 16 rows of 4096, delta and bias, in a chain of launches: 6.5 -> 4.6 us (weights read behind the
+// barrier (each warp adds the warps' sums up itself). 16 rows of 4096, delta and bias, in a chain of launches: 3.5 -> 2.4 us (weights read behind the
 // statistics, sums by one thread between two barriers before).
 // ------------------------------------------------------------------------------------------------------------------
 template <typename T> __device__ __forceinline__ void aln_unpack(const uint4& raw, float (&out)[8]) {
@@ -502,13 +502,19 @@ template <> __device__ __forceinline__ void aln_unpack<float>(const uint4&, floa
 
 template <typename T, int VECS>  // VECS vectors of 8 elements per thread: cols <= 256 * 8 * VECS
 __global__ void __launch_bounds__(256)
-    add_layer_norm_kernel(T* x, const T* delta, const T* bias, const T* w, const T* b, T* h, int cols, float eps) {
+    add_layer_norm_kernel(T* x, const int* idx, const T* table, int table_rows, const T* delta, const T* bias, const T* w, const T* b, T* h,
+                          int cols, float eps) {
   xl_grid_dependency_wait();
   xl_grid_launch_dependents();
   constexpr bool WIDE = sizeof(T) == 4;  // fp32 rows: two 16-byte pieces a vector, weights read where they are used
   __shared__ float red[2][8];
   const int row = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   T* xr = x + (long long)row * cols;
+  const T* src = xr;
+  if (idx) {  // the row comes from the table (zeros for an index outside it) and is stored
+    const int r = idx[row];
+    src = r >= 0 && r < table_rows ? table + (long long)r * cols : nullptr;
+  }
   float v[VECS][8];
   uint4 raw[4][VECS];  // delta, bias, w, b
   const T* from[4] = {delta ? delta + (long long)row * cols : nullptr, bias, w, b};
@@ -516,7 +522,9 @@ __global__ void __launch_bounds__(256)
   for (int i = 0; i < VECS; ++i) {
     const int c = (threadIdx.x + i * 256) * 8;
     if (c < cols) {
-      xl_load_vec<T, 8>(xr + c, v[i]);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) v[i][e] = 0.f;
+      if (src) xl_load_vec<T, 8>(src + c, v[i]);
 #pragma unroll
       for (int q = 0; q < 4; ++q)
         if (!WIDE && from[q]) raw[q][i] = *reinterpret_cast<const uint4*>(from[q] + c);
@@ -549,7 +557,7 @@ __global__ void __launch_bounds__(256)
           for (int e = 0; e < 8; ++e) v[i][e] += d[e];
         }
       }
-      if (delta || bias) {
+      if (delta || bias || idx) {
         xl_store_vec<T, 8>(xr + c, v[i]);
 #pragma unroll
         for (int e = 0; e < 8; ++e) v[i][e] = xl_to_float(xl_from_float<T>(v[i][e]));  // what later readers of x see
@@ -582,18 +590,28 @@ __global__ void __launch_bounds__(256)
   }
 }
 
-// x (rows, cols) is updated in place when delta or bias is given; h (rows, cols) receives the normalised rows.
-XL_API int xl_add_layer_norm(void* x, const void* delta, const void* bias, const void* w, const void* b, void* h,
-                             int rows, int cols, float eps, int dtype, cudaStream_t s) {
+static int aln_launch(void* x, const int* idx, const void* table, int table_rows, const void* delta, const void* bias, const void* w,
+                      const void* b, void* h, int rows, int cols, float eps, int dtype, cudaStream_t s) {
   if (cols > 256 * 32 || (cols % 8) || rows < 1 || w == nullptr || b == nullptr) return -1;
   XL_DISPATCH_DTYPE(dtype, T, {
-    void (*kernel)(T*, const T*, const T*, const T*, const T*, T*, int, float) =
+    void (*kernel)(T*, const int*, const T*, int, const T*, const T*, const T*, const T*, T*, int, float) =
         cols <= 256 * 8 ? add_layer_norm_kernel<T, 1> : (cols <= 256 * 16 ? add_layer_norm_kernel<T, 2> : add_layer_norm_kernel<T, 4>);
-    const cudaError_t e = xl_launch_overlapped(kernel, dim3(rows), dim3(256), (size_t)0, s, (T*)x, (const T*)delta, (const T*)bias,
-                                               (const T*)w, (const T*)b, (T*)h, cols, eps);
+    const cudaError_t e = xl_launch_overlapped(kernel, dim3(rows), dim3(256), (size_t)0, s, (T*)x, idx, (const T*)table, table_rows,
+                                               (const T*)delta, (const T*)bias, (const T*)w, (const T*)b, (T*)h, cols, eps);
     if (e != cudaSuccess) return (int)e;
   });
   return (int)cudaGetLastError();
+}
+// x (rows, cols) is updated in place when delta or bias is given; h (rows, cols) receives the normalised rows.
+XL_API int xl_add_layer_norm(void* x, const void* delta, const void* bias, const void* w, const void* b, void* h,
+                             int rows, int cols, float eps, int dtype, cudaStream_t s) {
+  return aln_launch(x, nullptr, nullptr, 0, delta, bias, w, b, h, rows, cols, eps, dtype, s);
+}
+// x (rows, cols) = table[idx] (zeros for an index outside its table_rows), h the normalised rows; 16-byte aligned tables.
+XL_API int xl_gather_layer_norm(const int* idx, const void* table, int table_rows, void* x, const void* w, const void* b, void* h,
+                                int rows, int cols, float eps, int dtype, cudaStream_t s) {
+  if (!idx || !table || (((uintptr_t)table) & 15)) return -1;
+  return aln_launch(x, idx, table, table_rows, nullptr, nullptr, w, b, h, rows, cols, eps, dtype, s);
 }
 
 // ------------------------------------------------------------------------------------------------------------------
@@ -604,13 +622,20 @@ XL_API int xl_add_layer_norm(void* x, const void* delta, const void* bias, const
 // row), the CTAs' winners meet in the shared memory of the first one. What bounds it is latency: one CTA per row kept 16 rows of
 // 50400 16-bit logits on 16 SMs for 47 us (32000 fp32: 33 us); with eight CTAs per row a thread has three to four loads, all in
 // flight together: 4.0 us (3.2 us). Of equal maxima the lowest index wins; NaN never wins.
+// With `current` the choice is taken in the same launch: it becomes the row's current token and goes to row *pos + ahead - base of `buf`
+// (where there is such a row), and with `advance` the CTA of the last row to finish moves the position on.
+struct GreedyTake {
+  int *current, *buf, *pos;
+  int buf_rows, base, ahead, advance, rows;
+  unsigned int* counter;  // zero between launches
+};
 struct ArgBest { float v; int i; };
 __device__ __forceinline__ void arg_take(ArgBest& b, float v, int i) {
   if (v > b.v || (v == b.v && i < b.i)) { b.v = v; b.i = i; }
 }
 template <typename T>
 __global__ void __launch_bounds__(256)
-    argmax_rows_kernel(const T* logits, float* max_out, int* idx_out, int V, int valid, int index_offset) {
+    argmax_rows_kernel(const T* logits, float* max_out, int* idx_out, int V, int valid, int index_offset, const GreedyTake take) {
   constexpr int N = XlVec<T>::N;
   namespace cg = cooperative_groups;
   cg::cluster_group cluster = cg::this_cluster();
@@ -653,8 +678,21 @@ __global__ void __launch_bounds__(256)
   if (part == 0 && threadIdx.x == 0) {
     best = ctas[0];
     for (int k = 1; k < parts; ++k) arg_take(best, ctas[k].v, ctas[k].i);
-    max_out[row] = best.v;
-    idx_out[row] = best.i + index_offset;
+    if (take.current) {
+      const int at = *take.pos, r = at + take.ahead - take.base;
+      take.current[row] = best.i;
+      if (r >= 0 && r < take.buf_rows) take.buf[(long long)r * take.rows + row] = best.i;
+      if (take.advance) {
+        __threadfence();  // every row has read the position before the last one moves it
+        if (atomicAdd(take.counter, 1u) == (unsigned int)take.rows - 1) {
+          *take.counter = 0;
+          *take.pos = at + 1;
+        }
+      }
+    } else {
+      max_out[row] = best.v;
+      idx_out[row] = best.i + index_offset;
+    }
   }
 }
 __global__ void advance_position_kernel(int* pos) {
@@ -663,9 +701,8 @@ __global__ void advance_position_kernel(int* pos) {
   *pos += 1;
 }
 
-XL_API int xl_argmax_rows(const void* logits, float* max_out, int* idx_out, long long rows, int V, int valid,
-                          int index_offset, int dtype, cudaStream_t s) {
-  if (rows < 1) return 0;
+static int argmax_launch(const void* logits, float* max_out, int* idx_out, long long rows, int V, int valid, int index_offset,
+                         const GreedyTake& take, int dtype, cudaStream_t s) {
   // two loads per thread and CTA are enough work; no more CTAs than four per SM together
   const int per_pass = 256 * (dtype == XL_F32 ? 4 : 8);
   int parts = 1;
@@ -685,12 +722,25 @@ XL_API int xl_argmax_rows(const void* logits, float* max_out, int* idx_out, long
   for (long long r0 = 0; r0 < rows; r0 += 65535) {  // rows are the y axis of the grid
     cfg.gridDim.y = (unsigned)(rows - r0 < 65535 ? rows - r0 : 65535);
     XL_DISPATCH_DTYPE(dtype, T, {
-      const cudaError_t e = cudaLaunchKernelEx(&cfg, argmax_rows_kernel<T>, (const T*)logits + r0 * V, max_out + r0, idx_out + r0, V,
-                                               valid, index_offset);
+      const cudaError_t e = cudaLaunchKernelEx(&cfg, argmax_rows_kernel<T>, (const T*)logits + r0 * V, max_out ? max_out + r0 : nullptr,
+                                               idx_out ? idx_out + r0 : nullptr, V, valid, index_offset, take);
       if (e != cudaSuccess) return (int)e;
     });
   }
   return (int)cudaGetLastError();
+}
+XL_API int xl_argmax_rows(const void* logits, float* max_out, int* idx_out, long long rows, int V, int valid,
+                          int index_offset, int dtype, cudaStream_t s) {
+  if (rows < 1) return 0;
+  return argmax_launch(logits, max_out, idx_out, rows, V, valid, index_offset, GreedyTake{}, dtype, s);
+}
+// The greedy choice of every row taken (see GreedyTake): current (rows), buf (buf_rows, rows) int32, *pos the position. `counter`: a
+// zero-initialised word (left zeroed). At most 65535 rows.
+XL_API int xl_take_greedy(const void* logits, int* current, int* buf, int* pos, unsigned int* counter, int rows, int V, int valid,
+                          int buf_rows, int base, int ahead, int advance, int dtype, cudaStream_t s) {
+  if (rows < 1 || rows > 65535 || valid < 1 || valid > V || !current || !buf || !pos || !counter) return -1;
+  return argmax_launch(logits, nullptr, nullptr, rows, V, valid, 0, GreedyTake{current, buf, pos, buf_rows, base, ahead, advance, rows, counter},
+                       dtype, s);
 }
 XL_API int xl_advance_position(int* pos, cudaStream_t s) {
   const cudaError_t e = xl_launch_overlapped(advance_position_kernel, dim3(1), dim3(1), (size_t)0, s, pos);

@@ -174,8 +174,6 @@ class DecoderGenerator:
                 valid = vshard  # padded rows of the last shard are excluded below via the index check
                 m, idx = ops.argmax_rows(logits, valid, 0)
                 idx = idx + off if cfg.tp > 1 else idx
-                if cfg.tp == 1:
-                    return idx
                 # rows beyond the true vocabulary can only win if their (zero-weight) logit beats everything: mask them
                 in_vocab = ops.cast(ops.less(idx, xl.constant(cfg.vocab_size, xl.int32)), xl.float32)
                 m = m * in_vocab + (in_vocab - 1.0) * 1e30
@@ -185,6 +183,18 @@ class DecoderGenerator:
                 # smallest candidate index over the group = max of the negated candidates
                 win = ops.negate(ops.collectives.replicated_all_reduce(ops.negate(cand), "max", tp_group))
                 return ops.cast(win, xl.int32)
+
+            def take_token(hn, head, ins, decoding):
+                """The next token of every sequence: chosen, made the current one and stored; decoding, the position moves on first."""
+                if cfg.tp == 1:
+                    logits = linear_gq_window_t(hn, head["weight_compressed"], head["weight_scale_zero_t"], head["bias"])
+                    ops.take_greedy_(ins["cur"], logits, ins["out_buf"], ins["pos"], vshard, base=P, ahead=int(decoding), advance=decoding)
+                    return
+                tok = select_token(hn, head, ins["off"])
+                if decoding:
+                    ops.advance_position_(ins["pos"])
+                ops.var_updates.copy_var_update_(ins["cur"], tok)
+                ops.store_row_(ins["out_buf"], ins["pos"], tok, base=P)
 
             def rows(w: Dict[str, xl.Tensor], lo: int, hi: int) -> Dict[str, xl.Tensor]:
                 """Output rows [lo, hi) of a quantised weight (a contiguous slice of every one of its tensors)."""
@@ -208,11 +218,12 @@ class DecoderGenerator:
                     return ops.all_reduce_add_layer_norm_(x, delta, delta_bias, lnw, lnb, tp_group, eps=cfg.eps)
                 return ops.add_layer_norm_(x, delta, delta_bias, lnw, lnb, eps=cfg.eps)
 
-            def decode_block(x, delta, delta_bias, L, pos):
+            def decode_block(x, delta, delta_bias, L, pos, h=None):
                 """One token per sequence, four kernels: (all-reduce +) residual + LayerNorm; [qkv | gelu(fc_in)] in one
                 de-quantising GEMM; rotary, cache append and attention, written next to the fc_in output; [out | fc_out] in
-                one GEMM. Returns this rank's partial layer output; the next layer's first kernel reduces it."""
-                h = residual_norm(x, delta, delta_bias, L["ln_w"], L["ln_b"])
+                one GEMM. Returns this rank's partial layer output; the next layer's first kernel reduces it. `h`: the norm, if
+                it came with the embedding."""
+                h = residual_norm(x, delta, delta_bias, L["ln_w"], L["ln_b"]) if h is None else h
                 w1 = L["w1"]
                 buf = linear_gq_window_t(h, w1["weight_compressed"], w1["weight_scale_zero_t"], w1["bias"],
                                          act_from_col=3 * hd)
@@ -267,24 +278,23 @@ class DecoderGenerator:
                     x = prefill_block(x, L)
                 last = ops.reshape(x, (B, P, cfg.hidden))[:, P - 1]
                 hn = ops.layer_norm(last, ins["ln_f_w"], ins["ln_f_b"], eps=cfg.eps)
-                tok = select_token(hn, head, ins["off"])
-                ops.var_updates.copy_var_update_(ins["cur"], tok)
-                ops.store_row_(ins["out_buf"], ins["pos"], tok, base=P)
+                take_token(hn, head, ins, decoding=False)
 
             def decode_body(ins):
                 nonlocal sin_tab_i, cos_tab_i
                 sin_tab_i, cos_tab_i = ins["sin_tab"], ins["cos_tab"]
                 layers, head = unpack(ins)
-                x = embed(ins["cur"], ins["wte"], ins["off"])
-                delta = delta_bias = None
+                h = delta = delta_bias = None
+                if cfg.tp == 1:
+                    x, h = ops.gather_layer_norm(ins["wte"], ins["cur"], layers[0]["ln_w"], layers[0]["ln_b"], eps=cfg.eps)
+                else:
+                    x = embed(ins["cur"], ins["wte"], ins["off"])
                 for L in layers:
-                    delta = decode_block(x, delta, delta_bias, L, ins["pos"])
+                    delta = decode_block(x, delta, delta_bias, L, ins["pos"], h)
+                    h = None
                     delta_bias = L["w2"]["bias"]
                 hn = residual_norm(x, delta, delta_bias, ins["ln_f_w"], ins["ln_f_b"])
-                tok = select_token(hn, head, ins["off"])
-                ops.advance_position_(ins["pos"])
-                ops.var_updates.copy_var_update_(ins["cur"], tok)
-                ops.store_row_(ins["out_buf"], ins["pos"], tok, base=P)
+                take_token(hn, head, ins, decoding=True)
 
             prefill, pre_map = make_graph("prefill", prefill_body)
             decode, dec_map = make_graph("decode_step", decode_body)

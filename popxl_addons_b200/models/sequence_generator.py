@@ -111,10 +111,7 @@ class SequenceGenerator:
 
     def _sample(self, t, h):
         """Greedy choice for every slot: becomes the current token and a row of the output buffer."""
-        _, tok = ops.argmax_rows(self.model.logits(t, h), self.model.vocab, 0)
-        ops.var_updates.copy_var_update_(t("current"), tok)
-        ops.store_row_(t("generated"), t("step"), tok)
-        ops.advance_position_(t("step"))
+        ops.take_greedy_(t("current"), self.model.logits(t, h), t("generated"), t("step"), self.model.vocab)
 
     def _portion_program(self, T: int, sample: bool):
         def build(entry, t):

@@ -109,6 +109,8 @@ _attn_dec = _sig("xl_attn_decode", _c_p, _c_ll, _c_p, _c_p, _c_p, _c_p, _c_p, _c
 _ar_add_ln = _sig("xl_ar_add_layer_norm", _c_p, _c_p, _c_p, _c_p, _c_p, _c_p, _c_int, _c_int, _c_f, _c_int, _c_p, _c_p, _c_ll,
                   _c_p, _c_p, _c_int, _c_int, _c_int, _c_p, _c_p)
 _add_ln = _sig("xl_add_layer_norm", _c_p, _c_p, _c_p, _c_p, _c_p, _c_p, _c_int, _c_int, _c_f, _c_int, _c_p)
+_gather_ln = _sig("xl_gather_layer_norm", _c_p, _c_p, _c_int, _c_p, _c_p, _c_p, _c_p, _c_int, _c_int, _c_f, _c_int, _c_p)
+_take_greedy = _sig("xl_take_greedy", _c_p, _c_p, _c_p, _c_p, _c_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_p)
 _argmax = _sig("xl_argmax_rows", _c_p, _c_p, _c_p, _c_ll, _c_int, _c_int, _c_int, _c_int, _c_p)
 _advance = _sig("xl_advance_position", _c_p, _c_p)
 _store_row = _sig("xl_store_row", _c_p, _c_p, _c_int, _c_p, _c_int, _c_int, _c_p)
@@ -1297,6 +1299,38 @@ def add_layer_norm_cuda(x, *rest, has_delta, has_bias, eps):
     _check(rc, "add_layer_norm")
     _count("add_layer_norm")
     return h
+
+
+@native("gather_layer_norm")
+def gather_layer_norm_cuda(table, idx, w, b, eps):
+    if not _ok(table, w, b) or table.dim() != 2 or table.shape[1] > 8192 or idx.dtype != torch.int32 or not idx.is_contiguous() \
+            or not (table.dtype == w.dtype == b.dtype):
+        return NotImplemented
+    x = torch.empty((idx.numel(), table.shape[1]), dtype=table.dtype, device=table.device)
+    h = torch.empty_like(x)
+    rc = _gather_ln(idx.data_ptr(), table.data_ptr(), table.shape[0], x.data_ptr(), w.data_ptr(), b.data_ptr(), h.data_ptr(), x.shape[0],
+                    x.shape[1], float(eps), _CODE[x.dtype], _stream())
+    if rc == -1:
+        return NotImplemented
+    _check(rc, "gather_layer_norm")
+    _count("gather_rows+add_layer_norm")
+    return x, h
+
+
+@native("take_greedy_")
+def take_greedy_cuda(current, logits, buf, pos, valid, base, ahead, advance):
+    if not _ok(logits) or logits.dim() != 2 or any(t.dtype != torch.int32 or not t.is_contiguous() for t in (current, buf, pos)) \
+            or buf.dim() != 2 or not current.numel() == buf.shape[1] == logits.shape[0]:
+        return NotImplemented
+    rows, V = logits.shape
+    rc = _take_greedy(logits.data_ptr(), current.data_ptr(), buf.data_ptr(), pos.data_ptr(),
+                      counters(1, logits.device, "counters greedy", 1).data_ptr(), rows, V, valid, buf.shape[0], base, ahead,
+                      int(advance), _CODE[logits.dtype], _stream())
+    if rc == -1:
+        return NotImplemented
+    _check(rc, "take_greedy")
+    _count("argmax_rows+store_row+advance_position" if advance else "argmax_rows+store_row")
+    return current
 
 
 @native("argmax_rows")

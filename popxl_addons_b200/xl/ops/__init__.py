@@ -1396,6 +1396,7 @@ def cross_entropy_with_grad(logits: Tensor, labels: Tensor, loss_grad=1.0, reduc
     return loss, dlogits
 from .decode import (rotary_kv_append_, attention_decode_packed, argmax_rows, advance_position_, store_row_,  # noqa: E402
                      kv_cache_fill_, timestamp, attention_decode_into_, rotary_attention_decode_into_, add_layer_norm_,
+                     take_greedy_, gather_layer_norm,
                      all_reduce_add_layer_norm_)
 from .sequence import (embed_dyt_, linear_residual_dyt_, select_dyt, linear_rows, linear_swiglu, min_gru_,  # noqa: E402
                        diff_attention_, advance_by_, embed_rms_, linear_residual_rms_, select_rms, linear_split_glu,

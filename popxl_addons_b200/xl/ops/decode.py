@@ -57,6 +57,22 @@ def _argmax_rows_ref(logits, valid, index_offset):
     return m, (i + index_offset).to(torch.int32)
 
 
+def _take_greedy_ref(current, logits, buf, pos, valid, base, ahead, advance):
+    if logits.device.type == "meta":
+        return current
+    tok = _argmax_rows_ref(logits, valid, 0)[1]
+    current.copy_(tok.reshape(current.shape))
+    _store_row_ref(buf, pos + ahead, tok, base)
+    if advance:
+        pos.add_(1)
+    return current
+
+
+def _gather_layer_norm_ref(table, idx, w, b, eps):
+    x = torch.index_select(table, 0, idx.long().reshape(-1)) if table.device.type != "meta" else table.new_empty((idx.numel(), table.shape[1]))
+    return x, torch.nn.functional.layer_norm(x.float(), (x.shape[-1],), w.float(), b.float(), eps).to(x.dtype)
+
+
 def _advance_ref(pos):
     if pos.device.type != "meta":
         pos.add_(1)
@@ -125,6 +141,8 @@ OpDef("add_layer_norm_", impl=_add_layer_norm_ref)
 OpDef("rotary_kv_append_", impl=_rotary_kv_append_ref, inplace=True)
 OpDef("attention_decode_packed", impl=_attn_decode_packed_ref)
 OpDef("argmax_rows", impl=_argmax_rows_ref)
+OpDef("take_greedy_", impl=_take_greedy_ref, inplace=True)
+OpDef("gather_layer_norm", impl=_gather_layer_norm_ref)
 OpDef("advance_position_", impl=_advance_ref, inplace=True)
 OpDef("store_row_", impl=_store_row_ref, inplace=True)
 OpDef("kv_cache_fill_", impl=_kv_fill_ref, inplace=True)
@@ -214,6 +232,20 @@ def argmax_rows(logits: Tensor, valid: Optional[int] = None, index_offset: int =
     """Per row: maximum over the first `valid` columns (fp32) and its column index plus `index_offset` (int32)."""
     m, i = emit("argmax_rows", [logits], dict(valid=int(valid or logits.shape[-1]), index_offset=int(index_offset)))
     return m, i
+
+
+def take_greedy_(current: Tensor, logits: Tensor, buf: Tensor, pos: Tensor, valid: Optional[int] = None, base: int = 0, ahead: int = 0,
+                 advance: bool = True) -> Tensor:
+    """Greedy choice of every row over the first `valid` columns: it becomes `current` and row `pos + ahead - base` of `buf` (ignored when
+    out of range); then `pos` moves on by one with `advance`."""
+    return emit1("take_greedy_", [current, logits, buf, pos],
+                 dict(valid=int(valid or logits.shape[-1]), base=int(base), ahead=int(ahead), advance=bool(advance)))
+
+
+def gather_layer_norm(table: Tensor, idx: Tensor, weight: Tensor, bias: Tensor, eps: float = 1e-5) -> Tuple[Tensor, Tensor]:
+    """`x = table[idx]` and its layer norm, as one op."""
+    x, h = emit("gather_layer_norm", [table, idx, weight, bias], dict(eps=float(eps)))
+    return x, h
 
 
 def advance_position_(pos: Tensor) -> Tensor:

@@ -178,6 +178,43 @@ def test_argmax_store_row_advance(nat):
     assert int((buf != 0).any(dim=1).sum()) == 1
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("rows,V,valid", [(1, 1, 1), (1, 50400, 50399), (16, 33, 33), (40, 32000, 32000), (300, 1001, 777)])
+def test_take_greedy(nat, dtype, rows, V, valid):
+    """One CTA per row and clusters, many rows: the choice of the separate kernel, its place in the buffer, rows outside the buffer, and
+    the position, which moves only when all rows have read it; called in a row, with the counter back at zero."""
+    logits = torch.randn(rows, V, generator=torch.Generator(device="cuda").manual_seed(V), device="cuda").to(dtype)
+    want = nat.argmax_rows_cuda(logits, valid, 0)[1]
+    current, pos = torch.full((rows,), -1, dtype=torch.int32, device="cuda"), torch.tensor(6, dtype=torch.int32, device="cuda")
+    buf = torch.full((3, rows), -1, dtype=torch.int32, device="cuda")
+    for k, (ahead, advance, r) in enumerate([(0, True, 0), (1, True, 2), (0, False, 2), (1, True, None), (-7, True, None)]):
+        buf.fill_(-1)
+        at = int(pos)
+        assert nat.take_greedy_cuda(current, logits, buf, pos, valid, 6, ahead, advance) is current
+        assert torch.equal(current, want) and int(pos) == at + int(advance)
+        for i in range(3):
+            assert torch.equal(buf[i], want) if i == r else bool((buf[i] == -1).all())
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("rows,cols", [(1, 8), (3, 2048), (16, 2056), (5, 4104), (2, 8192)])
+def test_gather_layer_norm(nat, dtype, rows, cols):
+    """Rows to the bit, zeros for an index outside the table, and the norm against fp32, for each number of vectors a thread takes."""
+    g = torch.Generator(device="cuda").manual_seed(cols)
+    table, w, b = (torch.randn(*s, generator=g, device="cuda").to(dtype) for s in ((7, cols), (cols,), (cols,)))
+    idx = torch.arange(rows, dtype=torch.int32, device="cuda") % 7
+    if rows > 1:
+        idx[1] = 7
+    x, h = nat.gather_layer_norm_cuda(table, idx, w, b, 1e-5)
+    want = torch.where((idx < 7)[:, None], table[idx.long().clamp(max=6)], torch.zeros_like(table[:1]))
+    assert torch.equal(x, want)
+    norm = torch.nn.functional.layer_norm(want.float(), (cols,), w.float(), b.float(), 1e-5)
+    tol = {torch.float32: 1e-5, torch.bfloat16: 2.0 ** -8, torch.float16: 2.0 ** -11}[dtype]  # rounding of the result
+    torch.testing.assert_close(h.float(), norm, rtol=tol, atol=tol)
+    y = want.clone()
+    assert torch.equal(nat.add_layer_norm_cuda(y, w, b, has_delta=False, has_bias=False, eps=1e-5), h)
+
+
 @pytest.mark.parametrize("cuda_graphs", [False, True])
 def test_generation_on_gpu_matches_cpu_backend(cuda_graphs):
     from popxl_addons_b200.models.decoder import DecoderConfig
