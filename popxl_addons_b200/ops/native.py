@@ -721,11 +721,12 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, bias: Optional[torch.Tensor] = Non
         return NotImplemented
     if lda % 8 or ldb % 8 or a.data_ptr() % 16 or b.data_ptr() % 16 or (batched and (sa % 8 or sb % 8)):
         return NotImplemented
-    gaps = None
+    gaps, pairs = None, _GEMM_CTA_PAIRS and accumulate <= 2 and gather is None and not causal and N > 128
     if out is None:
         out_dtype = out_dtype or a.dtype
-        if plain and N % 8 and out_dtype in (torch.bfloat16, torch.float16):
-            # 16-bit rows that do not start on 16-byte boundaries: multiplied into padded rows, then copied together
+        if plain and N % 8 and out_dtype in (torch.bfloat16, torch.float16) and not pairs:
+            # 16-bit rows that do not start on 16-byte boundaries: the single-CTA kernel multiplies into padded rows, which are
+            # copied together; the pair kernel writes them as they are
             gaps = torch.empty((M, (N + 7) // 8 * 8), dtype=out_dtype, device=a.device)
             out = gaps[:, :N]
         else:
@@ -766,7 +767,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, bias: Optional[torch.Tensor] = Non
             g_mode, src_ptrs, flags, g_bps, g_copy = gather
             g_src, g_flags = src_ptrs.data_ptr(), flags.data_ptr()
             g_dst = a.data_ptr() if g_mode == 1 else b.data_ptr()
-    if _GEMM_CTA_PAIRS and accumulate <= 2 and gather is None and not causal and N > 128:
+    if pairs:
         rc = _gemm_pair(a.data_ptr(), b.data_ptr(), out_ptr, M, N, K, batch, a_mn, b_mn, lda, ldb, ldc, sa, sb, stride_c,
                         int(a.dtype == torch.float16), _CODE[out.dtype], bias.data_ptr() if bias is not None else None,
                         _CODE[bias.dtype] if bias is not None else 0, act, accumulate,
