@@ -11,7 +11,8 @@
 constexpr int EW_UNROLL = 4;  // 16-byte vectors per thread and iteration: keeps ~64 B per thread in flight
 
 template <typename T, typename F>
-__global__ void __launch_bounds__(256) ew_unary_kernel(const T* __restrict__ x, T* __restrict__ y, long long n, F f) {
+__global__ void __launch_bounds__(256) ew_unary_kernel(const T* x, T* y, long long n, F f) {
+  xl_grid_dependency_wait();
   xl_grid_launch_dependents();
   constexpr int N = XlVec<T>::N;
   const long long nvec = n / N;
@@ -41,7 +42,8 @@ __global__ void __launch_bounds__(256) ew_unary_kernel(const T* __restrict__ x, 
 
 template <typename T, typename F>
 __global__ void __launch_bounds__(256)
-    ew_binary_kernel(const T* __restrict__ x, const T* __restrict__ g, T* __restrict__ y, long long n, F f) {
+    ew_binary_kernel(const T* x, const T* g, T* y, long long n, F f) {
+  xl_grid_dependency_wait();
   xl_grid_launch_dependents();
   constexpr int N = XlVec<T>::N;
   const long long nvec = n / N;
@@ -132,34 +134,43 @@ struct SwiGlu {
 XL_API int xl_gelu_fwd(const void* x, void* y, long long n, int dtype, int tanh_approx, cudaStream_t s) {
   const int grid = xl_grid_for(n, 256 * 8);
   XL_DISPATCH_DTYPE(dtype, T, {
-    if (tanh_approx) ew_unary_kernel<T><<<grid, 256, 0, s>>>((const T*)x, (T*)y, n, GeluTanh());
-    else if (sizeof(T) == 2) ew_unary_kernel<T><<<grid, 256, 0, s>>>((const T*)x, (T*)y, n, GeluErfFast());
-    else ew_unary_kernel<T><<<grid, 256, 0, s>>>((const T*)x, (T*)y, n, GeluErf());
+    if (tanh_approx) XL_TRY((xl_launch_overlapped(ew_unary_kernel<T, GeluTanh>, dim3(grid), dim3(256),
+        (size_t)0, s, (const T*)x, (T*)y, n, GeluTanh())));
+    else if (sizeof(T) == 2) XL_TRY((xl_launch_overlapped(ew_unary_kernel<T, GeluErfFast>, dim3(grid), dim3(256),
+        (size_t)0, s, (const T*)x, (T*)y, n, GeluErfFast())));
+    else XL_TRY((xl_launch_overlapped(ew_unary_kernel<T, GeluErf>, dim3(grid), dim3(256),
+        (size_t)0, s, (const T*)x, (T*)y, n, GeluErf())));
   });
   return (int)cudaGetLastError();
 }
 XL_API int xl_gelu_bwd(const void* x, const void* g, void* dx, long long n, int dtype, int tanh_approx, cudaStream_t s) {
   const int grid = xl_grid_for(n, 256 * 8);
   XL_DISPATCH_DTYPE(dtype, T, {
-    if (tanh_approx) ew_binary_kernel<T><<<grid, 256, 0, s>>>((const T*)x, (const T*)g, (T*)dx, n, GeluTanhGrad());
-    else if (sizeof(T) == 2) ew_binary_kernel<T><<<grid, 256, 0, s>>>((const T*)x, (const T*)g, (T*)dx, n, GeluErfGradFast());
-    else ew_binary_kernel<T><<<grid, 256, 0, s>>>((const T*)x, (const T*)g, (T*)dx, n, GeluErfGrad());
+    if (tanh_approx) XL_TRY((xl_launch_overlapped(ew_binary_kernel<T, GeluTanhGrad>, dim3(grid), dim3(256),
+        (size_t)0, s, (const T*)x, (const T*)g, (T*)dx, n, GeluTanhGrad())));
+    else if (sizeof(T) == 2) XL_TRY((xl_launch_overlapped(ew_binary_kernel<T, GeluErfGradFast>, dim3(grid), dim3(256),
+        (size_t)0, s, (const T*)x, (const T*)g, (T*)dx, n, GeluErfGradFast())));
+    else XL_TRY((xl_launch_overlapped(ew_binary_kernel<T, GeluErfGrad>, dim3(grid), dim3(256),
+        (size_t)0, s, (const T*)x, (const T*)g, (T*)dx, n, GeluErfGrad())));
   });
   return (int)cudaGetLastError();
 }
 XL_API int xl_silu_fwd(const void* x, void* y, long long n, int dtype, cudaStream_t s) {
   const int grid = xl_grid_for(n, 256 * 8);
-  XL_DISPATCH_DTYPE(dtype, T, { ew_unary_kernel<T><<<grid, 256, 0, s>>>((const T*)x, (T*)y, n, Silu()); });
+  XL_DISPATCH_DTYPE(dtype, T, { XL_TRY((xl_launch_overlapped(ew_unary_kernel<T, Silu>, dim3(grid), dim3(256),
+      (size_t)0, s, (const T*)x, (T*)y, n, Silu()))); });
   return (int)cudaGetLastError();
 }
 XL_API int xl_silu_bwd(const void* x, const void* g, void* dx, long long n, int dtype, cudaStream_t s) {
   const int grid = xl_grid_for(n, 256 * 8);
-  XL_DISPATCH_DTYPE(dtype, T, { ew_binary_kernel<T><<<grid, 256, 0, s>>>((const T*)x, (const T*)g, (T*)dx, n, SiluGrad()); });
+  XL_DISPATCH_DTYPE(dtype, T, { XL_TRY((xl_launch_overlapped(ew_binary_kernel<T, SiluGrad>, dim3(grid), dim3(256),
+      (size_t)0, s, (const T*)x, (const T*)g, (T*)dx, n, SiluGrad()))); });
   return (int)cudaGetLastError();
 }
 XL_API int xl_swiglu_fwd(const void* gate, const void* up, void* y, long long n, int dtype, cudaStream_t s) {
   const int grid = xl_grid_for(n, 256 * 8);
-  XL_DISPATCH_DTYPE(dtype, T, { ew_binary_kernel<T><<<grid, 256, 0, s>>>((const T*)gate, (const T*)up, (T*)y, n, SwiGlu()); });
+  XL_DISPATCH_DTYPE(dtype, T, { XL_TRY((xl_launch_overlapped(ew_binary_kernel<T, SwiGlu>, dim3(grid), dim3(256),
+      (size_t)0, s, (const T*)gate, (const T*)up, (T*)y, n, SwiGlu()))); });
   return (int)cudaGetLastError();
 }
 
@@ -208,8 +219,9 @@ constexpr int NORM_MAX_ITERS = 8;
 
 template <typename T, bool RMS, int ITERS>
 __global__ void __launch_bounds__(NORM_THREADS)
-    norm_fwd_kernel(const T* __restrict__ x, const T* __restrict__ w, const T* __restrict__ b, T* __restrict__ y,
-                    float* __restrict__ mean_out, float* __restrict__ rstd_out, int cols, float eps) {
+    norm_fwd_kernel(const T* x, const T* w, const T* b, T* y,
+                    float* mean_out, float* rstd_out, int cols, float eps) {
+  xl_grid_dependency_wait();
   xl_grid_launch_dependents();
   constexpr int N = XlVec<T>::N;
   __shared__ float red[32];
@@ -287,8 +299,9 @@ XL_API int xl_layer_norm_fwd(const void* x, const void* w, const void* b, void* 
   const int iters = norm_iters(cols, dtype, NORM_MAX_ITERS);
   if (!iters) return -1;
   XL_DISPATCH_DTYPE(dtype, T, XL_DISPATCH_ITERS(iters, IT, {
-    norm_fwd_kernel<T, false, IT><<<(unsigned)rows, NORM_THREADS, 0, s>>>((const T*)x, (const T*)w, (const T*)b, (T*)y,
-                                                                           mean, rstd, cols, eps);
+    XL_TRY((xl_launch_overlapped(norm_fwd_kernel<T, false, IT>, dim3((unsigned)rows), dim3(NORM_THREADS),
+        (size_t)0, s, (const T*)x, (const T*)w, (const T*)b, (T*)y,
+                                                                           mean, rstd, cols, eps)));
   }));
   return (int)cudaGetLastError();
 }
@@ -297,8 +310,9 @@ XL_API int xl_rms_norm_fwd(const void* x, const void* w, void* y, float* rstd, l
   const int iters = norm_iters(cols, dtype, NORM_MAX_ITERS);
   if (!iters) return -1;
   XL_DISPATCH_DTYPE(dtype, T, XL_DISPATCH_ITERS(iters, IT, {
-    norm_fwd_kernel<T, true, IT><<<(unsigned)rows, NORM_THREADS, 0, s>>>((const T*)x, (const T*)w, nullptr, (T*)y,
-                                                                          nullptr, rstd, cols, eps);
+    XL_TRY((xl_launch_overlapped(norm_fwd_kernel<T, true, IT>, dim3((unsigned)rows), dim3(NORM_THREADS),
+        (size_t)0, s, (const T*)x, (const T*)w, nullptr, (T*)y,
+                                                                          nullptr, rstd, cols, eps)));
   }));
   return (int)cudaGetLastError();
 }
@@ -308,9 +322,10 @@ XL_API int xl_rms_norm_fwd(const void* x, const void* w, void* y, float* rstd, l
 // kernel reduces in a fixed order (deterministic).
 template <typename T, bool RMS, int ITERS>
 __global__ void __launch_bounds__(NORM_THREADS)
-    norm_bwd_kernel(const T* __restrict__ x, const T* __restrict__ w, const float* __restrict__ mean,
-                    const float* __restrict__ rstd, const T* __restrict__ g, T* __restrict__ dx,
-                    float* __restrict__ partial, long long rows, int cols) {
+    norm_bwd_kernel(const T* x, const T* w, const float* mean,
+                    const float* rstd, const T* g, T* dx,
+                    float* partial, long long rows, int cols) {
+  xl_grid_dependency_wait();
   xl_grid_launch_dependents();
   constexpr int N = XlVec<T>::N;
   __shared__ float red[32];
@@ -402,7 +417,8 @@ __global__ void __launch_bounds__(NORM_THREADS)
 // then the 8 group sums are added in a fixed order (deterministic).
 template <typename T>
 __global__ void __launch_bounds__(256)
-    norm_bwd_finish_kernel(const float* __restrict__ partial, T* __restrict__ dw, T* __restrict__ db, int nparts, int cols) {
+    norm_bwd_finish_kernel(const float* partial, T* dw, T* db, int nparts, int cols) {
+  xl_grid_dependency_wait();
   xl_grid_launch_dependents();
   __shared__ float sw[8][33], sb[8][33];
   const int lane = threadIdx.x & 31, grp = threadIdx.x >> 5;
@@ -437,9 +453,11 @@ static int norm_bwd_launch(const void* x, const void* w, const float* mean, cons
   if (!iters) return -1;
   const int parts = xl_norm_bwd_parts(rows);
   XL_DISPATCH_DTYPE(dtype, T, XL_DISPATCH_ITERS(iters, IT, {
-    norm_bwd_kernel<T, RMS, IT><<<parts, NORM_THREADS, 0, s>>>((const T*)x, (const T*)w, mean, rstd, (const T*)g,
-                                                              (T*)dx, partial, rows, cols);
-    norm_bwd_finish_kernel<T><<<(cols + 31) / 32, 256, 0, s>>>(partial, (T*)dw, (T*)db, parts, cols);
+    XL_TRY((xl_launch_overlapped(norm_bwd_kernel<T, RMS, IT>, dim3(parts), dim3(NORM_THREADS),
+        (size_t)0, s, (const T*)x, (const T*)w, mean, rstd, (const T*)g,
+                                                              (T*)dx, partial, rows, cols)));
+    XL_TRY((xl_launch_overlapped(norm_bwd_finish_kernel<T>, dim3((cols + 31) / 32), dim3(256),
+        (size_t)0, s, partial, (T*)dw, (T*)db, parts, cols)));
   }));
   return (int)cudaGetLastError();
 }
@@ -463,7 +481,8 @@ constexpr int COLSUM_THREADS = 256;
 // `partial[part][cols]`; the finish kernel adds the parts in a fixed order (deterministic).
 template <typename T>
 __global__ void __launch_bounds__(COLSUM_THREADS)
-    col_sum_kernel(const T* __restrict__ x, float* __restrict__ partial, long long rows, int cols, long long rows_per_part) {
+    col_sum_kernel(const T* x, float* partial, long long rows, int cols, long long rows_per_part) {
+  xl_grid_dependency_wait();
   xl_grid_launch_dependents();
   constexpr int N = XlVec<T>::N;
   __shared__ float red[COLSUM_THREADS / 32][32 * N + 1];
@@ -507,7 +526,8 @@ __global__ void __launch_bounds__(COLSUM_THREADS)
   }
 }
 template <typename T>
-__global__ void __launch_bounds__(256) col_sum_finish_kernel(const float* __restrict__ partial, T* __restrict__ out, int parts, int cols) {
+__global__ void __launch_bounds__(256) col_sum_finish_kernel(const float* partial, T* out, int parts, int cols) {
+  xl_grid_dependency_wait();
   xl_grid_launch_dependents();
   const int c = blockIdx.x * 256 + threadIdx.x;
   if (c >= cols) return;
@@ -534,8 +554,10 @@ XL_API int xl_col_sum(const void* x, void* out, float* partial, long long rows, 
   const long long rows_per_part = (rows + parts - 1) / parts;
   dim3 grid((cols + 32 * n - 1) / (32 * n), parts);
   XL_DISPATCH_DTYPE(dtype, T, {
-    col_sum_kernel<T><<<grid, COLSUM_THREADS, 0, s>>>((const T*)x, partial, rows, cols, rows_per_part);
-    col_sum_finish_kernel<T><<<(cols + 255) / 256, 256, 0, s>>>(partial, (T*)out, parts, cols);
+    XL_TRY((xl_launch_overlapped(col_sum_kernel<T>, dim3(grid), dim3(COLSUM_THREADS),
+        (size_t)0, s, (const T*)x, partial, rows, cols, rows_per_part)));
+    XL_TRY((xl_launch_overlapped(col_sum_finish_kernel<T>, dim3((cols + 255) / 256), dim3(256),
+        (size_t)0, s, partial, (T*)out, parts, cols)));
   });
   return (int)cudaGetLastError();
 }
@@ -729,7 +751,8 @@ XL_API int xl_sgd_step(void* w, int w_dtype, const void* g, int g_dtype, float* 
 // acc = acc * step/(step+1) + x/(step+1), `step` read on the device. Bound by HBM; four elements per thread and access.
 template <typename TA, typename TX, int V>
 __global__ void __launch_bounds__(256)
-    accumulate_mean_kernel(TA* __restrict__ acc, const TX* __restrict__ x, const float* __restrict__ step, long long n) {
+    accumulate_mean_kernel(TA* acc, const TX* x, const float* step, long long n) {
+  xl_grid_dependency_wait();
   xl_grid_launch_dependents();
   const float t = *step;
   const float a = t / (t + 1.f), b = 1.f / (t + 1.f);
@@ -746,18 +769,18 @@ __global__ void __launch_bounds__(256)
   if (blockIdx.x == 0 && i < n) acc[i] = xl_from_float<TA>(xl_to_float(acc[i]) * a + xl_to_float(x[i]) * b);
 }
 template <typename TA, typename TX>
-static void accumulate_mean_launch(void* acc, const void* x, const float* step, long long n, cudaStream_t s) {
+static cudaError_t accumulate_mean_launch(void* acc, const void* x, const float* step, long long n, cudaStream_t s) {
   const bool wide = !((((uintptr_t)acc) & (4 * sizeof(TA) - 1)) | (((uintptr_t)x) & (4 * sizeof(TX) - 1)));
-  if (wide) accumulate_mean_kernel<TA, TX, 4><<<xl_grid_for(n, 256 * 4), 256, 0, s>>>((TA*)acc, (const TX*)x, step, n);
-  else accumulate_mean_kernel<TA, TX, 1><<<xl_grid_for(n, 256 * 4), 256, 0, s>>>((TA*)acc, (const TX*)x, step, n);
+  return xl_launch_overlapped(wide ? accumulate_mean_kernel<TA, TX, 4> : accumulate_mean_kernel<TA, TX, 1>, dim3(xl_grid_for(n, 256 * 4)),
+                              dim3(256), (size_t)0, s, (TA*)acc, (const TX*)x, step, n);
 }
 XL_API int xl_accumulate_mean(void* acc, int acc_dtype, const void* x, int x_dtype, const float* step, long long n,
                               cudaStream_t s) {
   XL_DISPATCH_DTYPE(acc_dtype, TA, {
-    if (x_dtype == acc_dtype) accumulate_mean_launch<TA, TA>(acc, x, step, n, s);
-    else if (x_dtype == XL_BF16) accumulate_mean_launch<TA, __nv_bfloat16>(acc, x, step, n, s);
-    else if (x_dtype == XL_F16) accumulate_mean_launch<TA, __half>(acc, x, step, n, s);
-    else accumulate_mean_launch<TA, float>(acc, x, step, n, s);
+    if (x_dtype == acc_dtype) XL_TRY((accumulate_mean_launch<TA, TA>(acc, x, step, n, s)));
+    else if (x_dtype == XL_BF16) XL_TRY((accumulate_mean_launch<TA, __nv_bfloat16>(acc, x, step, n, s)));
+    else if (x_dtype == XL_F16) XL_TRY((accumulate_mean_launch<TA, __half>(acc, x, step, n, s)));
+    else XL_TRY((accumulate_mean_launch<TA, float>(acc, x, step, n, s)));
   });
   return (int)cudaGetLastError();
 }
@@ -801,8 +824,9 @@ XL_API int xl_grad_sumsq(const void* x, int dtype, const float* scale, float* ou
 // per thread with the tokens inside the heads: 59.7 us for the queries and keys of 2048 tokens, 32 heads of 128, 17.9 us this way.)
 template <typename T, int VP>
 __global__ void __launch_bounds__(256)
-    rotary_kernel(const T* x, const T* __restrict__ sin_t, const T* __restrict__ cos_t, T* y, uint32_t total, uint32_t H, uint32_t S, int D,
+    rotary_kernel(const T* x, const T* sin_t, const T* cos_t, T* y, uint32_t total, uint32_t H, uint32_t S, int D,
                   int R, int sin_batch, float sign, long long xb, long long xh, long long xs, long long yb, long long yh, long long ys) {
+  xl_grid_dependency_wait();
   xl_grid_launch_dependents();
   // in place only the rotated pairs are touched; out of place the pass-through features are copied as well
   const uint32_t per_row = (uint32_t)((x == y) ? R / 2 : D / 2) / VP;
@@ -874,9 +898,10 @@ XL_API int xl_rotary(const void* x, const void* sin_t, const void* cos_t, void* 
                       ((xb | xh | xs | yb | yh | ys) % (2 * VP)) == 0 && ((((uintptr_t)x) | ((uintptr_t)y)) & 15) == 0 &&
                       ((((uintptr_t)sin_t) | ((uintptr_t)cos_t)) & 7) == 0;
     if (wide)
-      rotary_kernel<T, VP><<<xl_grid_for(pairs / VP, 256), 256, 0, s>>>((const T*)x, (const T*)sin_t, (const T*)cos_t, (T*)y,
+      XL_TRY((xl_launch_overlapped(rotary_kernel<T, VP>, dim3(xl_grid_for(pairs / VP, 256)), dim3(256),
+          (size_t)0, s, (const T*)x, (const T*)sin_t, (const T*)cos_t, (T*)y,
                                                                         (uint32_t)(pairs / VP), (uint32_t)H, (uint32_t)S, D, R, sin_batch, sign,
-                                                                        xb, xh, xs, yb, yh, ys);
+                                                                        xb, xh, xs, yb, yh, ys)));
     else
       rotary_any_kernel<T><<<xl_grid_for(pairs, 256 * 4), 256, 0, s>>>((const T*)x, (const T*)sin_t, (const T*)cos_t, (T*)y, pairs, H, S, D, R,
                                                                        sin_batch, sign, xb, xh, xs, yb, yh, ys);
@@ -939,7 +964,8 @@ constexpr int SM_MAX_ITERS = 8;
 
 template <typename T, int ITERS>
 __global__ void __launch_bounds__(SM_THREADS)
-    attn_softmax_fwd_kernel(T* __restrict__ s, float* __restrict__ lse, int Sq, int Sk, float scale, int causal) {
+    attn_softmax_fwd_kernel(T* s, float* lse, int Sq, int Sk, float scale, int causal) {
+  xl_grid_dependency_wait();
   xl_grid_launch_dependents();
   constexpr int N = XlVec<T>::N;
   __shared__ float red[32];
@@ -1041,7 +1067,8 @@ XL_API int xl_attn_softmax_fwd(void* s_, float* lse, long long rows, int Sq, int
   const int iters = softmax_iters(Sk, dtype, SM_MAX_ITERS);
   if (!iters) return -1;
   XL_DISPATCH_DTYPE(dtype, T, XL_DISPATCH_ITERS(iters, IT, {
-    attn_softmax_fwd_kernel<T, IT><<<(unsigned)rows, SM_THREADS, 0, s>>>((T*)s_, lse, Sq, Sk, scale, causal);
+    XL_TRY((xl_launch_overlapped(attn_softmax_fwd_kernel<T, IT>, dim3((unsigned)rows), dim3(SM_THREADS),
+        (size_t)0, s, (T*)s_, lse, Sq, Sk, scale, causal)));
   }));
   return (int)cudaGetLastError();
 }
