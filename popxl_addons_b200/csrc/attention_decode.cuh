@@ -26,5 +26,19 @@ __device__ __forceinline__ uint32_t dd_pack(float lo, float hi) {
 }
 __device__ __forceinline__ float dd_lo(uint32_t v) { return __uint_as_float(v << 16); }
 __device__ __forceinline__ float dd_hi(uint32_t v) { return __uint_as_float(v & 0xffff0000u); }
+// four results; `pairs`: the row starts on a 4-byte boundary
+__device__ __forceinline__ void dd_store4(__nv_bfloat16* out, float a, float b, float c, float d, bool pairs) {
+  const uint32_t lo = dd_pack(a, b), hi = dd_pack(c, d);
+  if (pairs) {
+    reinterpret_cast<uint32_t*>(out)[0] = lo;
+    reinterpret_cast<uint32_t*>(out)[1] = hi;
+  } else {
+    uint16_t* o = reinterpret_cast<uint16_t*>(out);
+    o[0] = (uint16_t)lo;
+    o[1] = (uint16_t)(lo >> 16);
+    o[2] = (uint16_t)hi;
+    o[3] = (uint16_t)(hi >> 16);
+  }
+}
 
 }  // namespace

@@ -223,6 +223,13 @@ __global__ void __launch_bounds__(SPLIT == 1 ? 128 : SPLIT * 32)
 // Q1 K1^T with map 2's rows zero plus Q2 K2^T with map 1's rows zero, so one accumulator holds both maps, and its layout is
 // the operand layout of the second product P V, which both maps share. P enters that product as a sum of two bf16 numbers
 // (value and rounding error), so the weights keep more than 16 bits. Slices are merged by the CTA that arrives last.
+//
+// With a few hundred keys the time is a chain of latencies, not bytes, so everything that can be asked for at once is: the
+// rings hold cached keys only (they start to fill before the projections of this step are complete) and the new key and value
+// take their place in shared memory; a thread's share of the queries is in flight together; the warps' results are weighted
+// and combined in one pass, four features at a time.
+// 32 heads on 8 key heads, head sizes 64 / 128, before and after: 16 sequences at position 144 19.9 -> 6.8 us, at position 2000
+// 48.1 -> 38.7 us (131 MB: 3.4 TB/s); one sequence at position 8000 46.0 -> 18.1 us.
 constexpr int DD_WARPS = 4;
 constexpr int DD_KEYS = 16;       // keys per block
 constexpr int DD_HEADS = 8;       // query heads per CTA
@@ -239,7 +246,7 @@ struct DecodeParams {
   const float* lam;
   int H, G, dim, vdim, R, Smax, chunk;
   float scale, eps, out_scale;
-  float* part;             // [B * G * head chunks][splits][16][vdim + 2]
+  float* part;             // [B * G * head chunks][splits][16][vdim], then [B * G * head chunks][splits][16][2]: maximum, sum
   unsigned int* counters;  // [B * G * head chunks], zero between launches
   int stages;
   int read_ahead;  // positions, counts and the cached keys and values were complete before the previous launch
@@ -253,6 +260,7 @@ template <int KD, int VT>
 __global__ void __launch_bounds__(DD_WARPS * 32) diff_attn_decode_kernel(const DecodeParams p) {
   extern __shared__ __align__(16) uint8_t smem[];
   __shared__ __align__(16) __nv_bfloat16 sq[2][DD_HEADS][KD * 32];
+  __shared__ __align__(16) __nv_bfloat16 sk[2][KD * 32];  // the new key
   __shared__ float sm[DD_WARPS][16], sl[DD_WARPS][16];
   __shared__ float wt[DD_MAX_SPLITS * 16], wl[DD_MAX_SPLITS * 16];  // maxima, then weights, and sums of the slices
   __shared__ unsigned int is_last;
@@ -275,71 +283,79 @@ __global__ void __launch_bounds__(DD_WARPS * 32) diff_attn_decode_kernel(const D
   const __nv_bfloat16* kb = p.kc + ((long long)b * p.G + g) * 2 * p.Smax * p.dim;
   const __nv_bfloat16* vb = p.vc + ((long long)b * p.G + g) * p.Smax * p.vdim;
 
-  // ---- the ring of key / value blocks: a range without the new key starts to load right away --------------------------------
+  // ---- the ring of key / value blocks, cached rows only -----------------------------------------------------------------------
   const int stage_bytes = dd_stage_bytes(KD, p.vdim), vld = p.vdim + 8;
   uint8_t* ring = smem + (long long)warp * p.stages * stage_bytes;
   const int mine = (blk1 - blk0 - warp + DD_WARPS - 1) / DD_WARPS;  // this warp's blocks: blk0 + warp, + DD_WARPS, ...
   auto prefetch = [&](int n) {
     if (n < mine) {
       uint8_t* st = ring + (n % p.stages) * stage_bytes;
-      const int key0 = first + (blk0 + warp + n * DD_WARPS) * DD_KEYS;
+      const int key0 = first + (blk0 + warp + n * DD_WARPS) * DD_KEYS;  // rows from `pos` on are zero-filled
 #pragma unroll
       for (int m = 0; m < 2; ++m)
 #pragma unroll
         for (int t = 0; t < 2; ++t) {
-          const int key = min(key0 + t * 8 + quad, pos);  // rows past the end repeat the last one and are masked
-          const __nv_bfloat16* src = kb + ((long long)m * p.Smax + key) * p.dim;
+          const int key = key0 + t * 8 + quad;
+          const __nv_bfloat16* src = kb + (key < pos ? ((long long)m * p.Smax + key) * p.dim + j * 8 : 0);
 #pragma unroll
           for (int i = 0; i < KD; ++i) {
-            uint8_t* dst = st + (((m * 2 + t) * KD + i) * 32 + lane) * 16;
-            if (i * 32 + j * 8 < p.dim) dd_cp16(dst, src + i * 32 + j * 8);
-            else *reinterpret_cast<uint4*>(dst) = make_uint4(0, 0, 0, 0);
+            const bool on = key < pos && i * 32 + j * 8 < p.dim;
+            dd_cp16_zfill(st + (((m * 2 + t) * KD + i) * 32 + lane) * 16, on ? src + i * 32 : kb, on);
           }
         }
       uint8_t* sv = st + DD_KEYS * 2 * KD * 64;
       const int pieces = p.vdim / 8;
       for (int i = lane; i < DD_KEYS * pieces; i += 32) {
         const int k = i / pieces, c = i % pieces;
-        dd_cp16(sv + (k * vld + c * 8) * 2, vb + (long long)min(key0 + k, pos) * p.vdim + c * 8);
+        const bool on = key0 + k < pos;
+        dd_cp16_zfill(sv + (k * vld + c * 8) * 2, on ? vb + (long long)(key0 + k) * p.vdim + c * 8 : vb, on);
       }
     }
     asm volatile("cp.async.commit_group;" ::: "memory");  // possibly empty: keeps the group count per block fixed
   };
-  const bool appends = split == splits - 1;
-  if (!appends)
-    for (int n = 0; n < p.stages - 1; ++n) prefetch(n);
+  for (int n = 0; n < p.stages - 1; ++n) prefetch(n);
   xl_grid_dependency_wait();  // the new projections
   xl_grid_launch_dependents();
-  // ---- rotated queries to shared memory; the CTAs with the last keys append the new key and value (the same data each) ----
-  const int half = p.dim / 2;  // dim is even
-  auto rotated = [&](const __nv_bfloat16* s, int e, float& y0, float& y1) {
-    const float x0 = __bfloat162float(s[0]), x1 = __bfloat162float(s[1]);
+  // ---- rotated queries and new key to shared memory; the CTAs with the last keys append (the same data each) ------------------
+  const bool appends = split == splits - 1;
+  const float lambda = *p.lam;
+  uint4 v_new = make_uint4(0, 0, 0, 0);  // lane's piece of the new value, in every warp
+  {
+    constexpr int PAIRS = KD * 16, ROWS = DD_WARPS * 32 / PAIRS, PASSES = (2 * DD_HEADS + 2 + ROWS - 1) / ROWS;
+    const int e = (threadIdx.x % PAIRS) * 2, r0 = threadIdx.x / PAIRS;  // rows: 8 queries of map 1, 8 of map 2, 2 keys
+    uint32_t raw[PASSES];
+#pragma unroll
+    for (int i = 0; i < PASSES; ++i) {
+      const int hm = r0 + i * ROWS, m = hm < 2 * DD_HEADS ? hm / DD_HEADS : hm - 2 * DD_HEADS, r = hm % DD_HEADS;
+      const bool on = e < p.dim && (hm < 2 * DD_HEADS ? r < nh : hm < 2 * DD_HEADS + 2 && appends);
+      raw[i] = on ? *reinterpret_cast<const uint32_t*>(
+                        row + ((long long)(hm < 2 * DD_HEADS ? h0 + r : p.H + g) * 2 + m) * p.dim + e)
+                  : 0u;
+    }
+    if (appends && lane < p.vdim / 8)
+      v_new = *reinterpret_cast<const uint4*>(row + (long long)(p.H + p.G) * 2 * p.dim + (long long)g * p.vdim + lane * 8);
+    float c = 1.f, sn = 0.f;
     if (e < p.R) {
-      const float c = p.cos_t[(long long)pos * (p.R / 2) + e / 2], sn = p.sin_t[(long long)pos * (p.R / 2) + e / 2];
-      y0 = x0 * c - x1 * sn;
-      y1 = x1 * c + x0 * sn;
-    } else {
-      y0 = x0;
-      y1 = x1;
+      c = p.cos_t[(long long)pos * (p.R / 2) + e / 2];
+      sn = p.sin_t[(long long)pos * (p.R / 2) + e / 2];
     }
-  };
-  for (int i = threadIdx.x; i < 2 * DD_HEADS * KD * 16; i += blockDim.x) {
-    const int e = (i % (KD * 16)) * 2, hm = i / (KD * 16), m = hm / DD_HEADS, r = hm % DD_HEADS;
-    float y0 = 0.f, y1 = 0.f;
-    if (r < nh && e < p.dim) rotated(row + ((long long)(h0 + r) * 2 + m) * p.dim + e, e, y0, y1);
-    *reinterpret_cast<uint32_t*>(&sq[m][r][e]) = dd_pack(y0, y1);
-  }
-  if (appends) {
-    for (int i = threadIdx.x; i < 2 * half; i += blockDim.x) {
-      const int m = i / half, e = (i % half) * 2;
-      float y0, y1;
-      rotated(row + ((long long)(p.H + g) * 2 + m) * p.dim + e, e, y0, y1);
-      *reinterpret_cast<uint32_t*>(p.kc + ((((long long)b * p.G + g) * 2 + m) * p.Smax + pos) * p.dim + e) = dd_pack(y0, y1);
+#pragma unroll
+    for (int i = 0; i < PASSES; ++i) {
+      const int hm = r0 + i * ROWS;
+      if (hm >= 2 * DD_HEADS + 2) break;
+      const float x0 = dd_lo(raw[i]), x1 = dd_hi(raw[i]);
+      const uint32_t y = e < p.R ? dd_pack(x0 * c - x1 * sn, x1 * c + x0 * sn) : raw[i];
+      if (hm < 2 * DD_HEADS) {  // rows and features that are not in use: zero
+        *reinterpret_cast<uint32_t*>(&sq[hm / DD_HEADS][hm % DD_HEADS][e]) = y;
+      } else if (appends) {
+        const int m = hm - 2 * DD_HEADS;
+        *reinterpret_cast<uint32_t*>(&sk[m][e]) = y;
+        if (e < p.dim)
+          *reinterpret_cast<uint32_t*>(p.kc + ((((long long)b * p.G + g) * 2 + m) * p.Smax + pos) * p.dim + e) = y;
+      }
     }
-    const __nv_bfloat16* vsrc = row + (long long)(p.H + p.G) * 2 * p.dim + (long long)g * p.vdim;
-    __nv_bfloat16* vdst = p.vc + (((long long)b * p.G + g) * p.Smax + pos) * p.vdim;
-    for (int i = threadIdx.x; i < p.vdim; i += blockDim.x) vdst[i] = vsrc[i];
-    __threadfence();
+    if (appends && threadIdx.x < p.vdim / 8)
+      *reinterpret_cast<uint4*>(p.vc + (((long long)b * p.G + g) * p.Smax + pos) * p.vdim + threadIdx.x * 8) = v_new;
   }
   __syncthreads();
   uint4 q1[KD], q2[KD];
@@ -355,15 +371,23 @@ __global__ void __launch_bounds__(DD_WARPS * 32) diff_attn_decode_kernel(const D
     for (int e = 0; e < 4; ++e) o[t][e] = 0.f;
   float mx[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f};  // rows quad (map 1) and quad + 8 (map 2)
   const float sc = p.scale * 1.4426950408889634f;
-  if (appends)
-    for (int n = 0; n < p.stages - 1; ++n) prefetch(n);
   for (int n = 0; n < mine; ++n) {
     prefetch(n + p.stages - 1);
     if (p.stages == 2) asm volatile("cp.async.wait_group 1;" ::: "memory");
     else asm volatile("cp.async.wait_group 2;" ::: "memory");
     __syncwarp();
-    const uint8_t* st = ring + (n % p.stages) * stage_bytes;
-    const int key0 = first + (blk0 + warp + n * DD_WARPS) * DD_KEYS;
+    uint8_t* st = ring + (n % p.stages) * stage_bytes;
+    const int blk = blk0 + warp + n * DD_WARPS, key0 = first + blk * DD_KEYS;
+    if (blk == blocks - 1) {  // the new key and value take their place
+      const int k = pos - key0;
+      for (int i = lane; i < 2 * KD * 4; i += 32) {
+        const int m = i / (KD * 4), c = i % (KD * 4);
+        *reinterpret_cast<uint4*>(st + (((m * 2 + (k >> 3)) * KD + (c >> 2)) * 32 + (k & 7) * 4 + (c & 3)) * 16) =
+            *reinterpret_cast<const uint4*>(&sk[m][c * 8]);
+      }
+      if (lane < p.vdim / 8) *reinterpret_cast<uint4*>(st + DD_KEYS * 2 * KD * 64 + (k * vld + lane * 8) * 2) = v_new;
+      __syncwarp();
+    }
     float s[2][4];
 #pragma unroll
     for (int t = 0; t < 2; ++t) {
@@ -446,57 +470,67 @@ __global__ void __launch_bounds__(DD_WARPS * 32) diff_attn_decode_kernel(const D
     }
   }
   __syncthreads();  // all rings are idle: their memory holds the warps' outputs from here on
-  float* so = reinterpret_cast<float*>(smem);  // [DD_WARPS][16][vdim]
+  float* so = reinterpret_cast<float*>(smem);  // [DD_WARPS][16][vdim + 8]
+  const int old = p.vdim + 8;                  // the padding keeps the quads' stores in different banks
 #pragma unroll
   for (int t = 0; t < VT; ++t) {
     if (t * 8 < p.vdim) {
-      float* d = so + ((long long)warp * 16 + quad) * p.vdim + t * 8 + 2 * j;
-      d[0] = o[t][0];
-      d[1] = o[t][1];
-      d += 8 * p.vdim;
-      d[0] = o[t][2];
-      d[1] = o[t][3];
+      float* d = so + (warp * 16 + quad) * old + t * 8 + 2 * j;
+      *reinterpret_cast<float2*>(d) = make_float2(o[t][0], o[t][1]);
+      *reinterpret_cast<float2*>(d + 8 * old) = make_float2(o[t][2], o[t][3]);
     }
   }
-  __syncthreads();
-  // ---- merge of the warps; the slice's result goes to `part`, or stays here when there is one slice ------------------------
-  __shared__ float fm[16], fl[16];
-  const long long unit = (long long)b * gridDim.y + blockIdx.y;
-  const int pw = p.vdim + 2;
-  float* mypart = p.part + (unit * splits + split) * 16 * pw;
+  // ---- merge of the warps: their weights, and the sums of the weights --------------------------------------------------------
+  __shared__ float fw[DD_WARPS][16], fl[16];
+  const long long units = (long long)gridDim.z * gridDim.y, unit = (long long)b * gridDim.y + blockIdx.y;
+  float* stats = p.part + units * splits * 16 * p.vdim;
   if (threadIdx.x < 16) {
     const int r = threadIdx.x;
     float m = -INFINITY, ll = 0.f;
+#pragma unroll
     for (int w = 0; w < DD_WARPS; ++w) m = fmaxf(m, sm[w][r]);
-    for (int w = 0; w < DD_WARPS; ++w) ll += sm[w][r] == -INFINITY ? 0.f : sl[w][r] * exp2f(sm[w][r] - m);
-    fm[r] = m;
-    fl[r] = ll;
-    if (splits > 1) {
-      __stcg(mypart + r * pw, m);
-      __stcg(mypart + r * pw + 1, ll);
+#pragma unroll
+    for (int w = 0; w < DD_WARPS; ++w) {
+      const float f = sm[w][r] == -INFINITY ? 0.f : exp2f(sm[w][r] - m);
+      fw[w][r] = f;
+      ll += sm[w][r] == -INFINITY ? 0.f : sl[w][r] * f;
     }
+    fl[r] = ll;
+    if (splits > 1) __stcg(reinterpret_cast<float2*>(stats) + (unit * splits + split) * 16 + r, make_float2(m, ll));
   }
   __syncthreads();
-  for (int i = threadIdx.x; i < 2 * nh * p.vdim; i += blockDim.x) {
-    const int rr = i / p.vdim, c = i - rr * p.vdim, r = rr < nh ? rr : DD_HEADS + rr - nh;  // rows in use
-    float acc = 0.f;
+  // One warp per head. Row r (map 1) or r + 8 (map 2), features c .. c + 3, over this CTA's warps:
+  auto merged = [&](int r, int c) {
+    float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-    for (int w = 0; w < DD_WARPS; ++w)
-      acc += sm[w][r] == -INFINITY ? 0.f : so[((long long)w * 16 + r) * p.vdim + c] * exp2f(sm[w][r] - fm[r]);
-    if (splits > 1) __stcg(mypart + r * pw + 2 + c, acc);
-    else so[(long long)r * p.vdim + c] = acc;  // warp 0's copy: read and written by this thread only
-  }
+    for (int w = 0; w < DD_WARPS; ++w) {
+      const float f = fw[w][r];
+      const float4 x = *reinterpret_cast<const float4*>(so + (w * 16 + r) * old + c);
+      if (sm[w][r] != -INFINITY) a = make_float4(a.x + x.x * f, a.y + x.y * f, a.z + x.z * f, a.w + x.w * f);
+    }
+    return a;
+  };
+  constexpr int CH = (VT * 8 + 127) / 128;  // features c of a lane: (lane + 32 u) * 4 ..
   if (splits > 1) {
+    for (int r = warp; r < nh; r += DD_WARPS)
+#pragma unroll
+      for (int u = 0; u < CH; ++u) {
+        const int c = (lane + 32 * u) * 4;
+        if (c >= p.vdim) continue;
+#pragma unroll
+        for (int m = 0; m < 2; ++m)
+          __stcg(reinterpret_cast<float4*>(p.part + ((unit * splits + split) * 16 + r + 8 * m) * p.vdim + c), merged(r + 8 * m, c));
+      }
     __threadfence();
     __syncthreads();
     if (threadIdx.x == 0) is_last = atomicAdd(p.counters + unit, 1u) == (unsigned int)splits - 1;
     __syncthreads();
     if (!is_last) return;
     __threadfence();
-    const float* parts = p.part + unit * splits * 16 * pw;
     for (int i = threadIdx.x; i < splits * 16; i += blockDim.x) {
-      wt[i] = __ldcg(parts + (long long)i * pw);
-      wl[i] = __ldcg(parts + (long long)i * pw + 1);
+      const float2 v = __ldcg(reinterpret_cast<const float2*>(stats) + unit * splits * 16 + i);
+      wt[i] = v.x;
+      wl[i] = v.y;
     }
     __syncthreads();
     if (threadIdx.x < 16) {
@@ -509,32 +543,46 @@ __global__ void __launch_bounds__(DD_WARPS * 32) diff_attn_decode_kernel(const D
       }
       fl[threadIdx.x] = ll;
     }
-    __syncthreads();
-    for (int i = threadIdx.x; i < 2 * nh * p.vdim; i += blockDim.x) {
-      const int rr = i / p.vdim, c = i - rr * p.vdim, r = rr < nh ? rr : DD_HEADS + rr - nh;
-      const float* src = parts + (long long)r * pw + 2 + c;
-      float acc = 0.f;
-#pragma unroll 8
-      for (int k = 0; k < splits; ++k) acc += wt[k * 16 + r] * __ldcg(src + (long long)k * 16 * pw);
-      so[(long long)r * p.vdim + c] = acc;
-    }
     if (threadIdx.x == 0) p.counters[unit] = 0;
+    __syncthreads();
   }
-  __syncthreads();
-  // ---- a_1 - lambda a_2, divided by its root mean square: one warp per head -------------------------------------------------
-  const float lambda = *p.lam;
+  // ---- a_1 - lambda a_2, divided by its root mean square ---------------------------------------------------------------------
   for (int r = warp; r < nh; r += DD_WARPS) {
     const float i1 = 1.f / fl[r], i2 = lambda / fl[r + 8];
+    float4 v[CH];
     float ss = 0.f;
-    for (int c = lane; c < p.vdim; c += 32) {
-      const float v = so[(long long)r * p.vdim + c] * i1 - so[(long long)(r + 8) * p.vdim + c] * i2;
-      so[(long long)r * p.vdim + c] = v;
-      ss += v * v;
+#pragma unroll
+    for (int u = 0; u < CH; ++u) {
+      const int c = (lane + 32 * u) * 4;
+      v[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (c >= p.vdim) continue;
+      float4 a1 = v[u], a2 = v[u];
+      if (splits > 1) {
+        const float* src = p.part + (unit * splits * 16 + r) * p.vdim + c;
+#pragma unroll 4
+        for (int k = 0; k < splits; ++k, src += 16 * p.vdim) {
+          const float4 x1 = __ldcg(reinterpret_cast<const float4*>(src));
+          const float4 x2 = __ldcg(reinterpret_cast<const float4*>(src + 8 * p.vdim));
+          const float f1 = wt[k * 16 + r], f2 = wt[k * 16 + r + 8];
+          a1 = make_float4(a1.x + x1.x * f1, a1.y + x1.y * f1, a1.z + x1.z * f1, a1.w + x1.w * f1);
+          a2 = make_float4(a2.x + x2.x * f2, a2.y + x2.y * f2, a2.z + x2.z * f2, a2.w + x2.w * f2);
+        }
+      } else {
+        a1 = merged(r, c);
+        a2 = merged(r + 8, c);
+      }
+      v[u] = make_float4(a1.x * i1 - a2.x * i2, a1.y * i1 - a2.y * i2, a1.z * i1 - a2.z * i2, a1.w * i1 - a2.w * i2);
+      ss += v[u].x * v[u].x + v[u].y * v[u].y + v[u].z * v[u].z + v[u].w * v[u].w;
     }
     ss = xl_warp_sum(ss);
     const float f = p.out_scale / sqrtf(ss / p.vdim + p.eps);
-    for (int c = lane; c < p.vdim; c += 32)
-      p.out[(long long)b * p.ldo + (long long)(h0 + r) * p.vdim + c] = __float2bfloat16_rn(so[(long long)r * p.vdim + c] * f);
+    __nv_bfloat16* out = p.out + (long long)b * p.ldo + (long long)(h0 + r) * p.vdim;
+#pragma unroll
+    for (int u = 0; u < CH; ++u) {
+      const int c = (lane + 32 * u) * 4;
+      if (c >= p.vdim) continue;
+      dd_store4(out + c, v[u].x * f, v[u].y * f, v[u].z * f, v[u].w * f, ((uintptr_t)out & 3) == 0);
+    }
   }
 }
 
@@ -542,7 +590,7 @@ template <int KD, int VT> int dd_launch(DecodeParams p, int B, int splits, cudaS
   const int stage = dd_stage_bytes(KD, p.vdim) * DD_WARPS;
   p.stages = 3 * stage <= DD_RING_LIMIT ? 3 : 2;
   int bytes = p.stages * stage;
-  const int merge = DD_WARPS * 16 * p.vdim * 4;
+  const int merge = DD_WARPS * 16 * (p.vdim + 8) * 4;
   if (bytes < merge) bytes = merge;
   static XlPerDevice smem;
   XL_TRY(xl_allow_smem(diff_attn_decode_kernel<KD, VT>, bytes, smem));
@@ -607,7 +655,7 @@ XL_API int xl_diff_attn_general(const void* q, long long ldq, const void* kc, co
 
 // One token per sequence (rows of qkv = sequences), bf16. dim, vdim multiples of 8, dim <= 128, vdim <= 256, ld a multiple of
 // 8. The new key and value are rotated / appended by the kernel; q is not modified. part: B * G * ceil(H/G/8) * splits * 16 *
-// (vdim + 2) floats; counters: B * G * ceil(H/G/8) zero-initialised words (left zeroed). Sequences with count 0 are skipped.
+// (vdim + 2) floats, 16-byte aligned; counters: B * G * ceil(H/G/8) zero-initialised words (left zeroed). Sequences with count 0 are skipped.
 XL_API int xl_diff_attn_decode(const void* qkv, long long ld, const float* cos_t, const float* sin_t, void* kc, void* vc,
                                void* out, long long ldo, const int* pos, const int* count, const float* lam, int B, int H, int G,
                                int dim, int vdim, int R, int Smax, int chunk, float scale, float eps, float out_scale,
@@ -616,7 +664,7 @@ XL_API int xl_diff_attn_decode(const void* qkv, long long ld, const float* cos_t
       R < 0 || R > dim || (R & 1) || Smax < 1 || chunk < 0 || splits < 1 || splits > DD_MAX_SPLITS || (ld % 8))
     return -1;
   if (((uintptr_t)qkv & 15) || ((uintptr_t)kc & 15) || ((uintptr_t)vc & 15) || (R > 0 && (!cos_t || !sin_t))) return -1;
-  if (splits > 1 && (!part || !counters)) return -1;
+  if (splits > 1 && (!part || ((uintptr_t)part & 15) || !counters)) return -1;
   DecodeParams p = {};
   p.qkv = (const __nv_bfloat16*)qkv; p.ld = ld; p.cos_t = cos_t; p.sin_t = sin_t;
   p.kc = (__nv_bfloat16*)kc; p.vc = (__nv_bfloat16*)vc; p.out = (__nv_bfloat16*)out; p.ldo = ldo;

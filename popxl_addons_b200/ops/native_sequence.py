@@ -224,6 +224,20 @@ def min_gru_cuda(h, weight, bz, bx, state, pos, count, T):
     return y
 
 
+def _decode_slices(units, longest, whole, device) -> int:
+    """Into how many CTAs the keys of one (sequence, key head, chunk of query heads) are cut, at up to `longest` keys: one wave
+    of two CTAs per SM, a 16-key block for each of a CTA's four warps. Up to `whole` keys the merge costs more than it saves:
+    a caller's cache is often much longer than what it holds, and an empty slice costs its merge all the same (differential
+    attention, 16 x 8 and 8 key heads, 160 keys: 1 slice 6.7 and 5.7 us, 2 slices 8.6 and 6.6; windows, 8 key heads: 256 keys
+    in 1 and 4 slices 6.9 and 6.2 us, 40 keys 3.9 and 5.7; 384 keys 9.3 and 6.9). Where only two or three slices fit the wave
+    they have to be longer (windows, 16 x 8 key heads: 256 keys 8.1 and 9.2 us, 512 keys 12.9 and 12.8, 1024 keys 21.6 and
+    18.9 in 1 and 2 slices)."""
+    most = 2 * _sms(device) // units
+    if longest <= whole or most < 2:
+        return 1
+    return min(most, (longest + 63) // 64 if most >= 4 else max(1, longest // 192), 64)
+
+
 @native("diff_attention_")
 def diff_attention_cuda(qkv, cos, sin, kc, vc, pos, count, lam, T, heads, rotary_dim, chunk, scale, eps, out_scale):
     B, G, _, smax, dim = kc.shape
@@ -237,7 +251,7 @@ def diff_attention_cuda(qkv, cos, sin, kc, vc, pos, count, lam, T, heads, rotary
     if T == 1 and qkv.dtype == torch.bfloat16 and dim % 8 == 0 and vdim % 8 == 0 and dim <= 128 and vdim <= 256:
         units = B * G * ((heads // G + 7) // 8)
         longest = min(smax, chunk) if chunk else smax
-        splits = max(1, min(2 * _sms(qkv.device) // units, (longest + 63) // 64, 64))  # one wave, two CTAs per SM
+        splits = _decode_slices(units, longest, 192, qkv.device)
         done = counters(units, qkv.device, "counters sequence", 1 << 16)
         part = torch.empty(units * splits * 16 * (vdim + 2), dtype=torch.float32, device=qkv.device) if splits > 1 else None
         if units <= 1 << 16:
@@ -358,8 +372,7 @@ def window_attention_cuda(proj, q_norm, k_norm, kc, vc, pos, count, joint, T, he
     if T == 1 and proj.dtype == torch.bfloat16:
         units = B * G * ((heads // G + 15) // 16)
         longest = min(smax, window + keep_first) if window else smax
-        # one wave, two CTAs per SM; a slice of fewer keys costs more in the merge than it saves
-        splits = max(1, min(2 * _sms(proj.device) // units, (longest + 383) // 384, 64))
+        splits = _decode_slices(units, longest, 320, proj.device)
         done = counters(units, proj.device, "counters sequence", 1 << 16)
         part = torch.empty(units * splits * 16 * (vdim + 2), dtype=torch.float32, device=proj.device) if splits > 1 else None
         if units <= 1 << 16:

@@ -230,6 +230,25 @@ def test_diff_attention(backend, shape, plant):
         torch.testing.assert_close(kc[1, :, :, :n], kc[2, :, :, :n], rtol=0, atol=0)
 
 
+@pytest.mark.parametrize("n", [1, 17, 64, 65, 192, 193, 450])  # caches of one slice and of several; the new key alone in its block
+def test_diff_attention_of_the_last_token(backend, n):
+    """The last position of a cache that it fills to the end; its row of the cache holds NaN before."""
+    H, G, dim, vdim, eps, out_scale, lam, scale = 6, 2, 64, 128, 1e-5, 0.4, 0.83, 0.125
+    raw = torch.randn(n, (H + G) * 2 * dim + G * vdim, generator=torch.Generator().manual_seed(n)).to(backend[1])
+    want = diff_oracle(raw.double(), H, G, dim, vdim, 0, scale, 0, eps, out_scale, lam, [])[-1:]
+    dev, none = backend[0], torch.zeros(1, device=backend[0])
+    kc = torch.zeros(1, G, 2, n, dim, dtype=backend[1], device=dev)
+    vc = torch.zeros(1, G, n, vdim, dtype=backend[1], device=dev)
+    for at, T in ((0, n - 1), (n - 1, 1)):
+        kc[:, :, :, n - 1], vc[:, :, n - 1] = (0.0, 0.0) if T > 1 else (float("nan"),) * 2
+        if T:
+            got = op("diff_attention_", backend, raw[at:at + T].to(dev), none, none, kc, vc, i32(backend, at), i32(backend, T),
+                     torch.tensor([lam], device=dev), T=T, heads=H, rotary_dim=0, chunk=0, scale=scale, eps=eps,
+                     out_scale=out_scale)
+    close(got, want, backend, 3e-5, 4e-2)  # the tolerances of the portions above
+    assert torch.equal(vc[0, :, -1].cpu(), raw[-1, -G * vdim:].reshape(G, vdim))
+
+
 def test_rotary_frequencies_match_the_oracle():
     from popxl_addons_b200.ops.rotary_pos_embed import frequency_tables, rotary_frequencies
 

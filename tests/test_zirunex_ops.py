@@ -170,6 +170,27 @@ SHAPES = [  # H, G, dim, vdim, window, keep, positions
 ]
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("smax", [70, 900])  # one slice and several
+@pytest.mark.parametrize("vdim,heads", [(40, 3), (128, 4), (200, 18)])
+def test_window_attention_into_rows_of_any_alignment(smax, vdim, heads):
+    """An output row that starts on an odd element gets the same bits as rows on 16-byte boundaries; the row of the caches that the
+    new token takes holds NaN before."""
+    H, G, dim, gpu = heads, 1, 64, ("cuda", torch.bfloat16)
+    proj = rnd(gpu, 2, (H + G) * dim + G * vdim + H * vdim, seed=1)[0]
+    one = torch.ones(dim, device="cuda")
+    outs = []
+    for extra in (8, 0, 3):
+        kc, vc = (rnd(gpu, 2, G, smax, c, seed=c)[0] for c in (dim, vdim))
+        kc[:, :, smax - 1] = vc[:, :, smax - 1] = float("nan")
+        joint = torch.full((2, H * vdim + extra), 9.0, dtype=torch.bfloat16, device="cuda")
+        op("window_attention_", gpu, proj, one, one, kc, vc, i32(gpu, smax - 1, smax - 1), i32(gpu, 1, 1), joint, T=1, heads=H,
+           window=0, keep_first=0, scale=0.125, sink=-1.5, eps=1e-5)
+        outs.append(joint[:, :H * vdim].clone())
+        assert (joint[:, H * vdim:] == 9.0).all() and outs[-1].isfinite().all()
+    assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])
+
+
 @pytest.mark.parametrize("shape", SHAPES, ids=lambda s: "x".join(map(str, s)))
 @pytest.mark.parametrize("plant", ["none", "edges"])
 def test_window_attention(backend, shape, plant):  # noqa: F811
