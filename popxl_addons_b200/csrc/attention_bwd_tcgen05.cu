@@ -104,7 +104,6 @@ template <int D, int BKV>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
     attn_bwd_dq_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_do,
                                const __grid_constant__ CUtensorMap map_kv, const AttnBwdParams p) {
-  xl_grid_launch_dependents();
   using L = BwdSmem<D, BKV>;
   static_assert(D % 64 == 0 && D <= 256 && BKV % 32 == 0 && BKV <= 64 && D + 4 * BKV <= (int)TMEM_COLS, "unsupported tile");
   extern __shared__ uint8_t smem_raw[];
@@ -174,6 +173,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
   __syncthreads();
   tcgen05_fence_after();
   const uint32_t tmem_base = *tmem_base_slot;
+  xl_grid_launch_dependents();  // TMEM is held: a successor that allocates some on this SM cannot come first
   const uint32_t tmem_dq = tmem_base;                 // columns [0, D)
   const uint32_t tmem_s = tmem_base + D;              // two buffers of BKV columns
   const uint32_t tmem_dp = tmem_base + D + 2 * BKV;   // two buffers of BKV columns

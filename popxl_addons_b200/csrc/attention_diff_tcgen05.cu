@@ -55,7 +55,6 @@ template <int DK, int VD>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
     diff_attn_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                              const __grid_constant__ CUtensorMap map_v, const DiffParams p) {
-  xl_grid_launch_dependents();
   using L = DiffSmem<DK, VD>;
   static_assert(L::TOTAL <= 227 * 1024, "shared memory");
   extern __shared__ uint8_t smem_raw[];
@@ -111,6 +110,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
   __syncthreads();
   tcgen05_fence_after();
   const uint32_t tmem_base = *tmem_base_slot;
+  xl_grid_launch_dependents();  // TMEM is held: a successor that allocates some on this SM cannot come first
 
   if (warp == 0) {
     // lane 0: queries and key tiles, lane 1: value tiles; each waits only on its own ring

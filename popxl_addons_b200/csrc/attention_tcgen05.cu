@@ -80,7 +80,6 @@ template <int D, int BKV>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
     attn_fwd_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                             const __grid_constant__ CUtensorMap map_v, const AttnParams p) {
-  xl_grid_launch_dependents();
   using L = AttnSmem<D, BKV>;
   static_assert(D % 64 == 0 && D <= 256 && BKV % 64 == 0 && D + 2 * BKV <= (int)TMEM_COLS, "unsupported tile");
   extern __shared__ uint8_t smem_raw[];
@@ -144,6 +143,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
   __syncthreads();
   tcgen05_fence_after();
   const uint32_t tmem_base = *tmem_base_slot;
+  xl_grid_launch_dependents();  // TMEM is held: a successor that allocates some on this SM cannot come first
   const uint32_t tmem_o = tmem_base;          // columns [0, D)
   const uint32_t tmem_s = tmem_base + D;      // two buffers of BKV columns
 

@@ -171,11 +171,12 @@ template <> __device__ __forceinline__ float2 xl_pair_to_float2<__nv_bfloat16>(u
 // xl_grid_dependency_wait() before it touches anything the predecessor reads or writes. Operands that were complete before the
 // predecessor started (weights, as a rule) may be read ahead of that wait, which hides their latency in the predecessor's tail;
 // whether an operand was is the caller's knowledge: such kernels take a `read_ahead` argument, and with 0 they wait first.
-// xl_grid_launch_dependents() after that wait lets the
-// successor do the same, so at most two kernels of a chain are in flight. Both are no-ops in an ordinary launch, where a kernel may call
-// xl_grid_launch_dependents() at once: it started when all work before it had ended (element-wise and attention kernels do, for the
-// products behind them, whose start-up of barriers, TMEM and descriptors takes 2 us otherwise). No pointer of such
-// a kernel is `__restrict__`: through one, the compiler could move a read of the predecessor's results over the wait.
+// xl_grid_launch_dependents() after that wait lets the successor do the same, so at most two kernels of a chain are in flight. Both are
+// no-ops in an ordinary launch, where a kernel may call xl_grid_launch_dependents() at once: it started when all work before it had ended
+// (element-wise and attention kernels do, for the products behind them, whose start-up of barriers, TMEM and descriptors takes 2 us
+// otherwise). A kernel that allocates TMEM calls it behind the barrier that follows its allocation: a successor allocates before it
+// waits, and if its CTA came first on an SM, its columns would wait for this kernel's end and this kernel for its columns.
+// No pointer of such a kernel is `__restrict__`: through one, the compiler could move a read of the predecessor's results over the wait.
 __device__ __forceinline__ void xl_grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void xl_grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 

@@ -250,7 +250,6 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
   if (warp == 0) {
     // ------------------------------------------------ TMA producer ------------------------------------------------
     xl_grid_dependency_wait();
-    xl_grid_launch_dependents();
     if (elect_one()) {
       uint32_t stage = 0, phase = 0;
       bool ok = true;
@@ -289,7 +288,8 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
   } else if (warp == 1) {
     const uint32_t tmem_base = *tmem_base_slot;
-    xl_grid_dependency_wait();  // no bounded wait runs while the previous kernel still does
+    xl_grid_dependency_wait();    // no bounded wait runs while the previous kernel still does
+    xl_grid_launch_dependents();  // here, not with the first loads: TMEM is held (see common.cuh)
     // ------------------------------------------------ MMA issuer (leader CTA only) -------------------------------
     if (leader && elect_one()) {
       const uint32_t fmt = p.is_fp16 ? 0u : 1u;
