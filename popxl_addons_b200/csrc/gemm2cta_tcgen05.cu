@@ -179,8 +179,9 @@ __device__ __forceinline__ void tile_coords(int tile, int tiles_m, int tiles_n, 
 //   EPI_16   16-bit C, overwritten, rows on 16-byte boundaries
 //   EPI_F32  fp32 C (overwritten or accumulated into), rows on 16-byte boundaries
 //   EPI_16A  16-bit C that is accumulated into (the second of two summed products), rows on 16-byte boundaries
-//   EPI_ANY  the rest: fp32 and 16-bit rows of any alignment
-enum EpiKind : int { EPI_16 = 0, EPI_F32 = 1, EPI_ANY = 2, EPI_16A = 3 };
+//   EPI_ANY32, EPI_ANY16, EPI_ANY16A  the same three for rows of any alignment
+// (One instance for the last three spilled 88 bytes a thread: 4096 x 768 x 50257 in fp32 442 -> 496 us, added to 16 bits 3603 -> 5545.)
+enum EpiKind : int { EPI_16 = 0, EPI_F32 = 1, EPI_16A = 2, EPI_ANY32 = 3, EPI_ANY16 = 4, EPI_ANY16A = 5 };
 
 template <int PN, int EPI>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
@@ -402,10 +403,25 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
 #pragma unroll 1
       for (int c = c_begin; c < c_end; c += 32) {
         const int col0 = nb * PAIR_N + c;
-        if (col0 >= p.N) break;  // uniform over the warp
+        if (col0 >= p.N || row_base >= p.M) break;  // uniform over the warp
         uint32_t r[32];
         tmem_ld_32x32b_x32(taddr + c, r);
         tmem_ld_wait();
+        // rows of any alignment: the thread's 32 columns to (row, column ^ row), both phases free of bank conflicts
+        float* stage32 = (float*)stage;
+        auto stage_columns = [&]() {
+          with_bias_and_act(p.epi, [&](auto bias, auto act) {
+            const float bv = decltype(bias)::value && col0 + lane < p.N ? epilogue_bias(p.epi, col0 + lane) : 0.f;
+#pragma unroll
+            for (int j = 0; j < 32; ++j) {
+              float v = __fmul_rn(__uint_as_float(r[j]), p.alpha);
+              if (decltype(bias)::value) v = __fadd_rn(v, __shfl_sync(0xffffffffu, bv, j));
+              if (decltype(act)::value) v = apply_act(v, p.epi.act);
+              stage32[lane * 32 + (j ^ lane)] = v;
+            }
+          });
+          __syncwarp();
+        };
         if (EPI == EPI_16 && col0 + 32 <= p.N) {
           // 16-bit C, no accumulation: the thread's 32 columns (64 bytes) go to shared memory, 16-byte pieces rotated by
           // the row pair so that neither phase has bank conflicts; then 4 lanes store one row's 64 bytes, 8 rows per
@@ -494,68 +510,60 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
             if (rr < p.M) *(float4*)(cbase + (long long)rr * p.ldc + c) = out[i];
           }
           __syncwarp();  // the buffer is rewritten by the next chunk
-        } else if (EPI == EPI_ANY && p.epi.c_dtype == XL_F32) {
+        } else if (EPI == EPI_ANY32) {
           // Rows that do not start on 16-byte boundaries (an odd number of columns): still whole row pieces, one column per
           // lane and one row per instruction, the old contents requested ahead of all stores. From the registers every
           // instruction touched 32 rows: the running mean of a 768 x 50257 gradient over 4096 tokens took 0.61 ms even with one
           // row per instruction but without the requests ahead; 0.24 ms this way, as for 50264 columns.
-          float* stage32 = (float*)stage;  // (row, column ^ row): both phases free of bank conflicts
           const int col = col0 + lane, rows = min(32, p.M - row_base);
           const bool on = col < p.N;
           float* c32 = (float*)p.C + (long long)b * p.batch_stride_c + (long long)row_base * p.ldc + col;
+          stage_columns();  // first: its registers are free for the old contents then
           float before[32];
           if (p.epi.accumulate) {
 #pragma unroll
-            for (int i = 0; i < 32; ++i) before[i] = on && i < rows ? c32[i * p.ldc] : 0.f;
-          }
-          const float bv = on ? epilogue_bias(p.epi, col) : 0.f;
-#pragma unroll
-          for (int j = 0; j < 32; ++j) stage32[lane * 32 + (j ^ lane)] = __uint_as_float(r[j]) * p.alpha;
-          __syncwarp();
-          with_bias_and_act(p.epi, [&](auto, auto act) {
-#pragma unroll
-            for (int i0 = 0; i0 < 32; i0 += 8) {  // reads of shared memory first: the compiler keeps them behind earlier stores
-              float o[8];
-#pragma unroll
-              for (int i = 0; i < 8; ++i) o[i] = stage32[(i0 + i) * 32 + (lane ^ (i0 + i))];
-#pragma unroll
-              for (int i = 0; i < 8; ++i) {
-                float t = o[i] + bv;
-                if (decltype(act)::value) t = apply_act(t, p.epi.act);
-                if (p.epi.accumulate == 1) t += before[i0 + i];
-                else if (p.epi.accumulate == 2) t = before[i0 + i] * mean_a + t * mean_b;
-                if (on && i0 + i < rows) c32[(i0 + i) * p.ldc] = t;
-              }
+            for (int i = 0; i < 32; ++i) {
+              before[i] = on && i < rows ? *c32 : 0.f;
+              c32 += p.ldc;
             }
-          });
+            c32 -= 32 * p.ldc;
+          }
+#pragma unroll
+          for (int i0 = 0; i0 < 32; i0 += 8) {  // reads of shared memory first: the compiler keeps them behind earlier stores
+            float o[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) o[i] = stage32[(i0 + i) * 32 + (lane ^ (i0 + i))];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+              float t = o[i];
+              if (p.epi.accumulate == 1) t += before[i0 + i];
+              else if (p.epi.accumulate == 2) t = before[i0 + i] * mean_a + t * mean_b;
+              if (on && i0 + i < rows) *c32 = t;
+              c32 += p.ldc;
+            }
+          }
           __syncwarp();
-        } else if (EPI == EPI_ANY && !p.epi.accumulate) {
+        } else if (EPI == EPI_ANY16) {
           // 16-bit rows of any alignment: a row's 32 columns per instruction. Against padded rows that are copied together afterwards:
-          // 2048 x 1024 x 8191 69 -> 45 us, 4096 x 768 x 50257 456 -> 399 (229 with the padded rows alone). With two columns per lane and the
-          // ends of odd rows by themselves, half the stores for twice the arithmetic, 78 and 526.
-          float* stage32 = (float*)stage;
+          // 2048 x 1024 x 8191 59 -> 39 us, 4096 x 768 x 50257 459 -> 353 (229 with the padded rows alone), 40 x 768 x 50257 57 -> 52. With
+          // two columns per lane and the ends of odd rows by themselves, half the stores for twice the arithmetic, 78 and 526 in
+          // place of the first two.
           const int col = col0 + lane, rows = min(32, p.M - row_base);
           const bool on = col < p.N, bf = p.epi.c_dtype == XL_BF16;
           uint16_t* c16 = (uint16_t*)p.C + (long long)b * p.batch_stride_c + (long long)row_base * p.ldc + col;
-          const float bv = on ? epilogue_bias(p.epi, col) : 0.f;
+          stage_columns();
 #pragma unroll
-          for (int j = 0; j < 32; ++j) stage32[lane * 32 + (j ^ lane)] = __uint_as_float(r[j]) * p.alpha;
-          __syncwarp();
-          with_bias_and_act(p.epi, [&](auto, auto act) {
+          for (int i0 = 0; i0 < 32; i0 += 16) {
+            uint16_t o[16];
 #pragma unroll
-            for (int i0 = 0; i0 < 32; i0 += 16) {
-              uint16_t o[16];
-#pragma unroll
-              for (int i = 0; i < 16; ++i) {
-                float t = stage32[(i0 + i) * 32 + (lane ^ (i0 + i))] + bv;
-                if (decltype(act)::value) t = apply_act(t, p.epi.act);
-                o[i] = bf ? __bfloat16_as_ushort(__float2bfloat16_rn(t)) : __half_as_ushort(__float2half_rn(t));
-              }
-#pragma unroll
-              for (int i = 0; i < 16; ++i, c16 += p.ldc)
-                if (on && i0 + i < rows) __stcs(c16, o[i]);
+            for (int i = 0; i < 16; ++i) {
+              const float t = stage32[(i0 + i) * 32 + (lane ^ (i0 + i))];
+              o[i] = bf ? __bfloat16_as_ushort(__float2bfloat16_rn(t)) : __half_as_ushort(__float2half_rn(t));
             }
-          });
+#pragma unroll
+            for (int i = 0; i < 16; ++i, c16 += p.ldc)
+              if (on && i0 + i < rows) __stcs(c16, o[i]);
+          }
           __syncwarp();
         } else if (row_ok) {
           epilogue_store_32cols(p.epi, r, crow, col0, p.alpha, mean_a, mean_b);
@@ -703,15 +711,15 @@ XL_API int xl_gemm2cta_tcgen05(const void* a, const void* b, void* c, int M, int
   p.step = step; p.alpha = alpha; p.is_fp16 = ab_is_fp16; p.err = err;
   const int align = c_dtype == XL_F32 ? 4 : 8;  // elements of 16 bytes
   const bool aligned = (ldc % align) == 0 && (batch == 1 || (stride_c % align) == 0) && (((uintptr_t)c) & 15) == 0;
-  const int kind = !aligned ? EPI_ANY : c_dtype == XL_F32 ? EPI_F32 : accumulate ? EPI_16A : EPI_16;
-  if (pair_n == 128) {
-    if (kind == EPI_16) return launch_pairs<128, EPI_16>(ma, mb, p, max_pairs, s);
-    if (kind == EPI_F32) return launch_pairs<128, EPI_F32>(ma, mb, p, max_pairs, s);
-    if (kind == EPI_16A) return launch_pairs<128, EPI_16A>(ma, mb, p, max_pairs, s);
-    return launch_pairs<128, EPI_ANY>(ma, mb, p, max_pairs, s);
-  }
-  if (kind == EPI_16) return launch_pairs<256, EPI_16>(ma, mb, p, max_pairs, s);
-  if (kind == EPI_F32) return launch_pairs<256, EPI_F32>(ma, mb, p, max_pairs, s);
-  if (kind == EPI_16A) return launch_pairs<256, EPI_16A>(ma, mb, p, max_pairs, s);
-  return launch_pairs<256, EPI_ANY>(ma, mb, p, max_pairs, s);
+  const bool wide = c_dtype == XL_F32;
+  const auto launch = [&](auto pn) -> int {
+    constexpr int PN = decltype(pn)::value;
+    if (aligned) {
+      if (wide) return launch_pairs<PN, EPI_F32>(ma, mb, p, max_pairs, s);
+      return accumulate ? launch_pairs<PN, EPI_16A>(ma, mb, p, max_pairs, s) : launch_pairs<PN, EPI_16>(ma, mb, p, max_pairs, s);
+    }
+    if (wide) return launch_pairs<PN, EPI_ANY32>(ma, mb, p, max_pairs, s);
+    return accumulate ? launch_pairs<PN, EPI_ANY16A>(ma, mb, p, max_pairs, s) : launch_pairs<PN, EPI_ANY16>(ma, mb, p, max_pairs, s);
+  };
+  return pair_n == 128 ? launch(std::integral_constant<int, 128>()) : launch(std::integral_constant<int, 256>());
 }

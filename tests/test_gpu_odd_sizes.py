@@ -51,6 +51,29 @@ def test_products(nat, M, K, N, dtype):
     _near(nat.gemm(x, b), x.double() @ b.double(), dtype)
 
 
+@pytest.mark.parametrize("out_dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("M,N", [(1, 131), (31, 160), (33, 257), (128, 129), (140, 600), (300, 1031)])
+@pytest.mark.parametrize("gap", [0, 1, 8])
+def test_every_way_a_product_leaves_the_pair_kernel(nat, out_dtype, M, N, gap):
+    """Overwritten, added to and as a running mean, with bias and activation or without, into rows of `gap` more columns than are written
+    (aligned and not), down to a single row of a tile; the columns between the rows stay as they are."""
+    g = torch.Generator(device="cuda").manual_seed(M + N + gap)
+    K, step = 72, torch.tensor(3.0, device="cuda")
+    a, b, bias = ((torch.randn(*s, device="cuda", generator=g) * 0.3).bfloat16() for s in ((M, K), (K, N), (N,)))
+    buf = torch.randn(M, N + gap, device="cuda", generator=g).to(out_dtype)
+    plain = a.double() @ b.double()
+    before = nat.LAUNCHES["by_kernel"].get("gemm2cta_tcgen05", 0)
+    for want, kw in ((plain, {}), (torch.nn.functional.gelu(plain + bias.double()), dict(bias=bias, act=1)), (plain + bias.double(), dict(bias=bias))):
+        for acc in (0, 1, 2):
+            held, full = buf.double()[:, :N], buf.clone()
+            out = full[:, :N]
+            assert nat.gemm(a, b, out=out, accumulate=acc, step=step if acc == 2 else None, **kw) is out
+            sums = {0: want, 1: held + want, 2: held * 0.75 + want * 0.25}[acc]
+            _near(out, sums, out_dtype, scale=sums.abs().max() + 1, terms=K)
+            assert torch.equal(full[:, N:], buf[:, N:])
+    assert nat.LAUNCHES["by_kernel"]["gemm2cta_tcgen05"] == before + 9
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
 @pytest.mark.parametrize("rows,V", [(1, 5), (3, 7), (2, 8), (65, 4099), (66, 1001), (70, 8193), (4, 50257)])
 def test_cross_entropy_and_its_column_sums(nat, rows, V, dtype):
