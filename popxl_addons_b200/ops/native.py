@@ -6,6 +6,7 @@ does not cover (odd alignment, unsupported dtype); the session then runs the op'
 missing on a machine with a GPU the import fails loudly rather than silently running the reference everywhere.
 """
 import ctypes
+import functools
 import os
 import threading
 from collections import OrderedDict
@@ -1225,6 +1226,7 @@ def rotary_kv_append_cuda(qkv, sin_tab, cos_tab, k_cache, v_cache, pos, n_heads,
     return qkv
 
 
+@functools.lru_cache(maxsize=256)
 def _attn_decode_splits(bh: int, smax: int, head_dim: int, sms: int) -> int:
     """CTAs that share a (sequence, head): what takes the least time for a full cache. A CTA reads up to 55 KB a us, all together 6.4
     TB/s; starting one and merging what several leave cost about 1.5 us each (1 sequence of 2000, 16 heads of 256: 9.6 us with 8 CTAs per
