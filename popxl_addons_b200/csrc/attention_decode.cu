@@ -1,19 +1,22 @@
 // Decode attention: one query per (b, h) against the cached keys and values of positions [0, pos], one launch; optionally with the
 // rotation of the new query and key and the append of the new key and value in front of it.
 //
-// The positions of a (b, h) are consecutive memory, so a producer warp brings 16 KB of keys and as much of values at a time (32, 64 or 128
-// positions of 256, 128 or 64 features) with two plain bulk copies into a ring of 96 KB per CTA, two CTAs per SM. Cached positions do
-// not depend on the previous kernel as a rule; they are then on their way before it ends. Eight warps take a share of each stage: a
-// position is a group of 32, 16 or 8 lanes, 16 bytes of a key per lane, and every group has an online softmax of its own. The new
-// key and value come from the projections: the CTA of the last positions rotates and appends them and takes them from registers.
+// The positions of a (b, h) are consecutive memory, so a producer warp brings a stage of keys and as much of values at a time with two plain
+// bulk copies into a ring of three stages. Cached positions do not depend on the previous kernel as a rule; they are then on their way
+// before it ends. W = 8, 4 or 2 warps take a share of each stage (W = 8: 16 KB of keys, which is 32, 64 or 128 positions of 256, 128 or
+// 64 features, and 96 KB of ring per CTA): a position is a group of 32, 16 or 8 lanes, 16 bytes of a key per lane, and every group has an
+// online softmax of its own. The new key and value come from the projections: the CTA of the last positions rotates and appends them and
+// takes them from registers.
 // Grid (B * H, splits): CTAs that share a (b, h) leave (max, sum, unnormalised output) of their positions; the last one to finish
 // (a counter per (b, h), left at zero again) merges them in order.
 //
 // What bounds it is HBM, and for short caches the latency of the chain load - score - softmax - merge, so splits are few (chosen by the
-// caller). Chains of launches on one B200, us (rotation and append as a kernel of their own, keys and values through registers -> here):
+// caller), and where there are more CTAs than two per SM they are smaller, so that more chains run side by side (W by the caller, with
+// the figures). Chains of launches on one B200, us (rotation and append as a kernel of their own, keys and values through registers -> here):
 //   16 sequences of 528 positions, 16 heads of 256   37.3 -> 24.9 (5.6 TB/s)      1 sequence of 93, 16 heads of 128     7.3 -> 3.3
 //   16 of 528, 16 heads of 128                       20.3 -> 14.6                 1 of 2000, 16 heads of 256           37.2 -> 9.5
 //   16 of 1000, 32 heads of 64                       36.7 -> 26.6                 1 of 8000, 8 heads of 256            41.8 -> 15.5
+//   300 of 100, 8 heads of 64                        23.9 -> 17.4                 128 of 60, 16 heads of 64            13.8 -> 9.7
 #include "common.cuh"
 #include "tcgen05.cuh"
 
@@ -23,13 +26,13 @@ namespace {
 
 using namespace xl_tc;
 
-constexpr int AD_WARPS = 8, AD_UNROLL = 4;
-constexpr int AD_THREADS = (AD_WARPS + 1) * 32;
+constexpr int AD_UNROLL = 4;
 enum { ERR_AD_FULL = 64, ERR_AD_EMPTY = 65 };
 
-template <int D> struct AdCfg {
+template <int D, int W> struct AdCfg {
+  static constexpr int THREADS = (W + 1) * 32, CTAS = W == 8 ? 2 : 16 / W;  // per SM
   static constexpr int LANES = D / 8, GROUPS = 32 / LANES;  // lanes of a position, positions of a warp at a time
-  static constexpr int POS = AD_WARPS * AD_UNROLL * GROUPS, ROW = D * 2, HALF = POS * ROW, STAGE = 2 * HALF, STAGES = 3;
+  static constexpr int POS = W * AD_UNROLL * GROUPS, ROW = D * 2, HALF = POS * ROW, STAGE = 2 * HALF, STAGES = 3;
   static constexpr int SMEM = STAGES * STAGE + 128 /*alignment slack*/;
 };
 
@@ -55,13 +58,14 @@ __device__ __forceinline__ void ad_bulk_load(void* dst, const void* src, uint32_
                "r"(bytes), "r"(smem_u32(bar))
                : "memory");
 }
-__device__ __forceinline__ void ad_sync() { asm volatile("bar.sync 1, %0;" ::"n"(AD_WARPS * 32) : "memory"); }
+template <int W> __device__ __forceinline__ void ad_sync() { asm volatile("bar.sync 1, %0;" ::"n"(W * 32) : "memory"); }
 
-template <typename T, int D>
-__global__ void __launch_bounds__(AD_THREADS, 2) attn_decode_kernel(const __grid_constant__ AdParams p) {
-  using C = AdCfg<D>;
+// W: warps that attend
+template <typename T, int D, int W>
+__global__ void __launch_bounds__((AdCfg<D, W>::THREADS), (AdCfg<D, W>::CTAS)) attn_decode_kernel(const __grid_constant__ AdParams p) {
+  using C = AdCfg<D, W>;
   using Vec = AdVec<T>;
-  constexpr int LANES = C::LANES, GROUPS = C::GROUPS, STREAMS = AD_WARPS * GROUPS;
+  constexpr int LANES = C::LANES, GROUPS = C::GROUPS, STREAMS = W * GROUPS;
   extern __shared__ uint8_t ad_smem[];
   __shared__ uint64_t full_bar[C::STAGES], empty_bar[C::STAGES];
   __shared__ int abort_word;
@@ -75,7 +79,7 @@ __global__ void __launch_bounds__(AD_THREADS, 2) attn_decode_kernel(const __grid
   if (threadIdx.x == 0) {
     for (int s = 0; s < C::STAGES; ++s) {
       mbar_init(&full_bar[s], 1);
-      mbar_init(&empty_bar[s], AD_WARPS);
+      mbar_init(&empty_bar[s], W);
     }
     abort_word = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -98,7 +102,7 @@ __global__ void __launch_bounds__(AD_THREADS, 2) attn_decode_kernel(const __grid
     fresh = here && first < end && end == len;
   };
 
-  if (warp == AD_WARPS) {
+  if (warp == W) {
     if (elect_one()) {
       if (!p.read_ahead) xl_grid_dependency_wait();
       range();
@@ -127,7 +131,7 @@ __global__ void __launch_bounds__(AD_THREADS, 2) attn_decode_kernel(const __grid
   xl_grid_launch_dependents();
   range();
   const T* row = (const T*)p.qkv + (long long)b * p.ldq + h * D + at_d;
-  const bool newest = fresh && warp == AD_WARPS - 1;  // its first group takes the new position
+  const bool newest = fresh && warp == W - 1;  // its first group takes the new position
   Vec qv = *reinterpret_cast<const Vec*>(row), kn, vn;
   if (newest) {
     kn = *reinterpret_cast<const Vec*>(row + p.H * D);
@@ -229,11 +233,10 @@ __global__ void __launch_bounds__(AD_THREADS, 2) attn_decode_kernel(const __grid
   if (at_d == 0) { sm[stream] = m; sl[stream] = l; }
   *reinterpret_cast<float4*>(&so[stream][at_d]) = make_float4(o[0], o[1], o[2], o[3]);
   *reinterpret_cast<float4*>(&so[stream][at_d + 4]) = make_float4(o[4], o[5], o[6], o[7]);
-  ad_sync();
+  ad_sync<W>();
   T* out = (T*)p.out + (long long)b * p.ldo + h * D;
   float* mine = p.part + ((long long)bh * splits + split) * (D + 2);
-  const int d = threadIdx.x;
-  if (d < D) {
+  for (int d = threadIdx.x; d < D; d += W * 32) {
     float mm = -INFINITY;
 #pragma unroll
     for (int w = 0; w < STREAMS; ++w) mm = fmaxf(mm, sm[w]);
@@ -252,16 +255,16 @@ __global__ void __launch_bounds__(AD_THREADS, 2) attn_decode_kernel(const __grid
     }
   }
   if (splits == 1) return;
-  ad_sync();
+  ad_sync<W>();
   if (threadIdx.x == 0) {
     __threadfence();  // for the stores of all, which the barrier has ordered before it
     is_last = atomicAdd(p.counters + bh, 1u) == (unsigned int)splits - 1;
   }
-  ad_sync();
+  ad_sync<W>();
   if (!is_last) return;
   __threadfence();
   const float* part = p.part + (long long)bh * splits * (D + 2);
-  if (d < D) {
+  for (int d = threadIdx.x; d < D; d += W * 32) {
     float mm = -INFINITY;
 #pragma unroll 8
     for (int s = 0; s < splits; ++s) mm = fmaxf(mm, __ldcg(part + s * (D + 2)));
@@ -278,15 +281,19 @@ __global__ void __launch_bounds__(AD_THREADS, 2) attn_decode_kernel(const __grid
   if (threadIdx.x == 0) p.counters[bh] = 0;
 }
 
-template <typename T, int D> int ad_launch(const AdParams& p, int BH, int splits, cudaStream_t s) {
-  using C = AdCfg<D>;
+template <typename T, int D, int W> int ad_launch(const AdParams& p, int BH, int splits, cudaStream_t s) {
+  using C = AdCfg<D, W>;
   static XlPerDevice smem;
-  XL_TRY(xl_allow_smem(attn_decode_kernel<T, D>, C::SMEM, smem));
-  const cudaError_t e = xl_launch_overlapped(attn_decode_kernel<T, D>, dim3(BH, splits), dim3(AD_THREADS), (size_t)C::SMEM, s, p);
+  XL_TRY(xl_allow_smem(attn_decode_kernel<T, D, W>, C::SMEM, smem));
+  const cudaError_t e = xl_launch_overlapped(attn_decode_kernel<T, D, W>, dim3(BH, splits), dim3(C::THREADS), (size_t)C::SMEM, s, p);
   return e != cudaSuccess ? (int)e : (int)cudaGetLastError();
 }
-template <typename T> int ad_pick(const AdParams& p, int BH, int D, int splits, cudaStream_t s) {
-  return D == 256 ? ad_launch<T, 256>(p, BH, splits, s) : (D == 128 ? ad_launch<T, 128>(p, BH, splits, s) : ad_launch<T, 64>(p, BH, splits, s));
+template <typename T, int W> int ad_pick(const AdParams& p, int BH, int D, int splits, cudaStream_t s) {
+  return D == 256 ? ad_launch<T, 256, W>(p, BH, splits, s)
+                  : (D == 128 ? ad_launch<T, 128, W>(p, BH, splits, s) : ad_launch<T, 64, W>(p, BH, splits, s));
+}
+template <typename T> int ad_warps(const AdParams& p, int BH, int D, int splits, int warps, cudaStream_t s) {
+  return warps == 8 ? ad_pick<T, 8>(p, BH, D, splits, s) : (warps == 4 ? ad_pick<T, 4>(p, BH, D, splits, s) : ad_pick<T, 2>(p, BH, D, splits, s));
 }
 
 }  // namespace
@@ -295,16 +302,15 @@ template <typename T> int ad_pick(const AdParams& p, int BH, int D, int splits, 
 // may be the rows' v part. Caches (B, H, Smax, D) of 16-byte aligned rows. append: q and k are rotated (first R features of each head,
 // interleaved pairs, tables (Smax, R / 2) of the type of qkv; qkv itself stays) for position *pos_ptr, k and v written to the caches there;
 // else the cache holds position *pos_ptr already. scratch: B * H * splits * (D + 2) floats; counters: B * H zero-initialised words (left
-// zeroed); both only for splits > 1. D in {64, 128, 256}; ldq, ldo multiples of 8. read_ahead: *pos_ptr and the caches were complete before
+// zeroed); both only for splits > 1. warps: 2, 4 or 8 per CTA. D in {64, 128, 256}; ldq, ldo multiples of 8. read_ahead: *pos_ptr and the caches were complete before
 // the previous launch on the stream. Returns -1 for arguments it does not take.
 XL_API int xl_attn_decode(const void* qkv, long long ldq, const void* sin_t, const void* cos_t, void* k_cache, void* v_cache, void* out,
                           long long ldo, float* scratch, unsigned int* counters, const int* pos_ptr, int B, int H, int D, int R,
-                          int Smax, float scale, int splits, int append, int read_ahead, int dtype, int* err, cudaStream_t s) {
-  if ((D != 64 && D != 128 && D != 256) || splits < 1 || splits > 65535 || dtype == XL_F32 || (ldq % 8) || (ldo % 8)) return -1;
+                          int Smax, float scale, int splits, int warps, int append, int read_ahead, int dtype, int* err, cudaStream_t s) {
+  if ((D != 64 && D != 128 && D != 256) || (warps != 2 && warps != 4 && warps != 8) || splits < 1 || splits > 65535 || dtype == XL_F32 || (ldq % 8) || (ldo % 8)) return -1;
   if (splits > 1 && (scratch == nullptr || counters == nullptr)) return -1;
   if (append && (R < 0 || (R & 1) || R > D || (R && (!sin_t || !cos_t)))) return -1;
   if (((uintptr_t)qkv | (uintptr_t)k_cache | (uintptr_t)v_cache) & 15) return -1;
   const AdParams p{qkv, ldq, k_cache, v_cache, out, ldo, scratch, counters, pos_ptr, sin_t, cos_t, H, Smax, R, append, read_ahead, scale, err};
-  if (dtype == XL_BF16) return ad_pick<__nv_bfloat16>(p, B * H, D, splits, s);
-  return ad_pick<__half>(p, B * H, D, splits, s);
+  return dtype == XL_BF16 ? ad_warps<__nv_bfloat16>(p, B * H, D, splits, warps, s) : ad_warps<__half>(p, B * H, D, splits, warps, s);
 }

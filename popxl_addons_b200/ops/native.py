@@ -108,7 +108,7 @@ _gq_small = _sig("xl_gq_gemm_small_m", _c_p, _c_p, _c_p, _c_p, _c_p, _c_p, _c_in
 _rot_append = _sig("xl_rotary_append", _c_p, _c_ll, _c_p, _c_p, _c_p, _c_p, _c_p, _c_int, _c_int, _c_int, _c_int, _c_int,
                    _c_int, _c_p)
 _attn_dec = _sig("xl_attn_decode", _c_p, _c_ll, _c_p, _c_p, _c_p, _c_p, _c_p, _c_ll, _c_p, _c_p, _c_p, _c_int, _c_int, _c_int, _c_int,
-                 _c_int, _c_f, _c_int, _c_int, _c_int, _c_int, _c_p, _c_p)
+                 _c_int, _c_f, _c_int, _c_int, _c_int, _c_int, _c_int, _c_p, _c_p)
 _ar_add_ln = _sig("xl_ar_add_layer_norm", _c_p, _c_p, _c_p, _c_p, _c_p, _c_p, _c_int, _c_int, _c_f, _c_int, _c_p, _c_p, _c_ll,
                   _c_p, _c_p, _c_int, _c_int, _c_int, _c_p, _c_p)
 _add_ln = _sig("xl_add_layer_norm", _c_p, _c_p, _c_p, _c_p, _c_p, _c_p, _c_int, _c_int, _c_f, _c_int, _c_p)
@@ -1227,17 +1227,32 @@ def rotary_kv_append_cuda(qkv, sin_tab, cos_tab, k_cache, v_cache, pos, n_heads,
 
 
 @functools.lru_cache(maxsize=256)
-def _attn_decode_splits(bh: int, smax: int, head_dim: int, sms: int) -> int:
-    """CTAs that share a (sequence, head): what takes the least time for a full cache. A CTA reads up to 55 KB a us, all together 6.4
-    TB/s; starting one and merging what several leave cost about 1.5 us each (1 sequence of 2000, 16 heads of 256: 9.6 us with 8 CTAs per
-    head; 16 of 1000, 32 heads of 64: 41 us with 4, for which 1 is chosen)."""
+def _attn_decode_plan(bh: int, smax: int, head_dim: int, sms: int) -> Tuple[int, int]:
+    """CTAs that share a (sequence, head), and warps of a CTA.
+
+    CTAs: what takes the least time for a full cache. A CTA reads up to 55 KB a us, all together 6.4 TB/s; starting one and merging what
+    several leave cost about 1.5 us each (1 sequence of 2000, 16 heads of 256: 9.6 us with 8 CTAs per head). More heads than two per SM
+    have one CTA each: a cut for the sake of an even last wave costs more than it gives (320 heads of 256 in caches of 600, 4 CTAs per head
+    and 1: 47.4 and 43.8 us full, 21.4 and 7.0 with 40 positions).
+
+    Warps: 8, of which two CTAs fit on an SM. With more CTAs than that and short caches, what counts is how many start-up latencies run
+    side by side, so they get 4 warps, or 2 where they are many waves all the same. us with 8, 4 and 2 warps, caches full and an eighth
+    full: 800 heads of 64, 256 positions 16.7, 13.2, 12.0 and 9.0, 5.9, 4.3; 1280 heads of 64, 512 positions 35.8, 31.8, 40.1 and 15.1, 9.3,
+    7.4; 2000 heads of 128, 128 positions 31.7, 26.3, 25.0 and 17.2, 10.1, 7.4; 4096 heads of 64, 1000 positions 153, 142, 146, with 30 of
+    them 38.4, 19.2, 12.7. Above that 8 are the better ones: 640 heads of
+    128, 512 positions 33.3, 38.0, 34.4; 4096 heads of 128, 4000 positions 1140, 1165, 1177."""
     bytes_each = 4 * head_dim
 
     def us(n):
         rate = min(55e3, 6.4e6 / min(bh * n, 2 * sms)) / bytes_each  # positions a us
         return -(-bh * n // (2 * sms)) * (smax / n / rate + 1.5) + (1.5 if n > 1 else 0)
 
-    return min(range(1, max(1, min(smax // 64, 64)) + 1), key=lambda n: (round(us(n), 1), n))
+    if bh <= 2 * sms:
+        return min(range(1, max(1, min(smax // 64, 64)) + 1), key=lambda n: (round(us(n), 1), n)), 8
+    cache, many = smax * bytes_each >> 10, bh >= 12 * sms  # KB of a head
+    if many and cache <= 256:
+        return 1, 2 if cache <= 128 or head_dim < 256 else 4
+    return 1, 4 if cache <= 128 else 8
 
 
 def _attn_decode_launch(qkv, k_cache, v_cache, pos, n_heads, head_dim, scale, out, rotary=None):
@@ -1248,7 +1263,7 @@ def _attn_decode_launch(qkv, k_cache, v_cache, pos, n_heads, head_dim, scale, ou
         return NotImplemented
     B, smax = qkv.shape[0], k_cache.shape[2]
     bh = B * n_heads
-    splits = _attn_decode_splits(bh, smax, head_dim, _sms(qkv.device))
+    splits, warps = _attn_decode_plan(bh, smax, head_dim, _sms(qkv.device))
     ws = done = None
     if splits > 1:
         ws = workspace(bh * splits * (head_dim + 2) * 4, qkv.device, "attn_decode").data_ptr()
@@ -1256,7 +1271,7 @@ def _attn_decode_launch(qkv, k_cache, v_cache, pos, n_heads, head_dim, scale, ou
     sin, cos, rotary_dim = rotary or (None, None, 0)
     rc = _attn_dec(qkv.data_ptr(), qkv.stride(0), sin.data_ptr() if rotary_dim else None, cos.data_ptr() if rotary_dim else None,
                    k_cache.data_ptr(), v_cache.data_ptr(), out.data_ptr(), out.stride(0), ws, done, pos.data_ptr(), B, n_heads,
-                   head_dim, rotary_dim, smax, float(scale), splits, int(rotary is not None),
+                   head_dim, rotary_dim, smax, float(scale), splits, warps, int(rotary is not None),
                    int(rotary is not None and read_ahead.allowed(pos, k_cache, v_cache)), _CODE[qkv.dtype],
                    gemm_error_flag(qkv.device).data_ptr(), _stream())
     if rc == -1:

@@ -159,6 +159,40 @@ def test_rotation_append_and_attention_in_one_launch(nat, dtype, B, H, D, R, S, 
     nat.check_gemm_errors()
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("B,H,D,S,pos", [(19, 16, 64, 90, 64), (20, 16, 128, 90, 31), (20, 16, 256, 120, 97), (75, 16, 128, 40, 16), (225, 8, 256, 200, 130),
+                                         (300, 8, 64, 200, 100), (300, 8, 128, 48, 47), (450, 4, 64, 9, 0), (240, 8, 64, 70, 65), (230, 8, 256, 30, 8),
+                                         (20, 16, 256, 600, 97)])
+@pytest.mark.parametrize("append", [True, False])
+def test_attention_of_more_heads_than_the_sms_hold(nat, dtype, B, H, D, S, pos, append):
+    """CTAs of 4, of 2 and of 8 warps, one position on and behind the end of a stage, the first and the last of a cache; against fp32 as
+    above, twice, with the caches to the bit of the separate kernel."""
+    from popxl_addons_b200.ops.rotary_pos_embed import trig_tables
+
+    splits, warps = nat._attn_decode_plan(B * H, S, D, nat._sms(torch.device("cuda")))
+    assert splits == 1 and warps == (8 if S == 600 else 2 if B > 225 else 4)
+    g, hd, R = torch.Generator(device="cuda").manual_seed(B + S + pos), H * D, D // 2
+    buf = torch.randn(B, 3 * hd, generator=g, device="cuda").to(dtype)
+    k, v = (torch.randn(B, H, S, D, generator=g, device="cuda").to(dtype) for _ in range(2))
+    sin, cos = (torch.tensor(t, device="cuda").to(dtype) for t in trig_tables(S, R))
+    p = torch.tensor(pos, dtype=torch.int32, device="cuda")
+    qkv, k_r, v_r = buf.clone(), k.clone(), v.clone()
+    if append:
+        assert nat.rotary_kv_append_cuda(qkv, sin, cos, k_r, v_r, p, H, D, R) is not NotImplemented
+    want = _ref("attention_decode_packed")(qkv.float(), k_r.float(), v_r.float(), p, H, D, D ** -0.5)
+    for _ in range(2):
+        if append:
+            out = buf.clone()
+            assert nat.rotary_attention_decode_into_cuda(out, sin, cos, k, v, p, H, D, R, 2 * hd, D ** -0.5) is out
+            assert torch.equal(out[:, :2 * hd], buf[:, :2 * hd])
+            out = out[:, 2 * hd:]
+        else:
+            out = nat.attention_decode_packed_cuda(buf, k, v, p, H, D, D ** -0.5)
+        assert torch.equal(k, k_r) and torch.equal(v, v_r)
+        torch.testing.assert_close(out.float(), want, rtol=2.0 ** -7, atol=2.0 ** -8)
+    nat.check_gemm_errors()
+
+
 def test_argmax_store_row_advance(nat):
     torch.manual_seed(2)
     logits = torch.randn(16, 6300, device="cuda").bfloat16()
