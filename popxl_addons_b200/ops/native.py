@@ -1233,25 +1233,28 @@ def _attn_decode_plan(bh: int, smax: int, head_dim: int, sms: int) -> Tuple[int,
     CTAs: what takes the least time for a full cache. A CTA reads up to 55 KB a us, all together 6.4 TB/s; starting one and merging what
     several leave cost about 1.5 us each (1 sequence of 2000, 16 heads of 256: 9.6 us with 8 CTAs per head). More heads than two per SM
     have one CTA each: a cut for the sake of an even last wave costs more than it gives (320 heads of 256 in caches of 600, 4 CTAs per head
-    and 1: 47.4 and 43.8 us full, 21.4 and 7.0 with 40 positions).
+    and 1: 47.4 and 43.8 us full, 21.4 and 7.0 with 40 positions), but for a few waves of long ones (640 heads of 256, 2000 positions, 6,
+    2 and 1 CTAs per head: 219, 203, 213; 320 heads, 2500 positions, 9, 2 and 1: 136, 141, 163).
 
     Warps: 8, of which two CTAs fit on an SM. With more CTAs than that and short caches, what counts is how many start-up latencies run
     side by side, so they get 4 warps, or 2 where they are many waves all the same. us with 8, 4 and 2 warps, caches full and an eighth
     full: 800 heads of 64, 256 positions 16.7, 13.2, 12.0 and 9.0, 5.9, 4.3; 1280 heads of 64, 512 positions 35.8, 31.8, 40.1 and 15.1, 9.3,
     7.4; 2000 heads of 128, 128 positions 31.7, 26.3, 25.0 and 17.2, 10.1, 7.4; 4096 heads of 64, 1000 positions 153, 142, 146, with 30 of
-    them 38.4, 19.2, 12.7. Above that 8 are the better ones: 640 heads of
-    128, 512 positions 33.3, 38.0, 34.4; 4096 heads of 128, 4000 positions 1140, 1165, 1177."""
+    them 38.4, 19.2, 12.7. Above that 8 are the better ones: 640 heads of 128, 512 positions 33.3, 38.0, 34.4; 4096 heads of 128, 4000 positions 1140, 1165, 1177."""
     bytes_each = 4 * head_dim
 
     def us(n):
         rate = min(55e3, 6.4e6 / min(bh * n, 2 * sms)) / bytes_each  # positions a us
         return -(-bh * n // (2 * sms)) * (smax / n / rate + 1.5) + (1.5 if n > 1 else 0)
 
+    splits = min(range(1, max(1, min(smax // 64, 64)) + 1), key=lambda n: (round(us(n), 1), n))
     if bh <= 2 * sms:
-        return min(range(1, max(1, min(smax // 64, 64)) + 1), key=lambda n: (round(us(n), 1), n)), 8
+        return splits, 8
     cache, many = smax * bytes_each >> 10, bh >= 12 * sms  # KB of a head
     if many and cache <= 256:
         return 1, 2 if cache <= 128 or head_dim < 256 else 4
+    if cache > 768 and bh <= 5 * sms:
+        return min(splits, 2) if cache <= 2048 else splits, 8
     return 1, 4 if cache <= 128 else 8
 
 
