@@ -326,7 +326,8 @@ __global__ void __launch_bounds__(NORM_THREADS)
                     const float* rstd, const T* g, T* dx,
                     float* partial, long long rows, int cols) {
   xl_grid_dependency_wait();
-  xl_grid_launch_dependents();
+  // The sums of its parts start when it has ended: their CTAs among these ones, early, cost more than their start-up (LayerNorm in bf16, 2048 x 768
+  // 16.4 us, 14.3 this way; 16384 x 1024 62.7 and 58.3).
   constexpr int N = XlVec<T>::N;
   __shared__ float red[32];
   const int nvec = cols / N;
