@@ -4,14 +4,21 @@
 #include "common.cuh"
 
 #include <math.h>
+#include <type_traits>
 
 // ------------------------------------------------------------------------------------------------------------------
 // generic 1-/2-/3-operand elementwise driver
 // ------------------------------------------------------------------------------------------------------------------
 constexpr int EW_UNROLL = 4;  // 16-byte vectors per thread and iteration: keeps ~64 B per thread in flight
 
+// CTAs per SM that fp32 kernels leave registers for, 0: as it comes. A load behind the wait for the predecessor is not of memory that the
+// compiler may take for constant, and without a limit it spent 10 to 20 registers more on the order of loads and stores: 4 M values,
+// gelu_grad 10.5 -> 11.2 us, its tanh form 9.9 -> 10.8, silu 8.8 -> 9.5; with it 9.9, 9.3 and 8.3.
+template <typename F> constexpr int EW_UNARY_CTAS = 5;
+constexpr int EW_BINARY_CTAS = 4;
+
 template <typename T, typename F>
-__global__ void __launch_bounds__(256) ew_unary_kernel(const T* x, T* y, long long n, F f) {
+__global__ void __launch_bounds__(256, sizeof(T) == 4 ? EW_UNARY_CTAS<F> : 0) ew_unary_kernel(const T* x, T* y, long long n, F f) {
   xl_grid_dependency_wait();
   xl_grid_launch_dependents();
   constexpr int N = XlVec<T>::N;
@@ -41,7 +48,7 @@ __global__ void __launch_bounds__(256) ew_unary_kernel(const T* x, T* y, long lo
 }
 
 template <typename T, typename F>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, sizeof(T) == 4 ? EW_BINARY_CTAS : 0)
     ew_binary_kernel(const T* x, const T* g, T* y, long long n, F f) {
   xl_grid_dependency_wait();
   xl_grid_launch_dependents();
@@ -104,6 +111,7 @@ struct GeluTanh {
     return 0.5f * x * (1.f + tanhf(k * (x + 0.044715f * x * x * x)));
   }
 };
+template <> constexpr int EW_UNARY_CTAS<GeluTanh> = 0;  // 40 registers by itself: 86 us for 64 M values, 88 with 48
 struct GeluErfGrad {
   __device__ __forceinline__ float operator()(float x, float g) const {
     const float cdf = 0.5f * (1.f + erff(x * 0.70710678118654752f));
@@ -217,8 +225,9 @@ XL_API int xl_swiglu_bwd(const void* gate, const void* up, const void* g, void* 
 constexpr int NORM_THREADS = 256;
 constexpr int NORM_MAX_ITERS = 8;
 
+// The limit is for LayerNorm of fp16 rows of 4104 to 8192 columns, which took 58 registers: 4096 x 8192 32.3 us, 30.0 with it.
 template <typename T, bool RMS, int ITERS>
-__global__ void __launch_bounds__(NORM_THREADS)
+__global__ void __launch_bounds__(NORM_THREADS, ITERS == 4 && !RMS && std::is_same<T, __half>::value ? 5 : 0)
     norm_fwd_kernel(const T* x, const T* w, const T* b, T* y,
                     float* mean_out, float* rstd_out, int cols, float eps) {
   xl_grid_dependency_wait();
