@@ -183,9 +183,8 @@ XL_API int xl_swiglu_fwd(const void* gate, const void* up, void* y, long long n,
 }
 
 template <typename T>
-__global__ void __launch_bounds__(256) swiglu_bwd_kernel(const T* __restrict__ gate, const T* __restrict__ up,
-                                                        const T* __restrict__ g, T* __restrict__ dgate,
-                                                        T* __restrict__ dup, long long n) {
+__global__ void __launch_bounds__(256) swiglu_bwd_kernel(const T* gate, const T* up, const T* g, T* dgate, T* dup, long long n) {
+  xl_grid_dependency_wait();  // in an ordinary launch the trigger below cost 0.1 us of 2.3; overlapped, as the forward, 1.9
   xl_grid_launch_dependents();
   constexpr int N = XlVec<T>::N;
   const long long nvec = n / N;
@@ -214,7 +213,8 @@ XL_API int xl_swiglu_bwd(const void* gate, const void* up, const void* g, void* 
                          int dtype, cudaStream_t s) {
   const int grid = xl_grid_for(n, 256 * 8);
   XL_DISPATCH_DTYPE(dtype, T, {
-    swiglu_bwd_kernel<T><<<grid, 256, 0, s>>>((const T*)gate, (const T*)up, (const T*)g, (T*)dgate, (T*)dup, n);
+    XL_TRY((xl_launch_overlapped(swiglu_bwd_kernel<T>, dim3(grid), dim3(256),
+        (size_t)0, s, (const T*)gate, (const T*)up, (const T*)g, (T*)dgate, (T*)dup, n)));
   });
   return (int)cudaGetLastError();
 }

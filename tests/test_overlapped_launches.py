@@ -93,3 +93,36 @@ def test_portion_attention_ahead_of_few_rows_products(rows):
     torch.cuda.synchronize()
     assert all(torch.equal(a, b) for a, b in zip(got, want))
     native.check_gemm_errors()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("rows,F", [(3, 41), (128, 256), (1000, 1024)])
+def test_gated_units_wait_for_what_they_read(dtype, rows, F):
+    """The gradient of a gated unit on what the launches before it wrote, and products of what it writes, as a graph: the bits of the same
+    calls with the device idle in between."""
+    from popxl_addons_b200.ops import native as nat
+
+    gpu = ("cuda", dtype)
+    gate, up, g = (rnd(gpu, rows, F, seed=s)[0] for s in (1, 2, 3))
+
+    def chain(between):
+        a, outs = gate, []
+        for _ in range(4):
+            y = nat.swish_cuda(a)
+            between()
+            da, du = nat.swiglu_grad_cuda(y, up, g)
+            between()
+            a = nat.gelu_cuda(da)
+            between()
+            outs += [da, du, a]
+        return outs
+
+    want = chain(torch.cuda.synchronize)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got = chain(lambda: None)
+    for _ in range(3):
+        graph.replay()
+    torch.cuda.synchronize()
+    assert all(torch.equal(a, b) for a, b in zip(got, want))
