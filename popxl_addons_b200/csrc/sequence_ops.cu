@@ -105,14 +105,16 @@ __global__ void __launch_bounds__(256)
 }
 
 // ---- RMS norm: one CTA per row, the row in registers between the sum of squares and the output --------------------------
-constexpr int RMS_THREADS = 256;
+constexpr int RMS_THREADS = 256;  // of rows of up to 1024 packs; twice as many for longer ones
 
 // x (rows, cols) fp32 += mult * y, or without y: x = mult * table[token]; with w, h = x / sqrt(mean(x^2) + eps) * w.
 // NP packs of V columns per thread stay in registers; the columns of longer rows are read again. The loads of all packs are asked
 // for before the first store, which they might alias: one after the other they were a chain of NP trips to memory (bf16, 16 rows
-// of 4096 columns 3.1 -> 2.1 us, 40 of 2048 2.3 -> 1.6 us, 2560 of 2048 14.1 -> 11.4 us, 8192 of 4096 70 -> 63 us: 6.4 TB/s).
+// of 4096 columns 3.1 -> 2.1 us, 40 of 2048 2.3 -> 1.6 us, 2560 of 2048 14.1 -> 11.4 us, 8192 of 4096 70 -> 63 us: 6.4 TB/s). Eight packs
+// per thread took 100 registers, which left two CTAs of 256 threads on an SM: embedding 2560 rows of 5120 columns 23.7 -> 25.0 us, of
+// 12288 52.7 -> 56.5, 8192 of 8192 85.7 -> 94.5. Four packs and 512 threads: 22.9, 47.0 and 88.5.
 template <typename T, int V, int NP>
-__global__ void __launch_bounds__(RMS_THREADS)
+__global__ void __launch_bounds__(2 * RMS_THREADS)
     stream_rms_kernel(float* x, const T* y, float mult, const int* tokens, const T* table, int vocab, const float* w,
                       float eps, T* h, int cols) {
   __shared__ float red[32];
@@ -390,14 +392,13 @@ template <typename T, int V>
 int launch_rms(float* x, const void* y, float mult, const int* tokens, const void* table, int vocab, const float* w, float eps,
                void* h, long long rows, int cols, cudaStream_t s) {
   const int packs = (cols + V - 1) / V;
-  const int threads = packs >= RMS_THREADS ? RMS_THREADS : (packs + 31) / 32 * 32;
+  const int threads = packs > 4 * RMS_THREADS ? 2 * RMS_THREADS : packs >= RMS_THREADS ? RMS_THREADS : (packs + 31) / 32 * 32;
 #define XL_RMS(NP)                                                                                                         \
   XL_TRY(xl_launch_overlapped(stream_rms_kernel<T, V, NP>, dim3((unsigned)rows), dim3(threads), (size_t)0, s, x, (const T*)y,  \
                               mult, tokens, (const T*)table, vocab, w, eps, (T*)h, cols))
   if (packs <= RMS_THREADS) XL_RMS(1);
   else if (packs <= 2 * RMS_THREADS) XL_RMS(2);
-  else if (packs <= 4 * RMS_THREADS) XL_RMS(4);
-  else XL_RMS(8);
+  else XL_RMS(4);
 #undef XL_RMS
   return (int)cudaGetLastError();
 }

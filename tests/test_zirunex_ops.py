@@ -46,6 +46,26 @@ def test_residual_stream_ops(backend, rows, width):  # noqa: F811
     close(sel, plain.rms_unit(x.double().cpu()[[0, rows - 1, 0]], eps) * w64, backend)
 
 
+@pytest.mark.parametrize("width", [1023, 1025, 2050, 4092, 4096, 4100, 8192, 8196])  # one, two and four packs per thread, 256 and 512 threads
+def test_rms_at_the_edges_of_its_tiles(backend, width):  # noqa: F811
+    """A value at each end of a row that is a hundred times the others: lost or counted twice, it shows in the norm."""
+    dev, eps = backend[0], 1e-3
+    w, w64 = rnd(f32(backend), width, seed=2)
+    table = torch.randn(3, width, generator=torch.Generator().manual_seed(5))
+    table[0, 0] = table[1, -1] = 100.0
+    table, t64 = table.to(backend[1]).to(dev), table.to(backend[1]).double()
+    x = torch.zeros(3, width, device=dev)
+    h = op("embed_rms_", backend, x, i32(backend, 0, 1, 2), table, w, scale=3.5, eps=eps)
+    close(x, 3.5 * t64, backend, 1e-6, 1e-6)
+    close(h, plain.rms_unit(3.5 * t64, eps) * w64, backend)
+    a, a64 = rnd(backend, 3, 8, seed=7)
+    m, m64 = rnd(backend, width, 8, std=0.3, seed=8)
+    h = op("linear_residual_rms_", backend, x, a, m, w, mult=0.7, eps=eps, deferred=False)
+    want = 3.5 * t64 + 0.7 * (a64 @ m64.T)
+    close(x, want, backend, 2e-6, 4e-3)
+    close(h, plain.rms_unit(want, eps) * w64, backend)
+
+
 @pytest.mark.parametrize("rows,N,K", [(1, 7, 8), (3, 130, 72), (16, 640, 264), (9, 96, 4096)])
 def test_products_that_finish_a_deferred_norm(backend, rows, N, K):  # noqa: F811
     """A row that is a hundred times larger than the others: its norm must not leak into them."""
