@@ -224,8 +224,7 @@ __global__ void __launch_bounds__((AdCfg<D, W>::THREADS), (AdCfg<D, W>::CTAS)) a
       }
       m = m_new;
     }
-    __syncwarp();
-    if (lane == 0) mbar_arrive(&empty_bar[stage]);
+    mbar_arrive_reads_done(&empty_bar[stage]);
     if (++stage == C::STAGES) { stage = 0; phase ^= 1; }
   }
   // merge the groups of this CTA, a thread per feature

@@ -224,8 +224,7 @@ __global__ void __launch_bounds__(GS_THREADS, 1)
           }
         }
       }
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&empty_bar[stage]);
+      mbar_arrive_reads_done(&empty_bar[stage]);
       }
       if (++turn == GS_TEAMS) turn = 0;
       if (++stage == STAGES) { stage = 0; phase ^= 1; }

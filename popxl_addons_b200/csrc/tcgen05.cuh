@@ -42,6 +42,15 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
   return false;
 }
 
+// A warp that read a stage with ordinary loads gives it back: the fence makes sure that the reads of all lanes have taken place. Without it
+// loads whose values are needed late came after the arrival, and where the code in between had to be fetched from memory (a
+// kernel's first stage), the stage was refilled before them.
+__device__ __forceinline__ void mbar_arrive_reads_done(uint64_t* bar) {
+  __threadfence_block();
+  __syncwarp();
+  if ((threadIdx.x & 31) == 0) mbar_arrive(bar);
+}
+
 __device__ __forceinline__ void tmem_alloc(uint32_t* smem_result, uint32_t cols) {
   asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(smem_result)), "r"(cols)
                : "memory");

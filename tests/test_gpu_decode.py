@@ -193,6 +193,20 @@ def test_attention_of_more_heads_than_the_sms_hold(nat, dtype, B, H, D, S, pos, 
     nat.check_gemm_errors()
 
 
+@pytest.mark.parametrize("B,H,D,S,pos", [(16, 16, 256, 640, 528), (4, 16, 128, 900, 899), (16, 32, 64, 1024, 1000), (300, 8, 64, 500, 400)])
+def test_attention_of_caches_from_memory(nat, B, H, D, S, pos):
+    """Keys from memory, values just written, the kernel's own instructions from memory: the same bits as with all of it in L2."""
+    g = torch.Generator(device="cuda").manual_seed(S)
+    q, k, v = (torch.randn(*s, generator=g, device="cuda").bfloat16() for s in ((B, 3 * H * D), (B, H, S, D), (B, H, S, D)))
+    p = torch.tensor(pos, dtype=torch.int32, device="cuda")
+    want = nat.attention_decode_packed_cuda(q, k, v, p, H, D, D ** -0.5)
+    for _ in range(20):
+        torch.randn(20_000_000, device="cuda").double()
+        written = v * 1
+        assert torch.equal(nat.attention_decode_packed_cuda(q, k, written, p, H, D, D ** -0.5), want)
+    nat.check_gemm_errors()
+
+
 def test_argmax_store_row_advance(nat):
     torch.manual_seed(2)
     logits = torch.randn(16, 6300, device="cuda").bfloat16()

@@ -372,6 +372,23 @@ def test_int4_product_through_the_ring(nat, dtype, M, N, K, gs):
     nat.check_gemm_errors()
 
 
+@pytest.mark.parametrize("M,N,K,gs", [(16, 50400, 2048, 64), (16, 28672, 4096, 64), (9, 28672, 4096, 128), (8, 50400, 2048, 64), (1, 14336, 2048, 64)])
+def test_int4_product_of_weights_from_memory(nat, M, N, K, gs):
+    """Codes and the kernel's own instructions come from memory, the scales have just been written: the same bits as with all of it in L2. (A
+    stage that was refilled while a warp still read it gave every second such launch of 16 tokens other results.)"""
+    g = torch.Generator(device="cuda").manual_seed(N + M)
+    x = torch.randn(M, K, generator=g, device="cuda").bfloat16()
+    packed = torch.randint(0, 32768, (N, K // gs, gs // 4), generator=g, device="cuda").to(torch.int16).view(torch.uint16)
+    pairs = (torch.randn(K // gs, N, 2, generator=g, device="cuda") * 0.05).half()
+    nat.gq_gemm_small_m(x, packed, pairs, None, None)
+    want = nat.gq_gemm_small_m(x, packed, pairs, None, None)
+    for _ in range(20):
+        torch.randn(20_000_000, device="cuda").double()  # 240 MB: more than L2 holds
+        written = pairs * 1
+        assert torch.equal(nat.gq_gemm_small_m(x, packed, written, None, None), want)
+    nat.check_gemm_errors()
+
+
 @pytest.mark.parametrize("rows,N,K", [(1, 1, 4), (2, 7, 132), (3, 2367, 1028), (4, 32000, 1024), (5, 30, 2816), (8, 2369, 68), (11, 513, 2048),
                                       (16, 1024, 1020)])
 def test_few_rows_product_in_32_bits(nat, rows, N, K):
