@@ -396,7 +396,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
           }
         }
       }
-      ok = mbar_wait_pair(&tmem_full_bar[acc], acc_phase, abort_flag, peer_abort_addr, p.err, ERR2_TMEM_FULL_WAIT);
+      ok = __all_sync(0xffffffffu, mbar_wait_pair(&tmem_full_bar[acc], acc_phase, abort_flag, peer_abort_addr, p.err, ERR2_TMEM_FULL_WAIT));
       if (!ok) break;
       tcgen05_fence_after();
       const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + acc * PAIR_N;

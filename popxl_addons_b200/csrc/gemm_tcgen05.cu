@@ -616,7 +616,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
       tile_coords(tile, tiles_m, tiles_n, b, mb, nb, raster_group);
       if (p.gather_mode == 1) mb = (mb + gather_rot) % tiles_m;
       if (p.causal == 1 && nb * BLOCK_N > mb * BLOCK_M + BLOCK_M - 1) continue;
-      ok = mbar_wait(&tmem_full_bar[acc], acc_phase, abort_flag, p.err, ERR_TMEM_FULL_WAIT);
+      ok = mbar_wait_warp(&tmem_full_bar[acc], acc_phase, abort_flag, p.err, ERR_TMEM_FULL_WAIT);
       if (!ok) break;
       tcgen05_fence_after();
       const int row = mb * BLOCK_M + q * 32 + lane;

@@ -119,7 +119,7 @@ __global__ void __launch_bounds__(GS_THREADS, 1)
             const int k = ch * GS_K + b * 64 + (j * 2 + q) * 8, tok = t * 8 + g;
             v[b][t][q] = tok < p.M && k < p.K ? *reinterpret_cast<const uint4*>(x + tok * p.ldx + k) : make_uint4(0, 0, 0, 0);
           }
-      if (i >= STAGES && !mbar_wait(&empty_bar[stage], (i / STAGES - 1) & 1, abort_flag, err, ERR_GS_EMPTY_X)) break;
+      if (i >= STAGES && !mbar_wait_warp(&empty_bar[stage], (i / STAGES - 1) & 1, abort_flag, err, ERR_GS_EMPTY_X)) break;
       uint4* xf = reinterpret_cast<uint4*>(ring + stage * C::STAGE + C::X_AT);
       float* xs = reinterpret_cast<float*>(ring + stage * C::STAGE + C::XS_AT);
       const uint32_t ones[4] = {F::ONES, F::ONES, F::ONES, F::ONES};
@@ -179,7 +179,7 @@ __global__ void __launch_bounds__(GS_THREADS, 1)
       bias[e] = p.bias && n_base + lane * 4 + e < p.N ? xl_to_float(((const T*)p.bias)[n_base + lane * 4 + e]) : 0.f;
     for (int c = c0; c < c1 && ok; ++c) {
       if (turn == team) {
-      ok = mbar_wait(&full_bar[stage], phase, abort_flag, err, ERR_GS_FULL);
+      ok = mbar_wait_warp(&full_bar[stage], phase, abort_flag, err, ERR_GS_FULL);
       if (!ok) break;
       const uint8_t* st = ring + stage * C::STAGE;
 #pragma unroll

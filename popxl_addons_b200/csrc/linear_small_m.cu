@@ -297,7 +297,7 @@ __global__ void __launch_bounds__(64 + SmRing<NTOK>::EPI, 2)
         if ((et & 7) == 0 && r < p.M) row_scale[r] = 1.f / sqrtf(sq / p.K + p.eps);
       }
     }
-    if (mbar_wait(&acc_full, 0, abort_flag, p.err, ERR_SM_ACC_FULL)) {
+    if (mbar_wait_warp(&acc_full, 0, abort_flag, p.err, ERR_SM_ACC_FULL)) {
       tcgen05_fence_after();
 #pragma unroll 1
       for (int t0 = (warp - 2) / 4 * 16; t0 < NTOK && t0 < p.M; t0 += SM_EPI / 8) {

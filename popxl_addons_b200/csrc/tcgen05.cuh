@@ -42,6 +42,12 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
   return false;
 }
 
+// The same for a whole warp that goes on with warp-wide instructions (mma.sync, tcgen05.ld): its lanes leave the loop at different times,
+// and nothing else brings them back together.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* err, int code) {
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, err, code));
+}
+
 // A warp that read a stage with ordinary loads gives it back: the fence makes sure that the reads of all lanes have taken place. Without it
 // loads whose values are needed late came after the arrival, and where the code in between had to be fetched from memory (a
 // kernel's first stage), the stage was refilled before them.

@@ -47,6 +47,27 @@ def test_a_kernel_holds_its_tmem_before_its_successor_starts():
                 assert "__syncthreads()" in behind, f"{name} starts its successor while its allocation is under way"
 
 
+def test_whole_warps_wait_together():
+    """A bounded wait is a loop that lanes leave at different times, and warp-wide instructions follow it: a wait that is not a single
+    thread's is one of `mbar_wait_warp` or stands in a vote. (Blocks are told by their indentation.)"""
+    waits = 0
+    for path in sorted(glob.glob(os.path.join(CSRC, "*.cu"))):
+        lines = open(path).read().splitlines()
+        for n, line in enumerate(lines):
+            if not re.search(r"\bmbar_wait(_pair)?\(", line) or "__forceinline__" in line:
+                continue
+            waits += 1
+            depth, around = len(line) - len(line.lstrip()), [line]
+            for above in reversed(lines[:n]):
+                indent = len(above) - len(above.lstrip())
+                if above.strip() and indent < depth and not above.lstrip().startswith(("#", "//")):
+                    depth = indent
+                    around.append(above)
+            single = any(re.search(r"elect_one\(\)|\blane (<|==)|threadIdx\.x ==", a) for a in around)
+            assert single or any("__all_sync" in a for a in around[:2]), f"{os.path.basename(path)}:{n + 1}: {line.strip()}"
+    assert waits > 20
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("rows", [2, 8])  # the few-rows products behind them allocate 32 columns on an SM with room for both
 def test_portion_attention_ahead_of_few_rows_products(rows):
