@@ -334,9 +334,10 @@ template <typename T, typename S> int gs_pick(const GqParams& p, int ctas, int* 
 }  // namespace
 
 // Scales and zero points as pairs, rows of pairs of whole 16-byte pieces; a chunk of K holds whole groups or lies in one.
-bool gq_stream_takes(const GqParams& p) {
-  return p.sz_pairs && p.N % 4 == 0 && (p.group_size % GS_K == 0 || p.group_size == 64 || p.group_size == 128);
+XL_API int xl_gq_gemm_streams(int N, int group_size, int sz_pairs) {
+  return sz_pairs && N % 4 == 0 && (group_size % GS_K == 0 || group_size == 64 || group_size == 128);
 }
+bool gq_stream_takes(const GqParams& p) { return xl_gq_gemm_streams(p.N, p.group_size, p.sz_pairs); }
 
 int gq_stream_launch(const GqParams& p, int ctas, int dtype, int scale_dtype, int* err, cudaStream_t s) {
   if (dtype == XL_BF16)

@@ -103,6 +103,7 @@ _gemm_ar_pull = _sig("xl_gemm_tcgen05_ar_pull", _c_p, _c_p, _c_p, _c_p, _c_p, _c
 _symm_all_gather_mc = _sig("xl_symm_all_gather_mc", _c_p, _c_p, _c_ll, _c_p, _c_p, _c_int, _c_int, _c_int, _c_p, _c_p)
 _kv_fill = _sig("xl_kv_fill", _c_p, _c_ll, _c_p, _c_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_p)
 _gq_small_slots = _sig("xl_gq_gemm_small_m_slots", _c_int)
+_gq_streams = _sig("xl_gq_gemm_streams", _c_int, _c_int, _c_int)
 _gq_small = _sig("xl_gq_gemm_small_m", _c_p, _c_p, _c_p, _c_p, _c_p, _c_p, _c_int, _c_int, _c_int, _c_int, _c_ll, _c_ll,
                  _c_int, _c_int, _c_p, _c_p, _c_int, _c_int, _c_int, _c_int, _c_p, _c_p)
 _rot_append = _sig("xl_rotary_append", _c_p, _c_ll, _c_p, _c_p, _c_p, _c_p, _c_p, _c_int, _c_int, _c_int, _c_int, _c_int,
@@ -168,13 +169,11 @@ def _count(name: str):
 
 
 def count_replay(names):
-    """Account for the kernels of a captured graph each time it is replayed. "a+b" is one launch that does the work of the kernels a
-    and b: it counts once, and under both names."""
+    """Account for the kernels of a captured graph each time it is replayed."""
     LAUNCHES["count"] += len(names)
     by = LAUNCHES["by_kernel"]
-    for name in names:
-        for n in name.split("+"):
-            by[n] = by.get(n, 0) + 1
+    for n in names:
+        by[n] = by.get(n, 0) + 1
 
 
 def _check(rc: int, name: str):
@@ -1280,7 +1279,7 @@ def _attn_decode_launch(qkv, k_cache, v_cache, pos, n_heads, head_dim, scale, ou
     if rc == -1:
         return NotImplemented
     _check(rc, "attn_decode")
-    _count("rotary_append+attn_decode" if rotary else "attn_decode")
+    _count("rotary_attn_decode" if rotary else "attn_decode")
     return out
 
 
@@ -1340,7 +1339,7 @@ def gather_layer_norm_cuda(table, idx, w, b, eps):
     if rc == -1:
         return NotImplemented
     _check(rc, "gather_layer_norm")
-    _count("gather_rows+add_layer_norm")
+    _count("gather_layer_norm")
     return x, h
 
 
@@ -1356,7 +1355,7 @@ def take_greedy_cuda(current, logits, buf, pos, valid, base, ahead, advance):
     if rc == -1:
         return NotImplemented
     _check(rc, "take_greedy")
-    _count("argmax_rows+store_row+advance_position" if advance else "argmax_rows+store_row")
+    _count("take_greedy")
     return current
 
 
@@ -1442,7 +1441,7 @@ def gq_gemm_small_m(x, packed, scale, zero, bias, out=None, act_from_col=None, c
     if rc == -1:
         return NotImplemented
     _check(rc, "gq_gemm_small_m")
-    _count("gq_gemm_small_m")
+    _count("gq_gemm_stream" if _gq_streams(N, gs, int(transposed)) else "gq_gemm_small_m")
     return y
 
 

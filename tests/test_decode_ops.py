@@ -9,3 +9,20 @@ def test_the_split_of_a_cache_is_worked_out_once_per_shape():
     before = native._attn_decode_plan.cache_info().hits
     assert native._attn_decode_plan(48, 20000, 128, 148) == first
     assert native._attn_decode_plan.cache_info().hits == before + 1
+
+
+def test_a_launch_is_booked_under_its_own_name():
+    """A fused launch is one kernel: nothing is booked under the names of those whose work it does."""
+    import os
+    import re
+
+    from popxl_addons_b200.ops import native
+
+    before = {k: dict(v) if isinstance(v, dict) else v for k, v in native.LAUNCHES.items()}
+    native.count_replay(["one+two"])
+    grown = {k for k, v in native.LAUNCHES["by_kernel"].items() if v != before["by_kernel"].get(k, 0)}
+    assert native.LAUNCHES["count"] == before["count"] + 1 and grown == {"one+two"}
+    native.LAUNCHES["count"] -= 1
+    del native.LAUNCHES["by_kernel"]["one+two"]
+    for name in ("native.py", "native_sequence.py"):
+        assert not re.search(r'_count\([^)\n]*"\w+\+\w', open(os.path.join(os.path.dirname(native.__file__), name)).read())

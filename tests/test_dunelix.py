@@ -156,7 +156,7 @@ def test_kernels_run_on_the_gpu():
     gen.generate([C.prompt(cfg, 50), C.prompt(cfg, 33)], 4)
     ran = {k for k, v in native.LAUNCHES["by_kernel"].items() if v > before.get(k, 0)}
     assert {"stream_dyt", "min_gru", "swiglu_packed", "linear_small_m", "linear_small_m_residual", "linear_small_m_swiglu",
-            "linear_small_m_min_gru", "diff_attn_decode", "select_dyt", "argmax_rows", "advance_by"} <= ran
+            "linear_small_m_min_gru", "diff_attn_decode", "select_dyt", "take_greedy", "advance_by"} <= ran
     assert FALLBACKS == fell
 
 

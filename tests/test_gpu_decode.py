@@ -294,6 +294,6 @@ def test_generation_on_gpu_matches_cpu_backend(cuda_graphs):
     # first tokens agree everywhere and that most sequences agree completely.
     np.testing.assert_array_equal(got[:, 0], want[:, 0])
     assert (got == want).all(axis=1).mean() >= 0.5
-    for k in ("gq_gemm_small_m", "attn_decode", "rotary_append", "argmax_rows", "add_layer_norm"):
+    for k in ("gq_gemm_stream", "rotary_attn_decode", "take_greedy", "gather_layer_norm", "add_layer_norm"):
         assert native.LAUNCHES["by_kernel"].get(k, 0) > before.get(k, 0), f"{k} kernel did not run"
     assert gpu.decode_ms() > 0

@@ -182,7 +182,7 @@ def test_kernels_run_on_the_gpu():
     gen.generate([C.prompt(cfg, 50), C.prompt(cfg, 33)], 4)
     ran = {k for k, v in native.LAUNCHES["by_kernel"].items() if v > before.get(k, 0)}
     assert {"stream_rms", "clamped_glu", "qk_norm_append", "window_attn_tcgen05", "linear_small_m", "linear_small_m_residual",
-            "linear_small_m_split_glu", "window_attn_decode", "select_rms", "argmax_rows", "advance_by"} <= ran
+            "linear_small_m_split_glu", "window_attn_decode", "select_rms", "take_greedy", "advance_by"} <= ran
     assert "window_attn_general" not in ran and FALLBACKS == fell
 
 
