@@ -1283,14 +1283,28 @@ def _attn_decode_launch(qkv, k_cache, v_cache, pos, n_heads, head_dim, scale, ou
     return out
 
 
+def _op(name, *args, **attrs):
+    """Another op on the same device, by its kernel or else its reference: the parts of a fused op whose kernel does not take the operands."""
+    res = OPS[name].native["cuda"](*args, **attrs)
+    if res is NotImplemented:
+        note_fallback(name)
+        res = OPS[name].impl(*args, **attrs)
+    return res
+
+
 @native("rotary_attention_decode_into_")
 def rotary_attention_decode_into_cuda(buf, sin_tab, cos_tab, k_cache, v_cache, pos, n_heads, head_dim, rotary_dim, out_col, scale):
     hd = n_heads * head_dim
-    if rotary_dim and not (_ok(sin_tab, cos_tab) and sin_tab.dtype == cos_tab.dtype == buf.dtype):
-        return NotImplemented
-    res = _attn_decode_launch(buf, k_cache, v_cache, pos, n_heads, head_dim, scale, buf[:, out_col:out_col + hd],
-                              (sin_tab, cos_tab, rotary_dim))
-    return buf if res is not NotImplemented else NotImplemented
+    out = buf[:, out_col:out_col + hd]
+    # in one launch the heads finish in any order: what one writes must not be what another has yet to read
+    apart = out_col % hd == 0 or out_col >= 3 * hd
+    if apart and (not rotary_dim or _ok(sin_tab, cos_tab) and sin_tab.dtype == cos_tab.dtype == buf.dtype):
+        if _attn_decode_launch(buf, k_cache, v_cache, pos, n_heads, head_dim, scale, out, (sin_tab, cos_tab, rotary_dim)) is not NotImplemented:
+            return buf
+    qkv = buf[:, :3 * hd].clone(memory_format=torch.contiguous_format)  # the projections in `buf` stay as they are
+    _op("rotary_kv_append_", qkv, sin_tab, cos_tab, k_cache, v_cache, pos, n_heads=n_heads, head_dim=head_dim, rotary_dim=rotary_dim)
+    out.copy_(_op("attention_decode_packed", qkv, k_cache, v_cache, pos, n_heads=n_heads, head_dim=head_dim, scale=scale))
+    return buf
 
 
 @native("attention_decode_packed")

@@ -226,6 +226,35 @@ def test_argmax_store_row_advance(nat):
     assert int((buf != 0).any(dim=1).sum()) == 1
 
 
+@pytest.mark.parametrize("dtype,D,out_col", [(torch.bfloat16, 80, 2), (torch.float16, 32, 3), (torch.float32, 64, 2), (torch.bfloat16, 64, 0.5),
+                                             (torch.bfloat16, 64, 2.25), (torch.bfloat16, 128, 3), (torch.float16, 64, 0)])
+def test_rotation_append_and_attention_of_what_one_launch_does_not_take(nat, dtype, D, out_col):
+    """Heads that the one launch does not take are rotated and appended by a kernel all the same (of 16 bits), and so are results that lie
+    across the keys and values of other heads (`out_col` in widths of q): against fp32, the rest of the buffer untouched."""
+    from popxl_addons_b200.ops.rotary_pos_embed import trig_tables
+
+    B, H, S, pos, R = 3, 4, 70, 40, 16
+    g, hd = torch.Generator(device="cuda").manual_seed(D), H * D
+    at, one = int(out_col * hd), out_col in (0, 3) and D in (64, 128)
+    buf = torch.randn(B, 5 * hd, generator=g, device="cuda").to(dtype)
+    k, v = (torch.randn(B, H, S, D, generator=g, device="cuda").to(dtype) for _ in range(2))
+    sin, cos = (torch.tensor(t, device="cuda").to(dtype) for t in trig_tables(S, R))
+    p = torch.tensor(pos, dtype=torch.int32, device="cuda")
+    qkv, k_r, v_r = buf[:, :3 * hd].clone(memory_format=torch.contiguous_format), k.clone(), v.clone()
+    (_ref("rotary_kv_append_") if dtype == torch.float32 else nat.rotary_kv_append_cuda)(qkv, sin, cos, k_r, v_r, p, H, D, R)
+    want = _ref("attention_decode_packed")(qkv.float(), k_r.float(), v_r.float(), p, H, D, D ** -0.5)
+    before = dict(nat.LAUNCHES["by_kernel"])
+    out = buf.clone()
+    assert nat.rotary_attention_decode_into_cuda(out, sin, cos, k, v, p, H, D, R, at, D ** -0.5) is out
+    tol = 1e-5 if dtype == torch.float32 else 2.0 ** -7
+    torch.testing.assert_close(out[:, at:at + hd].float(), want, rtol=tol, atol=tol / 2)
+    assert torch.equal(k, k_r) and torch.equal(v, v_r)
+    assert torch.equal(out[:, :at], buf[:, :at]) and torch.equal(out[:, at + hd:], buf[:, at + hd:])
+    ran = {n for n, c in nat.LAUNCHES["by_kernel"].items() if c > before.get(n, 0)}
+    parts = set() if dtype == torch.float32 else {"rotary_append", "attn_decode"} if D in (64, 128) else {"rotary_append"}
+    assert ran == ({"rotary_attn_decode"} if one else parts)
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("rows,V,valid", [(1, 1, 1), (1, 50400, 50399), (16, 33, 33), (40, 32000, 32000), (300, 1001, 777)])
 def test_take_greedy(nat, dtype, rows, V, valid):
