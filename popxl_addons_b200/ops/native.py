@@ -1343,18 +1343,18 @@ def add_layer_norm_cuda(x, *rest, has_delta, has_bias, eps):
 
 @native("gather_layer_norm")
 def gather_layer_norm_cuda(table, idx, w, b, eps):
-    if not _ok(table, w, b) or table.dim() != 2 or table.shape[1] > 8192 or idx.dtype != torch.int32 or not idx.is_contiguous() \
-            or not (table.dtype == w.dtype == b.dtype):
-        return NotImplemented
-    x = torch.empty((idx.numel(), table.shape[1]), dtype=table.dtype, device=table.device)
-    h = torch.empty_like(x)
-    rc = _gather_ln(idx.data_ptr(), table.data_ptr(), table.shape[0], x.data_ptr(), w.data_ptr(), b.data_ptr(), h.data_ptr(), x.shape[0],
-                    x.shape[1], float(eps), _CODE[x.dtype], _stream())
-    if rc == -1:
-        return NotImplemented
-    _check(rc, "gather_layer_norm")
-    _count("gather_layer_norm")
-    return x, h
+    if _ok(table, w, b) and table.dim() == 2 and table.shape[1] <= 8192 and idx.dtype == torch.int32 and idx.is_contiguous() \
+            and table.dtype == w.dtype == b.dtype:
+        x = torch.empty((idx.numel(), table.shape[1]), dtype=table.dtype, device=table.device)
+        h = torch.empty_like(x)
+        rc = _gather_ln(idx.data_ptr(), table.data_ptr(), table.shape[0], x.data_ptr(), w.data_ptr(), b.data_ptr(), h.data_ptr(), x.shape[0],
+                        x.shape[1], float(eps), _CODE[x.dtype], _stream())
+        if rc != -1:
+            _check(rc, "gather_layer_norm")
+            _count("gather_layer_norm")
+            return x, h
+    x = _op("gather", table, idx.reshape(-1), axis=0, zero_OOR=True)
+    return x, _op("add_layer_norm_", x, w, b, has_delta=False, has_bias=False, eps=eps)
 
 
 @native("take_greedy_")

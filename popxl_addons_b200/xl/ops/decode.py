@@ -69,7 +69,11 @@ def _take_greedy_ref(current, logits, buf, pos, valid, base, ahead, advance):
 
 
 def _gather_layer_norm_ref(table, idx, w, b, eps):
-    x = torch.index_select(table, 0, idx.long().reshape(-1)) if table.device.type != "meta" else table.new_empty((idx.numel(), table.shape[1]))
+    x = table.new_empty((idx.numel(), table.shape[1]))
+    if table.device.type != "meta":
+        at = idx.long().reshape(-1)
+        inside = (at >= 0) & (at < table.shape[0])
+        x = torch.where(inside[:, None], torch.index_select(table, 0, at.clamp(0, table.shape[0] - 1)), torch.zeros_like(x))
     return x, torch.nn.functional.layer_norm(x.float(), (x.shape[-1],), w.float(), b.float(), eps).to(x.dtype)
 
 
@@ -243,7 +247,7 @@ def take_greedy_(current: Tensor, logits: Tensor, buf: Tensor, pos: Tensor, vali
 
 
 def gather_layer_norm(table: Tensor, idx: Tensor, weight: Tensor, bias: Tensor, eps: float = 1e-5) -> Tuple[Tensor, Tensor]:
-    """`x = table[idx]` and its layer norm, as one op."""
+    """`x = table[idx]` (a row of zeros for an index outside the table) and its layer norm, as one op."""
     x, h = emit("gather_layer_norm", [table, idx, weight, bias], dict(eps=float(eps)))
     return x, h
 

@@ -1,4 +1,8 @@
 """The ops of the decoding path on the host: what a launch works out before it starts, and their references."""
+import torch
+
+import popxl_addons_b200.xl.ops  # noqa: F401  (registers the ops)
+from popxl_addons_b200.xl.opdef import OPS
 
 
 def test_the_split_of_a_cache_is_worked_out_once_per_shape():
@@ -26,3 +30,11 @@ def test_a_launch_is_booked_under_its_own_name():
     del native.LAUNCHES["by_kernel"]["one+two"]
     for name in ("native.py", "native_sequence.py"):
         assert not re.search(r'_count\([^)\n]*"\w+\+\w', open(os.path.join(os.path.dirname(native.__file__), name)).read())
+
+
+def test_rows_outside_the_table_are_zeros():
+    """In the reference as in the kernel: the norm of such a row is the norm's bias."""
+    table, w, b = torch.randn(7, 10), torch.randn(10), torch.randn(10)
+    x, h = OPS["gather_layer_norm"].impl(table, torch.tensor([3, 7, 0, -1], dtype=torch.int32), w, b, 1e-5)
+    assert torch.equal(x[[0, 2]], table[[3, 0]]) and not x[1].any() and not x[3].any()
+    torch.testing.assert_close(h[[1, 3]], b.expand(2, 10))

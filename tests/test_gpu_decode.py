@@ -256,6 +256,21 @@ def test_rotation_append_and_attention_of_what_one_launch_does_not_take(nat, dty
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("cols", [9, 2050, 8200])
+def test_gather_layer_norm_of_other_widths(nat, dtype, cols):
+    """The rows come from the kernel whatever their width, zeros for an index outside the table as everywhere."""
+    g = torch.Generator(device="cuda").manual_seed(cols)
+    table, w, b = (torch.randn(*s, generator=g, device="cuda").to(dtype) for s in ((7, cols), (cols,), (cols,)))
+    idx = torch.tensor([3, 7, 0, -1], dtype=torch.int32, device="cuda")
+    before = nat.LAUNCHES["by_kernel"].get("gather_rows", 0)
+    x, h = nat.gather_layer_norm_cuda(table, idx, w, b, 1e-5)
+    assert nat.LAUNCHES["by_kernel"]["gather_rows"] == before + 1
+    want, norm = _ref("gather_layer_norm")(table, idx, w, b, 1e-5)
+    assert torch.equal(x, want) and not x[1].any() and not x[3].any()
+    torch.testing.assert_close(h, norm, rtol=2.0 ** -8, atol=2.0 ** -8)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("rows,V,valid", [(1, 1, 1), (1, 50400, 50399), (16, 33, 33), (40, 32000, 32000), (300, 1001, 777)])
 def test_take_greedy(nat, dtype, rows, V, valid):
     """One CTA per row and clusters, many rows: the choice of the separate kernel, its place in the buffer, rows outside the buffer, and
