@@ -1359,17 +1359,22 @@ def gather_layer_norm_cuda(table, idx, w, b, eps):
 
 @native("take_greedy_")
 def take_greedy_cuda(current, logits, buf, pos, valid, base, ahead, advance):
-    if not _ok(logits) or logits.dim() != 2 or any(t.dtype != torch.int32 or not t.is_contiguous() for t in (current, buf, pos)) \
-            or buf.dim() != 2 or not current.numel() == buf.shape[1] == logits.shape[0]:
+    if logits.dim() != 2 or buf.dim() != 2 or not current.numel() == buf.shape[1] == logits.shape[0] or not 1 <= valid <= logits.shape[1]:
         return NotImplemented
-    rows, V = logits.shape
-    rc = _take_greedy(logits.data_ptr(), current.data_ptr(), buf.data_ptr(), pos.data_ptr(),
-                      counters(1, logits.device, "counters greedy", 1).data_ptr(), rows, V, valid, buf.shape[0], base, ahead,
-                      int(advance), _CODE[logits.dtype], _stream())
-    if rc == -1:
-        return NotImplemented
-    _check(rc, "take_greedy")
-    _count("take_greedy")
+    if _ok(logits) and all(t.dtype == torch.int32 and t.is_contiguous() for t in (current, buf, pos)):
+        rows, V = logits.shape
+        rc = _take_greedy(logits.data_ptr(), current.data_ptr(), buf.data_ptr(), pos.data_ptr(),
+                          counters(1, logits.device, "counters greedy", 1).data_ptr(), rows, V, valid, buf.shape[0], base, ahead,
+                          int(advance), _CODE[logits.dtype], _stream())
+        if rc != -1:
+            _check(rc, "take_greedy")
+            _count("take_greedy")
+            return current
+    chosen = _op("argmax_rows", logits, valid=valid, index_offset=0)[1]
+    current.copy_(chosen.reshape(current.shape))
+    _op("store_row_", buf, pos, chosen, base=base - ahead)
+    if advance:
+        _op("advance_position_", pos)
     return current
 
 

@@ -270,6 +270,23 @@ def test_gather_layer_norm_of_other_widths(nat, dtype, cols):
     torch.testing.assert_close(h, norm, rtol=2.0 ** -8, atol=2.0 ** -8)
 
 
+@pytest.mark.parametrize("rows,V,odd", [(3, 40, "view"), (2, 33, "offset")])
+def test_take_greedy_of_logits_that_the_kernel_does_not_take(nat, rows, V, odd):
+    """Columns of wider rows, rows off their 16-byte boundary: the parts one by one, which a graph can still hold."""
+    wide = torch.randn(rows, V + 5, device="cuda")
+    logits = wide[:, :V] if odd == "view" else torch.cat([wide.reshape(-1)[:1], wide[:, :V].reshape(-1)])[1:].view(rows, V)
+    current, pos = torch.zeros(rows, dtype=torch.int32, device="cuda"), torch.tensor(4, dtype=torch.int32, device="cuda")
+    buf = torch.full((3, rows), -1, dtype=torch.int32, device="cuda")
+    nat.take_greedy_cuda(current, logits, buf, pos, V, 4, 1, True)  # whatever is asked for once
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        nat.take_greedy_cuda(current, logits, buf, pos, V, 4, 1, True)
+    buf.fill_(-1)
+    graph.replay()
+    want = logits.argmax(dim=1).int()
+    assert int(pos) == 6 and torch.equal(current, want) and torch.equal(buf[2], want) and bool((buf[:2] == -1).all())
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("rows,V,valid", [(1, 1, 1), (1, 50400, 50399), (16, 33, 33), (40, 32000, 32000), (300, 1001, 777)])
 def test_take_greedy(nat, dtype, rows, V, valid):
