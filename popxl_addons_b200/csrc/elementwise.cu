@@ -632,13 +632,13 @@ __global__ void __launch_bounds__(256)
   constexpr int U = V == 1 ? 1 : 2;
   float c1 = 1.f, c2 = 1.f;
   if (step != nullptr) {
-    const float t = *step + (ticket ? 1.f : 0.f);  // without a ticket it has counted already
+    const float t = *step + 1.f;
     if (a.bias_correction) {
       c1 = 1.f / (1.f - powf(a.beta1, t));
       c2 = 1.f / (1.f - powf(a.beta2, t));
     }
     __syncthreads();  // the count moves when all CTAs have read it
-    if (ticket && threadIdx.x == 0) {
+    if (threadIdx.x == 0) {
       __threadfence();
       if (atomicAdd(ticket, 1u) == gridDim.x - 1) {
         *ticket = 0;
@@ -708,32 +708,19 @@ static int adam_launch_m(void* w, const void* g, void* m, int m_dtype, float* v,
   return (int)cudaGetLastError();
 }
 
-static int adam_step(void* w, int w_dtype, const void* g, int g_dtype, void* m, int m_dtype, float* v, float* master, float* step,
-                     unsigned int* ticket, const AdamArgs& a, long long n, cudaStream_t s) {
-  if (g_dtype != w_dtype && g_dtype != XL_F32) return -1;
+// One AdamW step over `n` elements. `step` (device float, may be null) moves on by one in the same launch, before it is used for bias
+// correction; with it `ticket`, a zero-initialised word of the stream's own (left zeroed). `master` (fp32, may be null) carries the
+// full-precision weights when `w` is 16-bit.
+XL_API int xl_adam_step(void* w, int w_dtype, const void* g, int g_dtype, void* m, int m_dtype, float* v, float* master, float* step,
+                        unsigned int* ticket, float lr, float beta1, float beta2, float eps, float weight_decay, float grad_scale,
+                        int bias_correction, long long n, cudaStream_t s) {
+  if ((g_dtype != w_dtype && g_dtype != XL_F32) || (step && !ticket)) return -1;
+  const AdamArgs a{lr, beta1, beta2, eps, weight_decay, grad_scale, bias_correction};
   XL_DISPATCH_DTYPE(w_dtype, TW, {
     if (g_dtype == XL_F32) return adam_launch_m<TW, float>(w, g, m, m_dtype, v, master, step, ticket, a, n, s);
     return adam_launch_m<TW, TW>(w, g, m, m_dtype, v, master, step, ticket, a, n, s);
   });
   return (int)cudaGetLastError();
-}
-__global__ void step_increment_kernel(float* step) { *step += 1.f; }
-// One AdamW step over `n` elements. `step` (device float, may be null) is incremented first and used for bias
-// correction; `master` (fp32, may be null) carries the full-precision weights when `w` is 16-bit.
-XL_API int xl_adam_step(void* w, int w_dtype, const void* g, int g_dtype, void* m, int m_dtype, float* v, float* master,
-                        float* step, float lr, float beta1, float beta2, float eps, float weight_decay,
-                        float grad_scale, int bias_correction, long long n, cudaStream_t s) {
-  if (step) step_increment_kernel<<<1, 1, 0, s>>>(step);
-  return adam_step(w, w_dtype, g, g_dtype, m, m_dtype, v, master, step, nullptr,
-                   AdamArgs{lr, beta1, beta2, eps, weight_decay, grad_scale, bias_correction}, n, s);
-}
-// The same, `step` (not null) counted in the same launch. `ticket`: a zero-initialised word of the stream's own (left zeroed).
-XL_API int xl_adam_step_counted(void* w, int w_dtype, const void* g, int g_dtype, void* m, int m_dtype, float* v, float* master,
-                                float* step, unsigned int* ticket, float lr, float beta1, float beta2, float eps, float weight_decay,
-                                float grad_scale, int bias_correction, long long n, cudaStream_t s) {
-  if (!step || !ticket) return -1;
-  return adam_step(w, w_dtype, g, g_dtype, m, m_dtype, v, master, step, ticket,
-                   AdamArgs{lr, beta1, beta2, eps, weight_decay, grad_scale, bias_correction}, n, s);
 }
 
 template <typename TW, typename TG>

@@ -60,10 +60,8 @@ _ln_bwd = _sig("xl_layer_norm_bwd", _c_p, _c_p, _c_p, _c_p, _c_p, _c_p, _c_p, _c
 _rms_fwd = _sig("xl_rms_norm_fwd", _c_p, _c_p, _c_p, _c_p, _c_ll, _c_int, _c_f, _c_int, _c_p)
 _rms_bwd = _sig("xl_rms_norm_bwd", _c_p, _c_p, _c_p, _c_p, _c_p, _c_p, _c_p, _c_ll, _c_int, _c_int, _c_p)
 _norm_parts = _sig("xl_norm_bwd_parts", _c_ll)
-_adam = _sig("xl_adam_step", _c_p, _c_int, _c_p, _c_int, _c_p, _c_int, _c_p, _c_p, _c_p, _c_f, _c_f, _c_f, _c_f, _c_f,
+_adam = _sig("xl_adam_step", _c_p, _c_int, _c_p, _c_int, _c_p, _c_int, _c_p, _c_p, _c_p, _c_p, _c_f, _c_f, _c_f, _c_f, _c_f,
              _c_f, _c_int, _c_ll, _c_p)
-_adam_counted = _sig("xl_adam_step_counted", _c_p, _c_int, _c_p, _c_int, _c_p, _c_int, _c_p, _c_p, _c_p, _c_p, _c_f, _c_f, _c_f, _c_f,
-                     _c_f, _c_f, _c_int, _c_ll, _c_p)
 _sgd = _sig("xl_sgd_step", _c_p, _c_int, _c_p, _c_int, _c_p, _c_f, _c_f, _c_f, _c_f, _c_ll, _c_p)
 _col_sum = _sig("xl_col_sum", _c_p, _c_p, _c_p, _c_ll, _c_int, _c_int, _c_p)
 _col_sum_parts = _sig("xl_col_sum_parts", _c_ll, _c_int, _c_int)
@@ -458,14 +456,10 @@ def adam_cuda(w, g, m, v, *rest, has_step, has_master, bias_correction, **attrs)
         return NotImplemented
     if step is not None and step.dtype != torch.float32:
         return NotImplemented
-    ptrs = (w.data_ptr(), _CODE[w.dtype], g.data_ptr(), _CODE[g.dtype], m.data_ptr(), _CODE[m.dtype], v.data_ptr(),
-            master.data_ptr() if master is not None else None)
-    args = (float(s["lr"]), float(s["beta1"]), float(s["beta2"]), float(s["epsilon"]), float(s["weight_decay"]),
-            float(s["grad_scale"]), int(bool(bias_correction)), w.numel(), _stream())
-    if step is not None:
-        rc = _adam_counted(*ptrs, step.data_ptr(), counters(1, w.device, "counters adam", 1).data_ptr(), *args)
-    else:
-        rc = _adam(*ptrs, None, *args)
+    counted = (None, None) if step is None else (step.data_ptr(), counters(1, w.device, "counters adam", 1).data_ptr())
+    rc = _adam(w.data_ptr(), _CODE[w.dtype], g.data_ptr(), _CODE[g.dtype], m.data_ptr(), _CODE[m.dtype], v.data_ptr(),
+               master.data_ptr() if master is not None else None, *counted, float(s["lr"]), float(s["beta1"]), float(s["beta2"]),
+               float(s["epsilon"]), float(s["weight_decay"]), float(s["grad_scale"]), int(bool(bias_correction)), w.numel(), _stream())
     if rc == -1:
         return NotImplemented
     _check(rc, "adam_step")

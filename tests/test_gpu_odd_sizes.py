@@ -176,30 +176,28 @@ def test_greedy_choice(nat, rows, V, valid, dtype):
 @pytest.mark.parametrize("offset", [0, 1])
 @pytest.mark.parametrize("moment", [torch.float32, torch.bfloat16])
 def test_adam_writes_the_master_and_the_16_bit_weight(nat, n, offset, moment):
-    """Groups of four, the elements behind the last one and buffers that are not aligned; master and weight from one kernel.
-    Against the op's torch reference: a few fp32 roundings apart (1e-6), one bf16 step for the 16-bit outputs."""
+    """Groups of four, the elements behind the last one and buffers that are not aligned; master, weight and step count from one launch, twice,
+    with the ticket back at zero. Each step against the op's torch reference on the same values: a few fp32 roundings apart (1e-6), one
+    bf16 step for the 16-bit outputs."""
     from popxl_addons_b200.xl.opdef import OPS
 
     g = torch.Generator().manual_seed(n + offset)
-    base = [torch.randn(n + offset, generator=g) for _ in range(3)] + [torch.rand(n + offset, generator=g)]
+    master, grad, m, v = (torch.randn(n + offset, generator=g).cuda()[offset:] for _ in range(4))
+    w, m, v = torch.cat([master[:offset], master]).bfloat16()[offset:], m.to(moment), v.abs_()
+    step, ticket = torch.tensor(2.0, device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda")
     kw = dict(has_step=True, has_master=True, bias_correction=True, _tensor_scalars=(), lr=1e-2, beta1=0.9, beta2=0.95,
               epsilon=1e-5, weight_decay=0.01, grad_scale=0.5)
-    got = []
-    for dev in ("cpu", "cuda"):
-        master, grad, m, v = (b.to(dev).clone()[offset:] for b in base)
-        w = base[0].to(dev).bfloat16()[offset:].clone() if offset == 0 else base[0].to(dev).bfloat16()[offset:]
-        m = m.to(moment)
-        step = torch.tensor(2.0, device=dev)
-        if dev == "cpu":
-            OPS["adam_fused_"].impl(w, grad, m, v, step, master, **kw)
-        else:
-            rc = nat._adam(w.data_ptr(), nat._CODE[w.dtype], grad.data_ptr(), nat._CODE[grad.dtype], m.data_ptr(),
-                              nat._CODE[m.dtype], v.data_ptr(), master.data_ptr(), step.data_ptr(), 1e-2, 0.9, 0.95, 1e-5,
-                              0.01, 0.5, 1, n, nat._stream())
-            assert rc == 0
-        got.append([t.float().cpu() for t in (w, m, v, master, step)])
-    for a, b, tol in zip(*got, (2 ** -8, 1e-6 if moment == torch.float32 else 2 ** -8, 1e-6, 1e-6, 0)):
-        assert torch.allclose(a, b, rtol=tol, atol=tol), (a - b).abs().max()
+    for count in (3, 4):
+        want = [t.cpu() for t in (w, grad, m, v, step, master)]
+        OPS["adam_fused_"].impl(*want, **kw)
+        rc = nat._adam(w.data_ptr(), nat._CODE[w.dtype], grad.data_ptr(), nat._CODE[grad.dtype], m.data_ptr(), nat._CODE[m.dtype],
+                       v.data_ptr(), master.data_ptr(), step.data_ptr(), ticket.data_ptr(), 1e-2, 0.9, 0.95, 1e-5, 0.01, 0.5, 1, n,
+                       nat._stream())
+        assert rc == 0 and int(ticket) == 0 and float(step) == float(want[4]) == count
+        for a, b, tol in zip((w, m, v, master), (want[0], want[2], want[3], want[5]),
+                             (2 ** -8, 1e-6 if moment == torch.float32 else 2 ** -8, 1e-6, 1e-6)):
+            a, b = a.float().cpu(), b.float()
+            assert torch.allclose(a, b, rtol=tol, atol=tol), (a - b).abs().max()
 
 
 @pytest.mark.parametrize("n", [1, 3, 5, 1023, 4099])
