@@ -4,7 +4,7 @@
 //
 // Work = (tiles of 128 channels) x (K chunks of 256), tile-major, cut into equal contiguous ranges, one per CTA, one CTA per SM. A CTA
 // has a producer (TMA: 16 KB of codes and their scales per chunk, 7 or 8 chunks ahead, which is 130 to 145 KB per SM on its way),
-// warps that bring the tokens' chunk into the order of the MMA fragments together with the sums of x per block, and eight warps that
+// four warps that bring the tokens' chunk into the order of the MMA fragments together with the sums of x per block, and eight warps that
 // multiply: 4 groups of 32 channels x 2 halves of the chunk. The launch's first chunks are on their way while the previous
 // kernel still runs, if that does not write them. A tile shared by several CTAs is finished by the one that arrives last; it adds
 // the slots of all in CTA order, so results do not depend on timing.
@@ -26,7 +26,7 @@ namespace {
 using namespace xl_tc;
 
 constexpr int GS_ROWS = 128, GS_K = 256, GS_BLOCKS = GS_K / 64;
-constexpr int GS_TEAM = 8, GS_TEAMS = 1, GS_MULT = GS_TEAM * GS_TEAMS, GS_PREP = 4;  // warps
+constexpr int GS_MULT = 8, GS_PREP = 4;  // warps
 constexpr int GS_THREADS = (GS_MULT + GS_PREP + 1) * 32;
 enum { ERR_GS_FULL = 61, ERR_GS_EMPTY = 62, ERR_GS_EMPTY_X = 63 };
 
@@ -35,9 +35,9 @@ template <int NT> struct GsCfg {  // NT: tiles of 8 tokens
   static constexpr int W = GS_ROWS * GS_K / 2, SZ = GS_BLOCKS * GS_ROWS * 4, X = TOK * GS_K * 2, XS = GS_BLOCKS * TOK * 4;
   static constexpr int SZ_AT = W, X_AT = W + SZ, XS_AT = X_AT + X;
   static constexpr int STAGE = (XS_AT + XS + 1023) / 1024 * 1024;
-  static constexpr int STAGES = NT == 1 ? 8 : 7, PARTS = 2 * GS_TEAMS;
+  static constexpr int STAGES = NT == 1 ? 8 : 7;
   static constexpr int RED_LD = GS_ROWS + 4;
-  static constexpr int SMEM = STAGES * STAGE + PARTS * TOK * RED_LD * 4 + 1024 /*alignment slack*/;
+  static constexpr int SMEM = STAGES * STAGE + 2 * TOK * RED_LD * 4 + 1024 /*alignment slack*/;
 };
 
 __device__ __forceinline__ void gs_mult_sync() { asm volatile("bar.sync 1, %0;" ::"n"(GS_MULT * 32) : "memory"); }
@@ -64,7 +64,7 @@ __global__ void __launch_bounds__(GS_THREADS, 1)
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) {
       mbar_init(&full_bar[s], 2);  // the producer and the warp that places the tokens
-      mbar_init(&empty_bar[s], GS_TEAM);
+      mbar_init(&empty_bar[s], GS_MULT);
     }
     abort_word = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -148,7 +148,7 @@ __global__ void __launch_bounds__(GS_THREADS, 1)
 
   // ---------------------------------------------------- products ---------------------------------------------------
   float* red = reinterpret_cast<float*>(ring + STAGES * C::STAGE);
-  const int team = warp / GS_TEAM, rows0 = (warp & 3) * 32, half = (warp % GS_TEAM) >> 2;  // 32 channels x blocks 2 * half, 2 * half + 1 of every chunk
+  const int rows0 = (warp & 3) * 32, half = warp >> 2;  // 32 channels x blocks 2 * half, 2 * half + 1 of every chunk
   // Row g of an MMA tile is channel `perm`: the four rows of a half-warp are 2 apart, so that the swizzled 32-byte pieces they read
   // lie in different banks.
   const int perm = 2 * (g & 3) + (g >> 2);
@@ -161,7 +161,7 @@ __global__ void __launch_bounds__(GS_THREADS, 1)
     sz_at[b] = C::SZ_AT + ((blk >> shift) * GS_ROWS + rows0 + perm) * 4;
   }
   const int x_at = C::X_AT + (half * 2 * NT * 2 * 32 + lane) * 16, xs_at = C::XS_AT + (half * 2 * C::TOK + 2 * j) * 4;
-  int stage = 0, turn = 0;  // of the teams
+  int stage = 0;
   uint32_t phase = 0;
   bool ok = true;  // a warp that gave up still meets the others at the barriers
   const int first_tile = begin / chunks;
@@ -178,7 +178,6 @@ __global__ void __launch_bounds__(GS_THREADS, 1)
     for (int e = 0; e < 4; ++e)  // of the channels whose results this lane stores, long before
       bias[e] = p.bias && n_base + lane * 4 + e < p.N ? xl_to_float(((const T*)p.bias)[n_base + lane * 4 + e]) : 0.f;
     for (int c = c0; c < c1 && ok; ++c) {
-      if (turn == team) {
       ok = mbar_wait_warp(&full_bar[stage], phase, abort_flag, err, ERR_GS_FULL);
       if (!ok) break;
       const uint8_t* st = ring + stage * C::STAGE;
@@ -225,8 +224,6 @@ __global__ void __launch_bounds__(GS_THREADS, 1)
         }
       }
       mbar_arrive_reads_done(&empty_bar[stage]);
-      }
-      if (++turn == GS_TEAMS) turn = 0;
       if (++stage == STAGES) { stage = 0; phase ^= 1; }
     }
     // the two halves of K meet in shared memory
@@ -237,15 +234,12 @@ __global__ void __launch_bounds__(GS_THREADS, 1)
       for (int t = 0; t < NT; ++t)
 #pragma unroll
         for (int e = 0; e < 4; ++e)
-          red[((team * 2 + half) * C::TOK + t * 8 + 2 * j + (e & 1)) * C::RED_LD + rows0 + i * 16 + perm + (e >> 1) * 8] = acc[i][t][e];
+          red[(half * C::TOK + t * 8 + 2 * j + (e & 1)) * C::RED_LD + rows0 + i * 16 + perm + (e >> 1) * 8] = acc[i][t][e];
     gs_mult_sync();
     auto together = [&](int r, int col) {
       float4 v = *reinterpret_cast<const float4*>(red + r * C::RED_LD + col);
-#pragma unroll
-      for (int q = 1; q < C::PARTS; ++q) {
-        const float4 o = *reinterpret_cast<const float4*>(red + (q * C::TOK + r) * C::RED_LD + col);
-        v.x += o.x; v.y += o.y; v.z += o.z; v.w += o.w;
-      }
+      const float4 o = *reinterpret_cast<const float4*>(red + (C::TOK + r) * C::RED_LD + col);
+      v.x += o.x; v.y += o.y; v.z += o.z; v.w += o.w;
       return v;
     };
     const bool whole = c1 - c0 == chunks;

@@ -169,11 +169,11 @@ class DecoderGenerator:
                 return all_reduce(ops.gather(wte, idx, axis=0, zero_OOR=cfg.tp > 1))
 
             def select_token(hn, head, off):
-                """Vocabulary-sharded logits of the normalised hidden state, greedy choice agreed between the shards."""
+                """Vocabulary-sharded logits of the normalised hidden state, greedy choice agreed between the shards (tp > 1)."""
                 logits = linear_gq_window_t(hn, head["weight_compressed"], head["weight_scale_zero_t"], head["bias"])
                 valid = vshard  # padded rows of the last shard are excluded below via the index check
                 m, idx = ops.argmax_rows(logits, valid, 0)
-                idx = idx + off if cfg.tp > 1 else idx
+                idx = idx + off
                 # rows beyond the true vocabulary can only win if their (zero-weight) logit beats everything: mask them
                 in_vocab = ops.cast(ops.less(idx, xl.constant(cfg.vocab_size, xl.int32)), xl.float32)
                 m = m * in_vocab + (in_vocab - 1.0) * 1e30

@@ -776,7 +776,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, bias: Optional[torch.Tensor] = Non
         if rc >= 0:
             _check(rc, "gemm2cta_tcgen05")
             _count("gemm2cta_tcgen05")
-            return out if gaps is None else _without_gaps(out)
+            return out
     rc = _gemm_fused(a.data_ptr(), b.data_ptr(), out_ptr, M, N, K, batch, a_mn, b_mn, lda, ldb, ldc, sa, sb, stride_c,
                      int(a.dtype == torch.float16), _CODE[out.dtype], bias.data_ptr() if bias is not None else None,
                      _CODE[bias.dtype] if bias is not None else 0, act, accumulate,
