@@ -13,11 +13,13 @@
 //             28672 x 4096   4096 x 20480   50400 x 4096   14336 x 2048   2048 x 10240   50400 x 2048   4096 x 1024
 //   1 token   29.4 -> 22.5   21.7 -> 18.4   47.9 -> 35.6   11.6 -> 9.9    10.1 -> 8.1    30.5 -> 20.9   8.6 -> 5.2
 //   16 tokens 34.8 -> 29.7   27.2 -> 24.1   58.9 -> 47.2   15.1 -> 12.8   13.5 -> 10.7   36.5 -> 28.6   8.5 -> 7.1
-// The ring alone, without the products, takes 13.3 us for 28672 x 4096 (5 TB/s). What is left is the products: about 76 instructions per 16
-// channels x 64 k values, 41 of them on the integer pipe (28 to take eight codes out of a word at a time), which issues every other
-// cycle, and four or eight MMAs of 8.4 cycles. Twice as many warps, or codes as subnormal fp16 numbers (20 instead of 28 integer
-// instructions, x rescaled per chunk), gave 0 to 5 % with up to 8 tokens and lost with more; tcgen05 with the codes as its A operand in
-// TMEM took 33 and 42 us for 28672 x 4096 (one block of 64 k values at a time is a chain of hand-overs).
+// With weights that come from HBM in every launch (three sets in turn), 1 and 16 tokens: 28672 x 4096 31.9 -> 25.2, 40.1 -> 33.3; 14336 x
+// 2048 14.8 -> 10.6, 17.7 -> 14.0; 2048 x 10240 12.0 -> 8.3, 16.7 -> 11.4. The ring alone, without the products, takes 13.3 us for 28672 x
+// 4096 (5 TB/s). No unit is full (1 and 16 tokens: issue slots 38 and 37 % busy, integer pipe 38 and 32 %, tensor pipe 17 and 26 %, DRAM 29
+// and 23 %): what is left is a chunk's chain of wait, loads, eight codes of a word at a time, MMAs and scales in two warps per quarter
+// of an SM. Twice as many warps, or codes as subnormal fp16 numbers (20 instead of 28 integer instructions for eight codes, x
+// rescaled per chunk), gave 0 to 5 % with up to 8 tokens and lost with more; tcgen05 with the codes as its A operand in TMEM took 33 and
+// 42 us for 28672 x 4096 (one block of 64 k values at a time is a chain of hand-overs).
 #include "gq_codes.cuh"
 #include "tcgen05.cuh"
 
